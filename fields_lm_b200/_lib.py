@@ -1,6 +1,7 @@
-"""Loads ``libfields_read.so`` and declares the C ABI of ``include/fields_read.h``.
+"""Loads ``libfields_read.so`` and declares the C ABI of ``include/fields_read.h``; loads the torch
+layer over it, ``libfields_torch.so``.
 
-There is no fallback: if the CUDA library has not been built, loading raises.
+There is no fallback: if a library has not been built, loading raises.
 """
 from __future__ import annotations
 
@@ -9,6 +10,7 @@ from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "libfields_read.so"
+TORCH_LIB_PATH = PKG / "libfields_torch.so"
 
 _P = ctypes.c_void_p
 _I = ctypes.c_int
@@ -84,6 +86,35 @@ def load() -> ctypes.CDLL:
             "(needs nvcc). There is no CPU fallback for the Field kernels.")
     _lib = open_library(LIB_PATH)
     return _lib
+
+
+_native = None      # the torch layer's module
+_native_lib = None  # the build of the library it is bound to
+
+
+def native():
+    """The torch layer (``csrc/torch_ops.cpp``), bound to the library that :func:`load` returns."""
+    if _native_lib is not None and _native_lib is _lib:
+        return _native
+    return _bind_native()
+
+
+def _bind_native():
+    global _native, _native_lib
+    lib = load()
+    if _native is None:
+        if not TORCH_LIB_PATH.exists():
+            raise FieldsLibraryError(
+                f"{TORCH_LIB_PATH.name} has not been built; run `python -m fields_lm_b200.build`.")
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        spec = importlib.util.spec_from_file_location("libfields_torch", TORCH_LIB_PATH)
+        _native = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_native)
+    _native.bind(lib._name, FieldsLibraryError)
+    _native_lib = lib
+    return _native
 
 
 def check(status: int, what: str) -> None:

@@ -1,7 +1,8 @@
-"""Builds ``libfields_read.so`` (CUDA, sm_100a) next to this file.
+"""Builds ``libfields_read.so`` (CUDA, sm_100a) and ``libfields_torch.so`` (the torch layer over
+its C ABI, plain C++) next to this file.
 
-``python -m fields_lm_b200.build`` or :func:`build_library`. nvcc cross-compiles
-without a GPU; the shared object stays in-tree (ignored by git).
+``python -m fields_lm_b200.build`` or :func:`build_library` and :func:`build_torch_layer`. nvcc
+cross-compiles without a GPU; the shared objects stay in-tree (ignored by git).
 """
 from __future__ import annotations
 
@@ -70,6 +71,34 @@ def build_variants(force: bool = False, verbose: bool = False) -> Path:
     return _compile(VARIANTS_LIB, ["-DFIELDS_ALL_VARIANTS"], verbose)
 
 
+# The torch layer: operators, autograd nodes and allocations as native code over the C ABI.
+TORCH_LIB = PKG / "libfields_torch.so"
+TORCH_SOURCES = sorted(CSRC.glob("torch_*.cpp"))
+TORCH_HEADERS = sorted(CSRC.glob("torch_*.h")) + [PKG.parent / "include" / "fields_read.h"]
+
+
+def build_torch_layer(force: bool = False) -> Path:
+    newest = max(p.stat().st_mtime for p in TORCH_SOURCES + TORCH_HEADERS)
+    if not force and TORCH_LIB.exists() and TORCH_LIB.stat().st_mtime >= newest:
+        return TORCH_LIB
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    cuda_home = Path(_nvcc()).resolve().parent.parent
+    lib_dir = Path(torch.__file__).parent / "lib"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{cuda_home / 'include'}"]
+    cmd += [f"-isystem{p}" for p in cpp_extension.include_paths()]
+    cmd += ["-o", str(TORCH_LIB), *map(str, TORCH_SOURCES), f"-L{lib_dir}", "-ltorch_python", "-ltorch",
+            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{lib_dir}", "-ldl"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode:
+        raise RuntimeError("g++ failed:\n" + proc.stderr)
+    return TORCH_LIB
+
+
 if __name__ == "__main__":
     import sys
     print(build_library(force=True, verbose="-v" in sys.argv))
+    print(build_torch_layer(force=True))

@@ -1,0 +1,497 @@
+// The package's operators as native torch code: argument checks, allocations, autograd nodes and
+// the calls into the C ABI (include/fields_read.h), compiled against the torch headers into
+// libfields_torch.so.
+//
+// Why native: at small and medium sizes a call costs what the host spends on it. Through
+// torch.autograd.Function and ctypes one forward + backward of the operator took 145 us of host
+// time whatever its size (21 us of kernels at 1 x 256 tokens) and one decode step 15.5 us (1.5 us
+// of kernel). Arguments are parsed by hand (METH_FASTCALL) because a signature parser costs as much
+// as the rest of a decode step.
+//
+// The kernels stay in libfields_read.so, which knows nothing of torch; bind() is given the path of
+// the build to use, so the tests can point this layer at another build of the library.
+#include <torch/extension.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <dlfcn.h>
+
+#include <atomic>
+#include <string>
+
+#include "../../include/fields_read.h"
+
+namespace fields_torch {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------------------------------------
+// The library's entry points, looked up in the build that bind() names.
+// ---------------------------------------------------------------------------------------------
+#define FIELDS_API(X)                                                                             \
+    X(fields_status_string) X(fields_last_cuda_error) X(fields_read_workspace_bytes)              \
+    X(fields_read_forward) X(fields_read_backward) X(fields_read_state_rows)                      \
+    X(fields_read_backward_from_states) X(fields_read_forward_bf16)                               \
+    X(fields_read_forward_bf16_stats) X(fields_read_backward_bf16)                                \
+    X(fields_read_norm_grad_combine) X(fields_read_step) X(fields_read_step_bf16)                 \
+    X(fields_scan_workspace_bytes) X(fields_scan_forward) X(fields_scan_backward)
+
+struct Api {
+#define X(name) decltype(&::name) name;
+    FIELDS_API(X)
+#undef X
+};
+static std::atomic<const Api*> g_api{nullptr};
+static PyObject* g_error_type = nullptr;  // FieldsLibraryError
+
+static const Api& api() {
+    const Api* a = g_api.load(std::memory_order_acquire);
+    TORCH_CHECK(a, "the CUDA library has not been bound");
+    return *a;
+}
+
+// FieldsLibraryError with the library's own text, from any thread (a backward pass runs on an
+// engine thread, which carries the exception to the caller).
+static void check(int rc, const char* what) {
+    if (C10_LIKELY(rc == FIELDS_OK)) return;
+    std::string text = std::string(what) + ": " + api().fields_status_string(rc);
+    if (rc == FIELDS_ERR_LAUNCH) text += std::string(": ") + api().fields_last_cuda_error();
+    text += " (status " + std::to_string(rc) + ")";
+    pybind11::gil_scoped_acquire gil;
+    PyErr_SetString(g_error_type, text.c_str());
+    python_error e;
+    e.persist();
+    throw e;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Small helpers.
+// ---------------------------------------------------------------------------------------------
+static Tensor f32(const Tensor& t) {
+    if (t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
+    return t.contiguous().to(at::kFloat);
+}
+static Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+static float* fp(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+static void* vp(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+static void* stream_of(const Tensor& t) {
+    return c10::cuda::getCurrentCUDAStream(t.device().index()).stream();
+}
+static Tensor empty(at::IntArrayRef size, at::ScalarType type, c10::Device device) {
+    return at::detail::empty_cuda(size, type, device, std::nullopt);
+}
+static Tensor workspace(size_t bytes, c10::Device device) {
+    return empty({(int64_t)std::max<size_t>(bytes, 256)}, at::kByte, device);
+}
+static std::string shape(const Tensor& t) { return c10::str("(", t.sizes(), ")"); }
+
+struct Dims {
+    int B, L, C;
+};
+
+// Checks shared by the forms of the operator (the reference's, same file :923-938).
+static Dims check_operator(const Tensor& raw, at::ScalarType type, const char* type_name,
+                           const Tensor& tr, const Tensor& ti, const Tensor& gm) {
+    TORCH_CHECK(raw.is_cuda(), "Chunked Field kernel requires CUDA");
+    TORCH_CHECK_TYPE(raw.scalar_type() == type, "raw must be ", type_name, ", got ",
+                     raw.scalar_type());
+    TORCH_CHECK_VALUE(raw.dim() == 3 && raw.size(2) % 3 == 0, shape(raw));
+    const int64_t C = raw.size(2) / 3;
+    TORCH_CHECK_VALUE(tr.numel() == C && ti.numel() == C && gm.numel() == C, shape(raw), " ", shape(tr));
+    return Dims{(int)raw.size(0), (int)raw.size(1), (int)C};
+}
+
+// ---------------------------------------------------------------------------------------------
+// The operator on the fp32 boundary, with an optional carried state.
+// ---------------------------------------------------------------------------------------------
+struct ForwardArgs {
+    Tensor raw, tr, ti, gm, state_in;  // state_in may be undefined
+    Dims d;
+};
+
+static ForwardArgs forward_args(const Tensor& raw, const Tensor& tr, const Tensor& ti,
+                                const Tensor& gm, const Tensor& state_in) {
+    const Dims d = check_operator(raw, at::kFloat, "float32", tr, ti, gm);
+    if (state_in.defined())
+        TORCH_CHECK_VALUE(state_in.dim() == 2 && state_in.size(0) == d.B && state_in.size(1) == 2 * d.C,
+                          shape(raw), " ", shape(state_in));
+    return ForwardArgs{dense(raw), f32(tr), f32(ti), f32(gm),
+                       state_in.defined() ? f32(state_in) : state_in, d};
+}
+
+static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, bool want_state) {
+    const Api& f = api();
+    const auto [B, L, C] = a.d;
+    const c10::Device dev = a.raw.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    read = empty({B, L, 4 * C}, at::kFloat, dev);
+    if (want_state) state_out = empty({B, 2 * C}, at::kFloat, dev);
+    const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
+    const Tensor ws = workspace(n, dev);
+    check(f.fields_read_forward(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read),
+                                fp(state_out), vp(ws), n, B, L, C, stream_of(a.raw)),
+          "fields_read_forward");
+}
+
+struct FieldRead : torch::autograd::Function<FieldRead> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& raw_, const Tensor& tr_,
+                                 const Tensor& ti_, const Tensor& gm_,
+                                 const std::optional<Tensor>& state_, bool lean, bool want_state) {
+        const ForwardArgs a = forward_args(raw_, tr_, ti_, gm_, state_.value_or(Tensor()));
+        Tensor read, state_out;
+        run_forward(a, read, state_out, want_state);
+        lean = lean && a.d.C % 4 == 0;
+        Tensor kept = read;
+        if (lean)  // every eighth state row instead of `read`
+            kept = read.slice(1, 7, std::nullopt, 8).slice(2, 0, 2 * a.d.C).contiguous();
+        ctx->set_materialize_grads(false);
+        ctx->save_for_backward({a.raw, a.tr, a.ti, a.gm, kept, a.state_in});
+        if (want_state) return {read, state_out};
+        return {read};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const Api& f = api();
+        const variable_list saved = ctx->get_saved_variables();
+        const Tensor &raw = saved[0], &tr = saved[1], &ti = saved[2], &gm = saved[3], &read = saved[4],
+                     &state_in = saved[5];
+        const int B = (int)raw.size(0), L = (int)raw.size(1), C = (int)raw.size(2) / 3;
+        const bool lean = read.size(2) == 2 * C;  // rows of states, not of `read`
+        const c10::Device dev = raw.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const Tensor grad_read =
+            grads[0].defined() ? f32(grads[0])
+                               : at::zeros({B, L, 4 * C}, at::TensorOptions().dtype(at::kFloat).device(dev));
+        const Tensor grad_state = grads.size() > 1 && grads[1].defined() ? f32(grads[1]) : Tensor();
+        const Tensor grad_raw = empty({B, L, 3 * C}, at::kFloat, dev);
+        const Tensor g_tr = empty({C}, at::kFloat, dev), g_ti = empty({C}, at::kFloat, dev),
+                     g_gm = empty({C}, at::kFloat, dev);
+        Tensor g_sin;
+        if (state_in.defined() && ctx->needs_input_grad(4)) g_sin = empty({B, 2 * C}, at::kFloat, dev);
+        const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
+        const Tensor ws = workspace(n, dev);
+        auto* entry = lean ? f.fields_read_backward_from_states : f.fields_read_backward;
+        // (lean: `read` holds the kept state rows, possibly none for L < 8)
+        check(entry(fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), read.numel() ? fp(read) : nullptr,
+                    fp(grad_read), fp(grad_state), fp(grad_raw), fp(g_tr), fp(g_ti), fp(g_gm), fp(g_sin),
+                    vp(ws), n, B, L, C, stream_of(raw)),
+              "fields_read_backward");
+        return {grad_raw, g_tr, g_ti, g_gm, g_sin, Tensor(), Tensor()};
+    }
+};
+
+// ---------------------------------------------------------------------------------------------
+// The operator on the bfloat16 boundary; with STATS also the sum of squares of each token's outputs.
+// ---------------------------------------------------------------------------------------------
+static variable_list run_forward_bf16(const Tensor& raw, const Tensor& tr, const Tensor& ti,
+                                      const Tensor& gm, const Dims& d, bool stats) {
+    const Api& f = api();
+    const auto [B, L, C] = d;
+    const c10::Device dev = raw.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const Tensor read = empty({B, L, 4 * C}, at::kBFloat16, dev);
+    const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
+    const Tensor ws = workspace(n, dev);
+    if (!stats) {
+        check(f.fields_read_forward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), nullptr,
+                                         vp(ws), n, B, L, C, stream_of(raw)),
+              "fields_read_forward_bf16");
+        return {read};
+    }
+    const Tensor groups = empty({B, L, (C + 127) / 128}, at::kFloat, dev);
+    check(f.fields_read_forward_bf16_stats(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), fp(groups),
+                                           nullptr, vp(ws), n, B, L, C, stream_of(raw)),
+          "fields_read_forward_bf16_stats");
+    return {read, groups.sum(-1)};
+}
+
+// grad_raw, d tr, d ti, d gamma from the gradient of `read` (bfloat16, dense).
+static variable_list run_backward_bf16(const Tensor& raw, const Tensor& tr, const Tensor& ti,
+                                       const Tensor& gm, const Tensor& read, const Tensor& grad_read) {
+    const Api& f = api();
+    const int B = (int)raw.size(0), L = (int)raw.size(1), C = (int)raw.size(2) / 3;
+    const c10::Device dev = raw.device();
+    const Tensor grad_raw = empty({B, L, 3 * C}, at::kBFloat16, dev);
+    const Tensor g_tr = empty({C}, at::kFloat, dev), g_ti = empty({C}, at::kFloat, dev),
+                 g_gm = empty({C}, at::kFloat, dev);
+    const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
+    const Tensor ws = workspace(n, dev);
+    check(f.fields_read_backward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), vp(grad_read),
+                                      nullptr, vp(grad_raw), fp(g_tr), fp(g_ti), fp(g_gm), nullptr, vp(ws),
+                                      n, B, L, C, stream_of(raw)),
+          "fields_read_backward_bf16");
+    return {grad_raw, g_tr, g_ti, g_gm};
+}
+
+template <bool STATS>
+struct FieldReadBf16 : torch::autograd::Function<FieldReadBf16<STATS>> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& raw_, const Tensor& tr_,
+                                 const Tensor& ti_, const Tensor& gm_) {
+        const Dims d = check_operator(raw_, at::kBFloat16, "bfloat16", tr_, ti_, gm_);
+        if (STATS) TORCH_CHECK_VALUE(d.B > 0 && d.L > 0, shape(raw_));
+        const Tensor raw = dense(raw_), tr = f32(tr_), ti = f32(ti_), gm = f32(gm_);
+        const variable_list out = run_forward_bf16(raw, tr, ti, gm, d, STATS);
+        if (STATS) ctx->set_materialize_grads(false);
+        ctx->save_for_backward({raw, tr, ti, gm, out[0]});
+        return out;
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list saved = ctx->get_saved_variables();
+        const Tensor &raw = saved[0], &read = saved[4];
+        const c10::cuda::CUDAGuard guard(raw.device());
+        Tensor total = grads[0].defined() ? dense(grads[0]).to(at::kBFloat16) : Tensor();
+        if (STATS && grads[1].defined()) {
+            // d sumsq / d read = 2 read: folded into the gradient the recurrence receives
+            const Tensor own = total, sumsq = f32(grads[1]);
+            total = empty(read.sizes(), at::kBFloat16, raw.device());
+            check(api().fields_read_norm_grad_combine(vp(own), vp(read), fp(sumsq), vp(total),
+                                                      read.size(0) * read.size(1), (int)read.size(2),
+                                                      stream_of(raw)),
+                  "fields_read_norm_grad_combine");
+        }
+        if (!total.defined()) total = at::zeros_like(read);
+        return run_backward_bf16(raw, saved[1], saved[2], saved[3], read, total);
+    }
+};
+
+// ---------------------------------------------------------------------------------------------
+// The real-valued scan.
+// ---------------------------------------------------------------------------------------------
+// `a` as the library reads it: a dense tensor, or one value per (b, t) broadcast over the channels
+// (the expanded view the softpatch mixer passes), read through its own strides.
+struct ScanDecay {
+    Tensor a;
+    long long batch, step;
+    int chan;
+};
+
+static ScanDecay scan_decay(const Tensor& a) {
+    if (a.size(2) > 1 && a.stride(2) == 0) return ScanDecay{a, a.stride(0), a.stride(1), 0};
+    const Tensor d = dense(a);
+    return ScanDecay{d, d.size(1) * d.size(2), d.size(2), 1};
+}
+
+struct LinearScan : torch::autograd::Function<LinearScan> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& a_, const Tensor& b_,
+                                 const std::optional<Tensor>& state_) {
+        const int B = (int)b_.size(0), L = (int)b_.size(1), C = (int)b_.size(2);
+        Tensor state_in;
+        if (state_ && state_->defined()) {
+            TORCH_CHECK_VALUE(state_->dim() == 2 && state_->size(0) == B && state_->size(1) == C,
+                              shape(b_), " ", shape(*state_));
+            state_in = f32(*state_);
+        }
+        const Api& f = api();
+        const c10::Device dev = b_.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const Tensor b = dense(b_);
+        const ScanDecay d = scan_decay(a_);
+        const Tensor states = empty({B, L, C}, at::kFloat, dev), state_out = empty({B, C}, at::kFloat, dev);
+        const size_t n = f.fields_scan_workspace_bytes(B, L, C);
+        const Tensor ws = workspace(n, dev);
+        check(f.fields_scan_forward(fp(d.a), d.batch, d.step, d.chan, fp(b), fp(state_in), fp(states),
+                                    fp(state_out), vp(ws), n, B, L, C, stream_of(b)),
+              "fields_scan_forward");
+        ctx->set_materialize_grads(false);
+        ctx->save_for_backward({d.a, states, state_in});
+        return {states, state_out};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const Api& f = api();
+        const variable_list saved = ctx->get_saved_variables();
+        const ScanDecay d = scan_decay(saved[0]);
+        const Tensor &states = saved[1], &state_in = saved[2];
+        const int B = (int)states.size(0), L = (int)states.size(1), C = (int)states.size(2);
+        const c10::Device dev = states.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const Tensor g = grads[0].defined() ? f32(grads[0]) : at::zeros_like(states);
+        const Tensor g_out = grads[1].defined() ? f32(grads[1]) : Tensor();
+        const Tensor grad_a = empty({B, L, C}, at::kFloat, dev), grad_b = empty({B, L, C}, at::kFloat, dev);
+        Tensor g_in;
+        if (state_in.defined() && ctx->needs_input_grad(2)) g_in = empty({B, C}, at::kFloat, dev);
+        const size_t n = f.fields_scan_workspace_bytes(B, L, C);
+        const Tensor ws = workspace(n, dev);
+        check(f.fields_scan_backward(fp(d.a), d.batch, d.step, d.chan, fp(states), fp(state_in), fp(g),
+                                     fp(g_out), fp(grad_a), fp(grad_b), fp(g_in), vp(ws), n, B, L, C,
+                                     stream_of(states)),
+              "fields_scan_backward");
+        // dense gradient of `a`; for an expanded `a` autograd sums it over the broadcast channels
+        return {grad_a, grad_b, g_in};
+    }
+};
+
+// ---------------------------------------------------------------------------------------------
+// One recurrent step of incremental decoding: `state` advances in place.
+// ---------------------------------------------------------------------------------------------
+static Tensor step(const Tensor& raw_, const Tensor& tr_, const Tensor& ti_, const Tensor& gm_,
+                   const Tensor& state) {
+    TORCH_CHECK(raw_.is_cuda(), "Field decode step requires CUDA");
+    const at::ScalarType type = raw_.scalar_type();
+    TORCH_CHECK_TYPE(type == at::kFloat || type == at::kBFloat16,
+                     "raw_row must be float32 or bfloat16, got ", type);
+    TORCH_CHECK_TYPE(state.scalar_type() == at::kFloat && state.is_contiguous(),
+                     "state must be a contiguous float32 tensor");
+    TORCH_CHECK_VALUE(raw_.dim() == 2 && raw_.size(1) % 3 == 0, shape(raw_));
+    const int64_t B = raw_.size(0), C = raw_.size(1) / 3;
+    TORCH_CHECK_VALUE(state.dim() == 2 && state.size(0) == B && state.size(1) == 2 * C && tr_.numel() == C,
+                      shape(raw_), " ", shape(state), " ", shape(tr_));
+    const Api& f = api();
+    const c10::Device dev = raw_.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const Tensor raw = dense(raw_), tr = f32(tr_), ti = f32(ti_), gm = f32(gm_);
+    Tensor read = empty({B, 4 * C}, type, dev);
+    const int rc = type == at::kFloat
+                       ? f.fields_read_step(fp(raw), fp(tr), fp(ti), fp(gm), fp(state), fp(read), (int)B,
+                                            (int)C, stream_of(raw))
+                       : f.fields_read_step_bf16(vp(raw), fp(tr), fp(ti), fp(gm), fp(state), vp(read), (int)B,
+                                                 (int)C, stream_of(raw));
+    check(rc, "fields_read_step");
+    return read;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Python entry points.
+// ---------------------------------------------------------------------------------------------
+static void want_args(Py_ssize_t n, Py_ssize_t want) {
+    TORCH_CHECK_TYPE(n == want, "expected ", want, " arguments, got ", n);
+}
+static const Tensor& tensor_arg(PyObject* o) {
+    TORCH_CHECK_TYPE(THPVariable_Check(o), "expected a tensor, got ", Py_TYPE(o)->tp_name);
+    return THPVariable_Unpack(o);
+}
+static std::optional<Tensor> optional_arg(PyObject* o) {
+    if (o == Py_None) return std::nullopt;
+    return tensor_arg(o);
+}
+static PyObject* wrap(const Tensor& t) { return THPVariable_Wrap(t); }
+static PyObject* wrap2(const Tensor& a, const Tensor& b) {
+    PyObject* out = PyTuple_New(2);
+    if (!out) throw python_error();
+    PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(a));
+    PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(b));
+    return out;
+}
+static bool wants_grad(std::initializer_list<const Tensor*> ts) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor* t : ts)
+        if (t->defined() && t->requires_grad()) return true;
+    return false;
+}
+
+// field_read(raw, tr, ti, gamma, state_in or None, lean, want_state) -> read, or (read, state_out)
+static PyObject* py_field_read(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, 7);
+    const Tensor &raw = tensor_arg(args[0]), &tr = tensor_arg(args[1]), &ti = tensor_arg(args[2]),
+                 &gm = tensor_arg(args[3]);
+    const std::optional<Tensor> state_in = optional_arg(args[4]);
+    const bool lean = PyObject_IsTrue(args[5]) == 1, want_state = PyObject_IsTrue(args[6]) == 1;
+    Tensor read, state_out;
+    {
+        pybind11::gil_scoped_release no_gil;
+        const Tensor s = state_in.value_or(Tensor());
+        if (wants_grad({&raw, &tr, &ti, &gm, &s})) {
+            const variable_list out = FieldRead::apply(raw, tr, ti, gm, state_in, lean, want_state);
+            read = out[0];
+            if (want_state) state_out = out[1];
+        } else {
+            run_forward(forward_args(raw, tr, ti, gm, s), read, state_out, want_state);
+        }
+    }
+    return want_state ? wrap2(read, state_out) : wrap(read);
+    END_HANDLE_TH_ERRORS
+}
+
+// field_read_bf16(raw, tr, ti, gamma, stats) -> read, or (read, sumsq)
+static PyObject* py_field_read_bf16(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, 5);
+    const Tensor &raw = tensor_arg(args[0]), &tr = tensor_arg(args[1]), &ti = tensor_arg(args[2]),
+                 &gm = tensor_arg(args[3]);
+    const bool stats = PyObject_IsTrue(args[4]) == 1;
+    variable_list out;
+    {
+        pybind11::gil_scoped_release no_gil;
+        out = stats ? FieldReadBf16<true>::apply(raw, tr, ti, gm) : FieldReadBf16<false>::apply(raw, tr, ti, gm);
+    }
+    return stats ? wrap2(out[0], out[1]) : wrap(out[0]);
+    END_HANDLE_TH_ERRORS
+}
+
+// linear_scan(a, b, state_in or None) -> (states, state_out); shapes and types checked by the caller
+static PyObject* py_linear_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, 3);
+    const Tensor &a = tensor_arg(args[0]), &b = tensor_arg(args[1]);
+    const std::optional<Tensor> state_in = optional_arg(args[2]);
+    variable_list out;
+    {
+        pybind11::gil_scoped_release no_gil;
+        out = LinearScan::apply(a, b, state_in);
+    }
+    return wrap2(out[0], out[1]);
+    END_HANDLE_TH_ERRORS
+}
+
+// step(raw_row, tr, ti, gamma, state) -> read
+static PyObject* py_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, 5);
+    const Tensor &raw = tensor_arg(args[0]), &tr = tensor_arg(args[1]), &ti = tensor_arg(args[2]),
+                 &gm = tensor_arg(args[3]), &state = tensor_arg(args[4]);
+    Tensor read;
+    {
+        pybind11::gil_scoped_release no_gil;
+        read = step(raw, tr, ti, gm, state);
+    }
+    return wrap(read);
+    END_HANDLE_TH_ERRORS
+}
+
+// bind(path, error_type): use the build of the library at `path` from now on.
+static PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, 2);
+    const char* path = PyUnicode_AsUTF8(args[0]);
+    if (!path) throw python_error();
+    void* handle = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+    TORCH_CHECK(handle, "cannot open ", path, ": ", dlerror());
+    auto table = std::make_unique<Api>();
+#define X(name)                                                                   \
+    table->name = reinterpret_cast<decltype(&::name)>(dlsym(handle, #name));      \
+    TORCH_CHECK(table->name, path, " has no symbol " #name);
+    FIELDS_API(X)
+#undef X
+    Py_INCREF(args[1]);
+    g_error_type = args[1];
+    // (a backward pass may still hold the old table: one small struct per bound build stays alive)
+    g_api.store(table.release(), std::memory_order_release);
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
+#define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+static PyMethodDef g_methods[] = {
+    FAST("bind", py_bind),
+    FAST("field_read", py_field_read),
+    FAST("field_read_bf16", py_field_read_bf16),
+    FAST("linear_scan", py_linear_scan),
+    FAST("step", py_step),
+    {nullptr, nullptr, 0, nullptr},
+};
+static PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "libfields_torch", nullptr, -1, g_methods,
+                               nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace fields_torch
+
+PyMODINIT_FUNC PyInit_libfields_torch(void) { return PyModule_Create(&fields_torch::g_module); }

@@ -11,219 +11,32 @@ decoding need; the reference always starts from the zero state.
 """
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import Optional
 
 import torch
 
 from . import _lib
-
-_FWD, _BWD = 0, 1
 
 
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
-def _workspace(B: int, L: int, C: int, which: int, device) -> Tuple[torch.Tensor, int]:
-    nbytes = _lib.load().fields_read_workspace_bytes(B, L, C, which)
-    # the caching allocator hands out 512-byte aligned blocks
-    return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device), nbytes
-
-
 def _stream(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-class FieldReadFunction(torch.autograd.Function):
-    """read, state_out = F(raw, tr, ti, gamma, state_in[, lean]).
+class FieldReadFunction:
+    """read, state_out = F(raw, tr, ti, gamma, state_in[, lean]), differentiable (the autograd node
+    is native, ``csrc/torch_ops.cpp``).
 
     With ``lean`` the function does not keep ``read`` for its backward pass but only every
     eighth state row (1/16 of it); the backward kernel recomputes the states in between.
     """
 
     @staticmethod
-    def forward(ctx, raw, transition_r, transition_i, gamma, state_in, lean=False):
-        if not raw.is_cuda:
-            raise RuntimeError("Chunked Field kernel requires CUDA")
-        if raw.dtype != torch.float32:
-            raise TypeError(f"raw must be float32, got {raw.dtype}")
-        if raw.dim() != 3:
-            raise ValueError(tuple(raw.shape))
-        raw = raw.contiguous()
-        tr = transition_r.contiguous().float()
-        ti = transition_i.contiguous().float()
-        gm = gamma.contiguous().float()
-        B, L, three_c = raw.shape
-        if three_c % 3:
-            raise ValueError(tuple(raw.shape))
-        C = three_c // 3
-        if tr.numel() != C or ti.numel() != C or gm.numel() != C:
-            raise ValueError((tuple(raw.shape), tuple(tr.shape)))
-        if state_in is not None:
-            if tuple(state_in.shape) != (B, 2 * C):
-                raise ValueError((tuple(raw.shape), tuple(state_in.shape)))
-            state_in = state_in.contiguous().float()
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            read = torch.empty((B, L, 4 * C), device=raw.device, dtype=torch.float32)
-            state_out = torch.empty((B, 2 * C), device=raw.device, dtype=torch.float32)
-            ws, nbytes = _workspace(B, L, C, _FWD, raw.device)
-            rc = lib.fields_read_forward(_ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), _ptr(state_in),
-                                         _ptr(read), _ptr(state_out), _ptr(ws), nbytes,
-                                         B, L, C, _stream(raw.device))
-        _lib.check(rc, "fields_read_forward")
-        ctx.set_materialize_grads(False)
-        ctx.lean = bool(lean) and C % 4 == 0
-        if ctx.lean:
-            rows = lib.fields_read_state_rows(L)
-            kept = read[:, 7::8, :2 * C][:, :rows].contiguous()
-        else:
-            kept = read
-        ctx.save_for_backward(raw, tr, ti, gm, kept, state_in)
-        ctx.dims = (B, L, C)
-        return read, state_out
-
-    @staticmethod
-    def backward(ctx, grad_read, grad_state_out):
-        raw, tr, ti, gm, read, state_in = ctx.saved_tensors
-        B, L, C = ctx.dims
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            if grad_read is None:
-                grad_read = torch.zeros((B, L, 4 * C), device=raw.device, dtype=torch.float32)
-            grad_read = grad_read.contiguous().float()
-            if grad_state_out is not None:
-                grad_state_out = grad_state_out.contiguous().float()
-            grad_raw = torch.empty_like(raw)
-            g_par = torch.empty((3, C), device=raw.device, dtype=torch.float32)
-            g_sin = (torch.empty((B, 2 * C), device=raw.device, dtype=torch.float32)
-                     if state_in is not None and ctx.needs_input_grad[4] else None)
-            ws, nbytes = _workspace(B, L, C, _BWD, raw.device)
-            # lean: `read` holds the kept state rows (possibly none for L <= 8)
-            entry = lib.fields_read_backward_from_states if ctx.lean else lib.fields_read_backward
-            rc = entry(
-                _ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), _ptr(state_in),
-                _ptr(read) if read.numel() else None,
-                _ptr(grad_read), _ptr(grad_state_out), _ptr(grad_raw), _ptr(g_par[0]),
-                _ptr(g_par[1]), _ptr(g_par[2]), _ptr(g_sin), _ptr(ws), nbytes, B, L, C,
-                _stream(raw.device))
-        _lib.check(rc, "fields_read_backward")
-        return grad_raw, g_par[0], g_par[1], g_par[2], g_sin, None
-
-
-class FieldReadBf16Function(torch.autograd.Function):
-    """read = F(raw, tr, ti, gamma) with bfloat16 raw / read / gradients and an fp32 state."""
-
-    @staticmethod
-    def forward(ctx, raw, transition_r, transition_i, gamma):
-        if not raw.is_cuda:
-            raise RuntimeError("Chunked Field kernel requires CUDA")
-        if raw.dtype != torch.bfloat16:
-            raise TypeError(f"raw must be bfloat16, got {raw.dtype}")
-        if raw.dim() != 3 or raw.shape[2] % 3:
-            raise ValueError(tuple(raw.shape))
-        raw = raw.contiguous()
-        tr = transition_r.contiguous().float()
-        ti = transition_i.contiguous().float()
-        gm = gamma.contiguous().float()
-        B, L, three_c = raw.shape
-        C = three_c // 3
-        if tr.numel() != C or ti.numel() != C or gm.numel() != C:
-            raise ValueError((tuple(raw.shape), tuple(tr.shape)))
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            read = torch.empty((B, L, 4 * C), device=raw.device, dtype=torch.bfloat16)
-            ws, nbytes = _workspace(B, L, C, _FWD, raw.device)
-            rc = lib.fields_read_forward_bf16(_ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), None,
-                                              _ptr(read), None, _ptr(ws), nbytes, B, L, C,
-                                              _stream(raw.device))
-        _lib.check(rc, "fields_read_forward_bf16")
-        ctx.save_for_backward(raw, tr, ti, gm, read)
-        ctx.dims = (B, L, C)
-        return read
-
-    @staticmethod
-    def backward(ctx, grad_read):
-        raw, tr, ti, gm, read = ctx.saved_tensors
-        B, L, C = ctx.dims
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            grad_read = grad_read.contiguous().to(torch.bfloat16)
-            grad_raw = torch.empty_like(raw)
-            g_par = torch.empty((3, C), device=raw.device, dtype=torch.float32)
-            ws, nbytes = _workspace(B, L, C, _BWD, raw.device)
-            rc = lib.fields_read_backward_bf16(
-                _ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), None, _ptr(read), _ptr(grad_read), None,
-                _ptr(grad_raw), _ptr(g_par[0]), _ptr(g_par[1]), _ptr(g_par[2]), None, _ptr(ws),
-                nbytes, B, L, C, _stream(raw.device))
-        _lib.check(rc, "fields_read_backward_bf16")
-        return grad_raw, g_par[0], g_par[1], g_par[2]
-
-
-class FieldReadBf16StatsFunction(torch.autograd.Function):
-    """read, sumsq = F(raw, tr, ti, gamma): the bfloat16 operator plus, per token, the sum of the
-    squares of its 4C outputs (``sumsq [B, L]`` fp32, from the fp32 values before rounding)."""
-
-    @staticmethod
-    def forward(ctx, raw, transition_r, transition_i, gamma):
-        if not raw.is_cuda:
-            raise RuntimeError("Chunked Field kernel requires CUDA")
-        if raw.dtype != torch.bfloat16:
-            raise TypeError(f"raw must be bfloat16, got {raw.dtype}")
-        if raw.dim() != 3 or raw.shape[2] % 3 or raw.shape[0] == 0 or raw.shape[1] == 0:
-            raise ValueError(tuple(raw.shape))
-        raw = raw.contiguous()
-        tr = transition_r.contiguous().float()
-        ti = transition_i.contiguous().float()
-        gm = gamma.contiguous().float()
-        B, L, three_c = raw.shape
-        C = three_c // 3
-        if tr.numel() != C or ti.numel() != C or gm.numel() != C:
-            raise ValueError((tuple(raw.shape), tuple(tr.shape)))
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            read = torch.empty((B, L, 4 * C), device=raw.device, dtype=torch.bfloat16)
-            groups = torch.empty((B, L, (C + 127) // 128), device=raw.device, dtype=torch.float32)
-            ws, nbytes = _workspace(B, L, C, _FWD, raw.device)
-            rc = lib.fields_read_forward_bf16_stats(_ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), None,
-                                                    _ptr(read), _ptr(groups), None, _ptr(ws), nbytes,
-                                                    B, L, C, _stream(raw.device))
-            _lib.check(rc, "fields_read_forward_bf16_stats")
-            sumsq = groups.sum(dim=-1)
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(raw, tr, ti, gm, read)
-        ctx.dims = (B, L, C)
-        return read, sumsq
-
-    @staticmethod
-    def backward(ctx, grad_read, grad_sumsq):
-        raw, tr, ti, gm, read = ctx.saved_tensors
-        B, L, C = ctx.dims
-        lib = _lib.load()
-        with torch.cuda.device(raw.device):
-            # d sumsq / d read = 2 read: folded into the gradient the recurrence receives
-            if grad_sumsq is not None:
-                if grad_read is not None:
-                    grad_read = grad_read.contiguous().to(torch.bfloat16)
-                total = torch.empty_like(read)
-                rc = lib.fields_read_norm_grad_combine(_ptr(grad_read), _ptr(read),
-                                                       _ptr(grad_sumsq.contiguous().float()),
-                                                       _ptr(total), B * L, 4 * C,
-                                                       _stream(raw.device))
-                _lib.check(rc, "fields_read_norm_grad_combine")
-            elif grad_read is not None:
-                total = grad_read.contiguous().to(torch.bfloat16)
-            else:
-                total = torch.zeros_like(read)
-            grad_raw = torch.empty_like(raw)
-            g_par = torch.empty((3, C), device=raw.device, dtype=torch.float32)
-            ws, nbytes = _workspace(B, L, C, _BWD, raw.device)
-            rc = lib.fields_read_backward_bf16(
-                _ptr(raw), _ptr(tr), _ptr(ti), _ptr(gm), None, _ptr(read), _ptr(total), None,
-                _ptr(grad_raw), _ptr(g_par[0]), _ptr(g_par[1]), _ptr(g_par[2]), None, _ptr(ws),
-                nbytes, B, L, C, _stream(raw.device))
-        _lib.check(rc, "fields_read_backward_bf16")
-        return grad_raw, g_par[0], g_par[1], g_par[2]
+    def apply(raw, transition_r, transition_i, gamma, state_in, lean=False):
+        return _lib.native().field_read(raw, transition_r, transition_i, gamma, state_in, lean, True)
 
 
 def fused_field_read_bf16_stats(raw: torch.Tensor, transition_r: torch.Tensor,
@@ -231,7 +44,7 @@ def fused_field_read_bf16_stats(raw: torch.Tensor, transition_r: torch.Tensor,
     """``fused_field_read_bf16`` that also returns ``sumsq [B, L]`` (fp32): the sum of squares of
     each token's 4C outputs, which is all an RMS norm over ``read`` needs from it. Both outputs
     are differentiable."""
-    return FieldReadBf16StatsFunction.apply(raw, transition_r, transition_i, gamma)
+    return _lib.native().field_read_bf16(raw, transition_r, transition_i, gamma, True)
 
 
 class MixerEpilogueFunction(torch.autograd.Function):
@@ -296,14 +109,13 @@ def fused_field_read_bf16(raw: torch.Tensor, transition_r: torch.Tensor,
                           transition_i: torch.Tensor, gamma: torch.Tensor) -> torch.Tensor:
     """The operator on a bfloat16 boundary: ``raw [B, L, 3C]`` bf16 in, ``read [B, L, 4C]`` bf16
     out, fp32 state inside. For mixers that keep the write projection's bf16 output."""
-    return FieldReadBf16Function.apply(raw, transition_r, transition_i, gamma)
+    return _lib.native().field_read_bf16(raw, transition_r, transition_i, gamma, False)
 
 
 def fused_field_read(raw: torch.Tensor, transition_r: torch.Tensor, transition_i: torch.Tensor,
                      gamma: torch.Tensor, block_c: int = 32, chunk_t: int = 64) -> torch.Tensor:
     """Drop-in for the reference's ``fused_field_read``; returns ``read [B, L, 4C]`` fp32."""
-    read, _ = FieldReadFunction.apply(raw, transition_r, transition_i, gamma, None)
-    return read
+    return _lib.native().field_read(raw, transition_r, transition_i, gamma, None, False, False)
 
 
 def field_read_with_state(raw, transition_r, transition_i, gamma,
@@ -314,4 +126,4 @@ def field_read_with_state(raw, transition_r, transition_i, gamma,
     (the kernel recomputes the rest; about 7 % slower backward, 8 KB per token less saved by
     this operator). It pays when the consumer of ``read`` does not keep it either.
     """
-    return FieldReadFunction.apply(raw, transition_r, transition_i, gamma, state_in, lean)
+    return _lib.native().field_read(raw, transition_r, transition_i, gamma, state_in, lean, True)

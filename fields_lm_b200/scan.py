@@ -21,73 +21,6 @@ from typing import Callable, Optional
 import torch
 
 from . import _lib
-from .field_read import _ptr, _stream
-
-
-def _a_layout(a: torch.Tensor, B: int, L: int, C: int):
-    """``a`` as the library reads it: a dense tensor, or one value per (b, t) broadcast over the
-    channels (the expanded view the softpatch mixer passes). Returns (tensor, batch, step, chan)."""
-    if C > 1 and a.stride(2) == 0:
-        per_token = a[:, :, 0].contiguous()
-        return per_token, L, 1, 0
-    a = a.contiguous()
-    return a, L * C, C, 1
-
-
-class LinearScanFunction(torch.autograd.Function):
-    """states, state_out = F(a, b, state_in): ``s_t = a_t s_{t-1} + b_t`` along dim 1."""
-
-    @staticmethod
-    def forward(ctx, a, b, state_in):
-        B, L, C = b.shape
-        b = b.contiguous()
-        a_mem, a_batch, a_step, a_chan = _a_layout(a, B, L, C)
-        if state_in is not None:
-            if tuple(state_in.shape) != (B, C):
-                raise ValueError((tuple(b.shape), tuple(state_in.shape)))
-            state_in = state_in.contiguous().float()
-        lib = _lib.load()
-        with torch.cuda.device(b.device):
-            states = torch.empty_like(b)
-            state_out = torch.empty((B, C), device=b.device, dtype=torch.float32)
-            nbytes = lib.fields_scan_workspace_bytes(B, L, C)
-            ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=b.device)
-            rc = lib.fields_scan_forward(_ptr(a_mem), a_batch, a_step, a_chan, _ptr(b),
-                                         _ptr(state_in), _ptr(states), _ptr(state_out), _ptr(ws),
-                                         nbytes, B, L, C, _stream(b.device))
-        _lib.check(rc, "fields_scan_forward")
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(a_mem, states, state_in)
-        ctx.layout = (a_batch, a_step, a_chan)
-        ctx.dims = (B, L, C)
-        return states, state_out
-
-    @staticmethod
-    def backward(ctx, grad_states, grad_state_out):
-        a_mem, states, state_in = ctx.saved_tensors
-        a_batch, a_step, a_chan = ctx.layout
-        B, L, C = ctx.dims
-        lib = _lib.load()
-        dev = states.device
-        with torch.cuda.device(dev):
-            if grad_states is None:
-                grad_states = torch.zeros_like(states)
-            grad_states = grad_states.contiguous().float()
-            if grad_state_out is not None:
-                grad_state_out = grad_state_out.contiguous().float()
-            grad_a = torch.empty_like(states)
-            grad_b = torch.empty_like(states)
-            g_sin = (torch.empty((B, C), device=dev, dtype=torch.float32)
-                     if state_in is not None and ctx.needs_input_grad[2] else None)
-            nbytes = lib.fields_scan_workspace_bytes(B, L, C)
-            ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-            rc = lib.fields_scan_backward(_ptr(a_mem), a_batch, a_step, a_chan, _ptr(states),
-                                          _ptr(state_in), _ptr(grad_states), _ptr(grad_state_out),
-                                          _ptr(grad_a), _ptr(grad_b), _ptr(g_sin), _ptr(ws), nbytes,
-                                          B, L, C, _stream(dev))
-        _lib.check(rc, "fields_scan_backward")
-        # dense gradient of `a`; for an expanded `a` autograd sums it over the broadcast channels
-        return (grad_a if ctx.needs_input_grad[0] else None), grad_b, g_sin
 
 
 def _check(a: torch.Tensor, b: torch.Tensor, block: int) -> None:
@@ -104,7 +37,7 @@ def _check(a: torch.Tensor, b: torch.Tensor, block: int) -> None:
 def linear_scan(a: torch.Tensor, b: torch.Tensor, block: int = 32) -> torch.Tensor:
     """The reference's ``hierarchical_scan(a, b, block)`` for real fp32 CUDA tensors."""
     _check(a, b, block)
-    return LinearScanFunction.apply(a, b, None)[0]
+    return _lib.native().linear_scan(a, b, None)[0]
 
 
 def linear_scan_with_state(a: torch.Tensor, b: torch.Tensor,
@@ -112,7 +45,7 @@ def linear_scan_with_state(a: torch.Tensor, b: torch.Tensor,
     """The same scan from an incoming state ``[B, C]``; returns (states, state after the last
     step). An extension: the reference always starts from zero."""
     _check(a, b, 32)
-    return LinearScanFunction.apply(a, b, state_in)
+    return _lib.native().linear_scan(a, b, state_in)
 
 
 def scan_entry(original: Callable) -> Callable:
