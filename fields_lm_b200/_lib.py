@@ -55,6 +55,12 @@ SYMBOLS = {
     "fields_mixer_epilogue_bias_rows": (_SZ, [ctypes.c_longlong]),
     "fields_mixer_epilogue_forward": (_I, [_P] * 7 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
     "fields_mixer_epilogue_backward": (_I, [_P] * 11 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
+    "fields_stack_layout": (_I, [_P, _P]),
+    "fields_stack_step_norm": (_I, [_P, _LL, _P, _P, _P, ctypes.c_float, _LL, _I, _P]),
+    "fields_stack_close_mixer": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 5 +
+                                 [ctypes.c_float, _I, ctypes.c_float, _LL, _I, _P]),
+    "fields_stack_swiglu": (_I, [_P, _P, _LL, _I, _P]),
+    "fields_stack_close_ff": (_I, [_P] * 5 + [ctypes.c_float, _LL, _I, _P]),
     "fields_read_static_scratch_bytes": (_SZ, []),
     "fields_read_forward_noalloc": (_I, [_P] * 7 + [_I, _I, _I, _P]),
 }

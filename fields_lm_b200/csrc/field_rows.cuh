@@ -1,0 +1,323 @@
+// Row-wise glue of a Field block's inference path: everything between its matrix products.
+//
+// A block of the reference (field_only_v4_chunked_triton_wiki100.py:1198-1221) is, per token,
+//   y = x + out_proj(read_norm(read)) * sigmoid(gate_proj(x));   x' = y + w3(silu(u) * v),
+//   (u, v) = w12(ff_norm(y)).
+// Run as library calls that is about 35 elementwise and reduction kernels per block, each of them a
+// pass over [tokens, dim] (12 ms of a 13.3 ms prefill of 8 x 1,024 tokens through 18 blocks, 2.0 of
+// 2.5 ms of the kernels of a 256-row decode step). Here it is four kernels, each of which reads its
+// inputs once and leaves what the next matrix product wants, in bfloat16:
+//   layout_block   bfloat16 copies of a block's weights and its transition parameters
+//   step_norm      the decode recurrence of a row and its RMS norm      -> operand of out_proj
+//   close_mixer    residual and gate, then ff_norm                      -> operand of w12
+//   swiglu         silu(u) * v                                          -> operand of w3
+//   close_ff       residual, then a cast or the next norm               -> operand of what follows
+// The read_norm weight is folded into the out_proj copy (W diag(w)), so the norm is a per-token
+// scale: step_norm applies it to the row, close_mixer applies it to the product when the row's sum of
+// squares comes from the recurrence kernel (`groups`).
+//
+// All of it is bound by HBM for thousands of rows (close_mixer 14 B, swiglu 6 B per hidden unit,
+// close_ff 12 B per element) and by latency for a few hundred: a row is owned by one warp when there
+// are rows enough to fill the GPU that way, by four warps otherwise. Arithmetic is fp32 throughout.
+// Device only.
+#pragma once
+
+#include "field_math.cuh"
+
+#ifndef FIELDS_HOST_EMU
+
+namespace fields {
+
+constexpr int kRowThreads = 256;
+
+__device__ __forceinline__ Vec<4> load4(const float* p) { return vec_load<4>(p); }
+__device__ __forceinline__ Vec<4> load4(const uint16_t* p) { return io_load4(p); }
+
+// Ordinary (not streaming) store of four bfloat16: the next kernel reads them from L2.
+__device__ __forceinline__ void store_bf16x4(uint16_t* p, const Vec<4>& x) {
+    uint32_t lo, hi;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(x.v[1]), "f"(x.v[0]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(x.v[3]), "f"(x.v[2]));
+    *reinterpret_cast<uint2*>(p) = make_uint2(lo, hi);
+}
+
+// Sum over the W warps that own a row (W = 1: one warp; otherwise all warps of the block in groups of W).
+template <int W>
+__device__ __forceinline__ float row_sum(float v, float* scratch) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if constexpr (W > 1) {
+        const int warp = threadIdx.x >> 5;
+        if ((threadIdx.x & 31) == 0) scratch[warp] = v;
+        __syncthreads();
+        v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < W; ++w) v += scratch[warp / W * W + w];
+    }
+    return v;
+}
+
+struct CloseMixerParams {
+    const float* x;          // [N, D]
+    const uint16_t* acc;     // [N, D] bf16: output projection of the (scaled or unscaled) read rows
+    const uint16_t* gate;    // rows of gate_stride, bf16
+    const float* groups;     // [N, G] sums of squares of the read row, or null: acc is already scaled
+    const float* bias;       // [D] of the output projection
+    const float* gate_bias;  // [D] or null
+    const float* norm_w;     // [D] of ff_norm
+    float* y;                // [N, D] (may be x)
+    uint16_t* h;             // [N, D] bf16
+    long long N, gate_stride;
+    int D, G;
+    float eps, inv_features, norm_eps;
+};
+
+// W warps per row, V groups of four columns per lane: D <= 128 * W * V.
+template <int W, int V>
+__global__ void __launch_bounds__(kRowThreads) close_mixer(const CloseMixerParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float scratch[kRowThreads / 32];
+    constexpr int kRows = kRowThreads / 32 / W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long n = (long long)blockIdx.x * kRows + warp / W;
+    const bool row_ok = n < p.N;
+    const int col = ((warp % W) * 32 + lane) * 4;
+    float rstd = 1.0f;
+    if (row_ok && p.groups) {
+        float s = 0.0f;
+        for (int g = 0; g < p.G; ++g) s += p.groups[n * p.G + g];
+        rstd = rsqrtf(s * p.inv_features + p.eps);
+    }
+    Vec<4> y[V];
+    float sq = 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = col + j * 128 * W;
+        if (row_ok && c < p.D) {
+            const Vec<4> xv = load4(p.x + n * p.D + c);
+            const Vec<4> a = load4(p.acc + n * p.D + c);
+            const Vec<4> g = load4(p.gate + n * p.gate_stride + c);
+            const Vec<4> b = load4(p.bias + c);
+            const Vec<4> gb = p.gate_bias ? load4(p.gate_bias + c) : vec_fill<4>(0.0f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                y[j].v[k] = xv.v[k] + (a.v[k] * rstd + b.v[k]) * sigmoidf_fast(g.v[k] + gb.v[k]);
+                sq += y[j].v[k] * y[j].v[k];
+            }
+            vec_store<4>(p.y + n * p.D + c, y[j]);
+        }
+    }
+    const float inv = rsqrtf(row_sum<W>(sq, scratch) / (float)p.D + p.norm_eps);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = col + j * 128 * W;
+        if (row_ok && c < p.D) {
+            const Vec<4> w = load4(p.norm_w + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) y[j].v[k] = y[j].v[k] * inv * w.v[k];
+            store_bf16x4(p.h + n * p.D + c, y[j]);
+        }
+    }
+}
+
+struct CloseFfParams {
+    const float* x;        // [N, D]
+    const uint16_t* f;     // [N, D] bf16: output of the feed-forward, or null
+    const float* norm_w;   // [D] of the norm that follows, or null: plain cast
+    float* y;              // [N, D] x + f (may be x), or null
+    uint16_t* h;           // [N, D] bf16
+    long long N;
+    int D;
+    float norm_eps;
+};
+
+template <int W, int V>
+__global__ void __launch_bounds__(kRowThreads) close_ff(const CloseFfParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float scratch[kRowThreads / 32];
+    constexpr int kRows = kRowThreads / 32 / W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long n = (long long)blockIdx.x * kRows + warp / W;
+    const bool row_ok = n < p.N;
+    const int col = ((warp % W) * 32 + lane) * 4;
+    Vec<4> y[V];
+    float sq = 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = col + j * 128 * W;
+        if (row_ok && c < p.D) {
+            y[j] = load4(p.x + n * p.D + c);
+            if (p.f) {
+                const Vec<4> f = load4(p.f + n * p.D + c);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y[j].v[k] += f.v[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sq += y[j].v[k] * y[j].v[k];
+            if (p.y) vec_store<4>(p.y + n * p.D + c, y[j]);
+        }
+    }
+    float inv = 1.0f;
+    if (p.norm_w) inv = rsqrtf(row_sum<W>(sq, scratch) / (float)p.D + p.norm_eps);  // (uniform branch)
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = col + j * 128 * W;
+        if (row_ok && c < p.D) {
+            if (p.norm_w) {
+                const Vec<4> w = load4(p.norm_w + c);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y[j].v[k] = y[j].v[k] * inv * w.v[k];
+            }
+            store_bf16x4(p.h + n * p.D + c, y[j]);
+        }
+    }
+}
+
+struct SwigluParams {
+    const uint16_t* uv;  // [N, 2H] bf16: u | v
+    uint16_t* out;       // [N, H] bf16
+    long long N;
+    int H;
+};
+
+// One 16-byte access of each half and one of the result per thread and item; H % 8 == 0.
+__global__ void __launch_bounds__(kRowThreads) swiglu(const SwigluParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int per_row = p.H / 8;
+    const long long items = p.N * per_row;
+    const long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x;
+    if (i >= items) return;
+    const long long n = i / per_row;
+    const int c = (int)(i - n * per_row) * 8;
+    const uint4 u = *reinterpret_cast<const uint4*>(p.uv + n * 2 * p.H + c);
+    const uint4 v = *reinterpret_cast<const uint4*>(p.uv + n * 2 * p.H + p.H + c);
+    const Vec<4> u0 = bf16x4_unpack(u.x, u.y), u1 = bf16x4_unpack(u.z, u.w);
+    const Vec<4> v0 = bf16x4_unpack(v.x, v.y), v1 = bf16x4_unpack(v.z, v.w);
+    Vec<4> a, b;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        a.v[k] = u0.v[k] * sigmoidf_fast(u0.v[k]) * v0.v[k];
+        b.v[k] = u1.v[k] * sigmoidf_fast(u1.v[k]) * v1.v[k];
+    }
+    uint32_t o[4];
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[0]) : "f"(a.v[1]), "f"(a.v[0]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[1]) : "f"(a.v[3]), "f"(a.v[2]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[2]) : "f"(b.v[1]), "f"(b.v[0]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[3]) : "f"(b.v[3]), "f"(b.v[2]));
+    *reinterpret_cast<uint4*>(p.out + n * p.H + c) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+struct StepNormParams {
+    const uint16_t* raw;  // rows of raw_stride, bf16: z_r | z_i | z_v
+    const float* par;     // [3, C] Re lambda | Im lambda | gamma
+    float* state;         // [N, 2C] in and out
+    uint16_t* out;        // [N, 4C] bf16: read / rms(read)
+    long long N, raw_stride;
+    int C;
+    float eps;
+};
+
+// One recurrence step of a row (the arithmetic of DecodeStep) and its RMS norm; 128 threads per row,
+// four channels per thread and group: C <= 512 * V, C % 4 == 0.
+template <int V>
+__global__ void __launch_bounds__(128) step_norm(const StepNormParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float scratch[4];
+    const long long n = blockIdx.x;
+    const int C = p.C;
+    Vec<4> sr[V], si[V], dr[V], di[V];
+    float sq = 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = (int)threadIdx.x * 4 + j * 512;
+        if (c < C) {
+            const uint16_t* raw = p.raw + n * p.raw_stride + c;
+            const Vec<4> zr = load4(raw), zi = load4(raw + C), zv = load4(raw + 2 * C);
+            const Vec<4> lr = load4(p.par + c), li = load4(p.par + C + c), gm = load4(p.par + 2 * C + c);
+            float* st = p.state + n * 2 * C + c;
+            sr[j] = load4(st);
+            si[j] = load4(st + C);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const Gate g = make_gate(zr.v[k], zi.v[k], zv.v[k]);
+                float mr, mi;
+                cmul(lr.v[k], li.v[k], sr[j].v[k], si[j].v[k], mr, mi);
+                const float bs = gm.v[k] * g.vac;
+                sr[j].v[k] = (1.0f - g.vac) * mr + bs * g.inj_r;
+                si[j].v[k] = (1.0f - g.vac) * mi + bs * g.inj_i;
+                dr[j].v[k] = g.vac * mr;
+                di[j].v[k] = g.vac * mi;
+                sq += sr[j].v[k] * sr[j].v[k] + si[j].v[k] * si[j].v[k] + dr[j].v[k] * dr[j].v[k] +
+                      di[j].v[k] * di[j].v[k];
+            }
+            vec_store<4>(st, sr[j]);
+            vec_store<4>(st + C, si[j]);
+        }
+    }
+    const float inv = rsqrtf(row_sum<4>(sq, scratch) / (float)(4 * C) + p.eps);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int c = (int)threadIdx.x * 4 + j * 512;
+        if (c < C) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                sr[j].v[k] *= inv; si[j].v[k] *= inv; dr[j].v[k] *= inv; di[j].v[k] *= inv;
+            }
+            uint16_t* o = p.out + n * 4 * C + c;
+            store_bf16x4(o, sr[j]);
+            store_bf16x4(o + C, si[j]);
+            store_bf16x4(o + 2 * C, dr[j]);
+            store_bf16x4(o + 3 * C, di[j]);
+        }
+    }
+}
+
+// One contiguous piece of a block's weights on its way to bfloat16: n elements (a multiple of 4),
+// column j of a row of `cols` scaled by scale[j] if given. radius / theta pieces: see layout_block.
+struct LayoutPiece {
+    const float* src;
+    uint16_t* dst;
+    const float* scale;
+    long long n;
+    int cols;
+};
+constexpr int kLayoutPieces = 7;
+
+struct LayoutParams {
+    LayoutPiece piece[kLayoutPieces];
+    const float* radius_logit;  // [C]
+    const float* theta;         // [C]
+    float* par;                 // [3, C]
+    int C;
+};
+
+// blockIdx.y: the piece; the last y index computes the transition parameters (reference :1169-1173):
+// lambda = r e^{i theta}, r = clamp(sigmoid(logit), 0.5, 0.99995), gamma = sqrt(max(1 - r^2, 1e-4)).
+__global__ void __launch_bounds__(kRowThreads) layout_block(const LayoutParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.y == kLayoutPieces) {
+        for (int c = blockIdx.x * kRowThreads + threadIdx.x; c < p.C; c += gridDim.x * kRowThreads) {
+            const float r = fminf(fmaxf(1.0f / (1.0f + expf(-p.radius_logit[c])), 0.50f), 0.99995f);
+            const float t = p.theta[c];
+            p.par[c] = r * cosf(t);
+            p.par[p.C + c] = r * sinf(t);
+            p.par[2 * p.C + c] = sqrtf(fmaxf(1.0f - r * r, 1e-4f));
+        }
+        return;
+    }
+    const LayoutPiece q = p.piece[blockIdx.y];
+    const long long step = (long long)gridDim.x * kRowThreads * 4;
+    for (long long i = ((long long)blockIdx.x * kRowThreads + threadIdx.x) * 4; i < q.n; i += step) {
+        Vec<4> v = vec_load_stream<4>(q.src + i);
+        if (q.scale) {
+            const Vec<4> s = load4(q.scale + i % q.cols);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v.v[k] *= s.v[k];
+        }
+        store_bf16x4(q.dst + i, v);
+    }
+}
+
+}  // namespace fields
+
+#endif  // FIELDS_HOST_EMU

@@ -16,6 +16,7 @@
 #include "field_tensor.cuh"
 #include "field_scan.cuh"
 #include "field_epilogue.cuh"
+#include "field_rows.cuh"
 
 #include "../../include/fields_read.h"
 
@@ -214,10 +215,10 @@ static int check_cuda(cudaError_t e) {
 
 // One launch, with the programmatic-serialization attribute unless FIELDS_READ_PDL=0.
 template <class P>
-static int launch_on(void (*fn)(const P), unsigned grid, unsigned threads, size_t bytes, Stream st,
-                     const P& params) {
+static int launch_grid(void (*fn)(const P), dim3 grid, unsigned threads, Stream st, const P& params,
+                       size_t bytes = 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
@@ -227,6 +228,12 @@ static int launch_on(void (*fn)(const P), unsigned grid, unsigned threads, size_
     cfg.attrs = attr;
     cfg.numAttrs = dependent_launch_enabled() ? 1 : 0;
     return check_cuda(cudaLaunchKernelEx(&cfg, fn, params));
+}
+
+template <class P>
+static int launch_on(void (*fn)(const P), unsigned grid, unsigned threads, size_t bytes, Stream st,
+                     const P& params) {
+    return launch_grid<P>(fn, dim3(grid), threads, st, params, bytes);
 }
 
 template <class K>
@@ -1749,6 +1756,105 @@ int fields_read_norm_grad_combine(const void* grad_read, const void* read, const
                      grad_sumsq, static_cast<uint16_t*>(total), N, F};
     return launch_on<NormGradParams>(norm_grad_combine, (unsigned)blocks, kEpiThreads, 0,
                                      reinterpret_cast<Stream>(stream), p);
+}
+
+int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
+    if (!w || w->dim <= 0 || w->hidden <= 0) return FIELDS_ERR_ARGUMENT;
+    if (!w->write_w || !w->write_b || !w->gate_w || !w->out_w || !w->read_norm_w || !w->w12 || !w->w3 ||
+        !w->radius_logit || !w->theta || !w->in_w || !w->in_b || !w->out_w16 || !w->w12_16 || !w->w3_16 ||
+        !w->par)
+        return FIELDS_ERR_ARGUMENT;
+    const long long D = w->dim, H = w->hidden, C = D / 2;
+    const void* all[] = {w->write_w, w->write_b, w->gate_w, w->out_w, w->read_norm_w, w->w12, w->w3,
+                         w->in_w, w->in_b, w->out_w16, w->w12_16, w->w3_16};
+    if (D % 8 || H % 8) return FIELDS_ERR_UNSUPPORTED;
+    for (const void* q : all)
+        if (!aligned16(q)) return FIELDS_ERR_UNSUPPORTED;
+    uint16_t* in_w = static_cast<uint16_t*>(w->in_w);
+    LayoutParams p{};
+    p.piece[0] = {w->write_w, in_w, nullptr, 3 * C * D, (int)D};
+    p.piece[1] = {w->gate_w, in_w + 3 * C * D, nullptr, D * D, (int)D};
+    p.piece[2] = {w->write_b, static_cast<uint16_t*>(w->in_b), nullptr, 3 * C, (int)(3 * C)};
+    p.piece[3] = {w->out_w, static_cast<uint16_t*>(w->out_w16), w->read_norm_w, D * 2 * D, (int)(2 * D)};
+    p.piece[4] = {w->w12, static_cast<uint16_t*>(w->w12_16), nullptr, 2 * H * D, (int)D};
+    p.piece[5] = {w->w3, static_cast<uint16_t*>(w->w3_16), nullptr, D * H, (int)H};
+    p.piece[6] = {nullptr, nullptr, nullptr, 0, 4};
+    p.radius_logit = w->radius_logit; p.theta = w->theta; p.par = w->par; p.C = (int)C;
+    // as many blocks per piece as the GPU has SMs: the pieces run side by side
+    return launch_grid<LayoutParams>(layout_block, dim3(148, kLayoutPieces + 1), kRowThreads,
+                                     reinterpret_cast<Stream>(stream), p);
+}
+
+int fields_stack_step_norm(const void* raw, long long raw_stride, const float* par, float* state,
+                           void* out, float eps, long long N, int C, void* stream) {
+    if (N < 0 || C <= 0) return FIELDS_ERR_ARGUMENT;
+    if (N == 0) return FIELDS_OK;
+    if (!raw || !par || !state || !out) return FIELDS_ERR_ARGUMENT;
+    if (C % 4 || C > 2048 || raw_stride % 4 || N > 0x7fffffffLL || !aligned8(raw) || !aligned16(par) ||
+        !aligned16(state) || !aligned8(out))
+        return FIELDS_ERR_UNSUPPORTED;
+    StepNormParams p{static_cast<const uint16_t*>(raw), par, state, static_cast<uint16_t*>(out), N,
+                     raw_stride, C, eps};
+    return launch_on<StepNormParams>(C <= 512 ? step_norm<1> : step_norm<4>, (unsigned)N, 128, 0,
+                                     reinterpret_cast<Stream>(stream), p);
+}
+
+}  // extern "C"
+
+// Which of the row kernels: one warp per row where that already fills the GPU (148 SMs of 32 warps) and
+// a row fits a warp's registers, four warps per row otherwise (fewer rows: shorter chains per thread).
+template <class P>
+static int launch_rows(void (*one)(const P), void (*four)(const P), void (*wide)(const P), long long N,
+                       int D, void* stream, const P& p) {
+    const bool single = D <= 1024 && N >= 148 * 32;
+    const long long per_block = single ? kRowThreads / 32 : kRowThreads / 128;
+    const long long blocks = (N + per_block - 1) / per_block;
+    if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+    return launch_on<P>(single ? one : D <= 1024 ? four : wide, (unsigned)blocks, kRowThreads, 0,
+                        reinterpret_cast<Stream>(stream), p);
+}
+
+extern "C" {
+
+int fields_stack_close_mixer(const float* x, const void* acc, const void* gate, long long gate_stride,
+                             const float* groups, int G, const float* bias, const float* gate_bias,
+                             const float* norm_w, float* y, void* h, float eps, int features,
+                             float norm_eps, long long N, int D, void* stream) {
+    if (N < 0 || D <= 0 || features <= 0 || G < 0) return FIELDS_ERR_ARGUMENT;
+    if (N == 0) return FIELDS_OK;
+    if (!x || !acc || !gate || !bias || !norm_w || !y || !h) return FIELDS_ERR_ARGUMENT;
+    if (D % 4 || D > 4096 || gate_stride % 4 || !aligned16(x) || !aligned16(y) || !aligned16(bias) ||
+        !aligned16(gate_bias) || !aligned16(norm_w) || !aligned8(acc) || !aligned8(gate) || !aligned8(h))
+        return FIELDS_ERR_UNSUPPORTED;
+    CloseMixerParams p{x, static_cast<const uint16_t*>(acc), static_cast<const uint16_t*>(gate), groups,
+                       bias, gate_bias, norm_w, y, static_cast<uint16_t*>(h), N, gate_stride, D, G, eps,
+                       1.0f / (float)features, norm_eps};
+    return launch_rows<CloseMixerParams>(close_mixer<1, 8>, close_mixer<4, 2>, close_mixer<4, 8>, N, D,
+                                         stream, p);
+}
+
+int fields_stack_swiglu(const void* uv, void* out, long long N, int H, void* stream) {
+    if (N < 0 || H <= 0) return FIELDS_ERR_ARGUMENT;
+    if (N == 0) return FIELDS_OK;
+    if (!uv || !out) return FIELDS_ERR_ARGUMENT;
+    if (H % 8 || !aligned16(uv) || !aligned16(out)) return FIELDS_ERR_UNSUPPORTED;
+    const long long blocks = (N * (H / 8) + kRowThreads - 1) / kRowThreads;
+    if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+    SwigluParams p{static_cast<const uint16_t*>(uv), static_cast<uint16_t*>(out), N, H};
+    return launch_on<SwigluParams>(swiglu, (unsigned)blocks, kRowThreads, 0,
+                                   reinterpret_cast<Stream>(stream), p);
+}
+
+int fields_stack_close_ff(const float* x, const void* f, const float* norm_w, float* y, void* h,
+                          float norm_eps, long long N, int D, void* stream) {
+    if (N < 0 || D <= 0) return FIELDS_ERR_ARGUMENT;
+    if (N == 0) return FIELDS_OK;
+    if (!x || !h) return FIELDS_ERR_ARGUMENT;
+    if (D % 4 || D > 4096 || !aligned16(x) || !aligned16(y) || !aligned16(norm_w) || !aligned8(f) ||
+        !aligned8(h))
+        return FIELDS_ERR_UNSUPPORTED;
+    CloseFfParams p{x, static_cast<const uint16_t*>(f), norm_w, y, static_cast<uint16_t*>(h), N, D, norm_eps};
+    return launch_rows<CloseFfParams>(close_ff<1, 8>, close_ff<4, 2>, close_ff<4, 8>, N, D, stream, p);
 }
 #endif  // FIELDS_HOST_EMU
 

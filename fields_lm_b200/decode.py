@@ -44,16 +44,45 @@ class FieldStackDecoder:
                                 "stepped")
         self.model = model
         self.states = None
+        self._stack = None     # native runner of the blocks (csrc/torch_stack.cpp), where it applies
+        self._refused = False  # it did not apply when last asked for (asked again at a prefill)
 
     def reset(self) -> None:
         self.states = None
+        self._stack = None
+
+    @staticmethod
+    def _bf16_products(x: torch.Tensor) -> bool:
+        """Whether the caller's context is the one the native runner computes: fp32 activations
+        under bfloat16 autocast."""
+        return (x.is_cuda and x.dtype == torch.float32 and x.numel() > 0
+                and torch.is_autocast_enabled("cuda")
+                and torch.get_autocast_dtype("cuda") == torch.bfloat16)
+
+    def _native_stack(self, x: torch.Tensor):
+        """The runner for the model as it is now, or None."""
+        if self._stack is None or not self._stack.same_model():
+            from .stack import plan
+            self._stack = plan(self.model, x.device)
+            self._refused = self._stack is None
+        return self._stack
 
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, last_only: bool = True) -> torch.Tensor:
         """Runs the prompt ``tokens [B, T]`` and stores the blocks' end states. Returns the
-        logits of the last position ``[B, V]``, or of every position with ``last_only=False``."""
+        logits of the last position ``[B, V]``, or of every position with ``last_only=False``.
+
+        Under bfloat16 autocast the blocks run natively where they are what that path computes
+        (``fields_lm_b200.stack``); the weights are laid out for it here, and the steps that
+        follow use the same copies until a parameter changes."""
         from .mixer import block_prefill
         x = self.model.emb(tokens)
+        if self._bf16_products(x) and x.dim() == 3:
+            stack = self._native_stack(x)
+            if stack is not None:
+                stack.layout()
+                x, self.states = stack.prefill(x)
+                return self.model.lm_head(self.model.final_norm(x[:, -1] if last_only else x))
         states = []
         for block in self.model.blocks:
             x, state = block_prefill(block, x)
@@ -70,6 +99,15 @@ class FieldStackDecoder:
         if self.states is None:
             raise RuntimeError("call prefill() before step()")
         x = self.model.emb(tokens)
+        if not self._refused and self._bf16_products(x) and x.dim() == 2:
+            stack = self._stack
+            if stack is None or not stack.current():  # something has changed since the prefill
+                stack = self._native_stack(x)
+                if stack is not None:
+                    stack.layout()
+            if stack is not None:
+                out = stack.step(x, self.states)
+                return out if stack.has_head else self.model.lm_head(self.model.final_norm(out))
         for block, state in zip(self.model.blocks, self.states):
             x = block_step(block, x, state)
         return self.model.lm_head(self.model.final_norm(x))

@@ -1,0 +1,138 @@
+"""Recognises a stack of the reference's Field blocks that the native inference path can run.
+
+``plan(model)`` looks at a field-only language model (the reference's ``ByteLM``,
+``field_only_v4_chunked_triton_wiki100.py:1306-1344``) and returns a ``FieldStack``
+(``csrc/torch_stack.cpp``) that runs its blocks under bfloat16 autocast with a handful of launches
+per block, or None if any part of the model is not what that path computes: other module
+classes, hooks, parameters that are not dense fp32 tensors on one GPU, sizes the kernels do not
+take. The feed-forward and the norms are modules of the model's own, so each one is also run once
+on a small input and compared with the formula the kernels use.
+"""
+from __future__ import annotations
+
+from typing import List, Optional
+
+import torch
+import torch.nn.functional as F
+
+from . import _lib
+
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks")
+
+
+class _NotApplicable(Exception):
+    pass
+
+
+def _need(ok: bool) -> None:
+    if not ok:
+        raise _NotApplicable
+
+
+class _Survey:
+    """Collects what the plan depends on: parameters, the slots they sit in, hook dictionaries,
+    and how far each module is from the formula it is taken for."""
+
+    def __init__(self, device):
+        self.device = device
+        self.slots, self.hooks, self.errors = [], [], []
+
+    def child(self, module, name: str):
+        _need(name in module._modules)
+        child = module._modules[name]
+        self.slots.append((module._modules, name, child))
+        self.hooks += [getattr(child, h) for h in _HOOKS]
+        return child
+
+    def parameter(self, module, name: str, *shape: int) -> torch.Tensor:
+        _need(name in module._parameters)
+        p = module._parameters[name]
+        _need(isinstance(p, torch.Tensor) and p.dtype == torch.float32 and p.device == self.device
+              and tuple(p.shape) == shape and p.is_contiguous() and p.data_ptr() % 16 == 0)
+        self.slots.append((module._parameters, name, p))
+        return p
+
+    def linear(self, module, name: str, rows: int, cols: int, bias: bool):
+        lin = self.child(module, name)
+        _need(type(lin) is torch.nn.Linear and (lin.bias is not None) == bias)
+        weight = self.parameter(lin, "weight", rows, cols)
+        return (weight, self.parameter(lin, "bias", rows)) if bias else (weight, None)
+
+    def norm(self, module, name: str, dim: int):
+        norm = self.child(module, name)
+        _need(type(norm).__name__ == "RMSNorm" and isinstance(getattr(norm, "eps", None), float))
+        weight = self.parameter(norm, "weight", dim)
+        self.compare(norm, dim, lambda x: x * torch.rsqrt(x.square().mean(-1, keepdim=True) + norm.eps) * weight)
+        return weight, norm.eps
+
+    def compare(self, module, dim: int, formula) -> None:
+        x = torch.arange(2 * dim, device=self.device, dtype=torch.float32).mul_(0.7).sin_().view(2, dim)
+        want = formula(x)
+        got = module(x)
+        _need(got.shape == want.shape and got.dtype == want.dtype)
+        self.errors.append((got - want).abs().max() / want.abs().max().clamp_min(1e-6))
+
+
+def _block(s: _Survey, blocks, key: str, dim: int):
+    block = s.child(blocks, key)
+    _need(type(block).__name__ == "FieldBlock")
+    mixer = s.child(block, "mixer")
+    _need(type(mixer).__name__ == "IndependentVacancyField" and mixer.dim == dim
+          and 2 * mixer.channels == dim)
+    channels = dim // 2
+    write = s.linear(mixer, "write_proj", 3 * channels, dim, True)
+    gate = s.linear(mixer, "gate_proj", dim, dim, True)
+    out = s.linear(mixer, "out_proj", dim, 2 * dim, True)
+    read_norm, read_eps = s.norm(mixer, "read_norm", 2 * dim)
+    ff_norm, ff_eps = s.norm(block, "ff_norm", dim)
+    ff = s.child(block, "ff")
+    _need(type(ff).__name__ == "PackedSwiGLU" and "w3" in ff._modules)
+    hidden = ff._modules["w3"].weight.shape[1]
+    _need(hidden % 8 == 0)
+    w12, _ = s.linear(ff, "w12", 2 * hidden, dim, False)
+    w3, _ = s.linear(ff, "w3", dim, hidden, False)
+
+    def feed_forward(x):
+        u, v = F.linear(x, w12).chunk(2, dim=-1)
+        return F.linear(F.silu(u) * v, w3)
+
+    s.compare(ff, dim, feed_forward)
+    radius = s.parameter(mixer, "radius_logit", channels)
+    theta = s.parameter(mixer, "theta", channels)
+    return [*write, *gate, *out, read_norm, ff_norm, w12, w3, radius, theta], (read_eps, ff_eps), hidden
+
+
+@torch.no_grad()
+def plan(model: torch.nn.Module, device: torch.device) -> Optional[object]:
+    """The native runner for ``model``'s blocks, or None if they are not what it computes."""
+    if torch.cuda.is_current_stream_capturing():
+        return None  # the comparison below reads a value back
+    s = _Survey(device)
+    try:
+        with torch.autocast("cuda", enabled=False):
+            blocks = s.child(model, "blocks")
+            _need(len(blocks) > 0 and type(blocks) is torch.nn.ModuleList)
+            first = blocks[0]
+            dim = int(getattr(getattr(first, "mixer", None), "dim", 0))
+            _need(dim > 0 and dim % 8 == 0 and dim <= 4096)
+            params: List[list] = []
+            eps, widths = [], set()
+            for key in blocks._modules:
+                p, e, hidden = _block(s, blocks, key, dim)
+                params.append(p)
+                eps.append(e)
+                widths.add(hidden)
+            _need(len(widths) == 1)
+            tail, tail_eps = [], 0.0
+            head = model._modules.get("lm_head")
+            if type(head) is torch.nn.Linear and not any(getattr(head, h) for h in _HOOKS):
+                weight, tail_eps = s.norm(model, "final_norm", dim)
+                w, b = s.linear(model, "lm_head", head.weight.shape[0], dim, head.bias is not None)
+                tail = [weight, w] + ([] if b is None else [b])
+            s.hooks += [getattr(torch.nn.modules.module, "_global" + h) for h in _HOOKS]
+            _need(not any(s.hooks))
+            _need(float(torch.stack(s.errors).max()) < 1e-4)
+    except (_NotApplicable, AttributeError):
+        return None
+    sizes = [(h, 0) for h in s.hooks] + [(blocks._modules, len(params))]
+    return _lib.native().FieldStack(params, eps, s.slots, sizes, tail, tail_eps)

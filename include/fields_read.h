@@ -458,6 +458,40 @@ int fields_mixer_epilogue_backward(const float *grad_y, const void *acc, const v
                                    float *grad_bias_rows, float *grad_gate_bias_rows, float eps,
                                    int features, long long N, int D, void *stream);
 
+/*
+ * Inference through a stack of Field blocks in bfloat16 products and fp32 elementwise arithmetic: what
+ * lies between the matrix products of a block (field_only_v4_chunked_triton_wiki100.py:1198-1221), a
+ * kernel each. D = dim, C = D / 2, H = hidden width of the SwiGLU; D % 8 == 0, D <= 4096, H % 8 == 0;
+ * tensors dense and 16-byte aligned (FIELDS_ERR_UNSUPPORTED otherwise). bf16 operands are void *.
+ *
+ * fields_stack_layout: bfloat16 copies of a block's weights as the products want them, and its
+ *   transition parameters. in_w = write_proj over gate_proj, in_b = write_proj's bias over zeros (the
+ *   caller zeroed it: only the first 3C elements are written), out_w16 = out_proj diag(read_norm).
+ * fields_stack_step_norm: one recurrence step of N rows from raw (row stride raw_stride) and par
+ *   [3, C]; state [N, 2C] advances in place; out [N, 4C] = read / rms(read).
+ * fields_stack_close_mixer: y = x + (acc r + bias) * sigmoid(gate + gate_bias) and h = norm_w * y /
+ *   rms(y); r is the RMS scale of the row's read values if groups [N, G] gives their sums of squares,
+ *   1 if it is NULL.
+ * fields_stack_swiglu: out = silu(u) * v for uv [N, 2H] = u | v.
+ * fields_stack_close_ff: y = x + f (f NULL: x; y NULL: not stored) and h = y, or norm_w * y / rms(y).
+ */
+struct fields_stack_weights {
+    const float *write_w, *write_b, *gate_w, *out_w, *read_norm_w, *w12, *w3, *radius_logit, *theta;
+    void *in_w, *in_b, *out_w16, *w12_16, *w3_16;
+    float *par;
+    int dim, hidden;
+};
+int fields_stack_layout(const struct fields_stack_weights *weights, void *stream);
+int fields_stack_step_norm(const void *raw, long long raw_stride, const float *par, float *state,
+                           void *out, float eps, long long N, int C, void *stream);
+int fields_stack_close_mixer(const float *x, const void *acc, const void *gate, long long gate_stride,
+                             const float *groups, int G, const float *bias, const float *gate_bias,
+                             const float *norm_w, float *y, void *h, float eps, int features,
+                             float norm_eps, long long N, int D, void *stream);
+int fields_stack_swiglu(const void *uv, void *out, long long N, int H, void *stream);
+int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, float *y, void *h,
+                          float norm_eps, long long N, int D, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

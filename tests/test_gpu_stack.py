@@ -1,0 +1,88 @@
+"""The native inference path of FieldStackDecoder (csrc/torch_stack.cpp, field_rows.cuh) against the
+same decoder running the model's modules one by one (GPU)."""
+import pytest
+import torch
+
+import mirror
+from conftest import BF16_TOL
+from fields_lm_b200 import FieldStackDecoder, stack
+
+pytestmark = pytest.mark.gpu
+
+
+class LM(torch.nn.Module):
+    def __init__(self, dim, layers, hidden, bias=False):
+        super().__init__()
+        self.emb = torch.nn.Embedding(97, dim)
+        self.blocks = torch.nn.ModuleList(mirror.FieldBlock(dim, ff_hidden=hidden) for _ in range(layers))
+        self.final_norm = mirror.RMSNorm(dim)
+        self.lm_head = torch.nn.Linear(dim, 97, bias=bias)
+
+
+def _rel(a, b):
+    return float((a.float() - b.float()).abs().max() / b.float().abs().max().clamp_min(1e-6))
+
+
+def _run(model, tokens, prefix, native):
+    dec = FieldStackDecoder(model)
+    dec._refused = not native
+    plan = stack.plan
+    if not native:
+        stack.plan = lambda *a: None
+    try:
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            out = [dec.prefill(tokens[:, :prefix], last_only=False)[:, -1]]
+            out += [dec.step(tokens[:, t]) for t in range(prefix, tokens.shape[1])]
+    finally:
+        stack.plan = plan
+    assert (dec._stack is not None) == native
+    return out, dec
+
+
+# one block's rounding differences grow by at most their sum over the blocks: BF16_TOL holds for three
+@pytest.mark.parametrize("dim,hidden,B,L", [(64, 8, 1, 1), (64, 40, 5, 3), (200, 96, 3, 37), (1024, 2528, 2, 64),
+                                            (1024, 704, 601, 8), (1032, 352, 4, 5), (4096, 64, 2, 6)])
+def test_native_stack_matches_the_modules(dim, hidden, B, L):
+    torch.manual_seed(dim + B)
+    model = LM(dim, 3, hidden, bias=dim == 200).cuda()
+    for p in model.parameters():  # norm weights away from one
+        if p.dim() == 1 and p.numel() in (dim, 2 * dim):
+            p.data += 0.1 * torch.randn_like(p)
+    tokens = torch.randint(0, 97, (B, L + 3), device="cuda")
+    got, dec = _run(model, tokens, L, True)
+    want, ref = _run(model, tokens, L, False)
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        assert _rel(a, b) < BF16_TOL
+    for a, b in zip(dec.states, ref.states):
+        assert a.dtype == torch.float32 and _rel(a, b) < BF16_TOL
+
+
+def test_native_stack_follows_the_model():
+    """Weights written in place, replaced or hooked after the prefill are seen by the next step."""
+    torch.manual_seed(0)
+    model = LM(64, 2, 32).cuda()
+    tokens = torch.randint(0, 97, (4, 6), device="cuda")
+    _, dec = _run(model, tokens, 6, True)
+
+    def step():
+        states = [s.clone() for s in dec.states]
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            out = dec.step(tokens[:, 0])
+        dec.states = states
+        return out
+
+    before = step()
+    assert torch.equal(before, step())
+    with torch.no_grad():
+        model.blocks[1].ff.w3.weight.mul_(3.0)
+    changed = step()
+    assert _rel(changed, before) > BF16_TOL
+    with torch.no_grad():
+        model.blocks[1].ff.w3.weight.div_(3.0)
+    assert _rel(step(), before) < BF16_TOL
+    model.blocks[1].ff.w3.weight = torch.nn.Parameter(model.blocks[1].ff.w3.weight.detach() * 3.0)
+    assert _rel(step(), changed) < BF16_TOL
+    seen = []
+    model.blocks[0].ff_norm.register_forward_hook(lambda *a: seen.append(1))
+    assert _rel(step(), changed) < BF16_TOL and seen and dec._stack is None
