@@ -216,10 +216,18 @@ FL_HD void io_store4_stream(float* p, const Vec<4>& x) { vec_store_stream<4>(p, 
 
 FL_HD Vec<4> bf16x4_unpack(uint32_t lo, uint32_t hi) {
     Vec<4> r;
+#if FL_DEVICE_CODE
+    // one operation each: a shift, or a mask for the half that is already in place
+    r.v[0] = __uint_as_float(lo << 16);
+    r.v[1] = __uint_as_float(lo & 0xffff0000u);
+    r.v[2] = __uint_as_float(hi << 16);
+    r.v[3] = __uint_as_float(hi & 0xffff0000u);
+#else
     r.v[0] = bf16_bits_to_float((uint16_t)(lo & 0xffffu));
     r.v[1] = bf16_bits_to_float((uint16_t)(lo >> 16));
     r.v[2] = bf16_bits_to_float((uint16_t)(hi & 0xffffu));
     r.v[3] = bf16_bits_to_float((uint16_t)(hi >> 16));
+#endif
     return r;
 }
 
@@ -309,6 +317,30 @@ FL_HD F2 add2(const F2& a, const F2& b) {
 FL_HD F2 exp2_2(const F2& a) { return F2{fast_exp2(a.x), fast_exp2(a.y)}; }
 FL_HD F2 rcp2(const F2& a) { return F2{fast_rcp(a.x), fast_rcp(a.y)}; }
 
+// The bits of four bfloat16 as they lie in memory; pair(h) widens channels 2h and 2h + 1.
+struct Bits4 {
+    uint32_t lo, hi;
+    FL_HD F2 pair(int h) const {
+        const uint32_t w = h == 0 ? lo : hi;
+#if FL_DEVICE_CODE
+        return F2{__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)};
+#else
+        return F2{bf16_bits_to_float((uint16_t)(w & 0xffffu)), bf16_bits_to_float((uint16_t)(w >> 16))};
+#endif
+    }
+};
+FL_HD Bits4 load_bits4(const uint16_t* p) {
+    Bits4 r;
+#if FL_DEVICE_CODE
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    r.lo = t.x;
+    r.hi = t.y;
+#else
+    std::memcpy(&r, p, 8);
+#endif
+    return r;
+}
+
 // Gates of two channels. `rr`, `ri` are the reciprocals inside the tanh form
 // (tanh = 1 - 2 r), kept because 1 - tanh^2 = (1 - 2 r)(2 r - 1) + 1 needs them.
 struct Gate2 {
@@ -327,6 +359,31 @@ FL_HD Gate2 make_gate2(const F2& zr, const F2& zi, const F2& zv) {
     g.inj_r = fma2(g.rr, m2, one);
     g.inj_i = fma2(g.ri, m2, one);
     g.sig = sigmoid2(zv);
+    g.vac = mul2(g.sig, splat2(kVacMax));
+    g.keep = fma2(g.sig, splat2(-kVacMax), one);
+    return g;
+}
+
+// The same gates with one reciprocal for the three (1/a = bc / abc and so on): four special-function
+// operations per channel instead of six, for kernels that the special-function pipe bounds. The
+// exponents are capped so that the product of the denominators stays finite: beyond 2^30 both forms
+// give tanh = 1 in fp32; the sigmoid's smallest value becomes 2^-64.
+FL_HD F2 min2(const F2& a, float m) { return F2{a.x < m ? a.x : m, a.y < m ? a.y : m}; }
+
+FL_HD Gate2 make_gate2_shared(const F2& zr, const F2& zi, const F2& zv) {
+    Gate2 g;
+    const F2 one = splat2(1.0f), k2 = splat2(2.0f * kLog2e), m2 = splat2(-2.0f);
+    const F2 a = add2(exp2_2(min2(mul2(zr, k2), 30.0f)), one);
+    const F2 b = add2(exp2_2(min2(mul2(zi, k2), 30.0f)), one);
+    const F2 c = add2(exp2_2(min2(mul2(zv, splat2(-kLog2e)), 64.0f)), one);
+    const F2 ab = mul2(a, b);
+    const F2 r = rcp2(mul2(ab, c));
+    const F2 rc = mul2(r, c);
+    g.rr = mul2(rc, b);
+    g.ri = mul2(rc, a);
+    g.sig = mul2(r, ab);
+    g.inj_r = fma2(g.rr, m2, one);
+    g.inj_i = fma2(g.ri, m2, one);
     g.vac = mul2(g.sig, splat2(kVacMax));
     g.keep = fma2(g.sig, splat2(-kVacMax), one);
     return g;
@@ -368,6 +425,24 @@ FL_HD void cmul(float ar, float ai, float br, float bi, float& or_, float& oi) {
 FL_HD void cmul_conj(float ar, float ai, float br, float bi, float& or_, float& oi) {
     or_ = ar * br + ai * bi;
     oi = ar * bi - ai * br;
+}
+
+// (r + i j)^N, N >= 1.
+template <int N>
+FL_HD void cpow(float re, float im, float& or_, float& oi) {
+    if constexpr (N == 1) {
+        or_ = re;
+        oi = im;
+    } else {
+        float hr, hi;
+        cpow<N / 2>(re, im, hr, hi);
+        cmul(hr, hi, hr, hi, or_, oi);
+        if constexpr (N % 2) {
+            hr = or_;
+            hi = oi;
+            cmul(hr, hi, re, im, or_, oi);
+        }
+    }
 }
 
 // Affine map s -> A s + B on one complex channel.

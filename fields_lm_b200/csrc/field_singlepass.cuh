@@ -41,6 +41,7 @@ struct SpShape {
     int prefetch;  // non-zero: blocks warm L2 with the inputs of the tile that many positions ahead
     unsigned max_polls;  // bound of every wait for another block's publication
     int ticket;    // non-zero: blocks take their tile from a counter in the workspace header
+    int zp, gp;    // elements from one row of raw to the next, and of grad_raw (3C where they are dense)
 };
 
 // Prefetches `planes` consecutive 128-channel plane chunks of `steps` rows into L2:
@@ -98,22 +99,14 @@ FL_HD SpTile sp_decode(const SpShape& s, unsigned ticket) {
 
 // IO = float, or uint16_t for bfloat16 raw / read (the state, the maps and all arithmetic stay fp32).
 //
-// STAGED: the kernel runs as persistent blocks that take their tiles from a ticket counter in the
-// workspace header, one tile ahead: while a block works on a tile it already holds the ticket
-// of its next one. Every thread keeps one staging cell per (step, plane) of its rows in shared
-// memory; once the block has moved the current tile's rows from the cells into registers
-// (phase 0) every thread starts the cp.async copies of its rows of the NEXT tile into the same
-// cells. They land while the block publishes its map, looks back and runs the recurrence, so the
-// next tile starts from shared memory instead of waiting for HBM. Tickets are taken in time-major
-// tile order by blocks that are running, so every tile a block waits for is held by a running
-// block (as its current or its next tile): progress does not depend on how many blocks the GPU
-// holds at once or on the order it starts them in. The atomic of a ticket is issued at the top
-// of a tile and its result is used after phase 0, so its latency is off the critical path.
-// (Holding two tickets ahead, so that a thread could start the next tile's copies right after
-// its own cell loads, was measured and was much slower: 80 us against 43 us. A ticket taken
-// early is a tile that its chain's successors wait for while its block is still busy.)
-template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false,
-          bool STAGED = false>
+// What bounds it: a tile lives about 10 us (its loads, the look-back, its stores), so bandwidth is the
+// tile state that an SM holds divided by that. fp32 keeps a step's gate values in registers between the
+// two halves, 12 bytes per channel and step (the raw values are as large). bfloat16 keeps
+// the raw bits, half as much, and evaluates the gates a second time, with one reciprocal for the three
+// (the special-function pipe would bound it otherwise): 43.0 -> 36.2 us at 8 x 2,048 x 512, 189 ->
+// 142 us at 1 x 65,536. Blocks of four warps overlap their phases better than blocks of eight; holding
+// tickets and staging the next tile in shared memory (an earlier form) came to 43.0 us.
+template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false>
 struct FwdSinglePass {
     using Params = SpFwdParamsT<IO>;
     static constexpr int kThreads = 32 * WARPS;
@@ -121,51 +114,44 @@ struct FwdSinglePass {
     static constexpr int kTile = TS * WARPS;
     static constexpr int kPhases = STATS ? 5 : 4;
     static constexpr int kStatRow = 33;  // lane partials of one (warp, step), padded against bank conflicts
-    static_assert(!STATS || kTile * kStatRow <= WARPS * 4 * kGroup, "lane partials reuse the map area");
     static constexpr int kSplitPhase = 2;  // host emulation: phases < 2 of all blocks run first
-    static constexpr int kSumFloats = WARPS * 4 * kGroup;
+    // per warp: product of keep, Re B, Im B; later the lane partials of the statistics
+    static constexpr int kMapFloats = WARPS * 3 * kGroup;
+    static constexpr int kSumFloats = STATS && kTile * kStatRow > kMapFloats ? (kTile * kStatRow + 3) / 4 * 4 : kMapFloats;
+    static constexpr bool kPacked = sizeof(IO) == 2;  // hold the raw bits, evaluate the gates twice
     static constexpr int kCarryFloats = WARPS * 2 * kGroup;
-    static constexpr bool kStaged = STAGED;
-    static constexpr int kCellFloats = (int)sizeof(IO);  // four elements: 16 bytes of float, 8 of bfloat16
-    static constexpr int kStageFloats = STAGED ? TS * 3 * kThreads * kCellFloats : 0;
-    static constexpr int kSmemFloats = kSumFloats + kCarryFloats + kStageFloats + (STAGED ? 4 : 0);
-    // the word through which thread 0 hands the block's next ticket to the other threads
-    FL_HD static unsigned* ticket_at(float* smem) {
-        return reinterpret_cast<unsigned*>(smem + kSumFloats + kCarryFloats + kStageFloats);
-    }
+    static constexpr int kSmemFloats = kSumFloats + kCarryFloats;
     static constexpr int kClaimAfter = 2;  // the next tile is claimed after the look-back phase
     FL_HD static constexpr bool barrier_after(int ph) { return ph != 1; }
-    FL_HD static float* cell_at(float* smem, int idx, int thread) {
-        return smem + kSumFloats + kCarryFloats + ((size_t)idx * kThreads + thread) * kCellFloats;
-    }
-
-    // Starts the copies of this thread's rows of `tile` into its staging cells (one commit group).
-    FL_HD static void stage(const Params& p, int tile, int thread, float* smem) {
-        const SpShape& s = p.s;
-        const SpTile tl = sp_decode(s, (unsigned)tile);
-        const int lane = thread & 31, warp = thread >> 5;
-        const int c0 = tl.cg * kGroup + lane * 4;
-        if (c0 < s.C) {
-            const int tw = tl.n * kTile + warp * TS;
-            const IO* base = p.raw + ((size_t)tl.b * s.L) * 3 * s.C + c0;
-#pragma unroll
-            for (int u = 0; u < TS; ++u) {
-                if (tw + u < s.L) {
-                    const IO* row = base + (size_t)(tw + u) * 3 * s.C;
-                    async_copy4(cell_at(smem, u * 3 + 0, thread), row);
-                    async_copy4(cell_at(smem, u * 3 + 1, thread), row + s.C);
-                    async_copy4(cell_at(smem, u * 3 + 2, thread), row + 2 * s.C);
-                }
-            }
-        }
-        async_commit();
-    }
 
     struct State {
-        Vec<4> br[TS], bi[TS], vac[TS];  // raw on load, then gamma*v*inj and vacancy
+        // float: raw on load, then gamma*v*inj and vacancy; bfloat16: the raw bits of four channels
+        F2 br[kPacked ? 1 : TS][2], bi[kPacked ? 1 : TS][2], vac[kPacked ? 1 : TS][2];
+        Bits4 raw[kPacked ? TS : 1][3];
     };
 
-    FL_HD static float* sum_at(float* smem, int w, int k) { return smem + (w * 4 + k) * kGroup; }
+    FL_HD static void take(State& st, int u, int plane, const IO* src) {
+        if constexpr (kPacked) {
+            st.raw[u][plane] = load_bits4(src);
+        } else {
+            const Vec<4> z = vec_load_stream<4>(src);
+            F2(&d)[2] = plane == 0 ? st.br[u] : plane == 1 ? st.bi[u] : st.vac[u];
+            d[0] = lo2(z); d[1] = hi2(z);
+        }
+    }
+    FL_HD static Gate2 gate(const State& st, int u, int h) {
+        if constexpr (kPacked)
+            return make_gate2_shared(st.raw[u][0].pair(h), st.raw[u][1].pair(h), st.raw[u][2].pair(h));
+        else return make_gate2(st.br[u][h], st.bi[u][h], st.vac[u][h]);
+    }
+
+    // Steps of warp w of the tile that lie inside the sequence.
+    FL_HD static int steps_of(const SpShape& s, const SpTile& tl, int w) {
+        const int n = s.L - (tl.n * kTile + w * TS);
+        return n < 0 ? 0 : n < TS ? n : TS;
+    }
+
+    FL_HD static float* sum_at(float* smem, int w, int k) { return smem + (w * 3 + k) * kGroup; }
     FL_HD static float* carry_at(float* smem, int w, int k) {
         return smem + kSumFloats + (w * 2 + k) * kGroup;
     }
@@ -175,8 +161,8 @@ struct FwdSinglePass {
         const SpShape& s = p.s;
         const SpTile nx = sp_decode(s, (unsigned)tile);
         const int t0 = nx.n * kTile;
-        prefetch_rows(p.raw + ((size_t)nx.b * s.L + t0) * 3 * s.C + nx.cg * kGroup, kTile, s.L - t0, 3,
-                      (size_t)3 * s.C, (size_t)s.C, s.C - nx.cg * kGroup, thread, kThreads);
+        prefetch_rows(p.raw + ((size_t)nx.b * s.L + t0) * s.zp + nx.cg * kGroup, kTile, s.L - t0, 3,
+                      (size_t)s.zp, (size_t)s.C, s.C - nx.cg * kGroup, thread, kThreads);
     }
 
     template <int PH>
@@ -190,82 +176,75 @@ struct FwdSinglePass {
         const int tw = tl.n * kTile + warp * TS;
 
         if constexpr (PH == 0) {
-            Affine m[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) m[k] = affine_identity();
-            if constexpr (STAGED) {
-                // The rows were started into this thread's cells by the kernel entry while the
-                // block's previous tile ran (by this very call in the host emulation, where a
-                // copy is synchronous).
-#if !FL_DEVICE_CODE
-                stage(p, block, thread, smem);
-#endif
-                async_wait_pending<0>();
-                if (chan_ok) {
-#pragma unroll
-                    for (int u = 0; u < TS; ++u) {
-                        if (tw + u < s.L) {
-                            st.br[u] = cell_load4<IO>(cell_at(smem, u * 3 + 0, thread));
-                            st.bi[u] = cell_load4<IO>(cell_at(smem, u * 3 + 1, thread));
-                            st.vac[u] = cell_load4<IO>(cell_at(smem, u * 3 + 2, thread));
-                        }
-                    }
-                }
-                // (on the device the kernel entry starts the next tile's rows towards the cells
-                // after the barrier that follows this phase)
-            }
+            // The warp's map is s -> lambda^n P s + B with P the product of the n steps' keep factors:
+            // lambda is constant along the sequence, so only P and B are accumulated here and the
+            // power of lambda is applied where the warp maps are composed.
+            F2 prod[2] = {splat2(1.0f), splat2(1.0f)};
+            F2 Br[2] = {splat2(0.0f), splat2(0.0f)}, Bi[2] = {splat2(0.0f), splat2(0.0f)};
             if (chan_ok) {
-                const Vec<4> lr = vec_load<4>(p.tr + c0);
-                const Vec<4> li = vec_load<4>(p.ti + c0);
-                const Vec<4> gm = vec_load<4>(p.gamma + c0);
-                if constexpr (!STAGED) {
-                    const IO* base = p.raw + ((size_t)tl.b * s.L) * 3 * C + c0;
-#pragma unroll
-                    for (int u = 0; u < TS; ++u) {
-                        if (tw + u < s.L) {
-                            const IO* row = base + (size_t)(tw + u) * 3 * C;
-                            st.br[u] = io_load4_stream(row);
-                            st.bi[u] = io_load4_stream(row + C);
-                            st.vac[u] = io_load4_stream(row + 2 * C);
-                        }
-                    }
-                }
+                // (only bfloat16 rows may be columns of a wider matrix)
+                const size_t pitch = kPacked ? (size_t)s.zp : (size_t)3 * C;
+                const IO* row = p.raw + ((size_t)tl.b * s.L + tw) * pitch + c0;
 #pragma unroll
                 for (int u = 0; u < TS; ++u) {
                     if (tw + u < s.L) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const Gate g = make_gate(st.br[u].v[k], st.bi[u].v[k], st.vac[u].v[k]);
-                            const float keep = 1.0f - g.vac;
-                            const float bs = gm.v[k] * g.vac;
-                            st.br[u].v[k] = bs * g.inj_r;
-                            st.bi[u].v[k] = bs * g.inj_i;
-                            st.vac[u].v[k] = g.vac;
-                            m[k] = affine_then(m[k], keep * lr.v[k], keep * li.v[k],
-                                               st.br[u].v[k], st.bi[u].v[k]);
+                        for (int q = 0; q < 3; ++q) take(st, u, q, row + (size_t)q * C);
+                    }
+                    row += pitch;
+                }
+                const Vec<4> lr4 = vec_load<4>(p.tr + c0);
+                const Vec<4> li4 = vec_load<4>(p.ti + c0);
+                const Vec<4> gm4 = vec_load<4>(p.gamma + c0);
+                const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)}, gm[2] = {lo2(gm4), hi2(gm4)};
+                const F2 nli[2] = {mul2(li[0], splat2(-1.0f)), mul2(li[1], splat2(-1.0f))};
+#pragma unroll
+                for (int u = 0; u < TS; ++u) {
+                    if (tw + u < s.L) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const Gate2 g = gate(st, u, h);
+                            const F2 bs = mul2(gm[h], g.vac);
+                            const F2 br = mul2(bs, g.inj_r), bi = mul2(bs, g.inj_i);
+                            if constexpr (!kPacked) {
+                                st.br[u][h] = br;
+                                st.bi[u][h] = bi;
+                                st.vac[u][h] = g.vac;
+                            }
+                            prod[h] = mul2(prod[h], g.keep);
+                            const F2 mr = fma2(lr[h], Br[h], mul2(nli[h], Bi[h]));
+                            const F2 mi = fma2(lr[h], Bi[h], mul2(li[h], Br[h]));
+                            Br[h] = fma2(g.keep, mr, br);
+                            Bi[h] = fma2(g.keep, mi, bi);
                         }
                     }
                 }
             }
-            Vec<4> o0, o1, o2, o3;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                o0.v[k] = m[k].ar; o1.v[k] = m[k].ai; o2.v[k] = m[k].br; o3.v[k] = m[k].bi;
-            }
-            vec_store<4>(sum_at(smem, warp, 0) + lane * 4, o0);
-            vec_store<4>(sum_at(smem, warp, 1) + lane * 4, o1);
-            vec_store<4>(sum_at(smem, warp, 2) + lane * 4, o2);
-            vec_store<4>(sum_at(smem, warp, 3) + lane * 4, o3);
+            vec_store<4>(sum_at(smem, warp, 0) + lane * 4, join2(prod[0], prod[1]));
+            vec_store<4>(sum_at(smem, warp, 1) + lane * 4, join2(Br[0], Br[1]));
+            vec_store<4>(sum_at(smem, warp, 2) + lane * 4, join2(Bi[0], Bi[1]));
         } else if constexpr (PH == 1) {
             // tile aggregate, one thread per channel; the first tile of a chain publishes
             // only its end state
-            if (thread < kGroup && tl.cg * kGroup + thread < C && tl.n > 0) {
-                Affine a = affine_identity();
+            // (a tile that others follow is whole: every warp has TS steps)
+            const int ch = tl.cg * kGroup + thread;
+            if (thread < kGroup && ch < C && tl.n > 0) {
+                float pr, pi;
+                cpow<TS>(p.tr[ch], p.ti[ch], pr, pi);
+                float ar = 1.0f, ai = 0.0f, br = 0.0f, bi = 0.0f;
 #pragma unroll
-                for (int w = 0; w < WARPS; ++w)
-                    a = affine_then(a, sum_at(smem, w, 0)[thread], sum_at(smem, w, 1)[thread],
-                                    sum_at(smem, w, 2)[thread], sum_at(smem, w, 3)[thread]);
-                publish4(p.agg + ((size_t)tl.idx * kGroup + thread) * 4, a.ar, a.ai, a.br, a.bi);
+                for (int w = 0; w < WARPS; ++w) {
+                    const float k = sum_at(smem, w, 0)[thread];
+                    const float xr = k * pr, xi = k * pi;
+                    float tr_, ti_;
+                    cmul(xr, xi, br, bi, tr_, ti_);
+                    br = tr_ + sum_at(smem, w, 1)[thread];
+                    bi = ti_ + sum_at(smem, w, 2)[thread];
+                    cmul(xr, xi, ar, ai, tr_, ti_);
+                    ar = tr_;
+                    ai = ti_;
+                }
+                publish4(p.agg + ((size_t)tl.idx * kGroup + thread) * 4, ar, ai, br, bi);
             }
         } else if constexpr (PH == 2) {
             const int ch = tl.cg * kGroup + thread;
@@ -277,12 +256,25 @@ struct FwdSinglePass {
                 } else {
                     look_back(p.agg, p.incl, tl.chain * s.NT, tl.n, thread, p.ctrl, s.max_polls, sr, si);
                 }
+                float pr, pi;
+                const float lr = p.tr[ch], li = p.ti[ch];
+                cpow<TS>(lr, li, pr, pi);
 #pragma unroll
                 for (int w = 0; w < WARPS; ++w) {
                     carry_at(smem, w, 0)[thread] = sr;
                     carry_at(smem, w, 1)[thread] = si;
-                    affine_apply(Affine{sum_at(smem, w, 0)[thread], sum_at(smem, w, 1)[thread],
-                                        sum_at(smem, w, 2)[thread], sum_at(smem, w, 3)[thread]},
+                    const int n = steps_of(s, tl, w);
+                    if (n < TS) {  // only in a sequence's last tile
+                        pr = 1.0f; pi = 0.0f;
+                        for (int j = 0; j < n; ++j) {
+                            float tr_, ti_;
+                            cmul(pr, pi, lr, li, tr_, ti_);
+                            pr = tr_; pi = ti_;
+                        }
+                    }
+                    const float k = sum_at(smem, w, 0)[thread];
+                    affine_apply(Affine{k * pr, k * pi, sum_at(smem, w, 1)[thread],
+                                        sum_at(smem, w, 2)[thread]},
                                  sr, si);
                 }
                 publish2(p.incl + ((size_t)tl.idx * kGroup + thread) * 2, sr, si);
@@ -299,36 +291,48 @@ struct FwdSinglePass {
                 }
                 return;
             }
-            const Vec<4> lr = vec_load<4>(p.tr + c0);
-            const Vec<4> li = vec_load<4>(p.ti + c0);
-            Vec<4> sr = vec_load<4>(carry_at(smem, warp, 0) + lane * 4);
-            Vec<4> si = vec_load<4>(carry_at(smem, warp, 1) + lane * 4);
-            IO* obase = p.read + ((size_t)tl.b * s.L) * 4 * C + c0;
+            const Vec<4> lr4 = vec_load<4>(p.tr + c0);
+            const Vec<4> li4 = vec_load<4>(p.ti + c0);
+            const Vec<4> gm4 = kPacked ? vec_load<4>(p.gamma + c0) : lr4;
+            const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)}, gm[2] = {lo2(gm4), hi2(gm4)};
+            const F2 nli[2] = {mul2(li[0], splat2(-1.0f)), mul2(li[1], splat2(-1.0f))};
+            const Vec<4> sr4 = vec_load<4>(carry_at(smem, warp, 0) + lane * 4);
+            const Vec<4> si4 = vec_load<4>(carry_at(smem, warp, 1) + lane * 4);
+            F2 sr[2] = {lo2(sr4), hi2(sr4)}, si[2] = {lo2(si4), hi2(si4)};
+            IO* orow = p.read + ((size_t)tl.b * s.L + tw) * 4 * C + c0;
 #pragma unroll
             for (int u = 0; u < TS; ++u) {
                 if (tw + u < s.L) {
-                    Vec<4> dr, di;
-                    float sq = 0.0f;
+                    F2 dr[2], di[2], sq = splat2(0.0f);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        float mr, mi;
-                        cmul(lr.v[k], li.v[k], sr.v[k], si.v[k], mr, mi);
-                        const float v = st.vac[u].v[k];
-                        dr.v[k] = v * mr;
-                        di.v[k] = v * mi;
-                        sr.v[k] = (1.0f - v) * mr + st.br[u].v[k];
-                        si.v[k] = (1.0f - v) * mi + st.bi[u].v[k];
+                    for (int h = 0; h < 2; ++h) {
+                        const F2 mr = fma2(lr[h], sr[h], mul2(nli[h], si[h]));
+                        const F2 mi = fma2(lr[h], si[h], mul2(li[h], sr[h]));
+                        F2 v, keep, br, bi;
+                        if constexpr (kPacked) {
+                            const Gate2 g = gate(st, u, h);
+                            const F2 bs = mul2(gm[h], g.vac);
+                            v = g.vac; keep = g.keep;
+                            br = mul2(bs, g.inj_r); bi = mul2(bs, g.inj_i);
+                        } else {
+                            v = st.vac[u][h];
+                            keep = fma2(v, splat2(-1.0f), splat2(1.0f));
+                            br = st.br[u][h]; bi = st.bi[u][h];
+                        }
+                        dr[h] = mul2(v, mr);
+                        di[h] = mul2(v, mi);
+                        sr[h] = fma2(keep, mr, br);
+                        si[h] = fma2(keep, mi, bi);
                         if constexpr (STATS)
-                            sq += sr.v[k] * sr.v[k] + si.v[k] * si.v[k] + dr.v[k] * dr.v[k] +
-                                  di.v[k] * di.v[k];
+                            sq = fma2(sr[h], sr[h], fma2(si[h], si[h], fma2(dr[h], dr[h], fma2(di[h], di[h], sq))));
                     }
-                    IO* orow = obase + (size_t)(tw + u) * 4 * C;
-                    io_store4_stream(orow, sr);
-                    io_store4_stream(orow + C, si);
-                    io_store4_stream(orow + 2 * C, dr);
-                    io_store4_stream(orow + 3 * C, di);
+                    io_store4_stream(orow, join2(sr[0], sr[1]));
+                    io_store4_stream(orow + C, join2(si[0], si[1]));
+                    io_store4_stream(orow + 2 * C, join2(dr[0], dr[1]));
+                    io_store4_stream(orow + 3 * C, join2(di[0], di[1]));
                     // the map area is free after the look-back: one partial per lane and step
-                    if constexpr (STATS) smem[(warp * TS + u) * kStatRow + lane] = sq;
+                    if constexpr (STATS) smem[(warp * TS + u) * kStatRow + lane] = sq.x + sq.y;
+                    orow += (size_t)4 * C;
                 }
             }
         } else {  // PH == 4 (STATS): one sum per step of the tile, lanes added in order
@@ -357,7 +361,6 @@ struct FwdSinglePass {
 template <int TS, int WARPS, int U_, int MIN_BLOCKS, int STAGES, typename IO = float>
 struct FwdTwoSweep {
     using Params = SpFwdParamsT<IO>;
-    static constexpr bool kStaged = false;
     static constexpr int kThreads = 32 * WARPS;
     static constexpr int kMinBlocks = MIN_BLOCKS;
     static constexpr int kTile = TS * WARPS;
@@ -748,12 +751,12 @@ struct BwdSinglePass {
                 const Vec<4> li = vec_load<4>(p.ti + c0);
                 const F2 lr2[2] = {lo2(lr), hi2(lr)}, li2[2] = {lo2(li), hi2(li)};
                 const F2 nli2[2] = {mul2(li2[0], splat2(-1.0f)), mul2(li2[1], splat2(-1.0f))};
-                const IO* zbase = p.raw + ((size_t)tl.b * s.L) * 3 * C + 2 * C + c0;
+                const IO* zbase = p.raw + ((size_t)tl.b * s.L) * s.zp + 2 * C + c0;
                 const IO* gbase = p.grad_read + ((size_t)tl.b * s.L) * 4 * C + c0;
                 // Running row pointers of the next batch to issue (rows descend; the pointers may
                 // step below the tile after the last batch and are not dereferenced then).
                 int t_issue = tend;
-                const IO* zq = zbase + (ptrdiff_t)(tend - 1) * 3 * C;
+                const IO* zq = zbase + (ptrdiff_t)(tend - 1) * s.zp;
                 const IO* gq = gbase + (ptrdiff_t)(tend - 1) * 4 * C;
                 // batch of U1 steps ending just before t_issue, into ring slot `stage`
                 auto issue1 = [&](int, int stage) {
@@ -761,7 +764,7 @@ struct BwdSinglePass {
                     for (int u = 0; u < U1; ++u) {
                         if (t_issue - 1 - u >= tbeg) {
                             const IO* grow = gq - (ptrdiff_t)u * 4 * C;
-                            async_copy4(cell_at(smem, stage, u * 5 + 0, thread), zq - (ptrdiff_t)u * 3 * C);
+                            async_copy4(cell_at(smem, stage, u * 5 + 0, thread), zq - (ptrdiff_t)u * s.zp);
                             async_copy4(cell_at(smem, stage, u * 5 + 1, thread), grow);
                             async_copy4(cell_at(smem, stage, u * 5 + 2, thread), grow + C);
                             async_copy4(cell_at(smem, stage, u * 5 + 3, thread), grow + 2 * C);
@@ -769,7 +772,7 @@ struct BwdSinglePass {
                         }
                     }
                     t_issue -= U1;
-                    zq -= (ptrdiff_t)U1 * 3 * C;
+                    zq -= (ptrdiff_t)U1 * s.zp;
                     gq -= (ptrdiff_t)U1 * 4 * C;
                     async_commit();
                 };
@@ -798,7 +801,7 @@ struct BwdSinglePass {
                     for (int u = 0; u < U1; ++u) {
                         const int t = t0 - 1 - u;
                         if (t >= tbeg) {
-                            zv[u] = io_load4(zbase + (size_t)t * 3 * C);
+                            zv[u] = io_load4(zbase + (size_t)t * s.zp);
                             const IO* grow = gbase + (size_t)t * 4 * C;
                             ur[u] = io_load4(grow);
                             ui[u] = io_load4(grow + C);
@@ -868,12 +871,12 @@ struct BwdSinglePass {
                 const Vec<4> cr4 = vec_load<4>(carry_at(smem, slot, 0) + lane * 4);
                 const Vec<4> ci4 = vec_load<4>(carry_at(smem, slot, 1) + lane * 4);
                 F2 cr[2] = {lo2(cr4), hi2(cr4)}, ci[2] = {lo2(ci4), hi2(ci4)};
-                const IO* zbase = p.raw + ((size_t)tl.b * s.L) * 3 * C + c0;
+                const IO* zbase = p.raw + ((size_t)tl.b * s.L) * s.zp + c0;
                 const IO* gbase = p.grad_read + ((size_t)tl.b * s.L) * 4 * C + c0;
                 const IO* rbase = p.read + ((size_t)tl.b * s.L) * 4 * C + c0;
-                IO* obase = p.grad_raw + ((size_t)tl.b * s.L) * 3 * C + c0;
+                IO* obase = p.grad_raw + ((size_t)tl.b * s.L) * s.gp + c0;
                 int t_issue = tend;
-                const IO* zq = zbase + (ptrdiff_t)(tend - 1) * 3 * C;
+                const IO* zq = zbase + (ptrdiff_t)(tend - 1) * s.zp;
                 const IO* gq = gbase + (ptrdiff_t)(tend - 1) * 4 * C;
                 const IO* rq = rbase + (ptrdiff_t)(tend - 2) * 4 * C;  // row of s_{t-1}
                 auto issue2 = [&](int, int stage) {
@@ -881,7 +884,7 @@ struct BwdSinglePass {
                     for (int u = 0; u < U2; ++u) {
                         const int t = t_issue - 1 - u;
                         if (t >= tbeg) {
-                            const IO* zrow = zq - (ptrdiff_t)u * 3 * C;
+                            const IO* zrow = zq - (ptrdiff_t)u * s.zp;
                             const IO* grow = gq - (ptrdiff_t)u * 4 * C;
                             async_copy4(cell_at(smem, stage, u * 9 + 0, thread), zrow);
                             async_copy4(cell_at(smem, stage, u * 9 + 1, thread), zrow + C);
@@ -898,7 +901,7 @@ struct BwdSinglePass {
                         }
                     }
                     t_issue -= U2;
-                    zq -= (ptrdiff_t)U2 * 3 * C;
+                    zq -= (ptrdiff_t)U2 * s.zp;
                     gq -= (ptrdiff_t)U2 * 4 * C;
                     rq -= (ptrdiff_t)U2 * 4 * C;
                     async_commit();
@@ -942,7 +945,7 @@ struct BwdSinglePass {
                     for (int u = 0; u < U2; ++u) {
                         const int t = t0 - 1 - u;
                         if (t >= tbeg) {
-                            const IO* zrow = zbase + (size_t)t * 3 * C;
+                            const IO* zrow = zbase + (size_t)t * s.zp;
                             zr[u] = io_load4_stream(zrow);
                             zi[u] = io_load4_stream(zrow + C);
                             zv[u] = io_load4_stream(zrow + 2 * C);
@@ -977,7 +980,7 @@ struct BwdSinglePass {
                             bwd_step2(hi2(zr[u]), hi2(zi[u]), hi2(zv[u]), hi2(ur[u]), hi2(ui[u]),
                                       hi2(gr[u]), hi2(gi[u]), hi2(pr[u]), hi2(pi[u]), lr2[1], li2[1],
                                       nli2[1], gm2[1], cr[1], ci[1], acc[1], ozr[1], ozi[1], ozv[1]);
-                            IO* orow = obase + (size_t)t * 3 * C;
+                            IO* orow = obase + (size_t)t * s.gp;
                             io_store4_stream(orow, join2(ozr[0], ozr[1]));
                             io_store4_stream(orow + C, join2(ozi[0], ozi[1]));
                             io_store4_stream(orow + 2 * C, join2(ozv[0], ozv[1]));

@@ -98,14 +98,6 @@ static int fill_unset(void* p, size_t bytes, Stream) {
     return FIELDS_OK;
 }
 
-// A staged kernel in the emulation: one tile per block, every tile stages its own rows.
-template <class K>
-static int launch_persistent(const typename K::Params& p, long long grid, long long first_wave,
-                             Stream st) {
-    return launch_stateful<K>(p, grid, first_wave, st);
-}
-
-
 template <class K>
 static int resident_blocks() { return 4; }  // any positive distance exercises the prefetch path
 
@@ -301,36 +293,6 @@ __global__ void __launch_bounds__(K::kThreads, K::kMinBlocks) stateful_entry(con
     run_phases<K, K::kClaimAfter + 1, K::kPhases - 1>(p, tile, smem, st);
 }
 
-// Persistent form for kernels with staging cells (K::kStaged). Blocks take tiles from a ticket
-// counter (word 1 of the workspace header, which the fill leaves at 0xFFFFFFFF, so the first
-// ticket is 0), always one tile ahead: thread 0 issues the atomic for the next ticket at the top
-// of a tile and hands its result round after phase 0, when every thread starts the copies of
-// the next tile's rows into its staging cells.
-template <class K>
-__global__ void __launch_bounds__(K::kThreads, K::kMinBlocks) persistent_entry(const typename K::Params p) {
-    extern __shared__ __align__(16) float smem[];
-    typename K::State st;
-    const unsigned tiles = (unsigned)((long long)p.s.B * p.s.G * p.s.NT);
-    unsigned* hand = K::ticket_at(smem);
-    wait_for_previous_kernel();
-    if (threadIdx.x == 0) *hand = atomicAdd(p.ctrl + 1, 1u) + 1u;
-    __syncthreads();
-    unsigned tile = *hand;
-    if (tile < tiles) K::stage(p, (int)tile, (int)threadIdx.x, smem);
-    while (tile < tiles) {
-        unsigned next_ticket = 0;
-        if (threadIdx.x == 0) next_ticket = atomicAdd(p.ctrl + 1, 1u) + 1u;  // used after phase 0
-        K::template phase<0>(p, (int)tile, (int)threadIdx.x, smem, st);
-        if (threadIdx.x == 0) *hand = next_ticket;
-        __syncthreads();
-        const unsigned next = *hand;
-        if (next < tiles) K::stage(p, (int)next, (int)threadIdx.x, smem);
-        run_phases<K, 1, K::kPhases - 1>(p, (int)tile, smem, st);
-        __syncthreads();  // the map, carry and hand-over areas are written again by the next tile
-        tile = next;
-    }
-}
-
 // Kernels that need more than the default 48 KB of dynamic shared memory opt in once per device.
 // `ready` is the caller's per-kernel, per-device record (kernels of equal signature share a
 // function-pointer type, so the record cannot live in this template).
@@ -406,41 +368,6 @@ static int resident_blocks() {
         return 0;
     cached[dev] = per_sm * sms;
     return cached[dev];
-}
-
-// Launch of a staged kernel as persistent blocks: as many as the GPU holds at once (asked once
-// per device, after the opt-in to its shared memory; fewer resident blocks only make it slower,
-// the tickets keep it correct), never more than there are tiles.
-template <class K>
-static int launch_persistent(typename K::Params p, long long tiles, long long, Stream st) {
-    if (tiles <= 0) return FIELDS_OK;
-    if (tiles > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
-    constexpr size_t bytes = K::kSmemFloats * sizeof(float);
-    static bool ready[64] = {};
-    int rc = allow_shared_memory(persistent_entry<K>, bytes, ready);
-    if (rc) return rc;
-    static std::mutex mu;
-    static int cached[64] = {};
-    int dev = 0, resident = 0;
-    rc = check_cuda(cudaGetDevice(&dev));
-    if (rc) return rc;
-    if (dev < 0 || dev >= 64) return FIELDS_ERR_UNSUPPORTED;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (cached[dev] == 0) {
-            int per_sm = 0, sms = 0;
-            rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            if (!rc)
-                rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &per_sm, persistent_entry<K>, K::kThreads, bytes));
-            if (rc) return rc;
-            if (per_sm * sms <= 0) return FIELDS_ERR_UNSUPPORTED;
-            cached[dev] = per_sm * sms;
-        }
-        resident = cached[dev];
-    }
-    const long long grid = tiles < resident ? tiles : resident;
-    return launch_on<typename K::Params>(persistent_entry<K>, (unsigned)grid, K::kThreads, bytes, st, p);
 }
 
 // Persistent block program over an executor: the calling thread, then a block barrier.
@@ -657,6 +584,7 @@ static SpPlan make_sp_plan(int B, int L, int C, int tile_steps) {
     pl.s.B = B; pl.s.L = L; pl.s.C = C;
     pl.s.NT = (L + tile_steps - 1) / tile_steps;
     pl.s.G = (C + kGroup - 1) / kGroup;
+    pl.s.zp = pl.s.gp = 3 * C;
     pl.s.max_polls = kMaxPolls;
     pl.s.ticket = tile_ticket_from_env();
     pl.tiles = (long long)B * pl.s.G * pl.s.NT;
@@ -694,13 +622,15 @@ static Algo algo_from_env() { return kAlgoAuto; }
 // Instantiations of the single-pass kernels. The first of each list is the default; the
 // others are tuning alternatives selected with FIELDS_FWD_VARIANT / FIELDS_BWD_VARIANT.
 //   forward  <steps per warp, warps, blocks per SM the registers must allow>
-using FwdSp0 = FwdSinglePass<6, 8, 2>;        // tile 48 steps, 128 registers, no spills
+// Three blocks of four warps per SM at 168 registers hold 108 steps of 128 channels (four blocks at 128
+// registers with 24-step tiles: 96). At 1 x 65,536 x 512 189 -> 183 us against the earlier two blocks of
+// eight warps and 48-step tiles, at 1 x 16,384 54.2 -> 51.8, at 2 x 3,001 x 384 20.6 -> 19.5, equal at
+// 8 x 2,048. Longer tiles spill.
+using FwdSp0 = FwdSinglePass<9, 4, 3>;
 #ifdef FIELDS_ALL_VARIANTS
 using FwdSp1 = FwdSinglePass<4, 8, 2>;        // tile 32
 //   two-sweep forward <steps per warp, warps, unroll, blocks per SM, ring slots>
 using FwdSp2 = FwdTwoSweep<8, 4, 2, 4, 3>;    // tile 32, 16 warps per SM
-//   staged: persistent blocks, the next tile's rows land in shared memory during the current tile
-using FwdSp3 = FwdSinglePass<5, 8, 2, float, false, true>;  // tile 40, 74 KB per block
 #endif
 //   backward <steps per warp, warps, sweep-1 unroll, sweep-2 unroll, blocks per SM, rings, ring slots>
 using BwdSp0 = BwdSinglePass<8, 4, 2, 1, 3, true, 3>;  // tile 32, 3-slot cp.async rings, 12 warps per SM
@@ -714,17 +644,20 @@ using BwdSp2 = BwdRecompute<8, 4, 1, 3, 2>;   // 73 KB per block, 12 warps per S
 using BwdSp3 = BwdTileResident<4, 4, 3>;      // tile 16, 68 KB per block, 12 warps per SM
 #endif
 //   bfloat16 raw / read / grad_read / grad_raw (bits as uint16_t); state and arithmetic stay fp32
-// The bfloat16 forward runs staged (persistent blocks, tickets one tile ahead, the next tile's
-// rows landing in shared memory during the current tile): 40.6 us against 46.1 us for the
-// one-tile-per-block form at 8 x 2,048 tokens. The fp32 forward does not (46.3 -> 51.6 us staged:
-// it is within 10 % of a plain copy already and pays for 74 KB of shared-memory traffic per tile).
-using FwdSpBf16 = FwdSinglePass<5, 8, 2, uint16_t, false, true>;
-using FwdSpBf16Stats = FwdSinglePass<5, 8, 2, uint16_t, true, true>;  // also writes per-token sums of squares
+// The forward in two tile shapes: blocks of four warps (tile 40) overlap their phases better, blocks of
+// eight (tile 80) look back over half as many tiles. 36.2 / 37.6 us at 8 x 2,048 x 512 (1,640 small
+// tiles), 43.2 / 41.4 at 1 x 16,384, 150 / 142 at 1 x 65,536, 129 / 128 at 8 x 8,192. The second
+// needs tiles enough that a part-filled last round costs little: the line is at 3,500 small tiles.
+static bool deep_tiles(int B, int L, int C) {
+    return (long long)B * ((C + kGroup - 1) / kGroup) * ((L + 39) / 40) >= 3500;
+}
+template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;
+template <bool STATS> using FwdSpBf16Deep = FwdSinglePass<10, 8, 2, uint16_t, STATS>;  // STATS: per-token sums of squares too
 // bfloat16 ring cells are half the size, so a 64-step tile (4 warps x 16 steps) still leaves room for
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
 // 16-byte cells) on 8 x 2,048 tokens.
 using BwdSpBf16 = BwdSinglePass<16, 4, 2, 1, 3, true, 3, uint16_t>;
-constexpr int kSpMinTile = 32;     // smallest time tile of any forward instantiation above (workspace bound)
+constexpr int kSpMinTile = 24;     // smallest time tile of any forward instantiation above (workspace bound)
 constexpr int kSpMinTileBwd = 16;  // same for the backward
 
 #ifdef FIELDS_ALL_VARIANTS
@@ -751,9 +684,10 @@ template <class K, typename IO = float>
 static int run_forward_single_pass(const IO* raw, const float* tr, const float* ti,
                                    const float* gamma, const float* state_in, IO* read,
                                    float* state_out, void* workspace, int B, int L, int C,
-                                   Stream st, float* sumsq = nullptr) {
+                                   Stream st, float* sumsq = nullptr, long long pitch = 0) {
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
-    if constexpr (!K::kStaged) pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
+    pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
+    if (pitch) pl.s.zp = (int)pitch;
     char* ws = static_cast<char*>(workspace);
     unsigned* ctrl = reinterpret_cast<unsigned*>(ws);
     int rc = fill_unset(ws, pl.bytes, st);  // error word and every publication slot
@@ -762,8 +696,7 @@ static int run_forward_single_pass(const IO* raw, const float* tr, const float* 
                        reinterpret_cast<float*>(ws + pl.agg_off),
                        reinterpret_cast<float*>(ws + pl.incl_off), ctrl, pl.s};
     p.sumsq = sumsq;
-    if constexpr (K::kStaged) return launch_persistent<K>(p, pl.tiles, (long long)B * pl.s.G, st);
-    else return launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st);
+    return launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st);
 }
 
 template <class K, typename IO = float>
@@ -773,9 +706,12 @@ static int run_backward_single_pass(const IO* raw, const float* tr, const float*
                                     IO* grad_raw, float* grad_tr, float* grad_ti,
                                     float* grad_gamma, float* grad_state_in, void* workspace,
                                     int B, int L, int C, Stream st,
-                                    const float* states = nullptr) {
+                                    const float* states = nullptr, long long raw_pitch = 0,
+                                    long long grad_pitch = 0) {
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
+    if (raw_pitch) pl.s.zp = (int)raw_pitch;
+    if (grad_pitch) pl.s.gp = (int)grad_pitch;
     char* ws = static_cast<char*>(workspace);
     unsigned* ctrl = reinterpret_cast<unsigned*>(ws);
     int rc = fill_unset(ws, pl.bytes, st);
@@ -997,12 +933,10 @@ int fields_read_forward(const float* raw, const float* tr, const float* ti, cons
         switch (variant_from_env("FIELDS_FWD_VARIANT")) {
             case 1: FIELDS_FWD_SP(FwdSp1);
             case 2: FIELDS_FWD_SP(FwdSp2);
-            case 3: FIELDS_FWD_SP(FwdSp3);
-            default: FIELDS_FWD_SP(FwdSp0);
+            default: break;
         }
-#else
-        FIELDS_FWD_SP(FwdSp0);
 #endif
+        FIELDS_FWD_SP(FwdSp0);
 #undef FIELDS_FWD_SP
     }
     float* ws = static_cast<float*>(workspace);
@@ -1407,6 +1341,24 @@ int fields_read_selftest_wait(void* workspace, size_t workspace_bytes, unsigned 
 
 static bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
+}  // extern "C"
+
+template <bool STATS>
+static int run_forward_bf16(const void* raw, long long pitch, const float* tr, const float* ti, const float* gamma,
+                            const float* state_in, void* read, float* sumsq, float* state_out, void* workspace,
+                            int B, int L, int C, void* stream) {
+    const auto* z = static_cast<const uint16_t*>(raw);
+    auto* out = static_cast<uint16_t*>(read);
+    Stream st = reinterpret_cast<Stream>(stream);
+    if (deep_tiles(B, L, C))
+        return run_forward_single_pass<FwdSpBf16Deep<STATS>, uint16_t>(z, tr, ti, gamma, state_in, out, state_out,
+                                                                       workspace, B, L, C, st, sumsq, pitch);
+    return run_forward_single_pass<FwdSpBf16<STATS>, uint16_t>(z, tr, ti, gamma, state_in, out, state_out,
+                                                               workspace, B, L, C, st, sumsq, pitch);
+}
+
+extern "C" {
+
 int fields_read_forward_bf16(const void* raw, const float* tr, const float* ti, const float* gamma,
                              const float* state_in, void* read, float* state_out, void* workspace,
                              size_t workspace_bytes, int B, int L, int C, void* stream) {
@@ -1423,9 +1375,8 @@ int fields_read_forward_bf16(const void* raw, const float* tr, const float* ti, 
     if (!workspace || workspace_bytes < fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD) ||
         (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return FIELDS_ERR_WORKSPACE;
-    return run_forward_single_pass<FwdSpBf16, uint16_t>(
-        static_cast<const uint16_t*>(raw), tr, ti, gamma, state_in, static_cast<uint16_t*>(read),
-        state_out, workspace, B, L, C, reinterpret_cast<Stream>(stream));
+    return run_forward_bf16<false>(raw, 3LL * C, tr, ti, gamma, state_in, read, nullptr, state_out, workspace, B,
+                                   L, C, stream);
 }
 
 int fields_read_forward_bf16_stats(const void* raw, const float* tr, const float* ti,
@@ -1440,9 +1391,8 @@ int fields_read_forward_bf16_stats(const void* raw, const float* tr, const float
     if (!workspace || workspace_bytes < fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD) ||
         (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return FIELDS_ERR_WORKSPACE;
-    return run_forward_single_pass<FwdSpBf16Stats, uint16_t>(
-        static_cast<const uint16_t*>(raw), tr, ti, gamma, state_in, static_cast<uint16_t*>(read),
-        state_out, workspace, B, L, C, reinterpret_cast<Stream>(stream), sumsq);
+    return run_forward_bf16<true>(raw, 3LL * C, tr, ti, gamma, state_in, read, sumsq, state_out, workspace, B, L,
+                                  C, stream);
 }
 
 int fields_read_backward_bf16(const void* raw, const float* tr, const float* ti, const float* gamma,
