@@ -55,6 +55,13 @@ SYMBOLS = {
     "fields_mixer_epilogue_bias_rows": (_SZ, [ctypes.c_longlong]),
     "fields_mixer_epilogue_forward": (_I, [_P] * 7 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
     "fields_mixer_epilogue_backward": (_I, [_P] * 11 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
+    "fields_read_forward_bf16_rows": (_I, [_P, _LL] + [_P] * 8 + [_SZ, _I, _I, _I, _P]),
+    "fields_read_backward_bf16_rows": (_I, [_P, _LL] + [_P] * 6 + [_LL] + [_P] * 4 + [_SZ, _I, _I, _I, _P]),
+    "fields_mixer_grad_rows": (_SZ, [_LL]),
+    "fields_mixer_grad_scratch_bytes": (_SZ, [_I]),
+    "fields_mixer_open_grad": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 4 + [_LL, _P, _P, ctypes.c_float, _I, _LL,
+                                                                       _I, _P]),
+    "fields_mixer_close_grad": (_I, [_P, _LL, _I, _P]),
     "fields_stack_layout": (_I, [_P, _P]),
     "fields_stack_step_norm": (_I, [_P, _LL, _P, _P, _P, ctypes.c_float, _LL, _I, _P]),
     "fields_stack_close_mixer": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 5 +

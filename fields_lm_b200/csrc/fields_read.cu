@@ -17,6 +17,7 @@
 #include "field_scan.cuh"
 #include "field_epilogue.cuh"
 #include "field_rows.cuh"
+#include "field_mixer_grad.cuh"
 
 #include "../../include/fields_read.h"
 
@@ -1709,10 +1710,10 @@ int fields_read_norm_grad_combine(const void* grad_read, const void* read, const
 }
 
 int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
-    if (!w || w->dim <= 0 || w->hidden <= 0) return FIELDS_ERR_ARGUMENT;
-    if (!w->write_w || !w->write_b || !w->gate_w || !w->out_w || !w->read_norm_w || !w->w12 || !w->w3 ||
-        !w->radius_logit || !w->theta || !w->in_w || !w->in_b || !w->out_w16 || !w->w12_16 || !w->w3_16 ||
-        !w->par)
+    if (!w || w->dim <= 0 || w->hidden < 0) return FIELDS_ERR_ARGUMENT;
+    if (!w->write_w || !w->write_b || !w->gate_w || !w->out_w || !w->read_norm_w || !w->radius_logit ||
+        !w->theta || !w->in_w || !w->in_b || !w->out_w16 || !w->par ||
+        (w->hidden && (!w->w12 || !w->w3 || !w->w12_16 || !w->w3_16)))
         return FIELDS_ERR_ARGUMENT;
     const long long D = w->dim, H = w->hidden, C = D / 2;
     const void* all[] = {w->write_w, w->write_b, w->gate_w, w->out_w, w->read_norm_w, w->w12, w->w3,
@@ -1728,7 +1729,7 @@ int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
     p.piece[3] = {w->out_w, static_cast<uint16_t*>(w->out_w16), w->read_norm_w, D * 2 * D, (int)(2 * D)};
     p.piece[4] = {w->w12, static_cast<uint16_t*>(w->w12_16), nullptr, 2 * H * D, (int)D};
     p.piece[5] = {w->w3, static_cast<uint16_t*>(w->w3_16), nullptr, D * H, (int)H};
-    p.piece[6] = {nullptr, nullptr, nullptr, 0, 4};
+    p.piece[6] = {nullptr, static_cast<uint16_t*>(w->in_b) + 3 * C, nullptr, D, (int)D};
     p.radius_logit = w->radius_logit; p.theta = w->theta; p.par = w->par; p.C = (int)C;
     // as many blocks per piece as the GPU has SMs: the pieces run side by side
     return launch_grid<LayoutParams>(layout_block, dim3(148, kLayoutPieces + 1), kRowThreads,
@@ -1772,7 +1773,7 @@ int fields_stack_close_mixer(const float* x, const void* acc, const void* gate, 
                              float norm_eps, long long N, int D, void* stream) {
     if (N < 0 || D <= 0 || features <= 0 || G < 0) return FIELDS_ERR_ARGUMENT;
     if (N == 0) return FIELDS_OK;
-    if (!x || !acc || !gate || !bias || !norm_w || !y || !h) return FIELDS_ERR_ARGUMENT;
+    if (!x || !acc || !gate || !bias || !y || (h && !norm_w)) return FIELDS_ERR_ARGUMENT;
     if (D % 4 || D > 4096 || gate_stride % 4 || !aligned16(x) || !aligned16(y) || !aligned16(bias) ||
         !aligned16(gate_bias) || !aligned16(norm_w) || !aligned8(acc) || !aligned8(gate) || !aligned8(h))
         return FIELDS_ERR_UNSUPPORTED;
@@ -1799,12 +1800,143 @@ int fields_stack_close_ff(const float* x, const void* f, const float* norm_w, fl
                           float norm_eps, long long N, int D, void* stream) {
     if (N < 0 || D <= 0) return FIELDS_ERR_ARGUMENT;
     if (N == 0) return FIELDS_OK;
-    if (!x || !h) return FIELDS_ERR_ARGUMENT;
+    if (!x || (!h && !y)) return FIELDS_ERR_ARGUMENT;
     if (D % 4 || D > 4096 || !aligned16(x) || !aligned16(y) || !aligned16(norm_w) || !aligned8(f) ||
         !aligned8(h))
         return FIELDS_ERR_UNSUPPORTED;
+    if (!norm_w) {
+        const long long n = N * D, per = 4LL * 4 * kRowThreads, blocks = (n + per - 1) / per;
+        if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+        AddCastParams p{x, static_cast<const uint16_t*>(f), y, static_cast<uint16_t*>(h), n};
+        return launch_on<AddCastParams>(add_cast, (unsigned)blocks, kRowThreads, 0, reinterpret_cast<Stream>(stream), p);
+    }
     CloseFfParams p{x, static_cast<const uint16_t*>(f), norm_w, y, static_cast<uint16_t*>(h), N, D, norm_eps};
     return launch_rows<CloseFfParams>(close_ff<1, 8>, close_ff<4, 2>, close_ff<4, 8>, N, D, stream, p);
+}
+
+int fields_read_forward_bf16_rows(const void* raw, long long raw_pitch, const float* tr, const float* ti,
+                                  const float* gamma, const float* state_in, void* read, float* sumsq,
+                                  float* state_out, void* workspace, size_t workspace_bytes, int B, int L,
+                                  int C, void* stream) {
+    if (B <= 0 || L <= 0 || C <= 0 || raw_pitch < 3LL * C || raw_pitch > 0x7fffffffLL) return FIELDS_ERR_ARGUMENT;
+    if (!raw || !read || !tr || !ti || !gamma) return FIELDS_ERR_ARGUMENT;
+    if (C % 4 || raw_pitch % 4 || !aligned8(raw) || !aligned8(read) || !aligned16(tr) || !aligned16(ti) ||
+        !aligned16(gamma))
+        return FIELDS_ERR_UNSUPPORTED;
+    if (!workspace || workspace_bytes < fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD) ||
+        (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return FIELDS_ERR_WORKSPACE;
+    if (sumsq)
+        return run_forward_bf16<true>(raw, raw_pitch, tr, ti, gamma, state_in, read, sumsq, state_out, workspace, B,
+                                      L, C, stream);
+    return run_forward_bf16<false>(raw, raw_pitch, tr, ti, gamma, state_in, read, nullptr, state_out, workspace, B, L,
+                                   C, stream);
+}
+
+int fields_read_backward_bf16_rows(const void* raw, long long raw_pitch, const float* tr, const float* ti,
+                                   const float* gamma, const void* read, const void* grad_read, void* grad_raw,
+                                   long long grad_pitch, float* grad_tr, float* grad_ti, float* grad_gamma,
+                                   void* workspace, size_t workspace_bytes, int B, int L, int C, void* stream) {
+    if (B <= 0 || L <= 0 || C <= 0 || raw_pitch < 3LL * C || raw_pitch > 0x7fffffffLL || grad_pitch < 3LL * C ||
+        grad_pitch > 0x7fffffffLL)
+        return FIELDS_ERR_ARGUMENT;
+    if (!raw || !read || !grad_read || !grad_raw || !tr || !ti || !gamma || !grad_tr || !grad_ti || !grad_gamma)
+        return FIELDS_ERR_ARGUMENT;
+    if (C % 4 || raw_pitch % 4 || grad_pitch % 4 || !aligned8(raw) || !aligned8(read) || !aligned8(grad_read) ||
+        !aligned8(grad_raw) || !aligned16(tr) || !aligned16(ti) || !aligned16(gamma))
+        return FIELDS_ERR_UNSUPPORTED;
+    if (!workspace || workspace_bytes < fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD) ||
+        (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return FIELDS_ERR_WORKSPACE;
+    return run_backward_single_pass<BwdSpBf16, uint16_t>(
+        static_cast<const uint16_t*>(raw), tr, ti, gamma, nullptr, static_cast<const uint16_t*>(read),
+        static_cast<const uint16_t*>(grad_read), nullptr, static_cast<uint16_t*>(grad_raw), grad_tr, grad_ti,
+        grad_gamma, nullptr, workspace, B, L, C, reinterpret_cast<Stream>(stream), nullptr, raw_pitch, grad_pitch);
+}
+
+// Rows of one block of open_grad: one round of blocks over the GPU, within what its shared memory holds.
+static int grad_rows_per_block(long long N) {
+    long long per = (N + kGradBlocks - 1) / kGradBlocks;
+    per = (per + 3) / 4 * 4;
+    return (int)(per < 4 ? 4 : per > kGradRowsMax ? kGradRowsMax : per);
+}
+constexpr int kColumnBlocks = 296, kWeightBlocks = 64;  // row blocks of column_sums and out_weight_grad
+
+size_t fields_mixer_grad_rows(long long N) {
+    const long long per = grad_rows_per_block(N);
+    return N > 0 ? (size_t)((N + per - 1) / per) : 0;
+}
+
+size_t fields_mixer_grad_scratch_bytes(int D) {
+    return D > 0 ? ((size_t)kColumnBlocks * (3 * (D / 2)) + (size_t)kWeightBlocks * 2 * D) * sizeof(float) : 0;
+}
+
+int fields_mixer_open_grad(const float* grad_y, const void* acc, const void* gate, long long gate_pitch,
+                           const float* groups, int G, const float* bias, const float* gate_bias, void* grad_acc,
+                           void* grad_gate, long long grad_pitch, float* grad_sumsq, float* rows, float eps,
+                           int features, long long N, int D, void* stream) {
+    if (N <= 0 || D <= 0 || features <= 0 || G <= 0) return FIELDS_ERR_ARGUMENT;
+    if (!grad_y || !acc || !gate || !groups || !bias || !gate_bias || !grad_acc || !grad_gate || !grad_sumsq || !rows)
+        return FIELDS_ERR_ARGUMENT;
+    if (D % 4 || D > 4096 || gate_pitch % 4 || grad_pitch % 4 || !aligned16(grad_y) || !aligned16(bias) ||
+        !aligned16(gate_bias) || !aligned16(rows) || !aligned8(acc) || !aligned8(gate) || !aligned8(grad_acc) ||
+        !aligned8(grad_gate))
+        return FIELDS_ERR_UNSUPPORTED;
+    OpenGradParams p{grad_y, static_cast<const uint16_t*>(acc), static_cast<const uint16_t*>(gate), groups, bias,
+                     gate_bias, static_cast<uint16_t*>(grad_acc), static_cast<uint16_t*>(grad_gate), grad_sumsq,
+                     rows, N, gate_pitch, grad_pitch, D, G, grad_rows_per_block(N), eps, 1.0f / (float)features};
+    const size_t blocks = fields_mixer_grad_rows(N);
+    if (blocks > 0x7fffffffu) return FIELDS_ERR_UNSUPPORTED;
+    Stream st = reinterpret_cast<Stream>(stream);
+    if (D <= 4 * kRowThreads) {
+        int threads = (D / 4 + 31) / 32 * 32;
+        if (threads < kGradRowsMax) threads = kGradRowsMax;  // one thread per row at the end
+        return launch_on<OpenGradParams>(open_grad<1, 4>, (unsigned)blocks, (unsigned)threads, 0, st, p);
+    }
+    return launch_on<OpenGradParams>(open_grad<4, 1>, (unsigned)blocks, kRowThreads, 0, st, p);
+}
+
+int fields_mixer_close_grad(const struct fields_mixer_grads* g, long long N, int D, void* stream) {
+    if (!g || N <= 0 || D <= 0) return FIELDS_ERR_ARGUMENT;
+    if (!g->rows || !g->grad_raw || !g->grad_out || !g->out_w || !g->norm_w || !g->radius_logit || !g->theta ||
+        !g->grad_tr || !g->grad_ti || !g->grad_gamma || !g->grad_out_b || !g->grad_gate_b || !g->grad_write_b ||
+        !g->grad_norm_w || !g->grad_radius || !g->grad_theta || !g->scratch)
+        return FIELDS_ERR_ARGUMENT;
+    if (D % 8 || g->grad_pitch % 4 || !aligned8(g->grad_raw) || !aligned16(g->grad_out) || !aligned16(g->out_w) ||
+        !aligned16(g->norm_w) || !aligned16(g->scratch))
+        return FIELDS_ERR_UNSUPPORTED;
+    Stream st = reinterpret_cast<Stream>(stream);
+    const int C = D / 2, cols = 3 * C, wide = 2 * D, per_x = kRowThreads * 4;
+    float* col_rows = g->scratch;
+    float* weight_rows = col_rows + (size_t)kColumnBlocks * cols;
+    const long long per = (N + kColumnBlocks - 1) / kColumnBlocks;
+    if (per > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+    const int col_blocks = (int)((N + per - 1) / per);
+    ColumnSumParams cp{static_cast<const uint16_t*>(g->grad_raw), col_rows, N, g->grad_pitch, cols, (int)per};
+    int rc = launch_grid<ColumnSumParams>(column_sums, dim3((cols + per_x - 1) / per_x, col_blocks), kRowThreads, st, cp);
+    if (rc) return rc;
+    const int wper = (D + kWeightBlocks - 1) / kWeightBlocks, weight_blocks = (D + wper - 1) / wper;
+    OutWeightGradParams wp{g->grad_out, g->out_w, g->norm_w, weight_rows, D, wide, wper};
+    rc = launch_grid<OutWeightGradParams>(out_weight_grad, dim3((wide + per_x - 1) / per_x, weight_blocks), kRowThreads,
+                                          st, wp);
+    if (rc) return rc;
+    const int n = (int)fields_mixer_grad_rows(N);
+    FinishGradParams p{};
+    int first = 0;
+    auto add = [&](int k, const float* rows, float* out, int count, int width) {
+        p.set[k] = PartialRows{rows, out, count, width, first};
+        first += (width + 31) / 32;
+    };
+    add(0, g->rows, g->grad_out_b, n, D);
+    add(1, g->rows + (size_t)n * D, g->grad_gate_b, n, D);
+    add(2, col_rows, g->grad_write_b, col_blocks, cols);
+    add(3, weight_rows, g->grad_norm_w, weight_blocks, wide);
+    p.transition_block = first;
+    p.radius_logit = g->radius_logit; p.theta = g->theta;
+    p.g_tr = g->grad_tr; p.g_ti = g->grad_ti; p.g_gm = g->grad_gamma;
+    p.g_radius = g->grad_radius; p.g_theta = g->grad_theta; p.C = C;
+    return launch_on<FinishGradParams>(finish_grad, (unsigned)(first + (C + kRowThreads - 1) / kRowThreads), kRowThreads,
+                                       0, st, p);
 }
 #endif  // FIELDS_HOST_EMU
 

@@ -33,7 +33,9 @@ using torch::autograd::variable_list;
     X(fields_read_norm_grad_combine) X(fields_read_step) X(fields_read_step_bf16)                 \
     X(fields_scan_workspace_bytes) X(fields_scan_forward) X(fields_scan_backward)                 \
     X(fields_stack_layout) X(fields_stack_step_norm) X(fields_stack_close_mixer)                  \
-    X(fields_stack_swiglu) X(fields_stack_close_ff)
+    X(fields_stack_swiglu) X(fields_stack_close_ff) X(fields_read_forward_bf16_rows)              \
+    X(fields_read_backward_bf16_rows) X(fields_mixer_grad_rows) X(fields_mixer_grad_scratch_bytes) \
+    X(fields_mixer_open_grad) X(fields_mixer_close_grad)
 
 struct Api {
 #define X(name) decltype(&::name) name;

@@ -1,0 +1,168 @@
+// The fused Field mixer (bfloat16 boundary, norm behind the output projection) as one autograd node.
+//
+// As a composition of torch operations the mixer's forward + backward made 76 launches and was bound
+// by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is three matrix
+// products forward and four backward (library calls; the two projections of x are one product over
+// [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
+// field_mixer_grad.cuh between them. Weight gradients come out of the products in fp32.
+#include "torch_api.h"
+
+#include <ATen/ops/addmm_cuda_dispatch.h>
+#include <ATen/ops/mm_cuda_dispatch.h>
+
+namespace fields_torch {
+
+enum { kX, kWriteW, kWriteB, kRadius, kTheta, kNormW, kOutW, kOutB, kGateW, kGateB, kMixerInputs };
+
+// Whether every input is what the node works on: dense, aligned fp32 on one GPU, sizes that fit.
+static bool mixer_applies(const std::vector<Tensor>& in) {
+    const Tensor& x = in[kX];
+    if (x.dim() != 3 || x.numel() == 0 || !x.is_cuda()) return false;
+    const int64_t D = x.size(2), C = D / 2;
+    if (D % 8 || D > 4096 || x.size(0) > INT_MAX || x.size(1) > INT_MAX) return false;
+    const std::vector<int64_t> shapes[kMixerInputs] = {{},     {3 * C, D},     {3 * C}, {C},    {C},
+                                                       {2 * D}, {D, 2 * D},     {D},     {D, D}, {D}};
+    for (int i = 0; i < kMixerInputs; ++i) {
+        const Tensor& t = in[i];
+        if (t.scalar_type() != at::kFloat || t.device() != x.device() || t.layout() != at::kStrided) return false;
+        if (i == kX) continue;
+        if (t.sizes() != at::IntArrayRef(shapes[i]) || !t.is_contiguous() ||
+            reinterpret_cast<uintptr_t>(t.data_ptr()) % 16)
+            return false;
+    }
+    return true;
+}
+
+struct FusedMixer : torch::autograd::Function<FusedMixer> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x_, const Tensor& write_w, const Tensor& write_b,
+                                 const Tensor& radius, const Tensor& theta, const Tensor& norm_w, const Tensor& out_w,
+                                 const Tensor& out_b, const Tensor& gate_w, const Tensor& gate_b, double eps) {
+        const Api& f = api();
+        const Tensor x = dense(x_);
+        const int64_t B = x.size(0), L = x.size(1), D = x.size(2), N = B * L, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
+        const c10::Device dev = x.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        void* st = stream_of(x);
+        const Tensor in_w = empty({W, D}, at::kBFloat16, dev), in_b = empty({W}, at::kBFloat16, dev),
+                     out16 = empty({D, 2 * D}, at::kBFloat16, dev), par = empty({3, C}, at::kFloat, dev);
+        fields_stack_weights w{};
+        w.write_w = fp(write_w); w.write_b = fp(write_b); w.gate_w = fp(gate_w); w.out_w = fp(out_w);
+        w.read_norm_w = fp(norm_w); w.radius_logit = fp(radius); w.theta = fp(theta);
+        w.in_w = vp(in_w); w.in_b = vp(in_b); w.out_w16 = vp(out16); w.par = fp(par);
+        w.dim = (int)D; w.hidden = 0;
+        check(f.fields_stack_layout(&w, st), "fields_stack_layout");
+        const Tensor xb = empty({N, D}, at::kBFloat16, dev);
+        check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, (int)D, st),
+              "fields_stack_close_ff");
+        Tensor u = empty({N, W}, at::kBFloat16, dev);
+        at::cuda::addmm_out(u, in_b, xb, in_w.t(), 1, 1);
+        const Tensor read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
+        {
+            const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
+            const Tensor ws = workspace(n, dev);
+            float* p = fp(par);
+            check(f.fields_read_forward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, nullptr, vp(read), fp(groups), nullptr,
+                                                  vp(ws), n, (int)B, (int)L, (int)C, st),
+                  "fields_read_forward_bf16_rows");
+        }
+        Tensor acc = empty({N, D}, at::kBFloat16, dev);
+        at::cuda::mm_out(acc, read, out16.t());
+        const Tensor y = empty({B, L, D}, at::kFloat, dev);
+        check(f.fields_stack_close_mixer(fp(x), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
+                                         nullptr, fp(y), nullptr, (float)eps, (int)(2 * D), 0.0f, N, (int)D, st),
+              "fields_stack_close_mixer");
+        ctx->save_for_backward({xb, u, read, groups, acc, in_w, out16, par, radius, theta, norm_w, out_w, out_b, gate_b});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["length"] = L;
+        return {y};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const Api& f = api();
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &xb = s[0], &u = s[1], &read = s[2], &groups = s[3], &acc = s[4], &in_w = s[5], &out16 = s[6],
+                     &par = s[7], &radius = s[8], &theta = s[9], &norm_w = s[10], &out_w = s[11], &out_b = s[12],
+                     &gate_b = s[13];
+        const Tensor gy = f32(grads[0]);
+        const int64_t N = xb.size(0), D = xb.size(1), C = D / 2, W = 3 * C + D, G = groups.size(1);
+        const int64_t L = ctx->saved_data["length"].toInt(), B = N / L;
+        const float eps = (float)ctx->saved_data["eps"].toDouble();
+        const c10::Device dev = xb.device();
+        const c10::cuda::CUDAGuard guard(dev);
+        void* st = stream_of(xb);
+        auto f32s = [&](at::IntArrayRef size) { return empty(size, at::kFloat, dev); };
+
+        const Tensor grad_acc = empty({N, D}, at::kBFloat16, dev), grad_u = empty({N, W}, at::kBFloat16, dev),
+                     grad_sumsq = f32s({N}), rows = f32s({2, (int64_t)f.fields_mixer_grad_rows(N), D});
+        check(f.fields_mixer_open_grad(fp(gy), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
+                                       vp(grad_acc), gate_of(grad_u, C), W, fp(grad_sumsq), fp(rows), eps, (int)(2 * D),
+                                       N, (int)D, st),
+              "fields_mixer_open_grad");
+        Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
+        at::cuda::mm_out(grad_read, grad_acc, out16);
+        Tensor grad_out = f32s({D, 2 * D});
+        at::cuda::mm_out(grad_out, grad_acc.t(), read, at::kFloat);
+        check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), fp(grad_sumsq), vp(grad_read), N, (int)(4 * C), st),
+              "fields_read_norm_grad_combine");
+        const Tensor g_par = f32s({3, C});
+        float *p = fp(par), *g = fp(g_par);
+        {
+            const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
+            const Tensor ws = workspace(n, dev);
+            check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
+                                                   g, g + C, g + 2 * C, vp(ws), n, (int)B, (int)L, (int)C, st),
+                  "fields_read_backward_bf16_rows");
+        }
+        Tensor grad_x;
+        if (ctx->needs_input_grad(kX)) {
+            Tensor back = empty({N, D}, at::kBFloat16, dev);
+            at::cuda::mm_out(back, grad_u, in_w);
+            grad_x = f32s({B, L, D});
+            check(f.fields_stack_close_ff(fp(gy), vp(back), nullptr, fp(grad_x), nullptr, 0.0f, N, (int)D, st),
+                  "fields_stack_close_ff");
+        }
+        Tensor grad_in = f32s({W, D});
+        at::cuda::mm_out(grad_in, grad_u.t(), xb, at::kFloat);
+
+        const Tensor g_out_b = f32s({D}), g_gate_b = f32s({D}), g_write_b = f32s({3 * C}), g_norm = f32s({2 * D}),
+                     g_radius = f32s({C}), g_theta = f32s({C}),
+                     scratch = f32s({(int64_t)(f.fields_mixer_grad_scratch_bytes((int)D) / 4)});
+        fields_mixer_grads q{};
+        q.rows = fp(rows); q.grad_raw = vp(grad_u); q.grad_pitch = W; q.grad_out = fp(grad_out); q.out_w = fp(out_w);
+        q.norm_w = fp(norm_w); q.radius_logit = fp(radius); q.theta = fp(theta);
+        q.grad_tr = g; q.grad_ti = g + C; q.grad_gamma = g + 2 * C;
+        q.grad_out_b = fp(g_out_b); q.grad_gate_b = fp(g_gate_b); q.grad_write_b = fp(g_write_b);
+        q.grad_norm_w = fp(g_norm); q.grad_radius = fp(g_radius); q.grad_theta = fp(g_theta); q.scratch = fp(scratch);
+        check(f.fields_mixer_close_grad(&q, N, (int)D, st), "fields_mixer_close_grad");
+        return {grad_x,   grad_in.narrow(0, 0, 3 * C),   g_write_b, g_radius, g_theta, g_norm, grad_out,
+                g_out_b, grad_in.narrow(0, 3 * C, D), g_gate_b,  Tensor()};
+    }
+
+  private:
+    // the gate columns of [raw | gate]
+    static void* gate_of(const Tensor& u, int64_t C) { return static_cast<at::BFloat16*>(vp(u)) + 3 * C; }
+};
+
+// fused_mixer(x, write_w, write_b, radius_logit, theta, norm_w, out_w, out_b, gate_w, gate_b, eps) -> y, or None
+// where the node does not apply
+PyObject* py_fused_mixer(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    want_args(n, kMixerInputs + 1);
+    std::vector<Tensor> in;
+    in.reserve(kMixerInputs);
+    for (int i = 0; i < kMixerInputs; ++i) in.push_back(tensor_arg(args[i]));
+    const double eps = PyFloat_AsDouble(args[kMixerInputs]);
+    if (PyErr_Occurred()) throw python_error();
+    Tensor y;
+    {
+        pybind11::gil_scoped_release no_gil;
+        if (mixer_applies(in))
+            y = FusedMixer::apply(in[kX], in[kWriteW], in[kWriteB], in[kRadius], in[kTheta], in[kNormW], in[kOutW],
+                                  in[kOutB], in[kGateW], in[kGateB], eps)[0];
+    }
+    if (!y.defined()) Py_RETURN_NONE;
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+}  // namespace fields_torch

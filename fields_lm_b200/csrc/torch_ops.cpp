@@ -16,7 +16,8 @@
 
 namespace fields_torch {
 
-void add_stack(PyObject* module);  // torch_stack.cpp
+void add_stack(PyObject* module);                                                 // torch_stack.cpp
+PyObject* py_fused_mixer(PyObject*, PyObject* const* args, Py_ssize_t n);  // torch_mixer.cpp
 
 struct Dims {
     int B, L, C;
@@ -403,6 +404,7 @@ static PyMethodDef g_methods[] = {
     FAST("bind", py_bind),
     FAST("field_read", py_field_read),
     FAST("field_read_bf16", py_field_read_bf16),
+    FAST("fused_mixer", py_fused_mixer),
     FAST("linear_scan", py_linear_scan),
     FAST("step", py_step),
     {nullptr, nullptr, 0, nullptr},

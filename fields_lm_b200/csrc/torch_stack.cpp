@@ -31,7 +31,7 @@ struct Block {
     std::vector<Source> src;
     double read_eps = 0, ff_eps = 0;
     // bfloat16, transposed views for the products; `in` = write over gate, scaled `out`
-    Tensor in_w, in_b, write_t, gate_t, in_t, out_t, w12_t, w3_t, par;
+    Tensor in_w, in_b, in_t, out_t, w12_t, w3_t, par;
     float* f(int i) const { return fp(src[i].t); }
 };
 
@@ -82,10 +82,8 @@ class FieldStack {
             for (Source& s : b.src) s.version = s.t._version();
             if (!b.in_w.defined()) {
                 b.in_w = empty({3 * C + D, D}, at::kBFloat16, dev);
-                b.in_b = at::zeros({3 * C + D}, at::TensorOptions().dtype(at::kBFloat16).device(dev));
+                b.in_b = empty({3 * C + D}, at::kBFloat16, dev);
                 b.in_t = b.in_w.t();
-                b.write_t = b.in_w.narrow(0, 0, 3 * C).t();
-                b.gate_t = b.in_w.narrow(0, 3 * C, D).t();
                 b.out_t = empty({D, 2 * D}, at::kBFloat16, dev).t();
                 b.w12_t = empty({2 * H, D}, at::kBFloat16, dev).t();
                 b.w3_t = empty({D, H}, at::kBFloat16, dev).t();
@@ -112,32 +110,29 @@ class FieldStack {
     std::pair<Tensor, std::vector<Tensor>> prefill(const Tensor& x_) {
         const Api& f = api();
         const Tensor x = dense(x_);
-        const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, G = (C + 127) / 128;
+        const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
         void* st = stream_of(x);
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
-                     raw = empty({N, 3 * C}, at::kBFloat16, dev), gate = empty({N, D}, at::kBFloat16, dev),
                      read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         const size_t ws_bytes = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
-        Tensor acc = empty({N, D}, at::kBFloat16, dev), ws = workspace(ws_bytes, dev),
+        Tensor acc = empty({N, D}, at::kBFloat16, dev), ws = workspace(ws_bytes, dev), u = empty({N, W}, at::kBFloat16, dev),
                uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev);
         std::vector<Tensor> states;
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, st),
               "fields_stack_close_ff");
         const float* in = fp(x);
         for (const Block& b : blocks_) {
-            Tensor raw_out = raw, gate_out = gate;
-            at::cuda::addmm_out(raw_out, b.in_b.narrow(0, 0, 3 * C), xb, b.write_t, 1, 1);
-            at::cuda::mm_out(gate_out, xb, b.gate_t);
+            at::cuda::addmm_out(u, b.in_b, xb, b.in_t, 1, 1);
             const Tensor state = empty({B, D}, at::kFloat, dev);
             float* par = fp(b.par);
-            check(f.fields_read_forward_bf16_stats(vp(raw), par, par + C, par + 2 * C, nullptr, vp(read),
-                                                   fp(groups), fp(state), vp(ws), ws_bytes, (int)B, (int)L,
-                                                   (int)C, st),
-                  "fields_read_forward_bf16_stats");
+            check(f.fields_read_forward_bf16_rows(vp(u), W, par, par + C, par + 2 * C, nullptr, vp(read), fp(groups),
+                                                  fp(state), vp(ws), ws_bytes, (int)B, (int)L, (int)C, st),
+                  "fields_read_forward_bf16_rows");
             at::cuda::mm_out(acc, read, b.out_t);
-            check(f.fields_stack_close_mixer(in, vp(acc), vp(gate), D, fp(groups), (int)G,
+            const void* gate = static_cast<at::BFloat16*>(vp(u)) + 3 * C;
+            check(f.fields_stack_close_mixer(in, vp(acc), gate, W, fp(groups), (int)G,
                                              b.f(Block::kOutB), b.f(Block::kGateB), b.f(Block::kFfNorm), fp(y),
                                              vp(xb), (float)b.read_eps, 2 * D_, (float)b.ff_eps, N, D_, st),
                   "fields_stack_close_mixer");

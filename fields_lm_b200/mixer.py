@@ -25,6 +25,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _lib
 from .decode import field_read_step
 from .field_read import (field_read_with_state, fused_field_read_bf16,
                          fused_field_read_bf16_stats, mixer_epilogue)
@@ -36,6 +37,21 @@ def transition_parameters(radius_logit: torch.Tensor, theta: torch.Tensor):
     theta = theta.float()
     return (radius * torch.cos(theta), radius * torch.sin(theta),
             torch.sqrt((1.0 - radius.square()).clamp_min(1e-4)))
+
+
+def _native_mixer(m: nn.Module, x: torch.Tensor) -> Optional[torch.Tensor]:
+    """``fused_mixer_forward`` as one native autograd node (``csrc/torch_mixer.cpp``); None where
+    a projection is not a plain ``nn.Linear`` or a tensor is not what the node works on."""
+    write, out, gate = m.write_proj, m.out_proj, m.gate_proj
+    if not (type(write) is nn.Linear and type(out) is nn.Linear and type(gate) is nn.Linear
+            and not write._forward_hooks and not write._forward_pre_hooks
+            and not write._backward_hooks and not write._backward_pre_hooks):
+        return None
+    params = (write.weight, write.bias, m.radius_logit, m.theta, m.read_norm.weight, out.weight,
+              out.bias, gate.weight, gate.bias)
+    if any(type(p) is not nn.Parameter for p in params):
+        return None
+    return _lib.native().fused_mixer(x, *params, m.read_norm.eps)
 
 
 def fused_mixer_forward(m: nn.Module, x: torch.Tensor) -> Optional[torch.Tensor]:
@@ -55,6 +71,9 @@ def fused_mixer_forward(m: nn.Module, x: torch.Tensor) -> Optional[torch.Tensor]
             and torch.get_autocast_dtype("cuda") == torch.bfloat16
             and m.channels % 4 == 0 and m.dim % 4 == 0 and m.dim <= 4096):
         return None
+    y = _native_mixer(m, x)
+    if y is not None:
+        return y
     x_in = x.to(torch.bfloat16)  # both projections of x take the same copy
     raw = m.write_proj(x_in).contiguous()
     tr, ti, gamma = transition_parameters(m.radius_logit, m.theta)

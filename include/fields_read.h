@@ -465,15 +465,16 @@ int fields_mixer_epilogue_backward(const float *grad_y, const void *acc, const v
  * tensors dense and 16-byte aligned (FIELDS_ERR_UNSUPPORTED otherwise). bf16 operands are void *.
  *
  * fields_stack_layout: bfloat16 copies of a block's weights as the products want them, and its
- *   transition parameters. in_w = write_proj over gate_proj, in_b = write_proj's bias over zeros (the
- *   caller zeroed it: only the first 3C elements are written), out_w16 = out_proj diag(read_norm).
+ *   transition parameters. in_w = write_proj over gate_proj, in_b = write_proj's bias over zeros,
+ *   out_w16 = out_proj diag(read_norm). hidden = 0: without the feed-forward (w12, w3 may be NULL).
  * fields_stack_step_norm: one recurrence step of N rows from raw (row stride raw_stride) and par
  *   [3, C]; state [N, 2C] advances in place; out [N, 4C] = read / rms(read).
  * fields_stack_close_mixer: y = x + (acc r + bias) * sigmoid(gate + gate_bias) and h = norm_w * y /
  *   rms(y); r is the RMS scale of the row's read values if groups [N, G] gives their sums of squares,
- *   1 if it is NULL.
+ *   1 if it is NULL. norm_w and h NULL: y only.
  * fields_stack_swiglu: out = silu(u) * v for uv [N, 2H] = u | v.
- * fields_stack_close_ff: y = x + f (f NULL: x; y NULL: not stored) and h = y, or norm_w * y / rms(y).
+ * fields_stack_close_ff: y = x + f (f NULL: x; y NULL: not stored) and h = y, or norm_w * y / rms(y)
+ *   (h NULL: not stored).
  */
 struct fields_stack_weights {
     const float *write_w, *write_b, *gate_w, *out_w, *read_norm_w, *w12, *w3, *radius_logit, *theta;
@@ -491,6 +492,50 @@ int fields_stack_close_mixer(const float *x, const void *acc, const void *gate, 
 int fields_stack_swiglu(const void *uv, void *out, long long N, int H, void *stream);
 int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, float *y, void *h,
                           float norm_eps, long long N, int D, void *stream);
+
+/*
+ * fields_read_forward_bf16(_stats) and fields_read_backward_bf16 on rows that lie raw_pitch (and
+ * grad_pitch) elements apart, as columns of a wider matrix: raw and gate of a mixer are one product.
+ * Pitches are multiples of 4; sumsq may be NULL.
+ */
+int fields_read_forward_bf16_rows(const void *raw, long long raw_pitch, const float *tr,
+                                  const float *ti, const float *gamma, const float *state_in,
+                                  void *read, float *sumsq, float *state_out, void *workspace,
+                                  size_t workspace_bytes, int B, int L, int C, void *stream);
+int fields_read_backward_bf16_rows(const void *raw, long long raw_pitch, const float *tr,
+                                   const float *ti, const float *gamma, const void *read,
+                                   const void *grad_read, void *grad_raw, long long grad_pitch,
+                                   float *grad_tr, float *grad_ti, float *grad_gamma,
+                                   void *workspace, size_t workspace_bytes, int B, int L, int C,
+                                   void *stream);
+
+/*
+ * The fused mixer's backward pass around its matrix products (D = dim, C = D / 2, D % 8 == 0, D <= 4096).
+ *
+ * fields_mixer_open_grad: from grad_y, acc, gate (row stride gate_pitch) and the sums of squares
+ *   groups [N, G] of y = x + (acc rstd + bias) sigmoid(gate + gate_bias): grad_acc [N, D] and
+ *   grad_gate (row stride grad_pitch) in bfloat16, grad_sumsq [N], and partial rows of the gradients
+ *   of bias and gate_bias, [2][fields_mixer_grad_rows(N)][D].
+ * fields_mixer_close_grad: gradients of the parameters from those partial rows, from grad_raw (the
+ *   first 3C columns of rows grad_pitch apart, bfloat16), from grad_out (in: gradient of out_proj
+ *   diag(norm), out: that of out_proj) and from the gradients of the transition parameters. scratch:
+ *   fields_mixer_grad_scratch_bytes(D) bytes.
+ */
+size_t fields_mixer_grad_rows(long long N);
+size_t fields_mixer_grad_scratch_bytes(int D);
+int fields_mixer_open_grad(const float *grad_y, const void *acc, const void *gate, long long gate_pitch,
+                           const float *groups, int G, const float *bias, const float *gate_bias,
+                           void *grad_acc, void *grad_gate, long long grad_pitch, float *grad_sumsq,
+                           float *rows, float eps, int features, long long N, int D, void *stream);
+struct fields_mixer_grads {
+    const float *rows;
+    const void *grad_raw;
+    long long grad_pitch;
+    float *grad_out;
+    const float *out_w, *norm_w, *radius_logit, *theta, *grad_tr, *grad_ti, *grad_gamma;
+    float *grad_out_b, *grad_gate_b, *grad_write_b, *grad_norm_w, *grad_radius, *grad_theta, *scratch;
+};
+int fields_mixer_close_grad(const struct fields_mixer_grads *grads, long long N, int D, void *stream);
 
 #ifdef __cplusplus
 }

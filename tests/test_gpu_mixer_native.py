@@ -1,0 +1,75 @@
+"""The native fused mixer (csrc/torch_mixer.cpp, field_rows.cuh, field_mixer_grad.cuh) against the same
+mixer as a composition of torch operations, and the forward kernels at the edges of their tiles (GPU)."""
+import numpy as np
+import pytest
+import torch
+
+import mirror
+from conftest import BF16_TOL, FP32_TOL, rel_err
+from fields_lm_b200 import fused_field_read, fused_field_read_bf16, mixer
+from oracle import field_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _grads(m, x, gy, native):
+    """y and every gradient, natively or through the composed path."""
+    keep = mixer._native_mixer
+    if not native:
+        mixer._native_mixer = lambda *a: None
+    try:
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = mixer.fused_mixer_forward(m, x)
+    finally:
+        mixer._native_mixer = keep
+    assert ("FusedMixer" in type(y.grad_fn).__name__ or "FusedMixer" in y.grad_fn.name()) == native
+    params = dict(m.named_parameters())
+    grads = torch.autograd.grad(y, [x, *params.values()], gy)
+    return {"y": y.detach(), "x": grads[0], **dict(zip(params, grads[1:]))}
+
+
+# rows below, at and above one block of the gradient kernels, and of one warp or four per row; widths
+# below, at and above one group of columns per thread
+@pytest.mark.parametrize("dim,B,L", [(8, 1, 1), (64, 3, 7), (200, 2, 33), (1024, 2, 384), (1024, 5, 1003),
+                                     (2048, 1, 65), (4096, 1, 70)])
+def test_native_mixer_matches_the_composed_one(dim, B, L):
+    torch.manual_seed(dim + L)
+    m = mirror.IndependentVacancyField(dim).cuda()
+    with torch.no_grad():
+        m.read_norm.weight.add_(0.2 * torch.randn(2 * dim, device="cuda"))
+        m.radius_logit.add_(torch.randn(dim // 2, device="cuda"))
+        if dim >= 64:  # outside the clamp of the radius, where its gradient is zero
+            m.radius_logit[0], m.radius_logit[1] = -1.0, 12.0
+    x = torch.randn(B, L, dim, device="cuda", requires_grad=True)
+    gy = torch.randn(B, L, dim, device="cuda")
+    got, want = _grads(m, x, gy, True), _grads(m, x, gy, False)
+    for name in want:
+        assert got[name].shape == want[name].shape and got[name].dtype == want[name].dtype, name
+        assert rel_err(got[name].float().cpu().numpy(), want[name].float().cpu().numpy()) < BF16_TOL, name
+
+
+@pytest.mark.parametrize("L", [8, 9, 10, 35, 36, 37, 39, 40, 41, 79, 80, 81])
+def test_forward_at_the_edges_of_the_tiles(L):
+    rng = np.random.default_rng(L)
+    B, C = 2, 132
+    radius, theta = rng.uniform(0.5, 0.99995, C), rng.uniform(-np.pi, np.pi, C)
+    par = [(radius * np.cos(theta)).astype(np.float32), (radius * np.sin(theta)).astype(np.float32),
+           np.sqrt(np.maximum(1 - radius ** 2, 1e-4)).astype(np.float32)]
+    raw = torch.from_numpy(rng.standard_normal((B, L, 3 * C)).astype(np.float32)).bfloat16()
+    want, _ = field_oracle.forward(raw.float().numpy(), *par)
+    dev = [torch.from_numpy(p).cuda() for p in par]
+    assert rel_err(fused_field_read(raw.float().cuda(), *dev).cpu().numpy(), want) < FP32_TOL
+    # one rounding to bfloat16 of values computed in fp32
+    assert rel_err(fused_field_read_bf16(raw.cuda(), *dev).float().cpu().numpy(), want) < 2 ** -8
+
+
+def test_bf16_forward_with_long_tiles():
+    """3,500 tiles of 40 steps and more: blocks of eight warps."""
+    B, L, C = 2, 35_003, 260
+    torch.manual_seed(0)
+    raw = (0.577 * torch.randn(B, L, 3 * C, device="cuda")).bfloat16()
+    ring, theta = torch.linspace(0.85, 0.999, C), torch.linspace(0.03, 3.04, C)
+    par = [t.cuda() for t in (ring * theta.cos(), ring * theta.sin(), (1 - ring ** 2).sqrt())]
+    want = fused_field_read(raw.float(), *par)
+    got = fused_field_read_bf16(raw, *par).float()
+    assert float((got - want).abs().max()) <= 2 ** -8 * float(want.abs().max())
