@@ -21,6 +21,7 @@
 
 #include "../../include/fields_read.h"
 
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <string>
@@ -1193,18 +1194,70 @@ int fields_read_fold_summaries_backward(const float* summaries, const float* car
 // ---------------------------------------------------------------------------
 // Real-valued scan (field_scan.cuh): plan and launches.
 // ---------------------------------------------------------------------------
+// Blocks per cluster: as many as a sequence has tiles, while all of them fit the GPU at once (up to 16:
+// the exchange costs a block Q stores and Q folds per super-tile, and its latency once).
 static ScanShape make_scan_shape(int B, int L, int C, long long a_batch, long long a_step,
                                  int a_chan) {
     ScanShape s{};
     s.B = B; s.L = L; s.C = C;
-    s.NT = (L + kScanChunk - 1) / kScanChunk;
+    s.NT = (L + kScanTile - 1) / kScanTile;
     s.CG = (C + 31) / 32;
     s.a_batch = a_batch; s.a_step = a_step; s.a_chan = a_chan;
+#ifdef FIELDS_HOST_EMU
+    s.Q = s.NT;
+#else
+    s.Q = 1;
+    while (s.Q < kScanMaxCluster && s.Q < s.NT && (long long)B * s.CG * s.Q < 2 * 148) s.Q *= 2;
+#endif
+    s.K = (s.NT + s.Q - 1) / s.Q;
     return s;
 }
 
+// (what the host emulation exchanges maps through; the GPU kernels need no workspace, the size is kept)
 static size_t scan_workspace_floats(int B, int L, int C) {
-    return (size_t)3 * B * ((L + kScanChunk - 1) / kScanChunk) * C;
+    return (size_t)3 * B * ((L + 15) / 16) * C;
+}
+
+template <bool BWD>
+static int run_scan(ScanParams p, float* ws, Stream st) {
+    const ScanShape& s = p.s;
+    const long long blocks = (long long)s.B * s.CG * s.Q;
+#ifdef FIELDS_HOST_EMU
+    p.maps = ws;
+    return launch_stateful<ScanWalk<BWD>>(p, blocks, 0, st);
+#else
+    (void)ws;
+    if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+    static std::atomic<bool> ready[64];
+    int dev = 0;
+    int rc = check_cuda(cudaGetDevice(&dev));
+    if (rc) return rc;
+    if (dev < 0 || dev >= 64) return FIELDS_ERR_UNSUPPORTED;
+    if (s.Q > 8 && !ready[dev]) {  // clusters of more than eight blocks are an opt-in (idempotent)
+        rc = check_cuda(cudaFuncSetAttribute(scan_walk<BWD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        if (rc) return rc;
+        ready[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(ScanWalk<BWD>::kThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (dependent_launch_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (s.Q > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = s.Q;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return check_cuda(cudaLaunchKernelEx(&cfg, scan_walk<BWD>, p));
+#endif
 }
 
 static int scan_check(const void* workspace, size_t workspace_bytes, int B, int L, int C,
@@ -1269,16 +1322,10 @@ int fields_scan_forward(const float* a, long long a_batch, long long a_step, int
     if (!a || !drive || !states) return FIELDS_ERR_ARGUMENT;
     int rc = scan_check(workspace, workspace_bytes, B, L, C, a_batch, a_step, a_chan);
     if (rc) return rc;
-    const ScanShape s = make_scan_shape(B, L, C, a_batch, a_step, a_chan);
-    float* ws = static_cast<float*>(workspace);
-    const size_t plane = (size_t)B * s.NT * C;
-    ScanFwdParams p{a, drive, state_in, states, state_out, ws, ws + plane, ws + 2 * plane, s};
-    const long long chunk_blocks = (scan_items(s) + kScanWarps - 1) / kScanWarps;
-    const long long chan_blocks = ((long long)B * C + ScanCarry::kThreads - 1) / ScanCarry::kThreads;
-    rc = launch<ScanChunkMap>(p, chunk_blocks, st);
-    if (!rc) rc = launch<ScanCarry>(p, chan_blocks, st);
-    if (!rc) rc = launch<ScanEmit>(p, chunk_blocks, st);
-    return rc;
+    ScanParams p{};
+    p.a = a; p.x = drive; p.first = state_in; p.out = states; p.end = state_out;
+    p.s = make_scan_shape(B, L, C, a_batch, a_step, a_chan);
+    return run_scan<false>(p, static_cast<float*>(workspace), st);
 }
 
 int fields_scan_backward(const float* a, long long a_batch, long long a_step, int a_chan,
@@ -1304,18 +1351,11 @@ int fields_scan_backward(const float* a, long long a_batch, long long a_step, in
     if (!a || !states || !grad_states || !grad_a || !grad_drive) return FIELDS_ERR_ARGUMENT;
     int rc = scan_check(workspace, workspace_bytes, B, L, C, a_batch, a_step, a_chan);
     if (rc) return rc;
-    const ScanShape s = make_scan_shape(B, L, C, a_batch, a_step, a_chan);
-    float* ws = static_cast<float*>(workspace);
-    const size_t plane = (size_t)B * s.NT * C;
-    ScanBwdParams p{a, states, state_in, grad_states, grad_state_out, grad_a, grad_drive,
-                    grad_state_in, ws, ws + plane, ws + 2 * plane, s};
-    const long long chunk_blocks = (scan_items(s) + kScanWarps - 1) / kScanWarps;
-    const long long chan_blocks =
-        ((long long)B * C + ScanCarryBwd::kThreads - 1) / ScanCarryBwd::kThreads;
-    rc = launch<ScanChunkMapBwd>(p, chunk_blocks, st);
-    if (!rc) rc = launch<ScanCarryBwd>(p, chan_blocks, st);
-    if (!rc) rc = launch<ScanEmitBwd>(p, chunk_blocks, st);
-    return rc;
+    ScanParams p{};
+    p.a = a; p.x = grad_states; p.states = states; p.first = state_in; p.last = grad_state_out;
+    p.out = grad_drive; p.grad_a = grad_a; p.end = grad_state_in;
+    p.s = make_scan_shape(B, L, C, a_batch, a_step, a_chan);
+    return run_scan<true>(p, static_cast<float*>(workspace), st);
 }
 
 int fields_read_selftest_wait(void* workspace, size_t workspace_bytes, unsigned max_polls,

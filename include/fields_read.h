@@ -237,7 +237,7 @@ int fields_read_step_bf16(const void *raw, const float *tr, const float *ti, con
  *   workspace    fields_scan_workspace_bytes(B, L, C) bytes, 16-byte aligned
  * Backward: grad_a is written densely [B, L, C] also for a broadcast `a` (the caller sums over
  * the broadcast dimension, as autograd does for an expanded tensor); states is the forward output.
- * Three launches each way (chunk maps, carries, states); results are bitwise reproducible.
+ * One launch each way; results are bitwise reproducible.
  */
 size_t fields_scan_workspace_bytes(int B, int L, int C);
 int fields_scan_forward(const float *a, long long a_batch, long long a_step, int a_chan,
