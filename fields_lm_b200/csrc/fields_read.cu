@@ -1771,9 +1771,16 @@ int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
     p.piece[5] = {w->w3, static_cast<uint16_t*>(w->w3_16), nullptr, D * H, (int)H};
     p.piece[6] = {nullptr, static_cast<uint16_t*>(w->in_b) + 3 * C, nullptr, D, (int)D};
     p.radius_logit = w->radius_logit; p.theta = w->theta; p.par = w->par; p.C = (int)C;
-    // as many blocks per piece as the GPU has SMs: the pieces run side by side
-    return launch_grid<LayoutParams>(layout_block, dim3(148, kLayoutPieces + 1), kRowThreads,
-                                     reinterpret_cast<Stream>(stream), p);
+    p.piece[7] = {nullptr, nullptr, nullptr, 0, 4};
+    long long at = 0;
+    for (int k = 0; k < kLayoutPieces; ++k) {
+        p.first[k] = at;
+        at += (p.piece[k].n + kLayoutChunk - 1) / kLayoutChunk;
+    }
+    p.first[kLayoutPieces] = at;
+    const long long blocks = at + (C + kRowThreads - 1) / kRowThreads;
+    if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+    return launch_on<LayoutParams>(layout_block, (unsigned)blocks, kRowThreads, 0, reinterpret_cast<Stream>(stream), p);
 }
 
 int fields_stack_step_norm(const void* raw, long long raw_stride, const float* par, float* state,
