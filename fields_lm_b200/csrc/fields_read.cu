@@ -18,6 +18,7 @@
 #include "field_epilogue.cuh"
 #include "field_rows.cuh"
 #include "field_mixer_grad.cuh"
+#include "field_step_gemm.cuh"
 
 #include "../../include/fields_read.h"
 
@@ -1984,6 +1985,121 @@ int fields_mixer_close_grad(const struct fields_mixer_grads* g, long long N, int
     p.g_radius = g->grad_radius; p.g_theta = g->grad_theta; p.C = C;
     return launch_on<FinishGradParams>(finish_grad, (unsigned)(first + (C + kRowThreads - 1) / kRowThreads), kRowThreads,
                                        0, st, p);
+}
+
+int fields_step_w12_rows(int hidden) { return hidden > 0 ? (hidden + 19) / 20 * 40 : 0; }
+
+static bool step_sizes(int D, int H) { return D > 0 && D % 16 == 0 && D <= 4096 && H > 0 && H % 8 == 0; }
+
+int fields_step_layout(const struct fields_step_weights* w, void* stream) {
+    if (!w || !w->write_w || !w->write_b || !w->gate_w || !w->gate_b || !w->w12 || !w->ff_norm_w || !w->in_w ||
+        !w->w12_w || !w->in_b)
+        return FIELDS_ERR_ARGUMENT;
+    if (!step_sizes(w->dim, w->hidden) || !aligned16(w->write_w) || !aligned16(w->gate_w) || !aligned16(w->w12) ||
+        !aligned16(w->ff_norm_w) || !aligned16(w->in_w) || !aligned16(w->w12_w))
+        return FIELDS_ERR_UNSUPPORTED;
+    const int D = w->dim, C = D / 2;
+    StepLayoutParams p{w->write_w, w->write_b, w->gate_w, w->gate_b, w->w12, w->ff_norm_w,
+                       static_cast<uint16_t*>(w->in_w), static_cast<uint16_t*>(w->w12_w), w->in_b, D, C, w->hidden};
+    return launch_on<StepLayoutParams>(step_layout, (unsigned)(5 * C + fields_step_w12_rows(w->hidden)), kRowThreads, 0,
+                                       reinterpret_cast<Stream>(stream), p);
+}
+
+}  // extern "C"
+
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's encoder of tensor maps, looked up once.
+static EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess || found != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<EncodeTiled>(f);
+    }();
+    return fn;
+}
+
+// A dense bfloat16 matrix [rows, cols] in boxes of 64 columns x box_rows rows with the 128-byte swizzle.
+static bool operand_map(CUtensorMap* map, const void* base, long long rows, int cols, int box_rows) {
+    const EncodeTiled encode = encode_tiled();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {kStepKBlock, (cuuint32_t)box_rows}, ones[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, ones,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One product of the step: A [M, K] activations, B [n_rows, K] weights, `slices` column slices.
+template <class Epi>
+static int launch_step(const void* a, const void* b, int n_rows, int K, int slices, StepBlockParams p, Stream st) {
+    using T = StepTile<Epi>;
+    p.k_blocks = (K + kStepKBlock - 1) / kStepKBlock;
+    p.tiles_n = (slices + Epi::kSlices - 1) / Epi::kSlices;
+    const int tiles = p.tiles_n * ((p.M + kStepRows - 1) / kStepRows);
+    // K over as many blocks as share the GPU in one round, every one of them with a part of K
+    p.S = 1;
+    for (int S = 2; S <= Epi::kSlices && tiles * S <= 148; S *= 2)
+        if ((S - 1) * ((p.k_blocks + S - 1) / S) < p.k_blocks) p.S = S;
+    CUtensorMap a_map, b_map;
+    if (!operand_map(&a_map, a, p.M, K, kStepRows) || !operand_map(&b_map, b, n_rows, K, T::kNT))
+        return FIELDS_ERR_UNSUPPORTED;
+    static bool ready[64] = {};
+    const int rc = allow_shared_memory(step_gemm<Epi>, T::kSmemBytes, ready);
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * p.S));
+    cfg.blockDim = dim3(kStepThreads);
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (dependent_launch_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.S > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)p.S;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return check_cuda(cudaLaunchKernelEx(&cfg, step_gemm<Epi>, a_map, b_map, p));
+}
+
+extern "C" {
+
+int fields_step_block(const struct fields_step_args* g, void* stream) {
+    if (!g || g->rows < 0) return FIELDS_ERR_ARGUMENT;
+    if (g->rows == 0) return FIELDS_OK;
+    const void* all[] = {g->x, g->state, g->y, g->xb, g->yb, g->read, g->gate, g->act, g->read_sq, g->y_sq, g->in_w,
+                         g->out_w16, g->w12_w, g->w3_16, g->in_b, g->par, g->out_b};
+    for (const void* q : all)
+        if (!q) return FIELDS_ERR_ARGUMENT;
+    if (!step_sizes(g->dim, g->hidden) || g->rows > 512) return FIELDS_ERR_UNSUPPORTED;
+    for (const void* q : all)
+        if (!aligned16(q)) return FIELDS_ERR_UNSUPPORTED;
+    const int D = g->dim, C = D / 2, H = g->hidden;
+    auto h = [](void* q) { return static_cast<uint16_t*>(q); };
+    StepBlockParams p{};
+    p.x = g->x; p.gate = h(g->gate); p.read = h(g->read); p.state = g->state; p.y = g->y; p.yb = h(g->yb);
+    p.act = h(g->act); p.out = g->y; p.xb = h(g->xb); p.read_sq = g->read_sq; p.y_sq = g->y_sq;
+    p.in_b = g->in_b; p.par = g->par; p.out_b = g->out_b;
+    p.read_eps = g->read_eps; p.ff_eps = g->ff_eps; p.M = g->rows; p.D = D; p.C = C; p.H = H;
+    Stream st = reinterpret_cast<Stream>(stream);
+    int rc = launch_step<EpiIn>(g->xb, g->in_w, 5 * C, D, C / 8, p, st);
+    if (!rc) rc = launch_step<EpiOut>(g->read, g->out_w16, D, 2 * D, D / 8, p, st);
+    if (!rc) rc = launch_step<EpiUv>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st);
+    if (!rc) rc = launch_step<EpiFf>(g->act, g->w3_16, D, H, D / 8, p, st);
+    return rc;
 }
 #endif  // FIELDS_HOST_EMU
 

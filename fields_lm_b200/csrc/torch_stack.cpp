@@ -32,6 +32,8 @@ struct Block {
     double read_eps = 0, ff_eps = 0;
     // bfloat16, transposed views for the products; `in` = write over gate, scaled `out`
     Tensor in_w, in_b, in_t, out_t, w12_t, w3_t, par;
+    // rows of `in` and w12 in the order of the fused step, its biases (made by the first step after a layout)
+    Tensor step_in, step_w12, step_b;
     float* f(int i) const { return fp(src[i].t); }
 };
 
@@ -104,6 +106,7 @@ class FieldStack {
             if (tail_.size() > 2) head_b_ = tail_[2].t.detach().to(at::kBFloat16);
         }
         laid_out_ = true;
+        step_laid_out_ = false;
     }
 
     // x [B, L, D] fp32 -> the stack's output [B, L, D] and every block's end state [B, D].
@@ -148,45 +151,38 @@ class FieldStack {
     // One token per row: x [B, D] fp32; states advance in place. Returns the logits where the tail (final
     // norm and head) is part of the plan, else the stack's output.
     Tensor step(const Tensor& x_, const std::vector<Tensor>& states) {
-        const Api& f = api();
-        const Tensor x = dense(x_);
-        const int64_t N = x.size(0), D = D_, C = D / 2, W = 3 * C + D;
+        Tensor x = dense(x_);
+        const int64_t N = x.size(0), D = D_;
         TORCH_CHECK_VALUE(states.size() == blocks_.size(), "one state per block is needed");
-        for (const Tensor& s : states)
+        std::vector<Tensor> own = states;  // 16-byte aligned: a caller's may be any view
+        bool aligned = true;
+        for (const Tensor& s : states) {
             TORCH_CHECK_VALUE(s.is_cuda() && s.scalar_type() == at::kFloat && s.is_contiguous() && s.dim() == 2 &&
                                   s.size(0) == N && s.size(1) == D,
                               shape(s));
-        const c10::Device dev = x.device();
-        const c10::cuda::CUDAGuard guard(dev);
-        void* st = stream_of(x);
-        const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({N, D}, at::kFloat, dev),
-                     read = empty({N, 4 * C}, at::kBFloat16, dev);
-        Tensor acc = empty({N, D}, at::kBFloat16, dev), in = empty({N, W}, at::kBFloat16, dev),
-               uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev);
-        check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, st),
-              "fields_stack_close_ff");
-        const float* from = fp(x);
-        for (size_t i = 0; i < blocks_.size(); ++i) {
-            const Block& b = blocks_[i];
-            at::cuda::addmm_out(in, b.in_b, xb, b.in_t, 1, 1);
-            check(f.fields_stack_step_norm(vp(in), W, fp(b.par), fp(states[i]), vp(read), (float)b.read_eps, N,
-                                           (int)C, st),
-                  "fields_stack_step_norm");
-            at::cuda::mm_out(acc, read, b.out_t);
-            const void* gate = static_cast<at::BFloat16*>(vp(in)) + 3 * C;
-            check(f.fields_stack_close_mixer(from, vp(acc), gate, W, nullptr, 0, b.f(Block::kOutB),
-                                             b.f(Block::kGateB), b.f(Block::kFfNorm), fp(y), vp(xb), 0.0f, 1,
-                                             (float)b.ff_eps, N, D_, st),
-                  "fields_stack_close_mixer");
-            feed_forward(b, xb, uv, act, acc, N, st);
-            const bool last = i + 1 == blocks_.size();
-            const float* norm = last && !tail_.empty() ? fp(tail_[0].t) : nullptr;
-            check(f.fields_stack_close_ff(fp(y), vp(acc), norm, fp(y), vp(xb), (float)tail_eps_, N, D_, st),
-                  "fields_stack_close_ff");
-            from = fp(y);
+            aligned = aligned && reinterpret_cast<uintptr_t>(s.data_ptr()) % 16 == 0;
         }
+        const c10::cuda::CUDAGuard guard(x.device());
+        if (!aligned)
+            for (Tensor& s : own) s = s.clone();
+        if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16) x = x.clone();
+        // Four launches per block while its products have tiles (128 rows x 64 features) few enough that K
+        // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 708 us at 16 rows and 675 at 256
+        // against 763 and 768 with library products, but 986 against 787 at 384.
+        const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
+        if (fused && !step_laid_out_) step_layout(stream_of(x));
+        const Tensor xb = empty({N, D}, at::kBFloat16, x.device()), y = empty({N, D}, at::kFloat, x.device());
+        check(api().fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, stream_of(x)),
+              "fields_stack_close_ff");
+        if (fused) step_fused(x, own, xb, y);
+        else step_products(x, own, xb, y);
+        if (!aligned)
+            for (size_t i = 0; i < states.size(); ++i) states[i].copy_(own[i]);
         if (tail_.empty()) return y;
-        Tensor logits = empty({N, head_w_.size(1)}, at::kBFloat16, dev);
+        check(api().fields_stack_close_ff(fp(y), nullptr, fp(tail_[0].t), nullptr, vp(xb), (float)tail_eps_, N, D_,
+                                          stream_of(x)),
+              "fields_stack_close_ff");
+        Tensor logits = empty({N, head_w_.size(1)}, at::kBFloat16, x.device());
         if (head_b_.defined()) at::cuda::addmm_out(logits, head_b_, xb, head_w_, 1, 1);
         else at::cuda::mm_out(logits, xb, head_w_);
         return logits;
@@ -203,6 +199,81 @@ class FieldStack {
         return true;
     }
 
+    // Weights in the order of the fused step. Its first kernel reads them before it waits for the kernel
+    // ahead of it, so a kernel that waits for this one has to stand between the two (step()'s copy of x).
+    void step_layout(void* st) {
+        const Api& f = api();
+        const int64_t D = D_, C = D / 2;
+        const c10::Device dev = blocks_[0].in_w.device();
+        for (Block& b : blocks_) {
+            if (!b.step_in.defined()) {
+                b.step_in = empty({5 * C, D}, at::kBFloat16, dev);
+                b.step_w12 = empty({f.fields_step_w12_rows(H_), D}, at::kBFloat16, dev);
+                b.step_b = empty({5 * C}, at::kFloat, dev);
+            }
+            fields_step_weights w{};
+            w.write_w = b.f(Block::kWriteW); w.write_b = b.f(Block::kWriteB); w.gate_w = b.f(Block::kGateW);
+            w.gate_b = b.f(Block::kGateB); w.w12 = b.f(Block::kW12); w.ff_norm_w = b.f(Block::kFfNorm);
+            w.in_w = vp(b.step_in); w.w12_w = vp(b.step_w12); w.in_b = fp(b.step_b);
+            w.dim = D_; w.hidden = H_;
+            check(f.fields_step_layout(&w, st), "fields_step_layout");
+        }
+        step_laid_out_ = true;
+    }
+
+    // The blocks of a step, each a chain of four products with fused epilogues (field_step_gemm.cuh).
+    void step_fused(const Tensor& x, const std::vector<Tensor>& states, const Tensor& xb, const Tensor& y) {
+        const Api& f = api();
+        const int64_t N = x.size(0), D = D_, C = D / 2, H = H_;
+        const c10::Device dev = x.device();
+        void* st = stream_of(x);
+        const Tensor yb = empty({N, D}, at::kBFloat16, dev), read = empty({N, 4 * C}, at::kBFloat16, dev),
+                     gate = empty({N, D}, at::kBFloat16, dev), act = empty({N, H}, at::kBFloat16, dev),
+                     read_sq = empty({C / 8, N}, at::kFloat, dev), y_sq = empty({D / 8, N}, at::kFloat, dev);
+        fields_step_args g{};
+        g.x = fp(x); g.y = fp(y); g.xb = vp(xb); g.yb = vp(yb); g.read = vp(read); g.gate = vp(gate); g.act = vp(act);
+        g.read_sq = fp(read_sq); g.y_sq = fp(y_sq);
+        g.rows = (int)N; g.dim = D_; g.hidden = H_;
+        for (size_t i = 0; i < blocks_.size(); ++i) {
+            const Block& b = blocks_[i];
+            g.state = fp(states[i]);
+            g.in_w = vp(b.step_in); g.out_w16 = vp(b.out_t); g.w12_w = vp(b.step_w12); g.w3_16 = vp(b.w3_t);
+            g.in_b = fp(b.step_b); g.par = fp(b.par); g.out_b = b.f(Block::kOutB);
+            g.read_eps = (float)b.read_eps; g.ff_eps = (float)b.ff_eps;
+            check(f.fields_step_block(&g, st), "fields_step_block");
+            g.x = g.y;
+        }
+    }
+
+    // The same with library products, for what the fused step does not take.
+    void step_products(const Tensor& x, const std::vector<Tensor>& states, const Tensor& xb, const Tensor& y) {
+        const Api& f = api();
+        const int64_t N = x.size(0), D = D_, C = D / 2, W = 3 * C + D;
+        const c10::Device dev = x.device();
+        void* st = stream_of(x);
+        const Tensor read = empty({N, 4 * C}, at::kBFloat16, dev);
+        Tensor acc = empty({N, D}, at::kBFloat16, dev), in = empty({N, W}, at::kBFloat16, dev),
+               uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev);
+        const float* from = fp(x);
+        for (size_t i = 0; i < blocks_.size(); ++i) {
+            const Block& b = blocks_[i];
+            at::cuda::addmm_out(in, b.in_b, xb, b.in_t, 1, 1);
+            check(f.fields_stack_step_norm(vp(in), W, fp(b.par), fp(states[i]), vp(read), (float)b.read_eps, N,
+                                           (int)C, st),
+                  "fields_stack_step_norm");
+            at::cuda::mm_out(acc, read, b.out_t);
+            const void* gate = static_cast<at::BFloat16*>(vp(in)) + 3 * C;
+            check(f.fields_stack_close_mixer(from, vp(acc), gate, W, nullptr, 0, b.f(Block::kOutB),
+                                             b.f(Block::kGateB), b.f(Block::kFfNorm), fp(y), vp(xb), 0.0f, 1,
+                                             (float)b.ff_eps, N, D_, st),
+                  "fields_stack_close_mixer");
+            feed_forward(b, xb, uv, act, acc, N, st);
+            check(f.fields_stack_close_ff(fp(y), vp(acc), nullptr, fp(y), vp(xb), 0.0f, N, D_, st),
+                  "fields_stack_close_ff");
+            from = fp(y);
+        }
+    }
+
     void feed_forward(const Block& b, const Tensor& h, Tensor& uv, Tensor& act, Tensor& out, int64_t N, void* st) {
         at::cuda::mm_out(uv, h, b.w12_t);
         check(api().fields_stack_swiglu(vp(uv), vp(act), N, H_, st), "fields_stack_swiglu");
@@ -216,7 +287,7 @@ class FieldStack {
     Tensor head_w_, head_b_;
     double tail_eps_;
     int D_ = 0, H_ = 0;
-    bool laid_out_ = false;
+    bool laid_out_ = false, step_laid_out_ = false;
 };
 
 void add_stack(PyObject* module) {

@@ -494,6 +494,38 @@ int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, fl
                           float norm_eps, long long N, int D, void *stream);
 
 /*
+ * The single-token step of a block as four launches, each a tensor-core product whose epilogue goes on to
+ * the operand of the next (D = dim, C = D / 2, H = hidden; D % 16 == 0, D <= 4096, H % 8 == 0, up to
+ * 512 rows; tensors dense and 16-byte aligned; FIELDS_ERR_UNSUPPORTED otherwise).
+ *
+ * fields_step_layout: the rows of [write | gate] and of w12 diag(ff_norm) in the column order of the
+ *   products: in_w [5C, D] and w12_w [fields_step_w12_rows(H), D] bfloat16, in_b [5C].
+ * fields_step_block: x [M, D] in (the block's input; xb its bfloat16 copy), y [M, D] out (may be x) and
+ *   xb its copy; state [M, 2C] advances in place. out_w16, w3_16 and par as fields_stack_layout leaves
+ *   them. Scratch: yb [M, D], read [M, 4C], gate [M, D], act [M, H] bfloat16, read_sq [C / 8, M],
+ *   y_sq [D / 8, M].
+ */
+struct fields_step_weights {
+    const float *write_w, *write_b, *gate_w, *gate_b, *w12, *ff_norm_w;
+    void *in_w, *w12_w;
+    float *in_b;
+    int dim, hidden;
+};
+struct fields_step_args {
+    const float *x;
+    float *state, *y;
+    void *xb, *yb, *read, *gate, *act;
+    float *read_sq, *y_sq;
+    const void *in_w, *out_w16, *w12_w, *w3_16;
+    const float *in_b, *par, *out_b;
+    float read_eps, ff_eps;
+    int rows, dim, hidden;
+};
+int fields_step_w12_rows(int hidden);
+int fields_step_layout(const struct fields_step_weights *weights, void *stream);
+int fields_step_block(const struct fields_step_args *args, void *stream);
+
+/*
  * fields_read_forward_bf16(_stats) and fields_read_backward_bf16 on rows that lie raw_pitch (and
  * grad_pitch) elements apart, as columns of a wider matrix: raw and gate of a mixer are one product.
  * Pitches are multiples of 4; sumsq may be NULL.

@@ -40,8 +40,12 @@ def _run(model, tokens, prefix, native):
 
 
 # one block's rounding differences grow by at most their sum over the blocks: BF16_TOL holds for three
+# (fused step: rows around one tile of 128 and its limit of 512, widths that leave part of a column
+# tile, K shorter than the split; 200 and 1032 are widths it does not take)
 @pytest.mark.parametrize("dim,hidden,B,L", [(64, 8, 1, 1), (64, 40, 5, 3), (200, 96, 3, 37), (1024, 2528, 2, 64),
-                                            (1024, 704, 601, 8), (1032, 352, 4, 5), (4096, 64, 2, 6)])
+                                            (1024, 704, 601, 8), (1032, 352, 4, 5), (4096, 64, 2, 6),
+                                            (1024, 2528, 129, 2), (512, 1344, 512, 2), (16, 24, 127, 2),
+                                            (272, 360, 128, 3), (256, 704, 256, 2)])
 def test_native_stack_matches_the_modules(dim, hidden, B, L):
     torch.manual_seed(dim + B)
     model = LM(dim, 3, hidden, bias=dim == 200).cuda()
@@ -56,6 +60,21 @@ def test_native_stack_matches_the_modules(dim, hidden, B, L):
         assert _rel(a, b) < BF16_TOL
     for a, b in zip(dec.states, ref.states):
         assert a.dtype == torch.float32 and _rel(a, b) < BF16_TOL
+
+
+def test_step_on_states_that_are_not_aligned():
+    torch.manual_seed(2)
+    model = LM(64, 2, 32).cuda()
+    tokens = torch.randint(0, 97, (3, 6), device="cuda")
+    _, dec = _run(model, tokens, 6, True)
+    odd = []
+    for s in dec.states:
+        odd.append(torch.zeros(s.numel() + 1, device="cuda")[1:].view_as(s).copy_(s))
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = dec.step(tokens[:, 0])
+        after, dec.states = dec.states, odd
+        assert torch.equal(dec.step(tokens[:, 0]), want)
+    assert all(torch.equal(a, b) for a, b in zip(after, odd))
 
 
 def test_native_stack_follows_the_model():
