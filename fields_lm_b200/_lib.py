@@ -22,6 +22,7 @@ SYMBOLS = {
     "fields_status_string": (ctypes.c_char_p, [_I]),
     "fields_read_version": (_I, []),
     "fields_last_cuda_error": (ctypes.c_char_p, []),
+    "fields_read_use_kept": (_I, [_P]),
     "fields_read_workspace_bytes": (_SZ, [_I, _I, _I, _I]),
     "fields_read_forward": (_I, [_P] * 8 + [_SZ, _I, _I, _I, _P]),
     "fields_read_backward": (_I, [_P] * 14 + [_SZ, _I, _I, _I, _P]),

@@ -31,6 +31,10 @@
 
 namespace fields {
 
+#ifdef FIELDS_HOST_EMU
+struct uint4;
+#endif
+
 constexpr int kCtrlHeader = 64;  // unsigned words before the slots: [0] error word
 constexpr int kGroup = 128;      // channels per tile
 
@@ -41,6 +45,8 @@ struct SpShape {
     int prefetch;  // non-zero: blocks warm L2 with the inputs of the tile that many positions ahead
     unsigned max_polls;  // bound of every wait for another block's publication
     int ticket;    // non-zero: blocks take their tile from a counter in the workspace header
+    uint4* clean;       // memory that this launch fills with the unset pattern for the next one (kept workspaces)
+    unsigned clean_n;   // 16-byte words of it
     int zp, gp;    // elements from one row of raw to the next, and of grad_raw (3C where they are dense)
 };
 
@@ -164,6 +170,8 @@ struct FwdSinglePass {
         prefetch_rows(p.raw + ((size_t)nx.b * s.L + t0) * s.zp + nx.cg * kGroup, kTile, s.L - t0, 3,
                       (size_t)s.zp, (size_t)s.C, s.C - nx.cg * kGroup, thread, kThreads);
     }
+
+    FL_HD static void finish(const Params&, int, int, float*) {}
 
     template <int PH>
     FL_HD static void phase(const Params& p, int block, int thread, float* smem, State& st) {
@@ -388,6 +396,8 @@ struct FwdTwoSweep {
     }
 
     FL_HD static void prefetch(const Params&, int, int) {}
+
+    FL_HD static void finish(const Params&, int, int, float*) {}
 
     template <int PH>
     FL_HD static void phase(const Params& p, int block, int thread, float* smem, State&) {
@@ -660,16 +670,56 @@ struct SpBwdParamsT {
     float* grad_state_in;         // [B, 2C] or null
     float* agg;                   // [tiles][128][4]
     float* incl;                  // [tiles][128][2]
-    unsigned* ctrl;               // error word
+    unsigned* ctrl;               // error word; from word 2 one counter per channel group
     float* partial;               // [3][B][NT][C]
     SpShape s;
     // Optional replacement for `read` in the kernels that recompute the states: row j holds the
     // state after step kStateRowEvery * (j + 1) - 1, [B, state_rows, 2C] fp32. Null: use `read`.
     const float* states = nullptr;
     int state_rows = 0;
+    // Few tiles: the last block of a channel group to finish adds its partial rows (null: BwdReduce does).
+    float* grad_par[3] = {nullptr, nullptr, nullptr};
 };
 using SpBwdParams = SpBwdParamsT<float>;
 constexpr int kStateRowEvery = 8;
+
+// The end of a block of a backward kernel where the reduction is folded in: the last block of a channel
+// group to get here (a counter in the workspace header, back at its first value when that block is done)
+// adds the group's partial rows in order, in double like BwdReduce.
+template <typename IO>
+FL_HD void fold_partial_rows(const SpBwdParamsT<IO>& p, int cg, int thread, int* last) {
+#if FL_DEVICE_CODE
+    const SpShape& s = p.s;
+    const int rows = s.B * s.NT;
+    __threadfence();
+    __syncthreads();
+    if (thread == 0) *last = atomicAdd(p.ctrl + 2 + cg, 1u) + 2u == (unsigned)rows;  // the first gets 0xFFFFFFFF
+    __syncthreads();
+    if (!*last) return;
+    if (thread == 0) p.ctrl[2 + cg] = kUnsetBits;
+    __threadfence();
+    const int ch = cg * kGroup + thread;
+    if (thread >= kGroup || ch >= s.C) return;
+    double acc[3] = {0.0, 0.0, 0.0};
+    const size_t plane = (size_t)rows * s.C;
+    for (int r = 0; r < rows; r += 8) {
+        float v[8][3];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                v[j][k] = r + j < rows ? __ldcg(p.partial + k * plane + (size_t)(r + j) * s.C + ch) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[k] += (double)v[j][k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) p.grad_par[k][ch] = (float)acc[k];
+#else
+    (void)p; (void)cg; (void)thread; (void)last;
+#endif
+}
 
 template <int TS, int WARPS, int U1_, int U2_, int MIN_BLOCKS, bool ASYNC = false, int STAGES = 2,
           typename IO = float>
@@ -717,6 +767,10 @@ struct BwdSinglePass {
                       s.L - t_lo, 1, (size_t)3 * s.C, (size_t)s.C, width, thread, kThreads);
         prefetch_rows(p.grad_read + ((size_t)nx.b * s.L + t_lo) * 4 * s.C + nx.cg * kGroup, kTile,
                       s.L - t_lo, 4, (size_t)4 * s.C, (size_t)s.C, width, thread, kThreads);
+    }
+
+    FL_HD static void finish(const Params& p, int block, int thread, float* smem) {
+        if (p.grad_par[0]) fold_partial_rows(p, sp_decode(p.s, (unsigned)block).cg, thread, reinterpret_cast<int*>(carry_at(smem, 0, 0)));
     }
 
     template <int PH>
@@ -1072,6 +1126,10 @@ struct BwdRecompute {
         async_copy4(cell_at(smem, stage, u * 7 + 6, thread), grow + 3 * C);
     }
 
+    FL_HD static void finish(const Params& p, int block, int thread, float* smem) {
+        if (p.grad_par[0]) fold_partial_rows(p, sp_decode(p.s, (unsigned)block).cg, thread, reinterpret_cast<int*>(carry_at(smem, 0, 0)));
+    }
+
     template <int PH>
     FL_HD static void phase(const Params& p, int block, int thread, float* smem, State&) {
         const SpShape& s = p.s;
@@ -1322,6 +1380,10 @@ struct BwdTileResident {
         return smem + kSumFloats + kCarryFloats + ((size_t)(j * 7 + q) * kThreads + thread) * 4;
     }
     FL_HD static void prefetch(const Params&, int, int) {}
+
+    FL_HD static void finish(const Params& p, int block, int thread, float* smem) {
+        if (p.grad_par[0]) fold_partial_rows(p, sp_decode(p.s, (unsigned)block).cg, thread, reinterpret_cast<int*>(carry_at(smem, 0, 0)));
+    }
 
     template <int PH>
     FL_HD static void phase(const Params& p, int block, int thread, float* smem, State& st) {

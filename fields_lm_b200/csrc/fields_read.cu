@@ -75,7 +75,7 @@ static void emu_phase_range(const typename K::Params& p, int block, float* smem,
 // order meets an inclusive state at the first step back.
 template <class K>
 static int launch_stateful(const typename K::Params& p, long long grid, long long first_wave,
-                           Stream) {
+                           Stream, bool = false) {
     std::vector<double> smem_store((size_t)grid * (K::kSmemFloats / 2 + 1));
     std::vector<typename K::State> states((size_t)grid * K::kThreads);
     auto smem_of = [&](long long b) {
@@ -271,7 +271,10 @@ __device__ __forceinline__ void run_phases(const typename K::Params& p, int tile
 // sits at the head of every tile: measured +9.5 % on the forward, +3.7 % on the fp32 step and
 // +10 % on the bfloat16 step at 8 x 2,048 tokens, which is why it is off in the product and
 // selectable (FIELDS_TILE_TICKET=1) only in the test build, where the GPU tests run it.
-template <class K>
+// EXTRA: the block also does its share of cleaning a kept workspace, and the last block of a channel group folds
+// the partial rows. A second instantiation, because the code costs registers (the bfloat16 backward lost
+// its fourth block per SM to it: 55.6 -> 61.1 us at 8 x 2,048).
+template <class K, bool EXTRA = false>
 __global__ void __launch_bounds__(K::kThreads, K::kMinBlocks) stateful_entry(const typename K::Params p) {
     extern __shared__ __align__(16) float smem[];
     typename K::State st;
@@ -285,6 +288,7 @@ __global__ void __launch_bounds__(K::kThreads, K::kMinBlocks) stateful_entry(con
         if (threadIdx.x == 0) *ticket = (int)(atomicAdd(p.ctrl + 1, 1u) + 1u);
         __syncthreads();
         tile = *ticket;
+        if ((unsigned)tile >= gridDim.x) return;  // (one ticket per block: only a stale counter gets here)
     }
 #endif
     run_phases<K, 0, K::kClaimAfter>(p, tile, smem, st);
@@ -294,6 +298,11 @@ __global__ void __launch_bounds__(K::kThreads, K::kMinBlocks) stateful_entry(con
         if (next < (long long)p.s.B * p.s.G * p.s.NT) K::prefetch(p, (int)next, (int)threadIdx.x);
     }
     run_phases<K, K::kClaimAfter + 1, K::kPhases - 1>(p, tile, smem, st);
+    if constexpr (EXTRA) {
+        for (unsigned i = blockIdx.x * K::kThreads + threadIdx.x; i < p.s.clean_n; i += gridDim.x * K::kThreads)
+            p.s.clean[i] = make_uint4(kUnsetBits, kUnsetBits, kUnsetBits, kUnsetBits);
+        K::finish(p, tile, (int)threadIdx.x, smem);
+    }
 }
 
 // Kernels that need more than the default 48 KB of dynamic shared memory opt in once per device.
@@ -319,14 +328,15 @@ static int allow_shared_memory(Fn fn, size_t bytes, bool* ready) {
 
 // (the third argument, the number of chains, only matters to the host emulation)
 template <class K>
-static int launch_stateful(const typename K::Params& p, long long tiles, long long, Stream st) {
+static int launch_stateful(const typename K::Params& p, long long tiles, long long, Stream st, bool extra = false) {
     if (tiles <= 0) return FIELDS_OK;
     if (tiles > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
     constexpr size_t bytes = K::kSmemFloats * sizeof(float);
-    static bool ready[64] = {};
-    const int rc = allow_shared_memory(stateful_entry<K>, bytes, ready);
+    static bool ready[2][64] = {};
+    const auto fn = extra ? stateful_entry<K, true> : stateful_entry<K, false>;
+    const int rc = allow_shared_memory(fn, bytes, ready[extra]);
     if (rc) return rc;
-    return launch_on<typename K::Params>(stateful_entry<K>, (unsigned)tiles, K::kThreads, bytes, st, p);
+    return launch_on<typename K::Params>(fn, (unsigned)tiles, K::kThreads, bytes, st, p);
 }
 
 // Fills with the "not yet written" pattern. A kernel rather than a memset, so that it takes part
@@ -366,7 +376,7 @@ static int resident_blocks() {
     std::lock_guard<std::mutex> lock(mu);
     if (cached[dev] > 0) return cached[dev];
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stateful_entry<K>, K::kThreads,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stateful_entry<K, false>, K::kThreads,
                                                       K::kSmemFloats * sizeof(float)) != cudaSuccess)
         return 0;
     cached[dev] = per_sm * sms;
@@ -660,7 +670,7 @@ template <bool STATS> using FwdSpBf16Deep = FwdSinglePass<10, 8, 2, uint16_t, ST
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
 // 16-byte cells) on 8 x 2,048 tokens.
 using BwdSpBf16 = BwdSinglePass<16, 4, 2, 1, 3, true, 3, uint16_t>;
-constexpr int kSpMinTile = 24;     // smallest time tile of any forward instantiation above (workspace bound)
+constexpr int kSpMinTile = 32;     // smallest time tile of any forward instantiation above (workspace bound)
 constexpr int kSpMinTileBwd = 16;  // same for the backward
 
 #ifdef FIELDS_ALL_VARIANTS
@@ -683,6 +693,58 @@ static int prefetch_from_env(int resident) {
 static int prefetch_from_env(int) { return 0; }
 #endif
 
+// The calling thread's next pass runs on a kept workspace (fields_read_use_kept); null: the workspace holds
+// anything and is filled first.
+static thread_local fields_kept* g_next_kept = nullptr;
+
+struct ReadyWorkspace {
+    unsigned* ctrl;
+    float *agg, *incl, *partial;
+};
+
+// Makes a workspace ready for a pass of the single-pass kernels.
+static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspace* out) {
+    char* ws = static_cast<char*>(workspace);
+    fields_kept* k = g_next_kept;
+    g_next_kept = nullptr;
+    char* slots = ws + pl.agg_off;
+    const size_t slot_bytes = pl.bytes - pl.agg_off;
+    out->ctrl = reinterpret_cast<unsigned*>(ws);
+    out->partial = reinterpret_cast<float*>(ws + pl.bytes);
+    int rc = FIELDS_OK;
+    if (k) {
+        // A small pass publishes in one half, which is unset, and fills what was used of the other. Up to
+        // 1,024 tiles: there the fill launch shows, in host time above all (20.1 -> 19.2 us of GPU at
+        // 2 x 3,001 x 384, 13.6 -> 12.7 at 1 x 2,048 x 512); above, the code in the kernel costs as much.
+        if (slot_bytes > k->half_bytes) return FIELDS_ERR_WORKSPACE;
+        const unsigned h = k->parity & 1;
+        char* half[2] = {ws + pl.agg_off, ws + pl.agg_off + k->half_bytes};
+        slots = half[h];
+        out->partial = reinterpret_cast<float*>(half[1] + k->half_bytes);
+        const size_t used = k->dirty[1 - h];
+        if (pl.tiles <= 1024 && k->dirty[h] == 0) {
+            if (used > (size_t)pl.tiles * 16384) {  // a much larger pass was before: too much for these blocks
+                rc = fill_unset(half[1 - h], used, st);
+            } else {
+                pl.s.clean = reinterpret_cast<uint4*>(half[1 - h]);
+                pl.s.clean_n = (unsigned)(used / 16);
+            }
+            k->dirty[1 - h] = 0;
+            k->dirty[h] = slot_bytes;
+            k->parity = 1 - h;
+        } else {
+            rc = fill_unset(slots, slot_bytes, st);
+            if (k->dirty[h] < slot_bytes) k->dirty[h] = slot_bytes;
+            if (used == 0) k->parity = 1 - h;
+        }
+    } else {
+        rc = fill_unset(ws, pl.bytes, st);  // error word, counters and every publication slot
+    }
+    out->agg = reinterpret_cast<float*>(slots);
+    out->incl = reinterpret_cast<float*>(slots + (pl.incl_off - pl.agg_off));
+    return rc;
+}
+
 template <class K, typename IO = float>
 static int run_forward_single_pass(const IO* raw, const float* tr, const float* ti,
                                    const float* gamma, const float* state_in, IO* read,
@@ -691,15 +753,12 @@ static int run_forward_single_pass(const IO* raw, const float* tr, const float* 
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (pitch) pl.s.zp = (int)pitch;
-    char* ws = static_cast<char*>(workspace);
-    unsigned* ctrl = reinterpret_cast<unsigned*>(ws);
-    int rc = fill_unset(ws, pl.bytes, st);  // error word and every publication slot
+    ReadyWorkspace ws;
+    const int rc = ready_workspace(workspace, pl, st, &ws);
     if (rc) return rc;
-    SpFwdParamsT<IO> p{raw, tr, ti, gamma, state_in, read, state_out,
-                       reinterpret_cast<float*>(ws + pl.agg_off),
-                       reinterpret_cast<float*>(ws + pl.incl_off), ctrl, pl.s};
+    SpFwdParamsT<IO> p{raw, tr, ti, gamma, state_in, read, state_out, ws.agg, ws.incl, ws.ctrl, pl.s};
     p.sumsq = sumsq;
-    return launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st);
+    return launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st, pl.s.clean_n > 0);
 }
 
 template <class K, typename IO = float>
@@ -715,20 +774,24 @@ static int run_backward_single_pass(const IO* raw, const float* tr, const float*
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (raw_pitch) pl.s.zp = (int)raw_pitch;
     if (grad_pitch) pl.s.gp = (int)grad_pitch;
-    char* ws = static_cast<char*>(workspace);
-    unsigned* ctrl = reinterpret_cast<unsigned*>(ws);
-    int rc = fill_unset(ws, pl.bytes, st);
+    ReadyWorkspace ws;
+    int rc = ready_workspace(workspace, pl, st, &ws);
     if (rc) return rc;
-    float* partial = reinterpret_cast<float*>(ws + pl.bytes);
     SpBwdParamsT<IO> p{raw, tr, ti, gamma, state_in, read, grad_read, grad_state_out, grad_raw,
-                       grad_state_in, reinterpret_cast<float*>(ws + pl.agg_off),
-                       reinterpret_cast<float*>(ws + pl.incl_off), ctrl, partial, pl.s};
+                       grad_state_in, ws.agg, ws.incl, ws.ctrl, ws.partial, pl.s};
     p.states = states;
     p.state_rows = L / kStateRowEvery;
-    rc = launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st);
-    if (rc) return rc;
+#ifndef FIELDS_HOST_EMU
+    // Up to 16 partial rows the last block of a channel group adds them: a launch less, 2.5 us of GPU and as
+    // much of host time. (At 64 rows that block took 5 us longer than the reduction kernel.)
+    if ((long long)B * pl.s.NT <= 16 && pl.s.G <= kCtrlHeader - 2) {
+        p.grad_par[0] = grad_tr; p.grad_par[1] = grad_ti; p.grad_par[2] = grad_gamma;
+    }
+#endif
+    rc = launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st, pl.s.clean_n > 0 || p.grad_par[0]);
+    if (rc || p.grad_par[0]) return rc;
     BwdParams rp{};
-    rp.partial = partial;
+    rp.partial = ws.partial;
     rp.grad_tr = grad_tr; rp.grad_ti = grad_ti; rp.grad_gamma = grad_gamma;
     rp.s = Shape{B, L, C, K::kTile, pl.s.NT, pl.s.G};
     return launch<BwdReduce>(rp, 3LL * ((C + 31) / 32), st);
@@ -881,6 +944,19 @@ const char* fields_status_string(int status) {
 int fields_read_version(void) { return 100; }
 
 const char* fields_last_cuda_error(void) { return g_last_error; }
+
+int fields_read_use_kept(struct fields_kept* kept) {
+    if (kept && (kept->half_bytes % 256 || kept->half_bytes > ((size_t)1 << 32))) return FIELDS_ERR_ARGUMENT;
+#ifdef FIELDS_HOST_EMU
+    if (kept) return FIELDS_ERR_UNSUPPORTED;
+#endif
+    // (the test build's other kernel families use a workspace as plain scratch, and its ticket counter
+    // starts from the fill)
+    if (kept && ((algo_from_env() != kAlgoAuto && algo_from_env() != kAlgoSinglePass) || tile_ticket_from_env()))
+        return FIELDS_ERR_UNSUPPORTED;
+    g_next_kept = kept;
+    return FIELDS_OK;
+}
 
 size_t fields_read_workspace_bytes(int B, int L, int C, int pass) {
     if (B <= 0 || L <= 0 || C <= 0) return 0;

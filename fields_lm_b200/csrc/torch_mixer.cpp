@@ -59,10 +59,10 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         const Tensor read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
-            const Tensor ws = workspace(n, dev);
+            PassWorkspace ws(n, u, true);
             float* p = fp(par);
-            check(f.fields_read_forward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, nullptr, vp(read), fp(groups), nullptr,
-                                                  vp(ws), n, (int)B, (int)L, (int)C, st),
+            ws.check(f.fields_read_forward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, nullptr, vp(read), fp(groups), nullptr,
+                                                  ws.ptr(), n, (int)B, (int)L, (int)C, st),
                   "fields_read_forward_bf16_rows");
         }
         Tensor acc = empty({N, D}, at::kBFloat16, dev);
@@ -108,9 +108,9 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         float *p = fp(par), *g = fp(g_par);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
-            const Tensor ws = workspace(n, dev);
-            check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
-                                                   g, g + C, g + 2 * C, vp(ws), n, (int)B, (int)L, (int)C, st),
+            PassWorkspace ws(n, u, true);
+            ws.check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
+                                                   g, g + C, g + 2 * C, ws.ptr(), n, (int)B, (int)L, (int)C, st),
                   "fields_read_backward_bf16_rows");
         }
         Tensor grad_x;

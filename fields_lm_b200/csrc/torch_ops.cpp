@@ -61,9 +61,9 @@ static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, b
     read = empty({B, L, 4 * C}, at::kFloat, dev);
     if (want_state) state_out = empty({B, 2 * C}, at::kFloat, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
-    const Tensor ws = workspace(n, dev);
-    check(f.fields_read_forward(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read),
-                                fp(state_out), vp(ws), n, B, L, C, stream_of(a.raw)),
+    PassWorkspace ws(n, a.raw, C % 4 == 0 && all_aligned({fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in)}, 16));
+    ws.check(f.fields_read_forward(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read),
+                                fp(state_out), ws.ptr(), n, B, L, C, stream_of(a.raw)),
           "fields_read_forward");
 }
 
@@ -98,19 +98,19 @@ struct FieldRead : torch::autograd::Function<FieldRead> {
                                : at::zeros({B, L, 4 * C}, at::TensorOptions().dtype(at::kFloat).device(dev));
         const Tensor grad_state = grads.size() > 1 && grads[1].defined() ? f32(grads[1]) : Tensor();
         const Tensor grad_raw = empty({B, L, 3 * C}, at::kFloat, dev);
-        const Tensor g_tr = empty({C}, at::kFloat, dev), g_ti = empty({C}, at::kFloat, dev),
-                     g_gm = empty({C}, at::kFloat, dev);
+        const Tensor g_par = empty({3, C}, at::kFloat, dev);
         Tensor g_sin;
         if (state_in.defined() && ctx->needs_input_grad(4)) g_sin = empty({B, 2 * C}, at::kFloat, dev);
         const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
-        const Tensor ws = workspace(n, dev);
+        PassWorkspace ws(n, raw, C % 4 == 0 && all_aligned({fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), fp(read),
+                                                                  fp(grad_read)}, 16));
         auto* entry = lean ? f.fields_read_backward_from_states : f.fields_read_backward;
         // (lean: `read` holds the kept state rows, possibly none for L < 8)
-        check(entry(fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), read.numel() ? fp(read) : nullptr,
-                    fp(grad_read), fp(grad_state), fp(grad_raw), fp(g_tr), fp(g_ti), fp(g_gm), fp(g_sin),
-                    vp(ws), n, B, L, C, stream_of(raw)),
+        ws.check(entry(fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), read.numel() ? fp(read) : nullptr,
+                    fp(grad_read), fp(grad_state), fp(grad_raw), fp(g_par), fp(g_par) + C,
+                    fp(g_par) + 2 * C, fp(g_sin), ws.ptr(), n, B, L, C, stream_of(raw)),
               "fields_read_backward");
-        return {grad_raw, g_tr, g_ti, g_gm, g_sin, Tensor(), Tensor()};
+        return {grad_raw, part_of(g_par, 0, C), part_of(g_par, C, C), part_of(g_par, 2 * C, C), g_sin, Tensor(), Tensor()};
     }
 };
 
@@ -125,16 +125,16 @@ static variable_list run_forward_bf16(const Tensor& raw, const Tensor& tr, const
     const c10::cuda::CUDAGuard guard(dev);
     const Tensor read = empty({B, L, 4 * C}, at::kBFloat16, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
-    const Tensor ws = workspace(n, dev);
+    PassWorkspace ws(n, raw, true);
     if (!stats) {
-        check(f.fields_read_forward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), nullptr,
-                                         vp(ws), n, B, L, C, stream_of(raw)),
+        ws.check(f.fields_read_forward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), nullptr,
+                                         ws.ptr(), n, B, L, C, stream_of(raw)),
               "fields_read_forward_bf16");
         return {read};
     }
     const Tensor groups = empty({B, L, (C + 127) / 128}, at::kFloat, dev);
-    check(f.fields_read_forward_bf16_stats(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), fp(groups),
-                                           nullptr, vp(ws), n, B, L, C, stream_of(raw)),
+    ws.check(f.fields_read_forward_bf16_stats(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), fp(groups),
+                                           nullptr, ws.ptr(), n, B, L, C, stream_of(raw)),
           "fields_read_forward_bf16_stats");
     return {read, groups.sum(-1)};
 }
@@ -146,15 +146,14 @@ static variable_list run_backward_bf16(const Tensor& raw, const Tensor& tr, cons
     const int B = (int)raw.size(0), L = (int)raw.size(1), C = (int)raw.size(2) / 3;
     const c10::Device dev = raw.device();
     const Tensor grad_raw = empty({B, L, 3 * C}, at::kBFloat16, dev);
-    const Tensor g_tr = empty({C}, at::kFloat, dev), g_ti = empty({C}, at::kFloat, dev),
-                 g_gm = empty({C}, at::kFloat, dev);
+    const Tensor g_par = empty({3, C}, at::kFloat, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
-    const Tensor ws = workspace(n, dev);
-    check(f.fields_read_backward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), vp(grad_read),
-                                      nullptr, vp(grad_raw), fp(g_tr), fp(g_ti), fp(g_gm), nullptr, vp(ws),
-                                      n, B, L, C, stream_of(raw)),
+    PassWorkspace ws(n, raw, true);
+    ws.check(f.fields_read_backward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), vp(grad_read),
+                                      nullptr, vp(grad_raw), fp(g_par), fp(g_par) + C, fp(g_par) + 2 * C,
+                                      nullptr, ws.ptr(), n, B, L, C, stream_of(raw)),
           "fields_read_backward_bf16");
-    return {grad_raw, g_tr, g_ti, g_gm};
+    return {grad_raw, part_of(g_par, 0, C), part_of(g_par, C, C), part_of(g_par, 2 * C, C)};
 }
 
 template <bool STATS>

@@ -120,7 +120,7 @@ class FieldStack {
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
                      read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         const size_t ws_bytes = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
-        Tensor acc = empty({N, D}, at::kBFloat16, dev), ws = workspace(ws_bytes, dev), u = empty({N, W}, at::kBFloat16, dev),
+        Tensor acc = empty({N, D}, at::kBFloat16, dev), u = empty({N, W}, at::kBFloat16, dev),
                uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev);
         std::vector<Tensor> states;
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, st),
@@ -129,9 +129,10 @@ class FieldStack {
         for (const Block& b : blocks_) {
             at::cuda::addmm_out(u, b.in_b, xb, b.in_t, 1, 1);
             const Tensor state = empty({B, D}, at::kFloat, dev);
+            PassWorkspace ws(ws_bytes, u, true);
             float* par = fp(b.par);
-            check(f.fields_read_forward_bf16_rows(vp(u), W, par, par + C, par + 2 * C, nullptr, vp(read), fp(groups),
-                                                  fp(state), vp(ws), ws_bytes, (int)B, (int)L, (int)C, st),
+            ws.check(f.fields_read_forward_bf16_rows(vp(u), W, par, par + C, par + 2 * C, nullptr, vp(read), fp(groups),
+                                                  fp(state), ws.ptr(), ws_bytes, (int)B, (int)L, (int)C, st),
                   "fields_read_forward_bf16_rows");
             at::cuda::mm_out(acc, read, b.out_t);
             const void* gate = static_cast<at::BFloat16*>(vp(u)) + 3 * C;

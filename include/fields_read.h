@@ -54,6 +54,23 @@ const char *fields_status_string(int status);
 /* Library version as major * 10000 + minor * 100 + patch. */
 int fields_read_version(void);
 
+/*
+ * Kept workspaces. The blocks of a forward or backward pass on 128-bit (64-bit for bfloat16) accesses
+ * publish in the workspace, which a pass fills with a pattern before it starts. A caller that keeps a
+ * workspace for such passes alone, on one stream, can save that fill: it has 256 + 3 * half_bytes
+ * bytes (half_bytes a multiple of 256, at least fields_read_workspace_bytes of every pass) filled with
+ * 0xFF once, and a fields_kept zeroed but for half_bytes. fields_read_use_kept(k) before a pass makes the
+ * calling thread's next pass take the workspace as that and update *k: the two halves take turns, and a
+ * pass fills what the one before it used. Such a call must not be replayed from a captured graph.
+ * fields_read_use_kept(NULL) takes it back; after a pass that returned an error start from the fill.
+ */
+struct fields_kept {
+    size_t half_bytes;
+    size_t dirty[2];
+    unsigned parity;
+};
+int fields_read_use_kept(struct fields_kept *kept);
+
 /* Bytes of scratch the given pass needs for these extents (0 for empty inputs). */
 size_t fields_read_workspace_bytes(int B, int L, int C, int pass);
 

@@ -1,0 +1,97 @@
+"""Passes on the kept workspaces of the torch layer (csrc/torch_api.h): extents and dtypes in any order,
+several streams and threads, and graphs, against passes that fill a workspace of their own (GPU)."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import FP32_TOL, rel_err
+from fields_lm_b200 import field_read_with_state, fused_field_read, fused_field_read_bf16
+from oracle import field_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(B, L, C, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    ring, theta = torch.linspace(0.85, 0.999, C, device="cuda"), torch.linspace(0.03, 3.04, C, device="cuda")
+    par = [ring * theta.cos(), ring * theta.sin(), (1 - ring ** 2).sqrt()]
+    raw = 0.577 * torch.randn(B, L, 3 * C, device="cuda", generator=g)
+    return [t.requires_grad_(True) for t in (raw, *par)], torch.randn(B, L, 4 * C, device="cuda", generator=g)
+
+
+def _pass(leaves, grad):
+    read = fused_field_read(*leaves)
+    return [read.detach(), *torch.autograd.grad(read, leaves, grad)]
+
+
+# the fold of the parameter gradients into the last block: one row, the most it takes (16) and one more
+@pytest.mark.parametrize("B,L,C", [(1, 1, 4), (2, 250, 132), (16, 32, 260), (17, 31, 128), (1, 513, 512)])
+def test_folded_parameter_gradients_match_the_oracle(B, L, C):
+    leaves, grad = _case(B, L, C, L)
+    host = [t.detach().cpu().numpy() for t in leaves]
+    want = [field_oracle.forward(*host)[0], *field_oracle.backward(*host, grad.cpu().numpy())[:4]]
+    for _ in range(2):  # the counters are back at their first value
+        for g, w in zip(_pass(leaves, grad), want):
+            assert rel_err(g.cpu().numpy(), np.asarray(w)) < FP32_TOL
+
+
+def test_extents_and_forms_in_any_order():
+    shapes = [(1, 40, 512), (2, 3001, 384), (3, 777, 132), (1, 300, 7), (1, 40, 512), (8, 512, 512), (1, 1, 4)]
+    cases = [_case(*s, i) for i, s in enumerate(shapes)]
+    want = [[t.cpu() for t in _pass(*c)] for c in cases]
+    for i in [3, 1, 0, 5, 2, 6, 4, 1, 3, 0, 2, 5]:
+        leaves, grad = cases[i]
+        fused_field_read_bf16(leaves[0].detach().bfloat16(), *[t.detach() for t in leaves[1:]]) if shapes[i][2] % 4 == 0 else None
+        field_read_with_state(*leaves, None, lean=True)[0].sum().backward()
+        for g, w in zip(_pass(leaves, grad), want[i]):
+            assert rel_err(g.cpu().numpy(), w.numpy()) < 1e-6
+
+
+def test_streams_and_threads():
+    cases = [_case(2, 1500 + 100 * i, 256, i) for i in range(4)]
+    want = [[t.cpu() for t in _pass(*c)] for c in cases]
+    torch.cuda.synchronize()
+    shared = torch.cuda.Stream()
+    bad = []
+
+    def work(i):
+        stream = shared if i % 2 else torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    got = _pass(*cases[i])
+                    stream.synchronize()
+                    for g, w in zip(got, want[i]):
+                        assert rel_err(g.cpu().numpy(), w.numpy()) < 1e-6
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+
+
+def test_captured_passes_can_be_replayed():
+    leaves, grad = _case(2, 900, 256, 3)
+    par = [t.detach() for t in leaves[1:]]
+    raw = leaves[0].detach().clone()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side), torch.no_grad():
+        fused_field_read(raw, *par)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(graph, stream=side):
+        out = fused_field_read(raw, *par)
+    for seed in (11, 12, 13):
+        raw.copy_(_case(2, 900, 256, seed)[0][0].detach())
+        graph.replay()
+        torch.cuda.synchronize()
+        got = out.clone()
+        with torch.no_grad():
+            want = fused_field_read(raw, *par)
+        assert rel_err(got.cpu().numpy(), want.cpu().numpy()) < 1e-6
