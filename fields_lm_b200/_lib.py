@@ -26,6 +26,7 @@ SYMBOLS = {
     "fields_read_workspace_bytes": (_SZ, [_I, _I, _I, _I]),
     "fields_read_forward": (_I, [_P] * 8 + [_SZ, _I, _I, _I, _P]),
     "fields_read_backward": (_I, [_P] * 14 + [_SZ, _I, _I, _I, _P]),
+    "fields_read_forward_rows": (_I, [_P] * 9 + [_SZ, _I, _I, _I, _P]),
     "fields_read_state_rows": (_I, [_I]),
     "fields_read_backward_from_states": (_I, [_P] * 14 + [_SZ, _I, _I, _I, _P]),
     "fields_read_forward_bf16": (_I, [_P] * 8 + [_SZ, _I, _I, _I, _P]),
@@ -66,7 +67,7 @@ SYMBOLS = {
     "fields_mixer_open_grad": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 4 + [_LL, _P, _P, ctypes.c_float, _I, _LL,
                                                                        _I, _P]),
     "fields_mixer_close_grad": (_I, [_P, _LL, _I, _P]),
-    "fields_stack_layout": (_I, [_P, _P]),
+    "fields_stack_layout": (_I, [_P, _I, _P]),
     "fields_stack_step_norm": (_I, [_P, _LL, _P, _P, _P, ctypes.c_float, _LL, _I, _P]),
     "fields_stack_close_mixer": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 5 +
                                  [ctypes.c_float, _I, ctypes.c_float, _LL, _I, _P]),

@@ -37,6 +37,7 @@ struct uint4;
 
 constexpr int kCtrlHeader = 64;  // unsigned words before the slots: [0] error word
 constexpr int kGroup = 128;      // channels per tile
+constexpr int kStateRowEvery = 8;  // steps per saved state row of the backward from state rows
 
 struct SpShape {
     int B, L, C;
@@ -83,6 +84,8 @@ struct SpFwdParamsT {
     // Kernels built with STATS also write, per token and 128-channel group, the sum of squares of
     // the four output planes (fp32 values, before any rounding of `read`): [B, L, G].
     float* sumsq = nullptr;
+    // Kernels built with ROWS: [B, L / kStateRowEvery, 2C] fp32.
+    float* rows = nullptr;
 };
 using SpFwdParams = SpFwdParamsT<float>;
 
@@ -112,7 +115,8 @@ FL_HD SpTile sp_decode(const SpShape& s, unsigned ticket) {
 // (the special-function pipe would bound it otherwise): 43.0 -> 36.2 us at 8 x 2,048 x 512, 189 ->
 // 142 us at 1 x 65,536. Blocks of four warps overlap their phases better than blocks of eight; holding
 // tickets and staging the next tile in shared memory (an earlier form) came to 43.0 us.
-template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false>
+// ROWS: also writes the state after every kStateRowEvery-th step, what a backward pass from state rows keeps.
+template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false, bool ROWS = false>
 struct FwdSinglePass {
     using Params = SpFwdParamsT<IO>;
     static constexpr int kThreads = 32 * WARPS;
@@ -341,6 +345,14 @@ struct FwdSinglePass {
                     // the map area is free after the look-back: one partial per lane and step
                     if constexpr (STATS) smem[(warp * TS + u) * kStatRow + lane] = sq.x + sq.y;
                     orow += (size_t)4 * C;
+                    if constexpr (ROWS) {
+                        const int t = tw + u;
+                        if (t % kStateRowEvery == kStateRowEvery - 1) {
+                            float* row = p.rows + ((size_t)tl.b * (s.L / kStateRowEvery) + t / kStateRowEvery) * 2 * C + c0;
+                            vec_store<4>(row, join2(sr[0], sr[1]));
+                            vec_store<4>(row + C, join2(si[0], si[1]));
+                        }
+                    }
                 }
             }
         } else {  // PH == 4 (STATS): one sum per step of the tile, lanes added in order
@@ -681,7 +693,6 @@ struct SpBwdParamsT {
     float* grad_par[3] = {nullptr, nullptr, nullptr};
 };
 using SpBwdParams = SpBwdParamsT<float>;
-constexpr int kStateRowEvery = 8;
 
 // The end of a block of a backward kernel where the reduction is folded in: the last block of a channel
 // group to get here (a counter in the workspace header, back at its first value when that block is done)

@@ -640,6 +640,7 @@ static Algo algo_from_env() { return kAlgoAuto; }
 // eight warps and 48-step tiles, at 1 x 16,384 54.2 -> 51.8, at 2 x 3,001 x 384 20.6 -> 19.5, equal at
 // 8 x 2,048. Longer tiles spill.
 using FwdSp0 = FwdSinglePass<9, 4, 3>;
+using FwdSpRows = FwdSinglePass<9, 4, 3, float, false, true>;  // also writes state rows
 #ifdef FIELDS_ALL_VARIANTS
 using FwdSp1 = FwdSinglePass<4, 8, 2>;        // tile 32
 //   two-sweep forward <steps per warp, warps, unroll, blocks per SM, ring slots>
@@ -714,7 +715,7 @@ static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspac
     int rc = FIELDS_OK;
     if (k) {
         // A small pass publishes in one half, which is unset, and fills what was used of the other. Up to
-        // 1,024 tiles: there the fill launch shows, in host time above all (20.1 -> 19.2 us of GPU at
+        // 592 tiles (four per SM): there the fill launch shows, in host time above all (20.1 -> 19.2 us of GPU at
         // 2 x 3,001 x 384, 13.6 -> 12.7 at 1 x 2,048 x 512); above, the code in the kernel costs as much.
         if (slot_bytes > k->half_bytes) return FIELDS_ERR_WORKSPACE;
         const unsigned h = k->parity & 1;
@@ -722,7 +723,7 @@ static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspac
         slots = half[h];
         out->partial = reinterpret_cast<float*>(half[1] + k->half_bytes);
         const size_t used = k->dirty[1 - h];
-        if (pl.tiles <= 1024 && k->dirty[h] == 0) {
+        if (pl.tiles <= 592 && k->dirty[h] == 0) {
             if (used > (size_t)pl.tiles * 16384) {  // a much larger pass was before: too much for these blocks
                 rc = fill_unset(half[1 - h], used, st);
             } else {
@@ -749,7 +750,8 @@ template <class K, typename IO = float>
 static int run_forward_single_pass(const IO* raw, const float* tr, const float* ti,
                                    const float* gamma, const float* state_in, IO* read,
                                    float* state_out, void* workspace, int B, int L, int C,
-                                   Stream st, float* sumsq = nullptr, long long pitch = 0) {
+                                   Stream st, float* sumsq = nullptr, long long pitch = 0,
+                                   float* rows = nullptr) {
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (pitch) pl.s.zp = (int)pitch;
@@ -758,6 +760,7 @@ static int run_forward_single_pass(const IO* raw, const float* tr, const float* 
     if (rc) return rc;
     SpFwdParamsT<IO> p{raw, tr, ti, gamma, state_in, read, state_out, ws.agg, ws.incl, ws.ctrl, pl.s};
     p.sumsq = sumsq;
+    p.rows = rows;
     return launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st, pl.s.clean_n > 0);
 }
 
@@ -1107,6 +1110,21 @@ int fields_read_backward(const float* raw, const float* tr, const float* ti, con
 }
 
 
+int fields_read_forward_rows(const float* raw, const float* tr, const float* ti, const float* gamma,
+                             const float* state_in, float* read, float* state_out, float* states,
+                             void* workspace, size_t workspace_bytes, int B, int L, int C, void* stream) {
+    if (B <= 0 || L <= 0 || C <= 0) return FIELDS_ERR_ARGUMENT;
+    if (!raw || !tr || !ti || !gamma || !read || (!states && L >= kStateRowEvery)) return FIELDS_ERR_ARGUMENT;
+    if (C % 4 != 0 || !aligned16(raw) || !aligned16(read) || !aligned16(tr) || !aligned16(ti) || !aligned16(gamma) ||
+        !aligned16(states))
+        return FIELDS_ERR_UNSUPPORTED;
+    if (!workspace || workspace_bytes < fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD) ||
+        (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return FIELDS_ERR_WORKSPACE;
+    return run_forward_single_pass<FwdSpRows>(raw, tr, ti, gamma, state_in, read, state_out, workspace, B, L, C,
+                                              reinterpret_cast<Stream>(stream), nullptr, 0, states);
+}
+
 int fields_read_state_rows(int L) { return L > 0 ? L / kStateRowEvery : 0; }
 
 int fields_read_backward_from_states(const float* raw, const float* tr, const float* ti,
@@ -1341,6 +1359,9 @@ static int scan_check(const void* workspace, size_t workspace_bytes, int B, int 
                       long long a_batch, long long a_step, int a_chan) {
     if (a_chan != 0 && a_chan != 1) return FIELDS_ERR_ARGUMENT;
     if (a_batch < 0 || a_step < 0) return FIELDS_ERR_ARGUMENT;
+#ifndef FIELDS_HOST_EMU
+    if (!workspace && !workspace_bytes) return FIELDS_OK;  // the GPU kernels use none
+#endif
     if (!workspace || workspace_bytes < scan_workspace_floats(B, L, C) * sizeof(float) ||
         (reinterpret_cast<uintptr_t>(workspace) & 15u))
         return FIELDS_ERR_WORKSPACE;
@@ -1826,7 +1847,10 @@ int fields_read_norm_grad_combine(const void* grad_read, const void* read, const
                                      reinterpret_cast<Stream>(stream), p);
 }
 
-int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
+}  // extern "C"
+
+// The layout of one block; the number of thread blocks it takes in *blocks.
+static int layout_params(const struct fields_stack_weights* w, LayoutParams& p, long long* blocks) {
     if (!w || w->dim <= 0 || w->hidden < 0) return FIELDS_ERR_ARGUMENT;
     if (!w->write_w || !w->write_b || !w->gate_w || !w->out_w || !w->read_norm_w || !w->radius_logit ||
         !w->theta || !w->in_w || !w->in_b || !w->out_w16 || !w->par ||
@@ -1839,7 +1863,6 @@ int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
     for (const void* q : all)
         if (!aligned16(q)) return FIELDS_ERR_UNSUPPORTED;
     uint16_t* in_w = static_cast<uint16_t*>(w->in_w);
-    LayoutParams p{};
     p.piece[0] = {w->write_w, in_w, nullptr, 3 * C * D, (int)D};
     p.piece[1] = {w->gate_w, in_w + 3 * C * D, nullptr, D * D, (int)D};
     p.piece[2] = {w->write_b, static_cast<uint16_t*>(w->in_b), nullptr, 3 * C, (int)(3 * C)};
@@ -1855,9 +1878,28 @@ int fields_stack_layout(const struct fields_stack_weights* w, void* stream) {
         at += (p.piece[k].n + kLayoutChunk - 1) / kLayoutChunk;
     }
     p.first[kLayoutPieces] = at;
-    const long long blocks = at + (C + kRowThreads - 1) / kRowThreads;
-    if (blocks > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
-    return launch_on<LayoutParams>(layout_block, (unsigned)blocks, kRowThreads, 0, reinterpret_cast<Stream>(stream), p);
+    *blocks = at + (C + kRowThreads - 1) / kRowThreads;
+    return *blocks > 0x7fffffffLL ? FIELDS_ERR_UNSUPPORTED : FIELDS_OK;
+}
+
+extern "C" {
+
+int fields_stack_layout(const struct fields_stack_weights* w, int count, void* stream) {
+    if (!w || count <= 0) return FIELDS_ERR_ARGUMENT;
+    for (int i = 0; i < count; i += kLayoutBlocks) {
+        LayoutBatch batch{};
+        const int n = count - i < kLayoutBlocks ? count - i : kLayoutBlocks;
+        long long blocks = 0;
+        for (int k = 0; k < n; ++k) {
+            if (w[i + k].dim != w[0].dim || w[i + k].hidden != w[0].hidden) return FIELDS_ERR_ARGUMENT;
+            const int rc = layout_params(&w[i + k], batch.block[k], &blocks);
+            if (rc) return rc;
+        }
+        const int rc = launch_grid<LayoutBatch>(layout_block, dim3((unsigned)blocks, (unsigned)n), kRowThreads,
+                                                reinterpret_cast<Stream>(stream), batch);
+        if (rc) return rc;
+    }
+    return FIELDS_OK;
 }
 
 int fields_stack_step_norm(const void* raw, long long raw_stride, const float* par, float* state,

@@ -1,0 +1,33 @@
+// The library's matrix products of the torch layer, called directly: the same cuBLAS routine that at::mm
+// calls for these types, without its checks, wrappers and tensor views (8 us of host time per product
+// against 3; a block's prefill of a few hundred tokens was bound by them).
+#pragma once
+
+#include <ATen/cuda/CUDAContextLight.h>
+#include <ATen/cuda/Exceptions.h>
+
+#include "torch_api.h"
+
+namespace fields_torch {
+
+// A dense bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any.
+struct Operand {
+    const void* p;
+    bool transposed;  // stored [cols, rows]
+};
+inline Operand plain(const Tensor& t) { return Operand{vp(t), false}; }
+inline Operand transposed(const Tensor& t) { return Operand{vp(t), true}; }
+
+// out [M, N] = a [M, K] b [K, N], row-major, fp32 accumulation; out is bfloat16 or fp32. On the current stream.
+inline void product(const Tensor& out, Operand a, Operand b, int64_t M, int64_t N, int64_t K) {
+    const float one = 1.0f, zero = 0.0f;
+    // cuBLAS is column-major: out^T = b^T a^T
+    TORCH_CUDABLAS_CHECK(cublasGemmEx(
+        at::cuda::getCurrentCUDABlasHandle(), b.transposed ? CUBLAS_OP_T : CUBLAS_OP_N,
+        a.transposed ? CUBLAS_OP_T : CUBLAS_OP_N, (int)N, (int)M, (int)K, &one, b.p, CUDA_R_16BF,
+        (int)(b.transposed ? K : N), a.p, CUDA_R_16BF, (int)(a.transposed ? M : K), &zero, out.data_ptr(),
+        out.scalar_type() == at::kFloat ? CUDA_R_32F : CUDA_R_16BF, (int)N, CUBLAS_COMPUTE_32F,
+        CUBLAS_GEMM_DEFAULT_TENSOR_OP));
+}
+
+}  // namespace fields_torch

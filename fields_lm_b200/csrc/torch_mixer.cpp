@@ -5,10 +5,9 @@
 // products forward and four backward (library calls; the two projections of x are one product over
 // [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
 // field_mixer_grad.cuh between them. Weight gradients come out of the products in fp32.
-#include "torch_api.h"
+#include "torch_gemm.h"
 
 #include <ATen/ops/addmm_cuda_dispatch.h>
-#include <ATen/ops/mm_cuda_dispatch.h>
 
 namespace fields_torch {
 
@@ -50,7 +49,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         w.read_norm_w = fp(norm_w); w.radius_logit = fp(radius); w.theta = fp(theta);
         w.in_w = vp(in_w); w.in_b = vp(in_b); w.out_w16 = vp(out16); w.par = fp(par);
         w.dim = (int)D; w.hidden = 0;
-        check(f.fields_stack_layout(&w, st), "fields_stack_layout");
+        check(f.fields_stack_layout(&w, 1, st), "fields_stack_layout");
         const Tensor xb = empty({N, D}, at::kBFloat16, dev);
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, (int)D, st),
               "fields_stack_close_ff");
@@ -66,7 +65,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
                   "fields_read_forward_bf16_rows");
         }
         Tensor acc = empty({N, D}, at::kBFloat16, dev);
-        at::cuda::mm_out(acc, read, out16.t());
+        product(acc, plain(read), transposed(out16), N, D, 2 * D);
         const Tensor y = empty({B, L, D}, at::kFloat, dev);
         check(f.fields_stack_close_mixer(fp(x), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
                                          nullptr, fp(y), nullptr, (float)eps, (int)(2 * D), 0.0f, N, (int)D, st),
@@ -92,20 +91,23 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         void* st = stream_of(xb);
         auto f32s = [&](at::IntArrayRef size) { return empty(size, at::kFloat, dev); };
 
+        const int64_t n_rows = (int64_t)f.fields_mixer_grad_rows(N),
+                      n_scratch = (int64_t)(f.fields_mixer_grad_scratch_bytes((int)D) / 4);
         const Tensor grad_acc = empty({N, D}, at::kBFloat16, dev), grad_u = empty({N, W}, at::kBFloat16, dev),
-                     grad_sumsq = f32s({N}), rows = f32s({2, (int64_t)f.fields_mixer_grad_rows(N), D});
+                     // scratch: partial rows of open_grad, of close_grad, grad_sumsq, gradients of the transition
+                     temp = f32s({2 * n_rows * D + n_scratch + 3 * C + N});
+        float *rows = fp(temp), *scratch = rows + 2 * n_rows * D, *g = scratch + n_scratch, *grad_sumsq = g + 3 * C;
         check(f.fields_mixer_open_grad(fp(gy), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
-                                       vp(grad_acc), gate_of(grad_u, C), W, fp(grad_sumsq), fp(rows), eps, (int)(2 * D),
+                                       vp(grad_acc), gate_of(grad_u, C), W, grad_sumsq, rows, eps, (int)(2 * D),
                                        N, (int)D, st),
               "fields_mixer_open_grad");
         Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
-        at::cuda::mm_out(grad_read, grad_acc, out16);
+        product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
         Tensor grad_out = f32s({D, 2 * D});
-        at::cuda::mm_out(grad_out, grad_acc.t(), read, at::kFloat);
-        check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), fp(grad_sumsq), vp(grad_read), N, (int)(4 * C), st),
+        product(grad_out, transposed(grad_acc), plain(read), D, 2 * D, N);
+        check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
               "fields_read_norm_grad_combine");
-        const Tensor g_par = f32s({3, C});
-        float *p = fp(par), *g = fp(g_par);
+        float* p = fp(par);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
             PassWorkspace ws(n, u, true);
@@ -116,23 +118,29 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         Tensor grad_x;
         if (ctx->needs_input_grad(kX)) {
             Tensor back = empty({N, D}, at::kBFloat16, dev);
-            at::cuda::mm_out(back, grad_u, in_w);
+            product(back, plain(grad_u), plain(in_w), N, D, W);
             grad_x = f32s({B, L, D});
             check(f.fields_stack_close_ff(fp(gy), vp(back), nullptr, fp(grad_x), nullptr, 0.0f, N, (int)D, st),
                   "fields_stack_close_ff");
         }
         Tensor grad_in = f32s({W, D});
-        at::cuda::mm_out(grad_in, grad_u.t(), xb, at::kFloat);
+        product(grad_in, transposed(grad_u), plain(xb), W, D, N);
 
-        const Tensor g_out_b = f32s({D}), g_gate_b = f32s({D}), g_write_b = f32s({3 * C}), g_norm = f32s({2 * D}),
-                     g_radius = f32s({C}), g_theta = f32s({C}),
-                     scratch = f32s({(int64_t)(f.fields_mixer_grad_scratch_bytes((int)D) / 4)});
+        // the small gradients share an allocation
+        const Tensor small = f32s({4 * D + 5 * C});
+        int64_t at = 0;
+        auto part = [&](int64_t n) {
+            at += n;
+            return part_of(small, at - n, n);
+        };
+        const Tensor g_out_b = part(D), g_gate_b = part(D), g_norm = part(2 * D), g_write_b = part(3 * C),
+                     g_radius = part(C), g_theta = part(C);
         fields_mixer_grads q{};
-        q.rows = fp(rows); q.grad_raw = vp(grad_u); q.grad_pitch = W; q.grad_out = fp(grad_out); q.out_w = fp(out_w);
+        q.rows = rows; q.grad_raw = vp(grad_u); q.grad_pitch = W; q.grad_out = fp(grad_out); q.out_w = fp(out_w);
         q.norm_w = fp(norm_w); q.radius_logit = fp(radius); q.theta = fp(theta);
         q.grad_tr = g; q.grad_ti = g + C; q.grad_gamma = g + 2 * C;
         q.grad_out_b = fp(g_out_b); q.grad_gate_b = fp(g_gate_b); q.grad_write_b = fp(g_write_b);
-        q.grad_norm_w = fp(g_norm); q.grad_radius = fp(g_radius); q.grad_theta = fp(g_theta); q.scratch = fp(scratch);
+        q.grad_norm_w = fp(g_norm); q.grad_radius = fp(g_radius); q.grad_theta = fp(g_theta); q.scratch = scratch;
         check(f.fields_mixer_close_grad(&q, N, (int)D, st), "fields_mixer_close_grad");
         return {grad_x,   grad_in.narrow(0, 0, 3 * C),   g_write_b, g_radius, g_theta, g_norm, grad_out,
                 g_out_b, grad_in.narrow(0, 3 * C, D), g_gate_b,  Tensor()};

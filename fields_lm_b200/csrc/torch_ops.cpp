@@ -53,7 +53,8 @@ static ForwardArgs forward_args(const Tensor& raw, const Tensor& tr, const Tenso
                        state_in.defined() ? f32(state_in) : state_in, d};
 }
 
-static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, bool want_state) {
+// With `rows` also every eighth state row, written by the kernel where it can (undefined otherwise).
+static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, bool want_state, Tensor* rows = nullptr) {
     const Api& f = api();
     const auto [B, L, C] = a.d;
     const c10::Device dev = a.raw.device();
@@ -61,10 +62,18 @@ static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, b
     read = empty({B, L, 4 * C}, at::kFloat, dev);
     if (want_state) state_out = empty({B, 2 * C}, at::kFloat, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
-    PassWorkspace ws(n, a.raw, C % 4 == 0 && all_aligned({fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in)}, 16));
+    const bool vector = C % 4 == 0 && all_aligned({fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in)}, 16);
+    PassWorkspace ws(n, a.raw, vector);
+    if (rows && vector && B > 0 && L >= 8) {
+        *rows = empty({B, L / 8, 2 * C}, at::kFloat, dev);
+        ws.check(f.fields_read_forward_rows(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read), fp(state_out),
+                                            fp(*rows), ws.ptr(), n, B, L, C, stream_of(a.raw)),
+                 "fields_read_forward");
+        return;
+    }
     ws.check(f.fields_read_forward(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read),
-                                fp(state_out), ws.ptr(), n, B, L, C, stream_of(a.raw)),
-          "fields_read_forward");
+                                   fp(state_out), ws.ptr(), n, B, L, C, stream_of(a.raw)),
+             "fields_read_forward");
 }
 
 struct FieldRead : torch::autograd::Function<FieldRead> {
@@ -73,10 +82,11 @@ struct FieldRead : torch::autograd::Function<FieldRead> {
                                  const std::optional<Tensor>& state_, bool lean, bool want_state) {
         const ForwardArgs a = forward_args(raw_, tr_, ti_, gm_, state_.value_or(Tensor()));
         Tensor read, state_out;
-        run_forward(a, read, state_out, want_state);
         lean = lean && a.d.C % 4 == 0;
-        Tensor kept = read;
-        if (lean)  // every eighth state row instead of `read`
+        Tensor kept;
+        run_forward(a, read, state_out, want_state, lean ? &kept : nullptr);
+        if (!lean) kept = read;
+        else if (!kept.defined())  // every eighth state row instead of `read`
             kept = read.slice(1, 7, std::nullopt, 8).slice(2, 0, 2 * a.d.C).contiguous();
         ctx->set_materialize_grads(false);
         ctx->save_for_backward({a.raw, a.tr, a.ti, a.gm, kept, a.state_in});
@@ -207,7 +217,7 @@ static ScanDecay scan_decay(const Tensor& a) {
 
 struct LinearScan : torch::autograd::Function<LinearScan> {
     static variable_list forward(AutogradContext* ctx, const Tensor& a_, const Tensor& b_,
-                                 const std::optional<Tensor>& state_) {
+                                 const std::optional<Tensor>& state_, bool want_state) {
         const int B = (int)b_.size(0), L = (int)b_.size(1), C = (int)b_.size(2);
         Tensor state_in;
         if (state_ && state_->defined()) {
@@ -220,14 +230,14 @@ struct LinearScan : torch::autograd::Function<LinearScan> {
         const c10::cuda::CUDAGuard guard(dev);
         const Tensor b = dense(b_);
         const ScanDecay d = scan_decay(a_);
-        const Tensor states = empty({B, L, C}, at::kFloat, dev), state_out = empty({B, C}, at::kFloat, dev);
-        const size_t n = f.fields_scan_workspace_bytes(B, L, C);
-        const Tensor ws = workspace(n, dev);
+        const Tensor states = empty({B, L, C}, at::kFloat, dev);
+        const Tensor state_out = want_state ? empty({B, C}, at::kFloat, dev) : Tensor();
         check(f.fields_scan_forward(fp(d.a), d.batch, d.step, d.chan, fp(b), fp(state_in), fp(states),
-                                    fp(state_out), vp(ws), n, B, L, C, stream_of(b)),
+                                    fp(state_out), nullptr, 0, B, L, C, stream_of(b)),
               "fields_scan_forward");
         ctx->set_materialize_grads(false);
         ctx->save_for_backward({d.a, states, state_in});
+        if (!want_state) return {states};
         return {states, state_out};
     }
 
@@ -240,18 +250,16 @@ struct LinearScan : torch::autograd::Function<LinearScan> {
         const c10::Device dev = states.device();
         const c10::cuda::CUDAGuard guard(dev);
         const Tensor g = grads[0].defined() ? f32(grads[0]) : at::zeros_like(states);
-        const Tensor g_out = grads[1].defined() ? f32(grads[1]) : Tensor();
+        const Tensor g_out = grads.size() > 1 && grads[1].defined() ? f32(grads[1]) : Tensor();
         const Tensor grad_a = empty({B, L, C}, at::kFloat, dev), grad_b = empty({B, L, C}, at::kFloat, dev);
         Tensor g_in;
         if (state_in.defined() && ctx->needs_input_grad(2)) g_in = empty({B, C}, at::kFloat, dev);
-        const size_t n = f.fields_scan_workspace_bytes(B, L, C);
-        const Tensor ws = workspace(n, dev);
         check(f.fields_scan_backward(fp(d.a), d.batch, d.step, d.chan, fp(states), fp(state_in), fp(g),
-                                     fp(g_out), fp(grad_a), fp(grad_b), fp(g_in), vp(ws), n, B, L, C,
+                                     fp(g_out), fp(grad_a), fp(grad_b), fp(g_in), nullptr, 0, B, L, C,
                                      stream_of(states)),
               "fields_scan_backward");
         // dense gradient of `a`; for an expanded `a` autograd sums it over the broadcast channels
-        return {grad_a, grad_b, g_in};
+        return {grad_a, grad_b, g_in, Tensor()};
     }
 };
 
@@ -346,18 +354,23 @@ static PyObject* py_field_read_bf16(PyObject*, PyObject* const* args, Py_ssize_t
     END_HANDLE_TH_ERRORS
 }
 
-// linear_scan(a, b, state_in or None) -> (states, state_out); shapes and types checked by the caller
+// linear_scan(a, b, state_in or None, want_state) -> states, or (states, state_out)
 static PyObject* py_linear_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    want_args(n, 3);
+    want_args(n, 4);
     const Tensor &a = tensor_arg(args[0]), &b = tensor_arg(args[1]);
     const std::optional<Tensor> state_in = optional_arg(args[2]);
+    const bool want_state = PyObject_IsTrue(args[3]) == 1;
+    TORCH_CHECK(a.is_cuda() && b.is_cuda(), "linear_scan requires CUDA tensors");
+    TORCH_CHECK_TYPE(a.scalar_type() == at::kFloat && b.scalar_type() == at::kFloat, "a and b must be float32, got ",
+                     a.scalar_type(), " and ", b.scalar_type());
+    TORCH_CHECK_VALUE(a.dim() == 3 && a.sizes() == b.sizes(), shape(a), " ", shape(b));
     variable_list out;
     {
         pybind11::gil_scoped_release no_gil;
-        out = LinearScan::apply(a, b, state_in);
+        out = LinearScan::apply(a, b, state_in, want_state);
     }
-    return wrap2(out[0], out[1]);
+    return want_state ? wrap2(out[0], out[1]) : wrap(out[0]);
     END_HANDLE_TH_ERRORS
 }
 

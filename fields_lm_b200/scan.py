@@ -23,29 +23,18 @@ import torch
 from . import _lib
 
 
-def _check(a: torch.Tensor, b: torch.Tensor, block: int) -> None:
-    if block < 1 or block > 64:
-        raise ValueError("field_chunk must be in [1, 64]")
-    if not b.is_cuda or not a.is_cuda:
-        raise RuntimeError("linear_scan requires CUDA tensors")
-    if a.dtype != torch.float32 or b.dtype != torch.float32:
-        raise TypeError(f"a and b must be float32, got {a.dtype} and {b.dtype}")
-    if a.dim() != 3 or a.shape != b.shape:
-        raise ValueError((tuple(a.shape), tuple(b.shape)))
-
-
 def linear_scan(a: torch.Tensor, b: torch.Tensor, block: int = 32) -> torch.Tensor:
     """The reference's ``hierarchical_scan(a, b, block)`` for real fp32 CUDA tensors."""
-    _check(a, b, block)
-    return _lib.native().linear_scan(a, b, None)[0]
+    if block < 1 or block > 64:
+        raise ValueError("field_chunk must be in [1, 64]")
+    return _lib.native().linear_scan(a, b, None, False)
 
 
 def linear_scan_with_state(a: torch.Tensor, b: torch.Tensor,
                            state_in: Optional[torch.Tensor] = None):
     """The same scan from an incoming state ``[B, C]``; returns (states, state after the last
     step). An extension: the reference always starts from zero."""
-    _check(a, b, 32)
-    return _lib.native().linear_scan(a, b, state_in)
+    return _lib.native().linear_scan(a, b, state_in, True)
 
 
 def scan_entry(original: Callable) -> Callable:

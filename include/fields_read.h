@@ -122,6 +122,11 @@ int fields_read_backward(const float *raw, const float *tr, const float *ti,
  * (FIELDS_ERR_UNSUPPORTED otherwise); states may be NULL when L <= 8.
  */
 int fields_read_state_rows(int L);
+/* The forward that also writes those rows: fields_read_forward plus states [B, L / 8, 2C] out. */
+int fields_read_forward_rows(const float *raw, const float *tr, const float *ti,
+                             const float *gamma, const float *state_in, float *read,
+                             float *state_out, float *states, void *workspace,
+                             size_t workspace_bytes, int B, int L, int C, void *stream);
 int fields_read_backward_from_states(const float *raw, const float *tr, const float *ti,
                                      const float *gamma, const float *state_in,
                                      const float *states, const float *grad_read,
@@ -251,7 +256,7 @@ int fields_read_step_bf16(const void *raw, const float *tr, const float *ti, con
  *   state_in     [B, C] or NULL (zero, the reference's contract)
  *   states       [B, L, C] out: s_t for every step
  *   state_out    [B, C] or NULL
- *   workspace    fields_scan_workspace_bytes(B, L, C) bytes, 16-byte aligned
+ *   workspace    fields_scan_workspace_bytes(B, L, C) bytes, 16-byte aligned, or NULL with 0 bytes
  * Backward: grad_a is written densely [B, L, C] also for a broadcast `a` (the caller sums over
  * the broadcast dimension, as autograd does for an expanded tensor); states is the forward output.
  * One launch each way; results are bitwise reproducible.
@@ -481,7 +486,7 @@ int fields_mixer_epilogue_backward(const float *grad_y, const void *acc, const v
  * kernel each. D = dim, C = D / 2, H = hidden width of the SwiGLU; D % 8 == 0, D <= 4096, H % 8 == 0;
  * tensors dense and 16-byte aligned (FIELDS_ERR_UNSUPPORTED otherwise). bf16 operands are void *.
  *
- * fields_stack_layout: bfloat16 copies of a block's weights as the products want them, and its
+ * fields_stack_layout: for each of `count` blocks of one size, bfloat16 copies of a block's weights as the products want them, and its
  *   transition parameters. in_w = write_proj over gate_proj, in_b = write_proj's bias over zeros,
  *   out_w16 = out_proj diag(read_norm). hidden = 0: without the feed-forward (w12, w3 may be NULL).
  * fields_stack_step_norm: one recurrence step of N rows from raw (row stride raw_stride) and par
@@ -499,7 +504,7 @@ struct fields_stack_weights {
     float *par;
     int dim, hidden;
 };
-int fields_stack_layout(const struct fields_stack_weights *weights, void *stream);
+int fields_stack_layout(const struct fields_stack_weights *weights, int count, void *stream);
 int fields_stack_step_norm(const void *raw, long long raw_stride, const float *par, float *state,
                            void *out, float eps, long long N, int C, void *stream);
 int fields_stack_close_mixer(const float *x, const void *acc, const void *gate, long long gate_stride,
