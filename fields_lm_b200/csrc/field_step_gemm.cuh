@@ -153,7 +153,7 @@ __device__ __forceinline__ float table_share(const float* table, int count, int 
 //   fetch      what slice g needs from global memory, while the product still runs
 //   run        the rest
 struct EpiIn {  // slice: eight channels' z_r | z_i | z_v, then sixteen gate features
-    static constexpr int kSlice = 40, kSlices = 4, kStages = 4, kConst = 64;
+    static constexpr int kSlice = 40, kSlices = 2, kStages = 7, kConst = 64;
     static constexpr bool kScaled = false;
     struct Fetched {
         float sr[8], si[8];
@@ -205,8 +205,13 @@ struct EpiIn {  // slice: eight channels' z_r | z_i | z_v, then sixteen gate fea
     }
 };
 
+// EpiOut and EpiFf come with tiles of 64 and of 32 features (and EpiUv with two of its slices for the same row
+// counts). Where 64 leave so few tiles that K would be split
+// over clusters of eight (up to 128 rows at d_model 1,024), 32 with clusters of four are faster: a kernel's
+// clusters of eight took up to 14 us to get started (18 blocks, 16 rows: 661 -> 571 us; 128 rows: 681 -> 548).
+template <int SLICES>
 struct EpiOut {  // slice: eight features
-    static constexpr int kSlice = 8, kSlices = 8, kStages = 7, kConst = 8;
+    static constexpr int kSlice = 8, kSlices = SLICES, kStages = 7, kConst = 8;
     static constexpr bool kScaled = true;
     struct Fetched {
         float x[8], gate[8];
@@ -237,8 +242,9 @@ struct EpiOut {  // slice: eight features
     }
 };
 
+template <int SLICES>
 struct EpiUv {  // slice: u of twenty features, then v of the same
-    static constexpr int kSlice = 40, kSlices = 4, kStages = 4, kConst = 0;
+    static constexpr int kSlice = 40, kSlices = SLICES, kStages = SLICES == 4 ? 4 : 7, kConst = 0;
     static constexpr bool kScaled = true;
     struct Fetched {};
     float rstd;
@@ -266,8 +272,9 @@ struct EpiUv {  // slice: u of twenty features, then v of the same
     }
 };
 
+template <int SLICES>
 struct EpiFf {  // slice: eight features
-    static constexpr int kSlice = 8, kSlices = 8, kStages = 7, kConst = 0;
+    static constexpr int kSlice = 8, kSlices = SLICES, kStages = 7, kConst = 0;
     static constexpr bool kScaled = false;
     struct Fetched {
         float y[8];

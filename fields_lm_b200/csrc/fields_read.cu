@@ -2214,9 +2214,13 @@ int fields_step_block(const struct fields_step_args* g, void* stream) {
     p.read_eps = g->read_eps; p.ff_eps = g->ff_eps; p.M = g->rows; p.D = D; p.C = C; p.H = H;
     Stream st = reinterpret_cast<Stream>(stream);
     int rc = launch_step<EpiIn>(g->xb, g->in_w, 5 * C, D, C / 8, p, st);
-    if (!rc) rc = launch_step<EpiOut>(g->read, g->out_w16, D, 2 * D, D / 8, p, st);
-    if (!rc) rc = launch_step<EpiUv>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st);
-    if (!rc) rc = launch_step<EpiFf>(g->act, g->w3_16, D, H, D / 8, p, st);
+    const bool narrow = (g->rows + kStepRows - 1) / kStepRows * ((D + 63) / 64) * 8 <= 148;
+    if (!rc) rc = narrow ? launch_step<EpiOut<4>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st)
+                         : launch_step<EpiOut<8>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st);
+    if (!rc) rc = narrow ? launch_step<EpiUv<2>>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st)
+                         : launch_step<EpiUv<4>>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st);
+    if (!rc) rc = narrow ? launch_step<EpiFf<4>>(g->act, g->w3_16, D, H, D / 8, p, st)
+                         : launch_step<EpiFf<8>>(g->act, g->w3_16, D, H, D / 8, p, st);
     return rc;
 }
 #endif  // FIELDS_HOST_EMU
