@@ -15,6 +15,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #ifdef FIELDS_HOST_EMU
 #define FL_HD inline
@@ -264,6 +265,50 @@ FL_HD void io_store4_stream(uint16_t* p, const Vec<4>& x) {
     const uint32_t w[2] = {lo, hi};
     std::memcpy(p, w, 8);
 #endif
+}
+
+// A float tensor without 128-bit access: channel counts that are not a multiple of four, pointers off a
+// 16-byte boundary. The kernels take it as an element type of its own; a thread's four channels are then four
+// 32-bit accesses, of which the first `n` exist. For the other types n is four and not looked at.
+struct F32Any {
+    float v;
+};
+template <typename IO>
+FL_HD int channels_at(int c0, int C) {
+    if constexpr (std::is_same<IO, F32Any>::value) return C - c0 < 4 ? C - c0 : 4;
+    return 4;
+}
+template <typename IO>
+FL_HD Vec<4> io_load4(const IO* p, int n) {
+    if constexpr (std::is_same<IO, F32Any>::value) {
+        Vec<4> r;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r.v[k] = k < n ? p[k].v : 0.0f;
+        return r;
+    } else {
+        return io_load4(p);
+    }
+}
+template <typename IO>
+FL_HD Vec<4> io_load4_stream(const IO* p, int n) {
+    if constexpr (std::is_same<IO, F32Any>::value) return io_load4(p, n);
+    else return io_load4_stream(p);
+}
+template <typename IO>
+FL_HD void io_store4_stream(IO* p, const Vec<4>& x, int n) {
+    if constexpr (std::is_same<IO, F32Any>::value) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < n) p[k].v = x.v[k];
+    } else {
+        io_store4_stream(p, x);
+    }
+}
+// Four parameters or state values that go with tensors of element type IO.
+template <typename IO>
+FL_HD Vec<4> par_load4(const float* p, int n) {
+    if constexpr (std::is_same<IO, F32Any>::value) return io_load4(reinterpret_cast<const F32Any*>(p), n);
+    else return vec_load<4>(p);
 }
 
 // ---------------------------------------------------------------------------

@@ -140,11 +140,11 @@ struct FwdSinglePass {
         Bits4 raw[kPacked ? TS : 1][3];
     };
 
-    FL_HD static void take(State& st, int u, int plane, const IO* src) {
+    FL_HD static void take(State& st, int u, int plane, const IO* src, int nch) {
         if constexpr (kPacked) {
             st.raw[u][plane] = load_bits4(src);
         } else {
-            const Vec<4> z = vec_load_stream<4>(src);
+            const Vec<4> z = io_load4_stream(src, nch);
             F2(&d)[2] = plane == 0 ? st.br[u] : plane == 1 ? st.bi[u] : st.vac[u];
             d[0] = lo2(z); d[1] = hi2(z);
         }
@@ -185,6 +185,7 @@ struct FwdSinglePass {
         const int C = s.C;
         const int c0 = tl.cg * kGroup + lane * 4;
         const bool chan_ok = c0 < C;
+        const int nch = channels_at<IO>(c0, C);  // of this thread's four channels
         const int tw = tl.n * kTile + warp * TS;
 
         if constexpr (PH == 0) {
@@ -201,13 +202,13 @@ struct FwdSinglePass {
                 for (int u = 0; u < TS; ++u) {
                     if (tw + u < s.L) {
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) take(st, u, q, row + (size_t)q * C);
+                        for (int q = 0; q < 3; ++q) take(st, u, q, row + (size_t)q * C, nch);
                     }
                     row += pitch;
                 }
-                const Vec<4> lr4 = vec_load<4>(p.tr + c0);
-                const Vec<4> li4 = vec_load<4>(p.ti + c0);
-                const Vec<4> gm4 = vec_load<4>(p.gamma + c0);
+                const Vec<4> lr4 = par_load4<IO>(p.tr + c0, nch);
+                const Vec<4> li4 = par_load4<IO>(p.ti + c0, nch);
+                const Vec<4> gm4 = par_load4<IO>(p.gamma + c0, nch);
                 const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)}, gm[2] = {lo2(gm4), hi2(gm4)};
                 const F2 nli[2] = {mul2(li[0], splat2(-1.0f)), mul2(li[1], splat2(-1.0f))};
 #pragma unroll
@@ -303,9 +304,9 @@ struct FwdSinglePass {
                 }
                 return;
             }
-            const Vec<4> lr4 = vec_load<4>(p.tr + c0);
-            const Vec<4> li4 = vec_load<4>(p.ti + c0);
-            const Vec<4> gm4 = kPacked ? vec_load<4>(p.gamma + c0) : lr4;
+            const Vec<4> lr4 = par_load4<IO>(p.tr + c0, nch);
+            const Vec<4> li4 = par_load4<IO>(p.ti + c0, nch);
+            const Vec<4> gm4 = kPacked ? par_load4<IO>(p.gamma + c0, nch) : lr4;
             const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)}, gm[2] = {lo2(gm4), hi2(gm4)};
             const F2 nli[2] = {mul2(li[0], splat2(-1.0f)), mul2(li[1], splat2(-1.0f))};
             const Vec<4> sr4 = vec_load<4>(carry_at(smem, warp, 0) + lane * 4);
@@ -338,10 +339,10 @@ struct FwdSinglePass {
                         if constexpr (STATS)
                             sq = fma2(sr[h], sr[h], fma2(si[h], si[h], fma2(dr[h], dr[h], fma2(di[h], di[h], sq))));
                     }
-                    io_store4_stream(orow, join2(sr[0], sr[1]));
-                    io_store4_stream(orow + C, join2(si[0], si[1]));
-                    io_store4_stream(orow + 2 * C, join2(dr[0], dr[1]));
-                    io_store4_stream(orow + 3 * C, join2(di[0], di[1]));
+                    io_store4_stream(orow, join2(sr[0], sr[1]), nch);
+                    io_store4_stream(orow + C, join2(si[0], si[1]), nch);
+                    io_store4_stream(orow + 2 * C, join2(dr[0], dr[1]), nch);
+                    io_store4_stream(orow + 3 * C, join2(di[0], di[1]), nch);
                     // the map area is free after the look-back: one partial per lane and step
                     if constexpr (STATS) smem[(warp * TS + u) * kStatRow + lane] = sq.x + sq.y;
                     orow += (size_t)4 * C;
@@ -795,6 +796,7 @@ struct BwdSinglePass {
         const int C = s.C;
         const int c0 = tl.cg * kGroup + lane * 4;
         const bool chan_ok = c0 < C;
+        const int nch = channels_at<IO>(c0, C);  // of this thread's four channels
         const int tbeg = time_tile * kTile + warp * TS;           // first step of the warp
         const int tend = tbeg + TS < s.L ? tbeg + TS : s.L;       // one past its last valid step
 
@@ -812,8 +814,8 @@ struct BwdSinglePass {
             }
             Affine2 m[2] = {affine2_identity(), affine2_identity()};
             if (chan_ok) {
-                const Vec<4> lr = vec_load<4>(p.tr + c0);
-                const Vec<4> li = vec_load<4>(p.ti + c0);
+                const Vec<4> lr = par_load4<IO>(p.tr + c0, nch);
+                const Vec<4> li = par_load4<IO>(p.ti + c0, nch);
                 const F2 lr2[2] = {lo2(lr), hi2(lr)}, li2[2] = {lo2(li), hi2(li)};
                 const F2 nli2[2] = {mul2(li2[0], splat2(-1.0f)), mul2(li2[1], splat2(-1.0f))};
                 const IO* zbase = p.raw + ((size_t)tl.b * s.L) * s.zp + 2 * C + c0;
@@ -829,11 +831,11 @@ struct BwdSinglePass {
                     for (int u = 0; u < U1; ++u) {
                         if (t_issue - 1 - u >= tbeg) {
                             const IO* grow = gq - (ptrdiff_t)u * 4 * C;
-                            async_copy4(cell_at(smem, stage, u * 5 + 0, thread), zq - (ptrdiff_t)u * s.zp);
-                            async_copy4(cell_at(smem, stage, u * 5 + 1, thread), grow);
-                            async_copy4(cell_at(smem, stage, u * 5 + 2, thread), grow + C);
-                            async_copy4(cell_at(smem, stage, u * 5 + 3, thread), grow + 2 * C);
-                            async_copy4(cell_at(smem, stage, u * 5 + 4, thread), grow + 3 * C);
+                            async_copy4(cell_at(smem, stage, u * 5 + 0, thread), zq - (ptrdiff_t)u * s.zp, nch);
+                            async_copy4(cell_at(smem, stage, u * 5 + 1, thread), grow, nch);
+                            async_copy4(cell_at(smem, stage, u * 5 + 2, thread), grow + C, nch);
+                            async_copy4(cell_at(smem, stage, u * 5 + 3, thread), grow + 2 * C, nch);
+                            async_copy4(cell_at(smem, stage, u * 5 + 4, thread), grow + 3 * C, nch);
                         }
                     }
                     t_issue -= U1;
@@ -866,12 +868,12 @@ struct BwdSinglePass {
                     for (int u = 0; u < U1; ++u) {
                         const int t = t0 - 1 - u;
                         if (t >= tbeg) {
-                            zv[u] = io_load4(zbase + (size_t)t * s.zp);
+                            zv[u] = io_load4(zbase + (size_t)t * s.zp, nch);
                             const IO* grow = gbase + (size_t)t * 4 * C;
-                            ur[u] = io_load4(grow);
-                            ui[u] = io_load4(grow + C);
-                            gr[u] = io_load4(grow + 2 * C);
-                            gi[u] = io_load4(grow + 3 * C);
+                            ur[u] = io_load4(grow, nch);
+                            ui[u] = io_load4(grow + C, nch);
+                            gr[u] = io_load4(grow + 2 * C, nch);
+                            gi[u] = io_load4(grow + 3 * C, nch);
                         }
                     }
                     }
@@ -927,9 +929,9 @@ struct BwdSinglePass {
             const F2 zero2 = splat2(0.0f);
             BwdAcc2 acc[2] = {{zero2, zero2, zero2, zero2}, {zero2, zero2, zero2, zero2}};
             if (chan_ok) {
-                const Vec<4> lr = vec_load<4>(p.tr + c0);
-                const Vec<4> li = vec_load<4>(p.ti + c0);
-                const Vec<4> gm = vec_load<4>(p.gamma + c0);
+                const Vec<4> lr = par_load4<IO>(p.tr + c0, nch);
+                const Vec<4> li = par_load4<IO>(p.ti + c0, nch);
+                const Vec<4> gm = par_load4<IO>(p.gamma + c0, nch);
                 const F2 lr2[2] = {lo2(lr), hi2(lr)}, li2[2] = {lo2(li), hi2(li)};
                 const F2 nli2[2] = {mul2(li2[0], splat2(-1.0f)), mul2(li2[1], splat2(-1.0f))};
                 const F2 gm2[2] = {lo2(gm), hi2(gm)};
@@ -951,17 +953,17 @@ struct BwdSinglePass {
                         if (t >= tbeg) {
                             const IO* zrow = zq - (ptrdiff_t)u * s.zp;
                             const IO* grow = gq - (ptrdiff_t)u * 4 * C;
-                            async_copy4(cell_at(smem, stage, u * 9 + 0, thread), zrow);
-                            async_copy4(cell_at(smem, stage, u * 9 + 1, thread), zrow + C);
-                            async_copy4(cell_at(smem, stage, u * 9 + 2, thread), zrow + 2 * C);
-                            async_copy4(cell_at(smem, stage, u * 9 + 3, thread), grow);
-                            async_copy4(cell_at(smem, stage, u * 9 + 4, thread), grow + C);
-                            async_copy4(cell_at(smem, stage, u * 9 + 5, thread), grow + 2 * C);
-                            async_copy4(cell_at(smem, stage, u * 9 + 6, thread), grow + 3 * C);
+                            async_copy4(cell_at(smem, stage, u * 9 + 0, thread), zrow, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 1, thread), zrow + C, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 2, thread), zrow + 2 * C, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 3, thread), grow, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 4, thread), grow + C, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 5, thread), grow + 2 * C, nch);
+                            async_copy4(cell_at(smem, stage, u * 9 + 6, thread), grow + 3 * C, nch);
                             if (t > 0) {
                                 const IO* prow = rq - (ptrdiff_t)u * 4 * C;
-                                async_copy4(cell_at(smem, stage, u * 9 + 7, thread), prow);
-                                async_copy4(cell_at(smem, stage, u * 9 + 8, thread), prow + C);
+                                async_copy4(cell_at(smem, stage, u * 9 + 7, thread), prow, nch);
+                                async_copy4(cell_at(smem, stage, u * 9 + 8, thread), prow + C, nch);
                             }
                         }
                     }
@@ -997,8 +999,8 @@ struct BwdSinglePass {
                                     pi[u] = cell_load4<IO>(cell_at(smem, stage, u * 9 + 8, thread));
                                 } else if (p.state_in) {
                                     const float* prow = p.state_in + (size_t)tl.b * 2 * C + c0;
-                                    pr[u] = vec_load<4>(prow);
-                                    pi[u] = vec_load<4>(prow + C);
+                                    pr[u] = par_load4<IO>(prow, nch);
+                                    pi[u] = par_load4<IO>(prow + C, nch);
                                 } else {
                                     pr[u] = vec_fill<4>(0.0f);
                                     pi[u] = vec_fill<4>(0.0f);
@@ -1011,22 +1013,22 @@ struct BwdSinglePass {
                         const int t = t0 - 1 - u;
                         if (t >= tbeg) {
                             const IO* zrow = zbase + (size_t)t * s.zp;
-                            zr[u] = io_load4_stream(zrow);
-                            zi[u] = io_load4_stream(zrow + C);
-                            zv[u] = io_load4_stream(zrow + 2 * C);
+                            zr[u] = io_load4_stream(zrow, nch);
+                            zi[u] = io_load4_stream(zrow + C, nch);
+                            zv[u] = io_load4_stream(zrow + 2 * C, nch);
                             const IO* grow = gbase + (size_t)t * 4 * C;
-                            ur[u] = io_load4_stream(grow);
-                            ui[u] = io_load4_stream(grow + C);
-                            gr[u] = io_load4_stream(grow + 2 * C);
-                            gi[u] = io_load4_stream(grow + 3 * C);
+                            ur[u] = io_load4_stream(grow, nch);
+                            ui[u] = io_load4_stream(grow + C, nch);
+                            gr[u] = io_load4_stream(grow + 2 * C, nch);
+                            gi[u] = io_load4_stream(grow + 3 * C, nch);
                             if (t > 0) {
                                 const IO* prow = rbase + (size_t)(t - 1) * 4 * C;
-                                pr[u] = io_load4_stream(prow);
-                                pi[u] = io_load4_stream(prow + C);
+                                pr[u] = io_load4_stream(prow, nch);
+                                pi[u] = io_load4_stream(prow + C, nch);
                             } else if (p.state_in) {
                                 const float* prow = p.state_in + (size_t)tl.b * 2 * C + c0;
-                                pr[u] = vec_load<4>(prow);
-                                pi[u] = vec_load<4>(prow + C);
+                                pr[u] = par_load4<IO>(prow, nch);
+                                pi[u] = par_load4<IO>(prow + C, nch);
                             } else {
                                 pr[u] = vec_fill<4>(0.0f);
                                 pi[u] = vec_fill<4>(0.0f);
@@ -1046,9 +1048,9 @@ struct BwdSinglePass {
                                       hi2(gr[u]), hi2(gi[u]), hi2(pr[u]), hi2(pi[u]), lr2[1], li2[1],
                                       nli2[1], gm2[1], cr[1], ci[1], acc[1], ozr[1], ozi[1], ozv[1]);
                             IO* orow = obase + (size_t)t * s.gp;
-                            io_store4_stream(orow, join2(ozr[0], ozr[1]));
-                            io_store4_stream(orow + C, join2(ozi[0], ozi[1]));
-                            io_store4_stream(orow + 2 * C, join2(ozv[0], ozv[1]));
+                            io_store4_stream(orow, join2(ozr[0], ozr[1]), nch);
+                            io_store4_stream(orow + C, join2(ozi[0], ozi[1]), nch);
+                            io_store4_stream(orow + 2 * C, join2(ozv[0], ozv[1]), nch);
                         }
                     }
                 }

@@ -105,6 +105,26 @@ FL_HD void async_copy4(float* cell, const uint16_t* src) {
 #endif
 }
 
+// The same where only the first n elements may exist (see F32Any).
+template <typename IO>
+FL_HD void async_copy4(float* cell, const IO* src, int n) {
+    if constexpr (std::is_same<IO, F32Any>::value) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k < n) {
+#if FL_DEVICE_CODE
+                const unsigned saddr = (unsigned)__cvta_generic_to_shared(cell + k);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(src + k) : "memory");
+#else
+                cell[k] = src[k].v;
+#endif
+            }
+        }
+    } else {
+        async_copy4(cell, src);
+    }
+}
+
 // Reads back a cell filled by async_copy4 from a source of element type IO.
 template <typename IO>
 FL_HD Vec<4> cell_load4(const float* cell) {

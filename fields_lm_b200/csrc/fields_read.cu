@@ -546,6 +546,7 @@ static long long tile_blocks(const Shape& s) {
     return (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
 }
 
+#ifdef FIELDS_ALL_VARIANTS
 template <int VEC>
 static int run_forward(const FwdParams& p, Stream st) {
     const Shape& s = p.s;
@@ -569,6 +570,7 @@ static int run_backward(const BwdParams& p, Stream st) {
     if (rc) return rc;
     return launch<BwdReduce>(p, 3LL * ((s.C + 31) / 32), st);
 }
+#endif
 
 
 // ---------------------------------------------------------------------------
@@ -611,10 +613,10 @@ static SpPlan make_sp_plan(int B, int L, int C, int tile_steps) {
 
 enum Algo { kAlgoAuto = 0, kAlgoThreePhase = 1, kAlgoSinglePass = 2, kAlgoWalk = 3 };
 
-// The product library runs one kernel family: single pass wherever 128-bit accesses are
-// possible, the scalar three-phase kernels otherwise. The measured alternatives (other tile
+// The product library runs one kernel family, single pass (with 32-bit accesses where 128-bit ones are not
+// possible). The measured alternatives (other tile
 // shapes, the two-sweep forward, the direct-load and tile-resident backward, the chain walkers,
-// the vectorised three-phase kernels, L2 prefetch) are compiled only into the test build
+// the three-phase kernels, L2 prefetch) are compiled only into the test build
 // (FIELDS_ALL_VARIANTS), which picks them per call from the environment:
 //   FIELDS_READ_ALGO = three_phase | single_pass | walk, FIELDS_FWD_VARIANT, FIELDS_BWD_VARIANT,
 //   FIELDS_READ_PREFETCH.
@@ -638,8 +640,15 @@ static Algo algo_from_env() { return kAlgoAuto; }
 // Three blocks of four warps per SM at 168 registers hold 108 steps of 128 channels (four blocks at 128
 // registers with 24-step tiles: 96). At 1 x 65,536 x 512 189 -> 183 us against the earlier two blocks of
 // eight warps and 48-step tiles, at 1 x 16,384 54.2 -> 51.8, at 2 x 3,001 x 384 20.6 -> 19.5, equal at
-// 8 x 2,048. Longer tiles spill.
+// 8 x 2,048. From eight rounds of blocks on, where the last one weighs little, 40-step tiles are a little
+// faster in spite of a few spilled registers: 183 -> 179 us at 1 x 65,536, 175 -> 171 at 4 x 16,384.
 using FwdSp0 = FwdSinglePass<9, 4, 3>;
+using FwdSpDeep = FwdSinglePass<10, 4, 3>;
+static long long tiles_of(int B, int L, int C, int steps) {
+    return (long long)B * ((C + kGroup - 1) / kGroup) * ((L + steps - 1) / steps);
+}
+// Tensors without 128-bit access (F32Any), forward and backward: the same kernels with four 32-bit accesses.
+using FwdSpAny = FwdSinglePass<6, 4, 3, F32Any>;
 using FwdSpRows = FwdSinglePass<9, 4, 3, float, false, true>;  // also writes state rows
 #ifdef FIELDS_ALL_VARIANTS
 using FwdSp1 = FwdSinglePass<4, 8, 2>;        // tile 32
@@ -648,6 +657,7 @@ using FwdSp2 = FwdTwoSweep<8, 4, 2, 4, 3>;    // tile 32, 16 warps per SM
 #endif
 //   backward <steps per warp, warps, sweep-1 unroll, sweep-2 unroll, blocks per SM, rings, ring slots>
 using BwdSp0 = BwdSinglePass<8, 4, 2, 1, 3, true, 3>;  // tile 32, 3-slot cp.async rings, 12 warps per SM
+using BwdSpAny = BwdSinglePass<8, 4, 2, 1, 3, true, 3, F32Any>;
 #ifdef FIELDS_ALL_VARIANTS
 using BwdSp1 = BwdSinglePass<8, 4, 2, 1, 4>;           // direct loads, 16 warps per SM
 #endif
@@ -663,7 +673,7 @@ using BwdSp3 = BwdTileResident<4, 4, 3>;      // tile 16, 68 KB per block, 12 wa
 // tiles), 43.2 / 41.4 at 1 x 16,384, 150 / 142 at 1 x 65,536, 129 / 128 at 8 x 8,192. The second
 // needs tiles enough that a part-filled last round costs little: the line is at 3,500 small tiles.
 static bool deep_tiles(int B, int L, int C) {
-    return (long long)B * ((C + kGroup - 1) / kGroup) * ((L + 39) / 40) >= 3500;
+    return tiles_of(B, L, C, 40) >= 3500;
 }
 template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;
 template <bool STATS> using FwdSpBf16Deep = FwdSinglePass<10, 8, 2, uint16_t, STATS>;  // STATS: per-token sums of squares too
@@ -1018,16 +1028,22 @@ int fields_read_forward(const float* raw, const float* tr, const float* ti, cons
             default: break;
         }
 #endif
+        if (tiles_of(B, L, C, 40) >= 8 * 3 * 148) FIELDS_FWD_SP(FwdSpDeep);
         FIELDS_FWD_SP(FwdSp0);
 #undef FIELDS_FWD_SP
     }
+    if (algo != kAlgoThreePhase)
+        return run_forward_single_pass<FwdSpAny, F32Any>(reinterpret_cast<const F32Any*>(raw), tr, ti, gamma, state_in,
+                                                         reinterpret_cast<F32Any*>(read), state_out, workspace, B, L, C,
+                                                         st);
+#ifdef FIELDS_ALL_VARIANTS
     float* ws = static_cast<float*>(workspace);
     FwdParams p{raw, tr, ti, gamma, state_in, read, state_out,
                 ws + pl.sum_off, ws + pl.carry_off, pl.s};
-#ifdef FIELDS_ALL_VARIANTS
-    if (vec4) return run_forward<4>(p, st);
+    return vec4 ? run_forward<4>(p, st) : run_forward<1>(p, st);
+#else
+    return FIELDS_ERR_UNSUPPORTED;  // (not reached)
 #endif
-    return run_forward<1>(p, st);
 }
 
 int fields_read_backward(const float* raw, const float* tr, const float* ti, const float* gamma,
@@ -1099,14 +1115,21 @@ int fields_read_backward(const float* raw, const float* tr, const float* ti, con
 #endif
 #undef FIELDS_BWD_SP
     }
+    if (algo_from_env() != kAlgoThreePhase) {
+        auto any = [](const float* q) { return reinterpret_cast<const F32Any*>(q); };
+        return run_backward_single_pass<BwdSpAny, F32Any>(any(raw), tr, ti, gamma, state_in, any(read), any(grad_read),
+                                                          grad_state_out, reinterpret_cast<F32Any*>(grad_raw), grad_tr,
+                                                          grad_ti, grad_gamma, grad_state_in, workspace, B, L, C, st);
+    }
+#ifdef FIELDS_ALL_VARIANTS
     float* ws = static_cast<float*>(workspace);
     BwdParams p{raw, tr, ti, gamma, state_in, read, grad_read, grad_state_out, grad_raw,
                 grad_state_in, ws + pl.sum_off, ws + pl.carry_off, ws + pl.partial_off,
                 grad_tr, grad_ti, grad_gamma, pl.s};
-#ifdef FIELDS_ALL_VARIANTS
-    if (vec4) return run_backward<4>(p, st);
+    return vec4 ? run_backward<4>(p, st) : run_backward<1>(p, st);
+#else
+    return FIELDS_ERR_UNSUPPORTED;  // (not reached)
 #endif
-    return run_backward<1>(p, st);
 }
 
 

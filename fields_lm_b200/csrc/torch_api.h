@@ -109,15 +109,14 @@ inline bool all_aligned(std::initializer_list<const void*> ptrs, uintptr_t bytes
 // One is kept per stream (fields_read_use_kept), for the last few streams, up to a size: that saves an
 // allocation and a fill launch per pass, about 4 us of host time and 2 us on the GPU. It is held
 // (locked) while a pass is issued, because a pass may be two launches. Passes that are captured into a
-// graph, larger ones, and the scalar kernels (`vector` false: they use a workspace as plain scratch) get
-// one of their own, as does every pass where the library refuses.
+// graph and larger ones get one of their own, as does every pass where the library refuses.
 class PassWorkspace {
   public:
-    PassWorkspace(size_t need, const Tensor& on, bool vector) : bytes_(need) {
+    PassWorkspace(size_t need, const Tensor& on) : bytes_(need) {
         const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(on.device().index());
         // (torch's own streams: another library's may be destroyed while work is pending)
         const bool own_stream = stream.id() == 0 || (stream.id() & 1);
-        if (vector && need <= kMostBytes && own_stream &&
+        if (need <= kMostBytes && own_stream &&
             c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
             kept_ = entry(on.device().index(), stream.id());
             lock_ = std::unique_lock<std::mutex>(kept_->mu);

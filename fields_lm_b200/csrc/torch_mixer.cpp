@@ -58,7 +58,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         const Tensor read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
-            PassWorkspace ws(n, u, true);
+            PassWorkspace ws(n, u);
             float* p = fp(par);
             ws.check(f.fields_read_forward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, nullptr, vp(read), fp(groups), nullptr,
                                                   ws.ptr(), n, (int)B, (int)L, (int)C, st),
@@ -110,7 +110,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         float* p = fp(par);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
-            PassWorkspace ws(n, u, true);
+            PassWorkspace ws(n, u);
             ws.check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
                                                    g, g + C, g + 2 * C, ws.ptr(), n, (int)B, (int)L, (int)C, st),
                   "fields_read_backward_bf16_rows");

@@ -62,9 +62,8 @@ static void run_forward(const ForwardArgs& a, Tensor& read, Tensor& state_out, b
     read = empty({B, L, 4 * C}, at::kFloat, dev);
     if (want_state) state_out = empty({B, 2 * C}, at::kFloat, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
-    const bool vector = C % 4 == 0 && all_aligned({fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in)}, 16);
-    PassWorkspace ws(n, a.raw, vector);
-    if (rows && vector && B > 0 && L >= 8) {
+    PassWorkspace ws(n, a.raw);
+    if (rows && all_aligned({fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in)}, 16) && B > 0 && L >= 8) {
         *rows = empty({B, L / 8, 2 * C}, at::kFloat, dev);
         ws.check(f.fields_read_forward_rows(fp(a.raw), fp(a.tr), fp(a.ti), fp(a.gm), fp(a.state_in), fp(read), fp(state_out),
                                             fp(*rows), ws.ptr(), n, B, L, C, stream_of(a.raw)),
@@ -112,8 +111,7 @@ struct FieldRead : torch::autograd::Function<FieldRead> {
         Tensor g_sin;
         if (state_in.defined() && ctx->needs_input_grad(4)) g_sin = empty({B, 2 * C}, at::kFloat, dev);
         const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
-        PassWorkspace ws(n, raw, C % 4 == 0 && all_aligned({fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), fp(read),
-                                                                  fp(grad_read)}, 16));
+        PassWorkspace ws(n, raw);
         auto* entry = lean ? f.fields_read_backward_from_states : f.fields_read_backward;
         // (lean: `read` holds the kept state rows, possibly none for L < 8)
         ws.check(entry(fp(raw), fp(tr), fp(ti), fp(gm), fp(state_in), read.numel() ? fp(read) : nullptr,
@@ -135,7 +133,7 @@ static variable_list run_forward_bf16(const Tensor& raw, const Tensor& tr, const
     const c10::cuda::CUDAGuard guard(dev);
     const Tensor read = empty({B, L, 4 * C}, at::kBFloat16, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_FORWARD);
-    PassWorkspace ws(n, raw, true);
+    PassWorkspace ws(n, raw);
     if (!stats) {
         ws.check(f.fields_read_forward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), nullptr,
                                          ws.ptr(), n, B, L, C, stream_of(raw)),
@@ -158,7 +156,7 @@ static variable_list run_backward_bf16(const Tensor& raw, const Tensor& tr, cons
     const Tensor grad_raw = empty({B, L, 3 * C}, at::kBFloat16, dev);
     const Tensor g_par = empty({3, C}, at::kFloat, dev);
     const size_t n = f.fields_read_workspace_bytes(B, L, C, FIELDS_PASS_BACKWARD);
-    PassWorkspace ws(n, raw, true);
+    PassWorkspace ws(n, raw);
     ws.check(f.fields_read_backward_bf16(vp(raw), fp(tr), fp(ti), fp(gm), nullptr, vp(read), vp(grad_read),
                                       nullptr, vp(grad_raw), fp(g_par), fp(g_par) + C, fp(g_par) + 2 * C,
                                       nullptr, ws.ptr(), n, B, L, C, stream_of(raw)),

@@ -131,7 +131,7 @@ class FieldStack {
         for (const Block& b : blocks_) {
             at::cuda::addmm_out(u, b.in_b, xb, b.in_t, 1, 1);
             const Tensor state = empty({B, D}, at::kFloat, dev);
-            PassWorkspace ws(ws_bytes, u, true);
+            PassWorkspace ws(ws_bytes, u);
             float* par = fp(b.par);
             ws.check(f.fields_read_forward_bf16_rows(vp(u), W, par, par + C, par + 2 * C, nullptr, vp(read), fp(groups),
                                                   fp(state), ws.ptr(), ws_bytes, (int)B, (int)L, (int)C, st),
