@@ -549,6 +549,51 @@ struct BwdReduce {
     }
 };
 
+// BwdReduce, and beside it blocks that fill what is used of a kept workspace with the unset pattern, so that
+// neither the next forward nor the next backward needs a fill launch (two launches a step). The sums leave
+// most of the GPU idle. Step of the operator through the package, before and after: 130.6 -> 128.8 us at
+// 8 x 2,048 x 512, 93.4 -> 91.6 in bfloat16, 72.4 -> 66.9 at 3 x 777 x 132, 88.7 -> 83.1 at 2 x 3,001 x 384 from state rows.
+struct BwdReduceParams : BwdParams {
+    unsigned* clean[2];    // 16-byte aligned
+    unsigned clean_n[2];   // 16-byte words
+    int reduce_blocks;     // blocks from here on clean
+    int clean_blocks;
+};
+
+struct BwdReduceClean {
+    using Params = BwdReduceParams;
+    static constexpr int kThreads = BwdReduce::kThreads;
+    static constexpr int kPhases = 2;
+    static constexpr int kSmemFloats = BwdReduce::kSmemFloats;
+    static constexpr int kWordsPerThread = 4;
+    static int blocks_for(long long words) {
+        const long long n = (words + kThreads * kWordsPerThread - 1) / (kThreads * kWordsPerThread);
+        return (int)(n < 296 ? n : 296);  // what the GPU holds at once
+    }
+
+    FL_HD static void phase0(const Params& p, int block, int thread, float* smem) {
+        if (block < p.reduce_blocks) {
+            BwdReduce::phase0(p, block, thread, smem);
+            return;
+        }
+        const unsigned stride = (unsigned)p.clean_blocks * kThreads;
+        const unsigned first = (unsigned)(block - p.reduce_blocks) * kThreads + thread;
+        for (int h = 0; h < 2; ++h) {
+            for (unsigned i = first; i < p.clean_n[h]; i += stride) {
+#if FL_DEVICE_CODE
+                reinterpret_cast<uint4*>(p.clean[h])[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+#else
+                std::memset(p.clean[h] + (size_t)i * 4, 0xFF, 16);
+#endif
+            }
+        }
+    }
+
+    FL_HD static void phase1(const Params& p, int block, int thread, float* smem) {
+        if (block < p.reduce_blocks) BwdReduce::phase1(p, block, thread, smem);
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Span summary: the affine map of a whole span per (batch, channel), composed from
 // the chunk maps that FwdSummary wrote. One block owns 32 channels of one batch row;

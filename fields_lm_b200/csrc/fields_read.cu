@@ -711,10 +711,13 @@ static thread_local fields_kept* g_next_kept = nullptr;
 struct ReadyWorkspace {
     unsigned* ctrl;
     float *agg, *incl, *partial;
+    fields_kept* kept;  // null: not a kept workspace
+    char* half[2];
 };
 
-// Makes a workspace ready for a pass of the single-pass kernels.
-static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspace* out) {
+// Makes a workspace ready for a pass of the single-pass kernels. cleaned_after: a kernel behind the pass fills
+// what is used of a kept workspace (BwdReduceClean).
+static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspace* out, bool cleaned_after = false) {
     char* ws = static_cast<char*>(workspace);
     fields_kept* k = g_next_kept;
     g_next_kept = nullptr;
@@ -722,18 +725,23 @@ static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspac
     const size_t slot_bytes = pl.bytes - pl.agg_off;
     out->ctrl = reinterpret_cast<unsigned*>(ws);
     out->partial = reinterpret_cast<float*>(ws + pl.bytes);
+    out->kept = k;
     int rc = FIELDS_OK;
     if (k) {
-        // A small pass publishes in one half, which is unset, and fills what was used of the other. Up to
-        // 592 tiles (four per SM): there the fill launch shows, in host time above all (20.1 -> 19.2 us of GPU at
-        // 2 x 3,001 x 384, 13.6 -> 12.7 at 1 x 2,048 x 512); above, the code in the kernel costs as much.
+        // A pass publishes in one half. Where that half is unset no fill is needed; a small pass (up to 592
+        // tiles, four per SM) also fills what was used of the other: there the fill launch shows, in host time
+        // above all (20.1 -> 19.2 us of GPU at 2 x 3,001 x 384, 13.6 -> 12.7 at 1 x 2,048 x 512); above, the code in
+        // the kernel costs as much, and the half stays as it is until the reduction of a backward pass fills
+        // both, or a pass meets it and fills it first.
         if (slot_bytes > k->half_bytes) return FIELDS_ERR_WORKSPACE;
         const unsigned h = k->parity & 1;
-        char* half[2] = {ws + pl.agg_off, ws + pl.agg_off + k->half_bytes};
+        char** half = out->half;
+        half[0] = ws + pl.agg_off;
+        half[1] = half[0] + k->half_bytes;
         slots = half[h];
         out->partial = reinterpret_cast<float*>(half[1] + k->half_bytes);
         const size_t used = k->dirty[1 - h];
-        if (pl.tiles <= 592 && k->dirty[h] == 0) {
+        if (pl.tiles <= 592 && k->dirty[h] == 0 && !cleaned_after) {
             if (used > (size_t)pl.tiles * 16384) {  // a much larger pass was before: too much for these blocks
                 rc = fill_unset(half[1 - h], used, st);
             } else {
@@ -744,7 +752,7 @@ static int ready_workspace(void* workspace, SpPlan& pl, Stream st, ReadyWorkspac
             k->dirty[h] = slot_bytes;
             k->parity = 1 - h;
         } else {
-            rc = fill_unset(slots, slot_bytes, st);
+            if (k->dirty[h]) rc = fill_unset(slots, slot_bytes, st);
             if (k->dirty[h] < slot_bytes) k->dirty[h] = slot_bytes;
             if (used == 0) k->parity = 1 - h;
         }
@@ -787,27 +795,37 @@ static int run_backward_single_pass(const IO* raw, const float* tr, const float*
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (raw_pitch) pl.s.zp = (int)raw_pitch;
     if (grad_pitch) pl.s.gp = (int)grad_pitch;
+    // Up to 16 partial rows the last block of a channel group adds them: a launch less, 2.5 us of GPU and as
+    // much of host time. (At 64 rows that block took 5 us longer than the reduction kernel.)
+#ifdef FIELDS_HOST_EMU
+    const bool fold = false;
+#else
+    const bool fold = (long long)B * pl.s.NT <= 16 && pl.s.G <= kCtrlHeader - 2;
+#endif
     ReadyWorkspace ws;
-    int rc = ready_workspace(workspace, pl, st, &ws);
+    int rc = ready_workspace(workspace, pl, st, &ws, !fold);
     if (rc) return rc;
     SpBwdParamsT<IO> p{raw, tr, ti, gamma, state_in, read, grad_read, grad_state_out, grad_raw,
                        grad_state_in, ws.agg, ws.incl, ws.ctrl, ws.partial, pl.s};
     p.states = states;
     p.state_rows = L / kStateRowEvery;
-#ifndef FIELDS_HOST_EMU
-    // Up to 16 partial rows the last block of a channel group adds them: a launch less, 2.5 us of GPU and as
-    // much of host time. (At 64 rows that block took 5 us longer than the reduction kernel.)
-    if ((long long)B * pl.s.NT <= 16 && pl.s.G <= kCtrlHeader - 2) {
-        p.grad_par[0] = grad_tr; p.grad_par[1] = grad_ti; p.grad_par[2] = grad_gamma;
-    }
-#endif
-    rc = launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st, pl.s.clean_n > 0 || p.grad_par[0]);
-    if (rc || p.grad_par[0]) return rc;
-    BwdParams rp{};
+    if (fold) { p.grad_par[0] = grad_tr; p.grad_par[1] = grad_ti; p.grad_par[2] = grad_gamma; }
+    rc = launch_stateful<K>(p, pl.tiles, (long long)B * pl.s.G, st, pl.s.clean_n > 0 || fold);
+    if (rc || fold) return rc;
+    BwdReduceClean::Params rp{};
     rp.partial = ws.partial;
     rp.grad_tr = grad_tr; rp.grad_ti = grad_ti; rp.grad_gamma = grad_gamma;
     rp.s = Shape{B, L, C, K::kTile, pl.s.NT, pl.s.G};
-    return launch<BwdReduce>(rp, 3LL * ((C + 31) / 32), st);
+    rp.reduce_blocks = 3 * ((C + 31) / 32);
+    if (fields_kept* k = ws.kept) {
+        for (int h = 0; h < 2; ++h) {
+            rp.clean[h] = reinterpret_cast<unsigned*>(ws.half[h]);
+            rp.clean_n[h] = (unsigned)(k->dirty[h] / 16);
+            k->dirty[h] = 0;
+        }
+        rp.clean_blocks = BwdReduceClean::blocks_for((long long)rp.clean_n[0] + rp.clean_n[1]);
+    }
+    return launch<BwdReduceClean>(rp, rp.reduce_blocks + rp.clean_blocks, st);
 }
 
 static size_t sp_backward_bytes(int B, int L, int C, int tile_steps) {

@@ -60,8 +60,8 @@ int fields_read_version(void);
  * workspace for such passes alone, on one stream, can save that fill: it has 256 + 3 * half_bytes
  * bytes (half_bytes a multiple of 256, at least fields_read_workspace_bytes of every pass) filled with
  * 0xFF once, and a fields_kept zeroed but for half_bytes. fields_read_use_kept(k) before a pass makes the
- * calling thread's next pass take the workspace as that and update *k: the two halves take turns, and a
- * pass fills what the one before it used. Such a call must not be replayed from a captured graph.
+ * calling thread's next pass take the workspace as that and update *k: the two halves take turns, and
+ * what was used is filled by a pass, beside its own work, for the ones after it. Such a call must not be replayed from a captured graph.
  * fields_read_use_kept(NULL) takes it back; after a pass that returned an error start from the fill.
  */
 struct fields_kept {

@@ -49,6 +49,22 @@ def test_extents_and_forms_in_any_order():
             assert rel_err(g.cpu().numpy(), w.numpy()) < 1e-6
 
 
+# the reduction of a backward pass fills both halves: after passes without it (none, one, two, more of them),
+# below and above the extent up to which a pass fills for itself, and with halves of unlike extent
+@pytest.mark.parametrize("B,L,C", [(17, 31, 132), (2, 1500, 384), (8, 2048, 512)])
+def test_halves_after_forwards_alone(B, L, C):
+    leaves, grad = _case(B, L, C, 5)
+    host = [t.detach().cpu().numpy() for t in leaves]
+    want = [field_oracle.forward(*host)[0], *field_oracle.backward(*host, grad.cpu().numpy())[:4]]
+    other = [t.detach() for t in _case(3, 1900, 512, 6)[0]]
+    for forwards in (0, 1, 2, 3, 0, 0):
+        with torch.no_grad():
+            for i in range(forwards):
+                fused_field_read(*(other if i == 1 else leaves))
+        for g, w in zip(_pass(leaves, grad), want):
+            assert rel_err(g.cpu().numpy(), np.asarray(w)) < FP32_TOL
+
+
 def test_streams_and_threads():
     cases = [_case(2, 1500 + 100 * i, 256, i) for i in range(4)]
     want = [[t.cpu() for t in _pass(*c)] for c in cases]
