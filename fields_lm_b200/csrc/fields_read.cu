@@ -648,7 +648,7 @@ static long long tiles_of(int B, int L, int C, int steps) {
     return (long long)B * ((C + kGroup - 1) / kGroup) * ((L + steps - 1) / steps);
 }
 // Tensors without 128-bit access (F32Any), forward and backward: the same kernels with four 32-bit accesses.
-using FwdSpAny = FwdSinglePass<6, 4, 3, F32Any>;
+using FwdSpAny = FwdSinglePass<8, 4, 3, F32Any>;
 using FwdSpRows = FwdSinglePass<9, 4, 3, float, false, true>;  // also writes state rows
 #ifdef FIELDS_ALL_VARIANTS
 using FwdSp1 = FwdSinglePass<4, 8, 2>;        // tile 32
@@ -681,8 +681,10 @@ template <bool STATS> using FwdSpBf16Deep = FwdSinglePass<10, 8, 2, uint16_t, ST
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
 // 16-byte cells) on 8 x 2,048 tokens.
 using BwdSpBf16 = BwdSinglePass<16, 4, 2, 1, 3, true, 3, uint16_t>;
-constexpr int kSpMinTile = 32;     // smallest time tile of any forward instantiation above (workspace bound)
-constexpr int kSpMinTileBwd = 16;  // same for the backward
+// Smallest time tile of any instantiation above, for the workspace bound (the run functions assert it). The
+// bound also decides which extents fields_read_forward_noalloc takes.
+constexpr int kSpMinTile = 32;
+constexpr int kSpMinTileBwd = 16;
 
 #ifdef FIELDS_ALL_VARIANTS
 static int variant_from_env(const char* name) {
@@ -770,6 +772,7 @@ static int run_forward_single_pass(const IO* raw, const float* tr, const float* 
                                    float* state_out, void* workspace, int B, int L, int C,
                                    Stream st, float* sumsq = nullptr, long long pitch = 0,
                                    float* rows = nullptr) {
+    static_assert(K::kTile >= kSpMinTile, "fields_read_workspace_bytes counts the slots of tiles of kSpMinTile steps");
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (pitch) pl.s.zp = (int)pitch;
@@ -791,6 +794,7 @@ static int run_backward_single_pass(const IO* raw, const float* tr, const float*
                                     int B, int L, int C, Stream st,
                                     const float* states = nullptr, long long raw_pitch = 0,
                                     long long grad_pitch = 0) {
+    static_assert(K::kTile >= kSpMinTileBwd, "fields_read_workspace_bytes counts the slots of tiles of that many steps");
     SpPlan pl = make_sp_plan(B, L, C, K::kTile);
     pl.s.prefetch = prefetch_from_env(resident_blocks<K>());
     if (raw_pitch) pl.s.zp = (int)raw_pitch;

@@ -77,6 +77,36 @@ def test_scalar_path_equals_vector_path():
     assert rel_err(sa, sb) < 1e-6
 
 
+# odd widths and unaligned pointers take kernels with a tile of their own; workspaces of exactly the stated size
+@pytest.mark.parametrize("B,L,C,misalign", [(1, 777, 33, False), (2, 300, 25, False), (1, 500, 130, False),
+                                            (2, 400, 333, False), (1, 600, 132, True), (1, 35, 512, True),
+                                            (1, 3600, 128, False), (2, 81, 132, False)])
+def test_passes_stay_within_the_stated_workspace(B, L, C, misalign):
+    rng = np.random.default_rng(C)
+    lib, ptr = emu.lib(), emu._ptr
+    par = [emu._f32(t) for t in _params(C, rng)]
+
+    def tensor(*shape):
+        flat = emu._f32(np.concatenate([[0.0], rng.standard_normal(int(np.prod(shape)))]))
+        return flat[1:].reshape(shape) if misalign else emu._f32(flat[1:].reshape(shape))
+
+    def guarded(which):
+        n = lib.fields_read_workspace_bytes(B, L, C, which)
+        ws = emu._aligned(2 * n + 4096)  # (room for what an overrun would write)
+        ws[n:] = 0xA5
+        return ws, n
+
+    raw, read, grad, grad_raw = tensor(B, L, 3 * C), tensor(B, L, 4 * C), tensor(B, L, 4 * C), tensor(B, L, 3 * C)
+    ws, n = guarded(0)
+    assert lib.fields_read_forward(ptr(raw), *map(ptr, par), None, ptr(read), None, ptr(ws), n, B, L, C, None) == 0
+    assert (ws[n:] == 0xA5).all()
+    ws, n = guarded(1)
+    sums = [emu._f32(np.zeros(C)) for _ in range(3)]
+    assert lib.fields_read_backward(ptr(raw), *map(ptr, par), None, ptr(read), ptr(grad), None, ptr(grad_raw),
+                                    *map(ptr, sums), None, ptr(ws), n, B, L, C, None) == 0
+    assert (ws[n:] == 0xA5).all()
+
+
 def test_golden_small_cases(golden_small, algo):
     for name in golden_small["cases"]:
         c = {k: golden_small[f"{name}/{k}"] for k in

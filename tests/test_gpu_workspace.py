@@ -111,3 +111,18 @@ def test_captured_passes_can_be_replayed():
         with torch.no_grad():
             want = fused_field_read(raw, *par)
         assert rel_err(got.cpu().numpy(), want.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("B,L,C", [(1, 10_000, 33), (2, 3000, 333)])
+def test_odd_width_on_a_workspace_of_its_own(B, L, C):
+    """Passes whose slots take more than the least half, on a stream that has kept none yet."""
+    leaves, grad = _case(B, L, C, 7)
+    host = [t.detach().cpu().numpy() for t in leaves]
+    want = [field_oracle.forward(*host)[0], *field_oracle.backward(*host, grad.cpu().numpy())[:4]]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        got = _pass(leaves, grad)
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        assert rel_err(g.cpu().numpy(), np.asarray(w)) < FP32_TOL
