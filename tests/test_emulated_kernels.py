@@ -107,6 +107,26 @@ def test_passes_stay_within_the_stated_workspace(B, L, C, misalign):
     assert (ws[n:] == 0xA5).all()
 
 
+@pytest.mark.parametrize("plane", [0, 1, 2])
+@pytest.mark.parametrize("stats", [False, True])
+def test_nan_reaches_the_bf16_read(plane, stats):
+    """A NaN in one gate input: everything of that channel from its step on, nothing before and beside it."""
+    rng = np.random.default_rng(plane)
+    B, L, C, at, chan = 1, 100, 8, 10, 3
+    par = _params(C, rng)
+    raw = rng.standard_normal((B, L, 3 * C)).astype(np.float32)
+    raw[0, at, plane * C + chan] = np.nan
+    if stats:
+        bits, sumsq = emu.forward_bf16_stats(_bits(raw), *par)
+        assert np.isnan(sumsq[0, at:]).all() and not np.isnan(sumsq[0, :at]).any()
+    else:
+        bits = emu.forward_bf16(_bits(raw), *par)
+    got = np.isnan(_unbits(bits)).reshape(L, 4, C)
+    want = np.isnan(emu.forward(raw, *par)[0]).reshape(L, 4, C)
+    assert want.any() and not (want & ~got).any()  # (at step `at` itself the shared reciprocal takes all three gates)
+    assert not got[:at].any() and not np.delete(got, chan, axis=2).any()
+
+
 def test_golden_small_cases(golden_small, algo):
     for name in golden_small["cases"]:
         c = {k: golden_small[f"{name}/{k}"] for k in

@@ -73,3 +73,24 @@ def test_bf16_forward_with_long_tiles():
     want = fused_field_read(raw.float(), *par)
     got = fused_field_read_bf16(raw, *par).float()
     assert float((got - want).abs().max()) <= 2 ** -8 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("plane", [0, 1, 2])
+def test_nan_reaches_the_outputs(plane):
+    """A NaN in one gate input or one token: from that step on in the operator's channel and in the mixer."""
+    torch.manual_seed(plane)
+    B, L, C, at, chan = 2, 150, 64, 70, 5
+    ring, theta = torch.linspace(0.85, 0.999, C), torch.linspace(0.03, 3.04, C)
+    par = [t.cuda() for t in (ring * theta.cos(), ring * theta.sin(), (1 - ring ** 2).sqrt())]
+    raw = torch.randn(B, L, 3 * C, device="cuda")
+    raw[1, at, plane * C + chan] = float("nan")
+    want = fused_field_read(raw, *par).isnan().view(B, L, 4, C)
+    got = fused_field_read_bf16(raw.bfloat16(), *par).isnan().view(B, L, 4, C)
+    assert bool(want.any()) and not bool((want & ~got).any())
+    assert not bool(got[0].any() or got[1, :at].any() or got[..., torch.arange(C) != chan].any())
+    m = mirror.IndependentVacancyField(2 * C).cuda()
+    x = torch.randn(B, L, 2 * C, device="cuda")
+    x[1, at, chan] = float("nan")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        y = mixer.fused_mixer_forward(m, x)
+    assert bool(y[1, at:].isnan().all()) and not bool(y[0].isnan().any() or y[1, :at].isnan().any())
