@@ -409,31 +409,6 @@ FL_HD Gate2 make_gate2(const F2& zr, const F2& zi, const F2& zv) {
     return g;
 }
 
-// The same gates with one reciprocal for the three (1/a = bc / abc and so on): four special-function
-// operations per channel instead of six, for kernels that the special-function pipe bounds. The
-// exponents are capped so that the product of the denominators stays finite: beyond 2^30 both forms
-// give tanh = 1 in fp32; the sigmoid's smallest value becomes 2^-64. A NaN passes the cap and makes all three NaN.
-FL_HD F2 cap2(const F2& a, float m) { return F2{a.x > m ? m : a.x, a.y > m ? m : a.y}; }
-
-FL_HD Gate2 make_gate2_shared(const F2& zr, const F2& zi, const F2& zv) {
-    Gate2 g;
-    const F2 one = splat2(1.0f), k2 = splat2(2.0f * kLog2e), m2 = splat2(-2.0f);
-    const F2 a = add2(exp2_2(cap2(mul2(zr, k2), 30.0f)), one);
-    const F2 b = add2(exp2_2(cap2(mul2(zi, k2), 30.0f)), one);
-    const F2 c = add2(exp2_2(cap2(mul2(zv, splat2(-kLog2e)), 64.0f)), one);
-    const F2 ab = mul2(a, b);
-    const F2 r = rcp2(mul2(ab, c));
-    const F2 rc = mul2(r, c);
-    g.rr = mul2(rc, b);
-    g.ri = mul2(rc, a);
-    g.sig = mul2(r, ab);
-    g.inj_r = fma2(g.rr, m2, one);
-    g.inj_i = fma2(g.ri, m2, one);
-    g.vac = mul2(g.sig, splat2(kVacMax));
-    g.keep = fma2(g.sig, splat2(-kVacMax), one);
-    return g;
-}
-
 // Affine maps of two channels.
 struct Affine2 {
     F2 ar, ai, br, bi;

@@ -111,9 +111,11 @@ FL_HD SpTile sp_decode(const SpShape& s, unsigned ticket) {
 // What bounds it: a tile lives about 10 us (its loads, the look-back, its stores), so bandwidth is the
 // tile state that an SM holds divided by that. fp32 keeps a step's gate values in registers between the
 // two halves, 12 bytes per channel and step (the raw values are as large). bfloat16 keeps
-// the raw bits, half as much, and evaluates the gates a second time, with one reciprocal for the three
-// (the special-function pipe would bound it otherwise): 43.0 -> 36.2 us at 8 x 2,048 x 512, 189 ->
-// 142 us at 1 x 65,536. Blocks of four warps overlap their phases better than blocks of eight; holding
+// the raw bits, half as much, and evaluates the gates a second time. (One reciprocal for the three gates,
+// four special-function operations per channel instead of six, gained 4 % at 1 x 65,536 x 512 and nothing at
+// 8 x 2,048; its state was 1.9e-7 from 64-bit arithmetic instead of 1.3e-7, and a gate that is masked with -inf did
+// not close.) Forward, workspace fill included: 48.1 -> 44.1 us at 8 x 2,048 x 512 against the staged form
+// below, 185 -> 157 us at 1 x 65,536. Blocks of four warps overlap their phases better than blocks of eight; holding
 // tickets and staging the next tile in shared memory (an earlier form) came to 43.0 us.
 // ROWS: also writes the state after every kStateRowEvery-th step, what a backward pass from state rows keeps.
 template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false, bool ROWS = false>
@@ -150,8 +152,7 @@ struct FwdSinglePass {
         }
     }
     FL_HD static Gate2 gate(const State& st, int u, int h) {
-        if constexpr (kPacked)
-            return make_gate2_shared(st.raw[u][0].pair(h), st.raw[u][1].pair(h), st.raw[u][2].pair(h));
+        if constexpr (kPacked) return make_gate2(st.raw[u][0].pair(h), st.raw[u][1].pair(h), st.raw[u][2].pair(h));
         else return make_gate2(st.br[u][h], st.bi[u][h], st.vac[u][h]);
     }
 

@@ -123,8 +123,27 @@ def test_nan_reaches_the_bf16_read(plane, stats):
         bits = emu.forward_bf16(_bits(raw), *par)
     got = np.isnan(_unbits(bits)).reshape(L, 4, C)
     want = np.isnan(emu.forward(raw, *par)[0]).reshape(L, 4, C)
-    assert want.any() and not (want & ~got).any()  # (at step `at` itself the shared reciprocal takes all three gates)
+    assert want.any() and (got == want).all()
     assert not got[:at].any() and not np.delete(got, chan, axis=2).any()
+
+
+def test_closed_gates_of_the_bf16_forward():
+    """Vacancies down to the smallest and masks (the type's lowest value, -inf): each element of `read` is the fp32
+    one to its own rounding, zero where that is zero."""
+    rng = np.random.default_rng(5)
+    B, L, C = 1, 40, 8
+    par = _params(C, rng)
+    raw = _unbits(_bits(rng.standard_normal((B, L, 3 * C))))
+    closed = np.array([-40, -44, -45, -50, -60, -80, -87, -100, -1e30, -3.3895314e38, -np.inf], np.float32)
+    for t in range(3, L):
+        raw[0, t, 2 * C:] = np.roll(np.resize(closed, 3 * C), t)[:C]
+    raw = _unbits(_bits(raw))
+    want = emu.forward(raw, *par)[0]
+    got = _unbits(emu.forward_bf16(_bits(raw), *par))
+    assert (want[0, 3:, 2 * C:] == 0).any() and (want[0, 3:, 2 * C:] != 0).any()
+    # (below the smallest normal number bfloat16 has fewer bits, and the GPU flushes to zero)
+    assert (np.abs(got - want) <= np.maximum(2 ** -8 * np.abs(want), 2.0 ** -126)).all()
+    assert (got[want == 0] == 0).all()
 
 
 def test_golden_small_cases(golden_small, algo):
