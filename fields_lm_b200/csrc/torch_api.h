@@ -112,7 +112,7 @@ inline bool all_aligned(std::initializer_list<const void*> ptrs, uintptr_t bytes
 // graph and larger ones get one of their own, as does every pass where the library refuses.
 class PassWorkspace {
   public:
-    PassWorkspace(size_t need, const Tensor& on) : bytes_(need) {
+    PassWorkspace(size_t need, const Tensor& on) {
         const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(on.device().index());
         // (torch's own streams: another library's may be destroyed while work is pending)
         const bool own_stream = stream.id() == 0 || (stream.id() & 1);
@@ -120,18 +120,25 @@ class PassWorkspace {
             c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
             kept_ = entry(on.device().index(), stream.id());
             lock_ = std::unique_lock<std::mutex>(kept_->mu);
+            if (kept_->state.half_bytes < need || !kept_->ws.defined()) {
+                // (either call may throw: the entry changes when both are done)
+                size_t half = std::max(kLeastBytes, kept_->state.half_bytes);
+                while (half < need) half *= 2;
+                Tensor ws = empty({(int64_t)(256 + 3 * half)}, at::kByte, on.device());
+                C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0xFF, 256 + 2 * half, stream.stream()));
+                kept_->ws = std::move(ws);
+                kept_->state = fields_kept{half, {0, 0}, 0};
+            }
+            // the last step that can fail: a registration without a pass would be taken by the thread's next one
             if (api().fields_read_use_kept(&kept_->state) != FIELDS_OK) {
                 lock_.unlock();
                 kept_.reset();
-            } else if (kept_->state.half_bytes < need || !kept_->ws.defined()) {
-                size_t half = std::max(kLeastBytes, kept_->state.half_bytes);
-                while (half < need) half *= 2;
-                kept_->ws = empty({(int64_t)(256 + 3 * half)}, at::kByte, on.device());
-                kept_->state = fields_kept{half, {0, 0}, 0};
-                C10_CUDA_CHECK(cudaMemsetAsync(kept_->ws.data_ptr(), 0xFF, 256 + 2 * half, stream.stream()));
             }
         }
-        if (!kept_) own_ = workspace(need, on.device());
+        if (!kept_) {
+            own_ = workspace(need, on.device());
+            api().fields_read_use_kept(nullptr);  // nor one that a caller of the library has left
+        }
         ptr_ = kept_ ? kept_->ws.data_ptr() : own_.data_ptr();
     }
     ~PassWorkspace() {
@@ -141,7 +148,6 @@ class PassWorkspace {
     }
     PassWorkspace(const PassWorkspace&) = delete;
     void* ptr() const { return ptr_; }
-    size_t bytes() const { return bytes_; }
     // the status of the pass
     void check(int rc, const char* what) {
         done_ = rc == FIELDS_OK;
@@ -181,7 +187,6 @@ class PassWorkspace {
     std::unique_lock<std::mutex> lock_;  // released before kept_
     Tensor own_;
     void* ptr_;
-    size_t bytes_;
     bool done_ = false;
 };
 inline std::string shape(const Tensor& t) { return c10::str("(", t.sizes(), ")"); }

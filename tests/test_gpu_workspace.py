@@ -126,3 +126,27 @@ def test_odd_width_on_a_workspace_of_its_own(B, L, C):
     torch.cuda.synchronize()
     for g, w in zip(got, want):
         assert rel_err(g.cpu().numpy(), np.asarray(w)) < FP32_TOL
+
+
+def test_a_failed_allocation_leaves_nothing_behind():
+    """A pass that gets no memory for its kept workspace (96 MiB here), then one on a workspace of its own (above
+    the most that is kept) and the first one again."""
+    few, many = _case(1, 300_000, 4, 1), _case(1, 360_000, 4, 2)
+    par = [t.detach() for t in few[0][1:]]
+    small, large = few[0][0].detach(), many[0][0].detach()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (70 << 20)) / total)
+    try:
+        with torch.cuda.stream(stream), pytest.raises(torch.cuda.OutOfMemoryError):
+            fused_field_read(small, *par)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    with torch.cuda.stream(stream):
+        got = [fused_field_read(t, *par) for t in (large, small, large, small)]
+    torch.cuda.synchronize()
+    host = [p.cpu().numpy() for p in par]
+    for g, t in zip(got, (large, small, large, small)):
+        assert rel_err(g.cpu().numpy(), field_oracle.forward(t.cpu().numpy(), *host)[0]) < FP32_TOL
