@@ -5,7 +5,9 @@
 // (field_rows.cuh) instead of the ~48 launches that the block's modules make; the bfloat16 copies of
 // the weights that autocast makes on every call are laid out once per prefill and kept for the steps
 // that follow it. The owner (FieldStackDecoder) asks current() before a step: the copies are used
-// only while every module, parameter and hook is what it was and no parameter has been written to.
+// only while every module, parameter and hook is what it was and no parameter has been written to, as far as
+// torch counts it (a write through `.data` or by another library is not counted; the next prefill sees
+// it). Parameters without a count (inference tensors) are laid out for every step.
 #include "torch_gemm.h"
 
 #include <ATen/ops/addmm_cuda_dispatch.h>
@@ -17,9 +19,11 @@ namespace fields_torch {
 namespace py = pybind11;
 
 // A parameter (the module's own tensor), where its data lay when the plan was made and its version
-// when its copy was made.
+// when its copy was made. Inference tensors have no version: their copies are never up to date.
 struct Source {
     explicit Source(const Tensor& p) : t(p), data(p.data_ptr()) {}
+    void copied() { version = t.is_inference() ? 0 : t._version(); }
+    bool current() const { return !t.is_inference() && t._version() == version; }
     Tensor t;
     const void* data;
     uint64_t version = 0;
@@ -68,8 +72,7 @@ class FieldStack {
 
     // ... and whether the copies of the parameters are up to date.
     bool current() const {
-        return laid_out_ && same_model() &&
-               every_source([](const Source& s) { return s.t._version() == s.version; });
+        return laid_out_ && same_model() && every_source([](const Source& s) { return s.current(); });
     }
 
     // Whether step() goes on to the logits.
@@ -82,7 +85,7 @@ class FieldStack {
         const int64_t D = D_, C = D / 2, H = H_;
         std::vector<fields_stack_weights> all;
         for (Block& b : blocks_) {
-            for (Source& s : b.src) s.version = s.t._version();
+            for (Source& s : b.src) s.copied();
             if (!b.in_w.defined()) {
                 b.in_w = empty({3 * C + D, D}, at::kBFloat16, dev);
                 b.in_b = empty({3 * C + D}, at::kBFloat16, dev);
@@ -103,7 +106,7 @@ class FieldStack {
         }
         check(api().fields_stack_layout(all.data(), (int)all.size(), stream_of(blocks_[0].in_w)), "fields_stack_layout");
         if (!tail_.empty()) {
-            for (Source& s : tail_) s.version = s.t._version();
+            for (Source& s : tail_) s.copied();
             head_w_ = tail_[1].t.detach().to(at::kBFloat16).t();
             if (tail_.size() > 2) head_b_ = tail_[2].t.detach().to(at::kBFloat16);
         }

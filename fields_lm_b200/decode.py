@@ -74,7 +74,11 @@ class FieldStackDecoder:
 
         Under bfloat16 autocast the blocks run natively where they are what that path computes
         (``fields_lm_b200.stack``); the weights are laid out for it here, and the steps that
-        follow use the same copies until a parameter changes."""
+        follow use the same copies until a parameter changes: an in-place write as torch counts
+        it (``load_state_dict``, an optimizer, ``copy_`` under ``no_grad``) or another tensor in
+        its place. A write that torch does not count, through ``.data`` or into the memory by
+        other means, is seen by the next prefill only. Inference tensors, which have no count, are
+        laid out for every step."""
         from .mixer import block_prefill
         x = self.model.emb(tokens)
         if self._bf16_products(x) and x.dim() == 3:

@@ -105,3 +105,22 @@ def test_native_stack_follows_the_model():
     seen = []
     model.blocks[0].ff_norm.register_forward_hook(lambda *a: seen.append(1))
     assert _rel(step(), changed) < BF16_TOL and seen and dec._stack is None
+
+
+def test_model_of_inference_tensors():
+    """Parameters that have no version counter: the weights as they are at every step."""
+    torch.manual_seed(1)
+    plain = LM(64, 2, 32).cuda()
+    with torch.inference_mode():
+        model = LM(64, 2, 32).cuda()
+        model.load_state_dict(plain.state_dict())
+    assert all(p.is_inference() for p in model.parameters())
+    tokens = torch.randint(0, 97, (4, 8), device="cuda")
+    got, want = _run(model, tokens, 5, True), _run(plain, tokens, 5, True)
+    assert all(torch.equal(a, b) for a, b in zip(got[0], want[0]))
+    for m in (model, plain):
+        with torch.inference_mode():
+            m.blocks[1].ff.w3.weight.mul_(3.0)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert torch.equal(got[1].step(tokens[:, 0]), want[1].step(tokens[:, 0]))
+        assert torch.equal(got[1].prefill(tokens), want[1].prefill(tokens))
