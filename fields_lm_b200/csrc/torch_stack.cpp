@@ -75,6 +75,16 @@ class FieldStack {
         return laid_out_ && same_model() && every_source([](const Source& s) { return s.current(); });
     }
 
+    // The same plan without copies, for a graph that is being captured: its copies are laid out by the graph
+    // itself, from the weights of the moment it runs, into memory of its own.
+    std::unique_ptr<FieldStack> fresh() const {
+        auto other = std::make_unique<FieldStack>(*this);
+        for (Block& b : other->blocks_) b.in_w = b.in_b = b.in_t = b.out_t = b.w12_t = b.w3_t = b.par = b.step_in = b.step_w12 = b.step_b = Tensor();
+        other->head_w_ = other->head_b_ = Tensor();
+        other->laid_out_ = other->step_laid_out_ = false;
+        return other;
+    }
+
     // Whether step() goes on to the logits.
     bool has_head() const { return !tail_.empty(); }
 
@@ -305,6 +315,7 @@ void add_stack(PyObject* module) {
         .def_property_readonly("has_head", &FieldStack::has_head)
         .def("same_model", &FieldStack::same_model)
         .def("current", &FieldStack::current)
+        .def("fresh", &FieldStack::fresh)
         .def("layout", torch::wrap_pybind_function_no_gil([](FieldStack& s) { s.layout(); }))
         .def("prefill", torch::wrap_pybind_function_no_gil([](FieldStack& s, const Tensor& x) { return s.prefill(x); }))
         .def("step", torch::wrap_pybind_function_no_gil(

@@ -60,7 +60,11 @@ class FieldStackDecoder:
                 and torch.get_autocast_dtype("cuda") == torch.bfloat16)
 
     def _native_stack(self, x: torch.Tensor):
-        """The runner for the model as it is now, or None."""
+        """The runner for the model as it is now, or None; one of its own for a graph that is being
+        captured, whose replays have to follow the weights and must not depend on this object."""
+        if torch.cuda.is_current_stream_capturing():
+            usable = self._stack is not None and self._stack.same_model()
+            return self._stack.fresh() if usable else None  # (a plan cannot be made here)
         if self._stack is None or not self._stack.same_model():
             from .stack import plan
             self._stack = plan(self.model, x.device)
@@ -105,7 +109,8 @@ class FieldStackDecoder:
         x = self.model.emb(tokens)
         if not self._refused and self._bf16_products(x) and x.dim() == 2:
             stack = self._stack
-            if stack is None or not stack.current():  # something has changed since the prefill
+            if (stack is None or not stack.current()  # something has changed since the prefill
+                    or torch.cuda.is_current_stream_capturing()):
                 stack = self._native_stack(x)
                 if stack is not None:
                     stack.layout()

@@ -124,3 +124,44 @@ def test_model_of_inference_tensors():
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert torch.equal(got[1].step(tokens[:, 0]), want[1].step(tokens[:, 0]))
         assert torch.equal(got[1].prefill(tokens), want[1].prefill(tokens))
+
+
+def test_captured_step_and_prefill_follow_the_weights():
+    """A graph replays with the weights of that moment, and does not need the decoder it was captured from."""
+    torch.manual_seed(3)
+    model = LM(64, 2, 32).cuda()
+    tokens = torch.randint(0, 97, (4, 6), device="cuda")
+    _, dec = _run(model, tokens, 6, True)
+    kept = [s.clone() for s in dec.states]
+
+    def eager():
+        ref = FieldStackDecoder(model)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            first = ref.prefill(tokens)
+            ref.states = [s.clone() for s in kept]
+            return ref.step(tokens[:, 0]), first
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        eager()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False), torch.cuda.graph(graph, stream=side):
+        states, dec.states = dec.states, [s.clone() for s in dec.states]
+        out = dec.step(tokens[:, 0])
+        first = dec.prefill(tokens)
+    dec.states = states
+    assert not dec._refused
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        dec.prefill(tokens)  # what was captured is no layout of the decoder's own
+        assert _rel(dec.step(tokens[:, 0]), eager()[0]) < 1e-6
+    dec.reset()
+    for factor in (1.0, 3.0, 0.5):
+        with torch.no_grad():
+            model.blocks[1].ff.w3.weight.mul_(factor)
+            model.blocks[0].mixer.gate_proj.bias.add_(factor)
+        graph.replay()
+        torch.cuda.synchronize()
+        for got, want in zip((out, first), eager()):
+            assert _rel(got, want) < 1e-6
