@@ -212,8 +212,8 @@ struct FinishGradParams {
     const float* g_tr;
     const float* g_ti;
     const float* g_gm;
-    float* g_radius;
-    float* g_theta;
+    float* g_radius;  // or null
+    float* g_theta;   // or null
     int C;
 };
 
@@ -233,8 +233,8 @@ __global__ void __launch_bounds__(kRowThreads) finish_grad(const FinishGradParam
         const float gtr = p.g_tr[c], gti = p.g_ti[c];
         float gr = gtr * co + gti * si;
         if (q >= 1e-4f) gr -= p.g_gm[c] * r / gm;
-        p.g_theta[c] = r * (gti * co - gtr * si);
-        p.g_radius[c] = sig >= 0.50f && sig <= 0.99995f ? gr * sig * (1.0f - sig) : 0.0f;
+        if (p.g_theta) p.g_theta[c] = r * (gti * co - gtr * si);
+        if (p.g_radius) p.g_radius[c] = sig >= 0.50f && sig <= 0.99995f ? gr * sig * (1.0f - sig) : 0.0f;
         return;
     }
     int k = 0;

@@ -2109,9 +2109,10 @@ int fields_mixer_open_grad(const float* grad_y, const void* acc, const void* gat
 
 int fields_mixer_close_grad(const struct fields_mixer_grads* g, long long N, int D, void* stream) {
     if (!g || N <= 0 || D <= 0) return FIELDS_ERR_ARGUMENT;
-    if (!g->rows || !g->grad_raw || !g->grad_out || !g->out_w || !g->norm_w || !g->radius_logit || !g->theta ||
-        !g->grad_tr || !g->grad_ti || !g->grad_gamma || !g->grad_out_b || !g->grad_gate_b || !g->grad_write_b ||
-        !g->grad_norm_w || !g->grad_radius || !g->grad_theta || !g->scratch)
+    const bool biases = g->grad_out_b || g->grad_gate_b, transition = g->grad_radius || g->grad_theta;
+    if ((biases && !g->rows) || (g->grad_write_b && !g->grad_raw) || (g->grad_norm_w && !g->grad_out) ||
+        (g->grad_out && (!g->out_w || !g->norm_w)) || ((g->grad_write_b || g->grad_out) && !g->scratch) ||
+        (transition && (!g->radius_logit || !g->theta || !g->grad_tr || !g->grad_ti || !g->grad_gamma)))
         return FIELDS_ERR_ARGUMENT;
     if (D % 8 || g->grad_pitch % 4 || !aligned8(g->grad_raw) || !aligned16(g->grad_out) || !aligned16(g->out_w) ||
         !aligned16(g->norm_w) || !aligned16(g->scratch))
@@ -2120,34 +2121,40 @@ int fields_mixer_close_grad(const struct fields_mixer_grads* g, long long N, int
     const int C = D / 2, cols = 3 * C, wide = 2 * D, per_x = kRowThreads * 4;
     float* col_rows = g->scratch;
     float* weight_rows = col_rows + (size_t)kColumnBlocks * cols;
+    FinishGradParams p{};
+    int first = 0, rc;
+    // (a set without an output has no columns, and so no blocks)
+    auto add = [&](int k, const float* rows, float* out, int count, int width) {
+        p.set[k] = PartialRows{rows, out, count, out ? width : 0, first};
+        first += (p.set[k].cols + 31) / 32;
+    };
+    const int n = (int)fields_mixer_grad_rows(N);
+    add(0, g->rows, g->grad_out_b, n, D);
+    add(1, g->rows + (size_t)n * D, g->grad_gate_b, n, D);
     const long long per = (N + kColumnBlocks - 1) / kColumnBlocks;
     if (per > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
     const int col_blocks = (int)((N + per - 1) / per);
-    ColumnSumParams cp{static_cast<const uint16_t*>(g->grad_raw), col_rows, N, g->grad_pitch, cols, (int)per};
-    int rc = launch_grid<ColumnSumParams>(column_sums, dim3((cols + per_x - 1) / per_x, col_blocks), kRowThreads, st, cp);
-    if (rc) return rc;
-    const int wper = (D + kWeightBlocks - 1) / kWeightBlocks, weight_blocks = (D + wper - 1) / wper;
-    OutWeightGradParams wp{g->grad_out, g->out_w, g->norm_w, weight_rows, D, wide, wper};
-    rc = launch_grid<OutWeightGradParams>(out_weight_grad, dim3((wide + per_x - 1) / per_x, weight_blocks), kRowThreads,
-                                          st, wp);
-    if (rc) return rc;
-    const int n = (int)fields_mixer_grad_rows(N);
-    FinishGradParams p{};
-    int first = 0;
-    auto add = [&](int k, const float* rows, float* out, int count, int width) {
-        p.set[k] = PartialRows{rows, out, count, width, first};
-        first += (width + 31) / 32;
-    };
-    add(0, g->rows, g->grad_out_b, n, D);
-    add(1, g->rows + (size_t)n * D, g->grad_gate_b, n, D);
+    if (g->grad_write_b) {
+        ColumnSumParams cp{static_cast<const uint16_t*>(g->grad_raw), col_rows, N, g->grad_pitch, cols, (int)per};
+        rc = launch_grid<ColumnSumParams>(column_sums, dim3((cols + per_x - 1) / per_x, col_blocks), kRowThreads, st, cp);
+        if (rc) return rc;
+    }
     add(2, col_rows, g->grad_write_b, col_blocks, cols);
+    const int wper = (D + kWeightBlocks - 1) / kWeightBlocks, weight_blocks = (D + wper - 1) / wper;
+    if (g->grad_out) {
+        OutWeightGradParams wp{g->grad_out, g->out_w, g->norm_w, weight_rows, D, wide, wper};
+        rc = launch_grid<OutWeightGradParams>(out_weight_grad, dim3((wide + per_x - 1) / per_x, weight_blocks), kRowThreads,
+                                              st, wp);
+        if (rc) return rc;
+    }
     add(3, weight_rows, g->grad_norm_w, weight_blocks, wide);
     p.transition_block = first;
     p.radius_logit = g->radius_logit; p.theta = g->theta;
     p.g_tr = g->grad_tr; p.g_ti = g->grad_ti; p.g_gm = g->grad_gamma;
     p.g_radius = g->grad_radius; p.g_theta = g->grad_theta; p.C = C;
-    return launch_on<FinishGradParams>(finish_grad, (unsigned)(first + (C + kRowThreads - 1) / kRowThreads), kRowThreads,
-                                       0, st, p);
+    const int blocks = first + (transition ? (C + kRowThreads - 1) / kRowThreads : 0);
+    if (blocks == 0) return FIELDS_OK;
+    return launch_on<FinishGradParams>(finish_grad, (unsigned)blocks, kRowThreads, 0, st, p);
 }
 
 int fields_step_w12_rows(int hidden) { return hidden > 0 ? (hidden + 19) / 20 * 40 : 0; }

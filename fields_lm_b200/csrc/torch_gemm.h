@@ -10,10 +10,12 @@
 
 namespace fields_torch {
 
-// A dense bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any.
+// A bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any; rows as stored are
+// `pitch` elements apart (0: dense).
 struct Operand {
     const void* p;
     bool transposed;  // stored [cols, rows]
+    int64_t pitch = 0;
 };
 inline Operand plain(const Tensor& t) { return Operand{vp(t), false}; }
 inline Operand transposed(const Tensor& t) { return Operand{vp(t), true}; }
@@ -25,7 +27,8 @@ inline void product(const Tensor& out, Operand a, Operand b, int64_t M, int64_t 
     TORCH_CUDABLAS_CHECK(cublasGemmEx(
         at::cuda::getCurrentCUDABlasHandle(), b.transposed ? CUBLAS_OP_T : CUBLAS_OP_N,
         a.transposed ? CUBLAS_OP_T : CUBLAS_OP_N, (int)N, (int)M, (int)K, &one, b.p, CUDA_R_16BF,
-        (int)(b.transposed ? K : N), a.p, CUDA_R_16BF, (int)(a.transposed ? M : K), &zero, out.data_ptr(),
+        (int)(b.pitch ? b.pitch : b.transposed ? K : N), a.p, CUDA_R_16BF,
+        (int)(a.pitch ? a.pitch : a.transposed ? M : K), &zero, out.data_ptr(),
         out.scalar_type() == at::kFloat ? CUDA_R_32F : CUDA_R_16BF, (int)N, CUBLAS_COMPUTE_32F,
         CUBLAS_GEMM_DEFAULT_TENSOR_OP));
 }

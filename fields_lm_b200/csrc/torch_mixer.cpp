@@ -101,40 +101,52 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
                                        vp(grad_acc), gate_of(grad_u, C), W, grad_sumsq, rows, eps, (int)(2 * D),
                                        N, (int)D, st),
               "fields_mixer_open_grad");
-        Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
-        product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
-        Tensor grad_out = f32s({D, 2 * D});
-        product(grad_out, transposed(grad_acc), plain(read), D, 2 * D, N);
-        check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
-              "fields_read_norm_grad_combine");
+        // What a frozen parameter leaves out; the recurrence runs backward for x and what lies before it.
+        auto need = [&](int i) { return ctx->needs_input_grad(i); };
+        const bool recurrence = need(kX) || need(kWriteW) || need(kWriteB) || need(kRadius) || need(kTheta);
         float* p = fp(par);
-        {
+        if (recurrence) {
+            const Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
+            product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
+            check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
+                  "fields_read_norm_grad_combine");
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
             PassWorkspace ws(n, u);
             ws.check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
                                                    g, g + C, g + 2 * C, ws.ptr(), n, (int)B, (int)L, (int)C, st),
                   "fields_read_backward_bf16_rows");
         }
+        Tensor grad_out;
+        if (need(kOutW) || need(kNormW)) {
+            grad_out = f32s({D, 2 * D});
+            product(grad_out, transposed(grad_acc), plain(read), D, 2 * D, N);
+        }
         Tensor grad_x;
-        if (ctx->needs_input_grad(kX)) {
+        if (need(kX)) {
             Tensor back = empty({N, D}, at::kBFloat16, dev);
             product(back, plain(grad_u), plain(in_w), N, D, W);
             grad_x = f32s({B, L, D});
             check(f.fields_stack_close_ff(fp(gy), vp(back), nullptr, fp(grad_x), nullptr, 0.0f, N, (int)D, st),
                   "fields_stack_close_ff");
         }
-        Tensor grad_in = f32s({W, D});
-        product(grad_in, transposed(grad_u), plain(xb), W, D, N);
+        Tensor grad_write_w, grad_gate_w;  // (one product over both where both are wanted)
+        if (need(kWriteW) || need(kGateW)) {
+            const int64_t first = need(kWriteW) ? 0 : 3 * C, rows_in = (need(kGateW) ? W : 3 * C) - first;
+            const Tensor grad_in = f32s({rows_in, D});
+            product(grad_in, Operand{static_cast<at::BFloat16*>(vp(grad_u)) + first, true, W}, plain(xb), rows_in, D, N);
+            if (need(kWriteW)) grad_write_w = grad_in.narrow(0, 0, 3 * C);
+            if (need(kGateW)) grad_gate_w = grad_in.narrow(0, 3 * C - first, D);
+        }
 
         // the small gradients share an allocation
         const Tensor small = f32s({4 * D + 5 * C});
         int64_t at = 0;
-        auto part = [&](int64_t n) {
+        auto part = [&](int i, int64_t n) {
             at += n;
-            return part_of(small, at - n, n);
+            return need(i) ? part_of(small, at - n, n) : Tensor();
         };
-        const Tensor g_out_b = part(D), g_gate_b = part(D), g_norm = part(2 * D), g_write_b = part(3 * C),
-                     g_radius = part(C), g_theta = part(C);
+        const Tensor g_out_b = part(kOutB, D), g_gate_b = part(kGateB, D), g_norm = part(kNormW, 2 * D),
+                     g_write_b = part(kWriteB, 3 * C), g_radius = part(kRadius, C), g_theta = part(kTheta, C);
         fields_mixer_grads q{};
         q.rows = rows; q.grad_raw = vp(grad_u); q.grad_pitch = W; q.grad_out = fp(grad_out); q.out_w = fp(out_w);
         q.norm_w = fp(norm_w); q.radius_logit = fp(radius); q.theta = fp(theta);
@@ -142,8 +154,8 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         q.grad_out_b = fp(g_out_b); q.grad_gate_b = fp(g_gate_b); q.grad_write_b = fp(g_write_b);
         q.grad_norm_w = fp(g_norm); q.grad_radius = fp(g_radius); q.grad_theta = fp(g_theta); q.scratch = scratch;
         check(f.fields_mixer_close_grad(&q, N, (int)D, st), "fields_mixer_close_grad");
-        return {grad_x,   grad_in.narrow(0, 0, 3 * C),   g_write_b, g_radius, g_theta, g_norm, grad_out,
-                g_out_b, grad_in.narrow(0, 3 * C, D), g_gate_b,  Tensor()};
+        return {grad_x,   grad_write_w, g_write_b,   g_radius, g_theta, g_norm, need(kOutW) ? grad_out : Tensor(),
+                g_out_b, grad_gate_w,  g_gate_b,  Tensor()};
     }
 
   private:

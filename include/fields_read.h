@@ -573,7 +573,8 @@ int fields_read_backward_bf16_rows(const void *raw, long long raw_pitch, const f
  * fields_mixer_close_grad: gradients of the parameters from those partial rows, from grad_raw (the
  *   first 3C columns of rows grad_pitch apart, bfloat16), from grad_out (in: gradient of out_proj
  *   diag(norm), out: that of out_proj) and from the gradients of the transition parameters. scratch:
- *   fields_mixer_grad_scratch_bytes(D) bytes.
+ *   fields_mixer_grad_scratch_bytes(D) bytes. A result that is NULL is left out, and what only it
+ *   needs may be NULL (grad_out: with grad_norm_w).
  */
 size_t fields_mixer_grad_rows(long long N);
 size_t fields_mixer_grad_scratch_bytes(int D);

@@ -127,3 +127,40 @@ def test_state_of_the_bf16_forward_is_as_accurate_as_the_fp32_one():
                                         ws.data_ptr(), n, B, L, C, torch.cuda.current_stream().cuda_stream) == 0
     err = [float((s.double() - want).norm() / want.norm()) for s in (state, field_read_with_state(raw.float(), *par)[1])]
     assert err[0] < 1.15 * err[1], err  # (1.3e-7 both; 1.9e-7 with one reciprocal shared by the three gates)
+
+
+@pytest.mark.parametrize("wanted", [("x",), ("x", "write_proj.bias"), ("gate_proj.weight",), ("write_proj.weight",),
+                                    ("out_proj.weight", "gate_proj.bias"), ("read_norm.weight",), ("radius_logit",),
+                                    ("theta", "out_proj.bias"), ("write_proj.weight", "gate_proj.weight")])
+def test_frozen_parameters_cost_nothing(wanted):
+    """Gradients of some inputs alone are those of the full pass, and what only the others need is not computed: a
+    third of the weights' gradients is more than the difference that the allocator sees."""
+    torch.manual_seed(6)
+    D, B, L = 1024, 1, 40
+    m = mirror.IndependentVacancyField(D).cuda()
+    x = torch.randn(B, L, D, device="cuda", requires_grad=True)
+    gy = torch.randn(B, L, D, device="cuda")
+    full = _grads(m, x, gy, True)
+    leaves = {"x": x, **dict(m.named_parameters())}
+
+    def backward():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = mixer.fused_mixer_forward(m, x)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        needed = [t for t in leaves.values() if t.requires_grad]
+        got = torch.autograd.grad(y, needed, gy)
+        torch.cuda.synchronize()
+        return dict(zip([n for n, t in leaves.items() if t.requires_grad], got)), torch.cuda.max_memory_allocated() - before
+
+    _, most = backward()
+    for name, t in leaves.items():
+        t.requires_grad_(name in wanted)
+    got, peak = backward()
+    for name in wanted:
+        assert torch.equal(got[name], full[name]) or rel_err(got[name].cpu().numpy(), full[name].cpu().numpy()) < 1e-6
+    sizes = {"write_proj.weight": 3 * D * D // 2, "gate_proj.weight": D * D, "out_proj.weight": 2 * D * D}
+    spared = sum(n for name, n in sizes.items()
+                 if name not in wanted and not (name == "out_proj.weight" and "read_norm.weight" in wanted))
+    assert peak <= most - 4 * spared * 0.9
