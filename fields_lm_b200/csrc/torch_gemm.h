@@ -20,12 +20,37 @@ struct Operand {
 inline Operand plain(const Tensor& t) { return Operand{vp(t), false}; }
 inline Operand transposed(const Tensor& t) { return Operand{vp(t), true}; }
 
+// torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False, as at::mm heeds it: partial sums
+// of a product that is split along K are added in fp32.
+class ReductionMode {
+  public:
+    explicit ReductionMode(cublasHandle_t handle) : handle_(handle) {
+        if (at::globalContext().allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK)
+            return;
+        TORCH_CUDABLAS_CHECK(cublasGetMathMode(handle_, &before_));
+        TORCH_CUDABLAS_CHECK(cublasSetMathMode(
+            handle_, static_cast<cublasMath_t>(before_ | CUBLAS_MATH_DISALLOW_REDUCED_PRECISION_REDUCTION)));
+        set_ = true;
+    }
+    ~ReductionMode() {
+        if (set_) cublasSetMathMode(handle_, before_);
+    }
+    ReductionMode(const ReductionMode&) = delete;
+
+  private:
+    cublasHandle_t handle_;
+    cublasMath_t before_ = CUBLAS_DEFAULT_MATH;
+    bool set_ = false;
+};
+
 // out [M, N] = a [M, K] b [K, N], row-major, fp32 accumulation; out is bfloat16 or fp32. On the current stream.
 inline void product(const Tensor& out, Operand a, Operand b, int64_t M, int64_t N, int64_t K) {
     const float one = 1.0f, zero = 0.0f;
+    const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+    const ReductionMode mode(handle);
     // cuBLAS is column-major: out^T = b^T a^T
     TORCH_CUDABLAS_CHECK(cublasGemmEx(
-        at::cuda::getCurrentCUDABlasHandle(), b.transposed ? CUBLAS_OP_T : CUBLAS_OP_N,
+        handle, b.transposed ? CUBLAS_OP_T : CUBLAS_OP_N,
         a.transposed ? CUBLAS_OP_T : CUBLAS_OP_N, (int)N, (int)M, (int)K, &one, b.p, CUDA_R_16BF,
         (int)(b.pitch ? b.pitch : b.transposed ? K : N), a.p, CUDA_R_16BF,
         (int)(a.pitch ? a.pitch : a.transposed ? M : K), &zero, out.data_ptr(),
