@@ -127,7 +127,7 @@ class FieldStack {
     // x [B, L, D] fp32 -> the stack's output [B, L, D] and every block's end state [B, D].
     std::pair<Tensor, std::vector<Tensor>> prefill(const Tensor& x_) {
         const Api& f = api();
-        const Tensor x = dense(x_);
+        const Tensor x = activations(x_, 3);
         const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
@@ -167,13 +167,13 @@ class FieldStack {
     // One token per row: x [B, D] fp32; states advance in place. Returns the logits where the tail (final
     // norm and head) is part of the plan, else the stack's output.
     Tensor step(const Tensor& x_, const std::vector<Tensor>& states) {
-        Tensor x = dense(x_);
+        const Tensor x = activations(x_, 2);
         const int64_t N = x.size(0), D = D_;
         TORCH_CHECK_VALUE(states.size() == blocks_.size(), "one state per block is needed");
         std::vector<Tensor> own = states;  // 16-byte aligned: a caller's may be any view
         bool aligned = true;
         for (const Tensor& s : states) {
-            TORCH_CHECK_VALUE(s.is_cuda() && s.scalar_type() == at::kFloat && s.is_contiguous() && s.dim() == 2 &&
+            TORCH_CHECK_VALUE(s.device() == x.device() && s.scalar_type() == at::kFloat && s.is_contiguous() && s.dim() == 2 &&
                                   s.size(0) == N && s.size(1) == D,
                               shape(s));
             aligned = aligned && reinterpret_cast<uintptr_t>(s.data_ptr()) % 16 == 0;
@@ -181,7 +181,6 @@ class FieldStack {
         const c10::cuda::CUDAGuard guard(x.device());
         if (!aligned)
             for (Tensor& s : own) s = s.clone();
-        if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16) x = x.clone();
         // Four launches per block while its products have tiles (128 rows x 64 features) few enough that K
         // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 600 us at 16 rows and 670 at 256
         // against 763 and 768 with library products, but 986 against 787 at 384.
@@ -205,6 +204,15 @@ class FieldStack {
     }
 
   private:
+    // The embedding's output as the kernels take it: a width of another model is refused, as nn.Linear does.
+    Tensor activations(const Tensor& x, int64_t dims) const {
+        const c10::Device dev = blocks_[0].src[0].t.device();
+        TORCH_CHECK(x.dim() == dims && x.size(dims - 1) == D_ && x.scalar_type() == at::kFloat && x.device() == dev,
+                    "activations of shape ", shape(x), " on ", x.device(), " do not fit blocks of width ", D_, " on ", dev);
+        const Tensor d = dense(x);
+        return reinterpret_cast<uintptr_t>(d.data_ptr()) % 16 ? d.clone() : d;
+    }
+
     template <class F>
     bool every_source(F ok) const {
         for (const Block& b : blocks_)

@@ -165,3 +165,32 @@ def test_captured_step_and_prefill_follow_the_weights():
         torch.cuda.synchronize()
         for got, want in zip((out, first), eager()):
             assert _rel(got, want) < 1e-6
+
+
+@pytest.mark.parametrize("width", [32, 128])
+def test_activations_of_another_width_are_refused(width):
+    torch.manual_seed(4)
+    model = LM(64, 2, 32).cuda()
+    tokens = torch.randint(0, 97, (3, 6), device="cuda")
+    _, dec = _run(model, tokens, 6, True)
+    model.emb = torch.nn.Embedding(97, width).cuda()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        with pytest.raises(RuntimeError):
+            dec.step(tokens[:, 0])
+        with pytest.raises(RuntimeError):
+            dec.prefill(tokens)
+
+
+def test_activations_that_are_not_aligned():
+    class Shifted(torch.nn.Embedding):
+        def forward(self, tokens):
+            x = super().forward(tokens)
+            return torch.zeros(x.numel() + 1, device=x.device)[1:].view_as(x).copy_(x)
+
+    torch.manual_seed(5)
+    model = LM(64, 2, 32).cuda()
+    tokens = torch.randint(0, 97, (3, 8), device="cuda")
+    want, _ = _run(model, tokens, 5, True)
+    model.emb.__class__ = Shifted
+    got, _ = _run(model, tokens, 5, True)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
