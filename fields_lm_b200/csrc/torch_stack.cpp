@@ -45,8 +45,9 @@ class FieldStack {
   public:
     FieldStack(const std::vector<std::vector<Tensor>>& params, const std::vector<std::pair<double, double>>& eps,
                std::vector<std::tuple<py::object, py::object, py::object>> slots,
-               std::vector<std::pair<py::object, int64_t>> sizes, std::vector<Tensor> tail, double tail_eps)
-        : slots_(std::move(slots)), sizes_(std::move(sizes)), tail_eps_(tail_eps) {
+               std::vector<std::pair<py::object, int64_t>> sizes,
+               std::vector<std::pair<py::object, py::object>> classes, std::vector<Tensor> tail, double tail_eps)
+        : slots_(std::move(slots)), sizes_(std::move(sizes)), classes_(std::move(classes)), tail_eps_(tail_eps) {
         for (size_t i = 0; i < params.size(); ++i) {
             Block b;
             TORCH_CHECK_VALUE(params[i].size() == Block::kCount, "a block has ", (int)Block::kCount, " parameters");
@@ -60,13 +61,15 @@ class FieldStack {
         H_ = (int)blocks_[0].src[Block::kW3].t.size(1);
     }
 
-    // Whether the model still consists of the same modules and parameters where they were, with no
-    // hooks on them.
+    // Whether the model still consists of the same modules, attributes and parameters where they were, with
+    // the same code and no hooks on them.
     bool same_model() const {
         for (const auto& [dict, key, want] : slots_)
             if (PyDict_GetItem(dict.ptr(), key.ptr()) != want.ptr()) return false;
         for (const auto& [dict, size] : sizes_)
             if (PyDict_Size(dict.ptr()) != size) return false;
+        for (const auto& [cls, forward] : classes_)
+            if (py::object(cls.attr("forward")).ptr() != forward.ptr()) return false;
         return every_source([](const Source& s) { return s.t.data_ptr() == s.data; });
     }
 
@@ -307,6 +310,7 @@ class FieldStack {
     std::vector<Block> blocks_;
     std::vector<std::tuple<py::object, py::object, py::object>> slots_;  // (dict, key, the object there)
     std::vector<std::pair<py::object, int64_t>> sizes_;                  // dicts and the sizes they have to have
+    std::vector<std::pair<py::object, py::object>> classes_;             // and the `forward` they have to have
     std::vector<Source> tail_;  // final norm weight, head weight[, head bias]; may be empty
     Tensor head_w_, head_b_;
     double tail_eps_;
@@ -319,7 +323,8 @@ void add_stack(PyObject* module) {
     py::class_<FieldStack>(m, "FieldStack")
         .def(py::init<const std::vector<std::vector<Tensor>>&, const std::vector<std::pair<double, double>>&,
                       std::vector<std::tuple<py::object, py::object, py::object>>,
-                      std::vector<std::pair<py::object, int64_t>>, std::vector<Tensor>, double>())
+                      std::vector<std::pair<py::object, int64_t>>, std::vector<std::pair<py::object, py::object>>,
+                      std::vector<Tensor>, double>())
         .def_property_readonly("has_head", &FieldStack::has_head)
         .def("same_model", &FieldStack::same_model)
         .def("current", &FieldStack::current)

@@ -31,6 +31,11 @@ from .field_read import (field_read_with_state, fused_field_read_bf16,
                          fused_field_read_bf16_stats, mixer_epilogue)
 
 
+# hooks that torch calls for every module; write_proj is the one module that the mixer calls as such
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks",
+                 "_global_backward_pre_hooks")
+
+
 def transition_parameters(radius_logit: torch.Tensor, theta: torch.Tensor):
     """``lambda = r e^{i theta}``, ``gamma = sqrt(max(1 - r^2, 1e-4))`` (reference :1169-1173)."""
     radius = torch.sigmoid(radius_logit).clamp(0.50, 0.99995).float()
@@ -39,13 +44,21 @@ def transition_parameters(radius_logit: torch.Tensor, theta: torch.Tensor):
             torch.sqrt((1.0 - radius.square()).clamp_min(1e-4)))
 
 
+def plain_linear(module: nn.Module) -> bool:
+    """Whether calling ``module`` is ``F.linear`` on its parameters and nothing else (hooks aside):
+    no subclass, no ``forward`` of its own, none put in place of torch's."""
+    return (type(module) is nn.Linear and "forward" not in vars(module)
+            and nn.Linear.forward.__module__ == nn.Linear.__module__)
+
+
 def _native_mixer(m: nn.Module, x: torch.Tensor) -> Optional[torch.Tensor]:
     """``fused_mixer_forward`` as one native autograd node (``csrc/torch_mixer.cpp``); None where
     a projection is not a plain ``nn.Linear`` or a tensor is not what the node works on."""
     write, out, gate = m.write_proj, m.out_proj, m.gate_proj
-    if not (type(write) is nn.Linear and type(out) is nn.Linear and type(gate) is nn.Linear
+    if not (plain_linear(write) and type(out) is nn.Linear and type(gate) is nn.Linear
             and not write._forward_hooks and not write._forward_pre_hooks
-            and not write._backward_hooks and not write._backward_pre_hooks):
+            and not write._backward_hooks and not write._backward_pre_hooks
+            and not any(getattr(nn.modules.module, h) for h in _GLOBAL_HOOKS)):
         return None
     params = (write.weight, write.bias, m.radius_logit, m.theta, m.read_norm.weight, out.weight,
               out.bias, gate.weight, gate.bias)

@@ -1,23 +1,29 @@
 """Recognises a stack of the reference's Field blocks that the native inference path can run.
 
-``plan(model)`` looks at a field-only language model (the reference's ``ByteLM``,
+``plan(model, device)`` looks at a field-only language model (the reference's ``ByteLM``,
 ``field_only_v4_chunked_triton_wiki100.py:1306-1344``) and returns a ``FieldStack``
 (``csrc/torch_stack.cpp``) that runs its blocks under bfloat16 autocast with a handful of launches
 per block, or None if any part of the model is not what that path computes: other module
 classes, hooks, parameters that are not dense fp32 tensors on one GPU, sizes the kernels do not
 take. The feed-forward and the norms are modules of the model's own, so each one is also run once
-on a small input and compared with the formula the kernels use.
+on a small input and compared with the formula the kernels use. What that comparison rests on is
+part of the plan: the class's ``forward`` and the instance's attributes, which therefore have to be
+plain values, beside the parameters, children and hooks.
 """
 from __future__ import annotations
 
+import types
 from typing import List, Optional
 
 import torch
 import torch.nn.functional as F
 
 from . import _lib
+from .mixer import plain_linear
 
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks")
+_OWN = frozenset(vars(torch.nn.Module()))  # what every module's __dict__ holds
+_PLAIN = (int, float, bool, str, type(None), torch.dtype, types.FunctionType, types.BuiltinFunctionType)
 
 
 class _NotApplicable(Exception):
@@ -30,19 +36,37 @@ def _need(ok: bool) -> None:
 
 
 class _Survey:
-    """Collects what the plan depends on: parameters, the slots they sit in, hook dictionaries,
-    and how far each module is from the formula it is taken for."""
+    """Collects what the plan depends on: parameters, the slots they sit in, dictionaries and their
+    sizes (hooks: none), classes and their ``forward``, and how far each module is from the formula it
+    is taken for."""
 
     def __init__(self, device):
         self.device = device
-        self.slots, self.hooks, self.errors = [], [], []
+        self.slots, self.hooks, self.sizes, self.errors = [], [], [], []
+        self.classes = {}
 
     def child(self, module, name: str):
         _need(name in module._modules)
         child = module._modules[name]
         self.slots.append((module._modules, name, child))
         self.hooks += [getattr(child, h) for h in _HOOKS]
+        _need("forward" not in vars(child))  # (nor later: the size of the dictionary is kept)
+        self.sizes.append((vars(child), len(vars(child))))
         return child
+
+    def formula(self, module, parameters: set, children: set) -> None:
+        """A module that is taken for a formula: nothing in it beside these but plain attributes."""
+        for own, names in ((module._parameters, parameters), (module._modules, children), (module._buffers, set())):
+            _need({k for k, v in own.items() if v is not None} == names)
+            self.slots += [(own, k, None) for k, v in own.items() if v is None]
+            self.sizes.append((own, len(own)))
+        for key, value in vars(module).items():
+            if key not in _OWN:
+                items = value if type(value) is tuple else (value,)
+                _need(all(isinstance(v, _PLAIN) for v in items))
+            if key not in _OWN or key == "training":
+                self.slots.append((vars(module), key, value))
+        self.classes[type(module)] = type(module).forward
 
     def parameter(self, module, name: str, *shape: int) -> torch.Tensor:
         _need(name in module._parameters)
@@ -54,7 +78,8 @@ class _Survey:
 
     def linear(self, module, name: str, rows: int, cols: int, bias: bool):
         lin = self.child(module, name)
-        _need(type(lin) is torch.nn.Linear and (lin.bias is not None) == bias)
+        _need(plain_linear(lin) and (lin.bias is not None) == bias)
+        self.classes[torch.nn.Linear] = torch.nn.Linear.forward
         weight = self.parameter(lin, "weight", rows, cols)
         return (weight, self.parameter(lin, "bias", rows)) if bias else (weight, None)
 
@@ -62,6 +87,7 @@ class _Survey:
         norm = self.child(module, name)
         _need(type(norm).__name__ == "RMSNorm" and isinstance(getattr(norm, "eps", None), float))
         weight = self.parameter(norm, "weight", dim)
+        self.formula(norm, {"weight"}, set())
         self.compare(norm, dim, lambda x: x * torch.rsqrt(x.square().mean(-1, keepdim=True) + norm.eps) * weight)
         return weight, norm.eps
 
@@ -96,6 +122,7 @@ def _block(s: _Survey, blocks, key: str, dim: int):
         u, v = F.linear(x, w12).chunk(2, dim=-1)
         return F.linear(F.silu(u) * v, w3)
 
+    s.formula(ff, set(), {"w12", "w3"})
     s.compare(ff, dim, feed_forward)
     radius = s.parameter(mixer, "radius_logit", channels)
     theta = s.parameter(mixer, "theta", channels)
@@ -104,9 +131,8 @@ def _block(s: _Survey, blocks, key: str, dim: int):
 
 @torch.no_grad()
 def plan(model: torch.nn.Module, device: torch.device) -> Optional[object]:
-    """The native runner for ``model``'s blocks, or None if they are not what it computes."""
-    if torch.cuda.is_current_stream_capturing():
-        return None  # the comparison below reads a value back
+    """The native runner for ``model``'s blocks, or None if they are not what it computes. Reads a value
+    back, so not while a graph is being captured."""
     s = _Survey(device)
     try:
         with torch.autocast("cuda", enabled=False):
@@ -125,7 +151,7 @@ def plan(model: torch.nn.Module, device: torch.device) -> Optional[object]:
             _need(len(widths) == 1)
             tail, tail_eps = [], 0.0
             head = model._modules.get("lm_head")
-            if type(head) is torch.nn.Linear and not any(getattr(head, h) for h in _HOOKS):
+            if isinstance(head, torch.nn.Linear) and plain_linear(head) and not any(getattr(head, h) for h in _HOOKS):
                 weight, tail_eps = s.norm(model, "final_norm", dim)
                 w, b = s.linear(model, "lm_head", head.weight.shape[0], dim, head.bias is not None)
                 tail = [weight, w] + ([] if b is None else [b])
@@ -134,5 +160,5 @@ def plan(model: torch.nn.Module, device: torch.device) -> Optional[object]:
             _need(float(torch.stack(s.errors).max()) < 1e-4)
     except (_NotApplicable, AttributeError):
         return None
-    sizes = [(h, 0) for h in s.hooks] + [(blocks._modules, len(params))]
-    return _lib.native().FieldStack(params, eps, s.slots, sizes, tail, tail_eps)
+    sizes = [(h, 0) for h in s.hooks] + [(blocks._modules, len(params))] + s.sizes
+    return _lib.native().FieldStack(params, eps, s.slots, sizes, list(s.classes.items()), tail, tail_eps)
