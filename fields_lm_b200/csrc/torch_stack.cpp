@@ -46,8 +46,10 @@ class FieldStack {
     FieldStack(const std::vector<std::vector<Tensor>>& params, const std::vector<std::pair<double, double>>& eps,
                std::vector<std::tuple<py::object, py::object, py::object>> slots,
                std::vector<std::pair<py::object, int64_t>> sizes,
-               std::vector<std::pair<py::object, py::object>> classes, std::vector<Tensor> tail, double tail_eps)
-        : slots_(std::move(slots)), sizes_(std::move(sizes)), classes_(std::move(classes)), tail_eps_(tail_eps) {
+               std::vector<std::pair<py::object, py::object>> classes, std::vector<Tensor> tail, double tail_eps,
+               bool usable)
+        : slots_(std::move(slots)), sizes_(std::move(sizes)), classes_(std::move(classes)), tail_eps_(tail_eps),
+          usable_(usable) {
         for (size_t i = 0; i < params.size(); ++i) {
             Block b;
             TORCH_CHECK_VALUE(params[i].size() == Block::kCount, "a block has ", (int)Block::kCount, " parameters");
@@ -87,6 +89,9 @@ class FieldStack {
         other->laid_out_ = other->step_laid_out_ = false;
         return other;
     }
+
+    // Whether the model's modules compute what this class does; if not, the plan only stands for the refusal.
+    bool usable() const { return usable_; }
 
     // Whether step() goes on to the logits.
     bool has_head() const { return !tail_.empty(); }
@@ -314,6 +319,7 @@ class FieldStack {
     std::vector<Source> tail_;  // final norm weight, head weight[, head bias]; may be empty
     Tensor head_w_, head_b_;
     double tail_eps_;
+    bool usable_;
     int D_ = 0, H_ = 0;
     bool laid_out_ = false, step_laid_out_ = false;
 };
@@ -324,7 +330,8 @@ void add_stack(PyObject* module) {
         .def(py::init<const std::vector<std::vector<Tensor>>&, const std::vector<std::pair<double, double>>&,
                       std::vector<std::tuple<py::object, py::object, py::object>>,
                       std::vector<std::pair<py::object, int64_t>>, std::vector<std::pair<py::object, py::object>>,
-                      std::vector<Tensor>, double>())
+                      std::vector<Tensor>, double, bool>())
+        .def_property_readonly("usable", &FieldStack::usable)
         .def_property_readonly("has_head", &FieldStack::has_head)
         .def("same_model", &FieldStack::same_model)
         .def("current", &FieldStack::current)

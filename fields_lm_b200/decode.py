@@ -48,8 +48,7 @@ class FieldStackDecoder:
         self._refused = False  # it did not apply when last asked for (asked again at a prefill)
 
     def reset(self) -> None:
-        self.states = None
-        self._stack = None
+        self.states = None  # (the plan stays: it notices by itself when the model changes)
 
     @staticmethod
     def _bf16_products(x: torch.Tensor) -> bool:
@@ -63,13 +62,13 @@ class FieldStackDecoder:
         """The runner for the model as it is now, or None; one of its own for a graph that is being
         captured, whose replays have to follow the weights and must not depend on this object."""
         if torch.cuda.is_current_stream_capturing():
-            usable = self._stack is not None and self._stack.same_model()
+            usable = self._stack is not None and self._stack.usable and self._stack.same_model()
             return self._stack.fresh() if usable else None  # (a plan cannot be made here)
         if self._stack is None or not self._stack.same_model():
             from .stack import plan
             self._stack = plan(self.model, x.device)
-            self._refused = self._stack is None
-        return self._stack
+            self._refused = self._stack is None or not self._stack.usable
+        return None if self._refused else self._stack
 
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, last_only: bool = True) -> torch.Tensor:

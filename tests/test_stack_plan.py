@@ -92,3 +92,60 @@ def test_mixer_leaves_other_forwards_alone(monkeypatch):
     assert len(reached) == 1
     mixer._native_mixer(m, x)
     assert len(reached) == 2
+
+
+def test_comparison_does_not_rest_on_the_weights():
+    """A feed-forward of another formula is found out although its weights are zero, and one refusal is enough."""
+    class PackedSwiGLU(mirror.PackedSwiGLU):
+        def forward(self, x):
+            gate, value = self.w12(x).chunk(2, dim=-1)
+            return self.w3(F.gelu(gate) * value)
+
+    model = LM()
+    for block in model.blocks:
+        block.ff.__class__ = PackedSwiGLU
+        torch.nn.init.zeros_(block.ff.w3.weight)
+    plan = _plan(model)
+    assert not plan.usable and plan.same_model()
+    odd = LM()
+    odd.blocks[1].ff.__class__ = PackedSwiGLU  # one of several
+    assert not _plan(odd).usable
+    for m in (LM(), LM().requires_grad_(False)):
+        torch.nn.init.constant_(m.blocks[0].ff.w3.weight, float("nan"))  # to be loaded yet
+        assert _plan(m).usable
+
+
+def test_decoder_keeps_plan_and_refusal(monkeypatch):
+    from fields_lm_b200 import FieldStackDecoder
+    made = []
+    plan = stack.plan
+    monkeypatch.setattr(stack, "plan", lambda *a: made.append(1) or plan(*a))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    x = torch.zeros(1, 64)
+    model = LM()
+    dec = FieldStackDecoder(model)
+    first = dec._native_stack(x)
+    dec.reset()
+    assert first is not None and dec._native_stack(x) is first and made == [1]
+    model.blocks[0].ff_norm.eps = 1e-3
+    assert dec._native_stack(x) not in (None, first) and made == [1, 1]
+    mirror_forward = mirror.PackedSwiGLU.forward
+    monkeypatch.setattr(mirror.PackedSwiGLU, "forward", lambda self, x: 2 * mirror_forward(self, x))
+    assert dec._native_stack(x) is None and dec._native_stack(x) is None and made == [1, 1, 1] and dec._refused
+    monkeypatch.undo()
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert dec._native_stack(x) is not None and not dec._refused
+
+
+def test_comparison_leaves_the_model_alone():
+    class PackedSwiGLU(mirror.PackedSwiGLU):
+        def forward(self, x):
+            assert self is not model.blocks[0].ff
+            return super().forward(x[:, None])  # a formula that fails is a refusal
+
+    model = LM()
+    before = {k: (v, v.clone()) for k, v in model.state_dict(keep_vars=True).items()}
+    model.blocks[0].ff.__class__ = PackedSwiGLU
+    assert _plan(model) is None or not _plan(model).usable
+    for k, v in model.state_dict(keep_vars=True).items():
+        assert v is before[k][0] and torch.equal(v, before[k][1])
