@@ -47,6 +47,10 @@ class FieldStackDecoder:
         self._stack = None     # native runner of the blocks (csrc/torch_stack.cpp), where it applies
         self._refused = False  # it did not apply when last asked for (asked again at a prefill)
 
+    def __getstate__(self) -> dict:
+        # a copy or an unpickled decoder makes a plan of its own
+        return dict(vars(self), _stack=None, _refused=False)
+
     def reset(self) -> None:
         self.states = None  # (the plan stays: it notices by itself when the model changes)
 

@@ -1,5 +1,8 @@
 """What the plan of the native inference path accepts, and what it notices afterwards (``fields_lm_b200.stack``; no
 GPU: a plan only looks at the model)."""
+import copy
+import pickle
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -149,3 +152,15 @@ def test_comparison_leaves_the_model_alone():
     assert _plan(model) is None or not _plan(model).usable
     for k, v in model.state_dict(keep_vars=True).items():
         assert v is before[k][0] and torch.equal(v, before[k][1])
+
+
+def test_decoder_can_be_copied_and_pickled(monkeypatch):
+    from fields_lm_b200 import FieldStackDecoder
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    dec = FieldStackDecoder(LM())
+    dec.states = [torch.ones(1, 64), torch.ones(1, 64)]
+    plan = dec._native_stack(torch.zeros(1, 64))
+    for twin in (copy.copy(dec), copy.deepcopy(dec), pickle.loads(pickle.dumps(dec))):
+        assert twin._stack is None and torch.equal(twin.states[1], dec.states[1])
+        assert twin._native_stack(torch.zeros(1, 64)) is not None
+    assert dec._stack is plan
