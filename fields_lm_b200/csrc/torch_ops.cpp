@@ -305,10 +305,11 @@ static PyObject* wrap2(const Tensor& a, const Tensor& b) {
     PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(b));
     return out;
 }
+// Whether the autograd node has to see the call: for a gradient, or to refuse a forward-mode tangent (which
+// no_grad does not drop).
 static bool wants_grad(std::initializer_list<const Tensor*> ts) {
-    if (!at::GradMode::is_enabled()) return false;
     for (const Tensor* t : ts)
-        if (t->defined() && t->requires_grad()) return true;
+        if (t->defined() && ((at::GradMode::is_enabled() && t->requires_grad()) || t->_fw_grad(0).defined())) return true;
     return false;
 }
 

@@ -150,3 +150,17 @@ def test_a_failed_allocation_leaves_nothing_behind():
     host = [p.cpu().numpy() for p in par]
     for g, t in zip(got, (large, small, large, small)):
         assert rel_err(g.cpu().numpy(), field_oracle.forward(t.cpu().numpy(), *host)[0]) < FP32_TOL
+
+
+@pytest.mark.parametrize("which", range(4))
+@pytest.mark.parametrize("grad", [True, False])
+def test_forward_mode_tangents_are_refused(which, grad):
+    """None of the operators has a forward-mode derivative; a tangent is not dropped in silence."""
+    import torch.autograd.forward_ad as fwd
+    leaves = [t.detach() for t in _case(1, 20, 8, 1)[0]]
+    with fwd.dual_level(), torch.set_grad_enabled(grad):
+        leaves[which] = fwd.make_dual(leaves[which], torch.ones_like(leaves[which]))
+        with pytest.raises(RuntimeError):
+            fused_field_read(*leaves)
+        with pytest.raises(RuntimeError):
+            field_read_with_state(*leaves)
