@@ -227,14 +227,14 @@ __global__ void __launch_bounds__(kRowThreads) finish_grad(const FinishGradParam
         const int c = ((int)blockIdx.x - p.transition_block) * kRowThreads + (int)threadIdx.x;
         if (c >= p.C) return;
         const float sig = 1.0f / (1.0f + expf(-p.radius_logit[c]));
-        const float r = fminf(fmaxf(sig, 0.50f), 0.99995f);
+        const float r = clamp_nan(sig, 0.50f, 0.99995f);
         const float co = cosf(p.theta[c]), si = sinf(p.theta[c]);
-        const float q = 1.0f - r * r, gm = sqrtf(fmaxf(q, 1e-4f));
+        const float q = 1.0f - r * r, gm = sqrtf(clamp_nan(q, 1e-4f, 1.0f));
         const float gtr = p.g_tr[c], gti = p.g_ti[c];
         float gr = gtr * co + gti * si;
         if (q >= 1e-4f) gr -= p.g_gm[c] * r / gm;
         if (p.g_theta) p.g_theta[c] = r * (gti * co - gtr * si);
-        if (p.g_radius) p.g_radius[c] = sig >= 0.50f && sig <= 0.99995f ? gr * sig * (1.0f - sig) : 0.0f;
+        if (p.g_radius) p.g_radius[c] = (sig >= 0.50f && sig <= 0.99995f ? gr : 0.0f) * sig * (1.0f - sig);
         return;
     }
     int k = 0;

@@ -30,6 +30,9 @@ namespace fields {
 
 constexpr int kRowThreads = 256;
 
+// clamp as torch has it: a NaN stays one.
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) { return x < lo ? lo : x > hi ? hi : x; }
+
 __device__ __forceinline__ Vec<4> load4(const float* p) { return vec_load<4>(p); }
 __device__ __forceinline__ Vec<4> load4(const uint16_t* p) { return io_load4(p); }
 
@@ -350,11 +353,11 @@ __global__ void __launch_bounds__(kRowThreads) layout_block(const __grid_constan
     if (block >= p.first[kLayoutPieces]) {
         const int c = (int)(block - p.first[kLayoutPieces]) * kRowThreads + (int)threadIdx.x;
         if (c >= p.C) return;
-        const float r = fminf(fmaxf(1.0f / (1.0f + expf(-p.radius_logit[c])), 0.50f), 0.99995f);
+        const float r = clamp_nan(1.0f / (1.0f + expf(-p.radius_logit[c])), 0.50f, 0.99995f);
         const float t = p.theta[c];
         p.par[c] = r * cosf(t);
         p.par[p.C + c] = r * sinf(t);
-        p.par[2 * p.C + c] = sqrtf(fmaxf(1.0f - r * r, 1e-4f));
+        p.par[2 * p.C + c] = sqrtf(clamp_nan(1.0f - r * r, 1e-4f, 1.0f));
         return;
     }
     int k = 0;

@@ -164,3 +164,18 @@ def test_frozen_parameters_cost_nothing(wanted):
     spared = sum(n for name, n in sizes.items()
                  if name not in wanted and not (name == "out_proj.weight" and "read_norm.weight" in wanted))
     assert peak <= most - 4 * spared * 0.9
+
+
+@pytest.mark.parametrize("name", ["radius_logit", "theta"])
+def test_nan_parameters_reach_the_outputs(name):
+    """A NaN in the transition of one channel: the output and the gradients of that channel are NaN, as composed."""
+    torch.manual_seed(7)
+    m = mirror.IndependentVacancyField(64).cuda()
+    with torch.no_grad():
+        getattr(m, name)[5] = float("nan")
+    x = torch.randn(1, 20, 64, device="cuda", requires_grad=True)
+    gy = torch.randn_like(x)
+    got, want = _grads(m, x, gy, True), _grads(m, x, gy, False)
+    assert bool(want["y"].isnan().all()) and bool(want[name][5].isnan())
+    for key in want:
+        assert torch.equal(got[key].isnan(), want[key].isnan()), key
