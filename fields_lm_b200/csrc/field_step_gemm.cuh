@@ -106,6 +106,7 @@ struct StepBlockParams {
     int M, D, C, H;
     // tiling
     int tiles_n, S, k_blocks;
+    int wait_first;         // non-zero: parameters are read, and the next kernel let in, after the kernels before this one
 };
 
 __device__ __forceinline__ void store8(float* p, const float* v) {
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
     auto load_a = [&](int i) {
         tma_load2(stage_a(i), &a_map, (kb0 + i) * kStepKBlock, m0, full + (i % kStages) * 8);
     };
+    if (p.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (control) {
         for (int i = 0; i < kStages; ++i) {
             mbar_init(full + i * 8, 1);
@@ -352,7 +354,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
         mbar_init(got, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (S > 1) mbar_expect(got, (unsigned)((S - 1) * (own * kSlice + (Epi::kScaled ? 1 : 0)) * kStepRows * 4));
-        // weights do not depend on the kernels before this one
+        // weights do not depend on the kernels before this one (or those have been waited for)
         for (int i = 0; i < kStages && i < count; ++i) load_b(i);
     }
     __syncwarp();

@@ -166,13 +166,15 @@ using Stream = cudaStream_t;
 static thread_local const char* g_last_error = "no error";
 
 // Programmatic dependent launch. Every kernel of this library is launched with the
-// programmatic-serialization attribute and begins by waiting, before it touches any memory,
-// until the kernel before it on the stream has completed and its writes are visible. The
-// launch itself (grid set-up, block scheduling) then overlaps the end of the previous kernel
-// instead of following it. Because every kernel waits, the completion order of the stream is
-// kept along the whole chain. No kernel signals early: letting the next grid take SM slots
-// while this one still ran its last blocks was measured and was slower. The instruction does
-// nothing in a kernel launched without the attribute (FIELDS_READ_PDL=0).
+// programmatic-serialization attribute and waits until the kernel before it on the stream has
+// completed and its writes are visible. The launch itself (grid set-up, block scheduling) then
+// overlaps the end of the previous kernel instead of following it. Because every kernel waits, the
+// completion order of the stream is kept along the whole chain. All but one wait before they
+// touch any memory and do not signal early: letting the next grid take SM slots while this one
+// still ran its last blocks was measured and was slower for the recurrence. step_gemm does both: it
+// lets the next kernel in at its start and reads parameters ahead of its own wait, which its
+// caller has to allow (settled, in fields_step_args). The instruction does nothing in a kernel launched
+// without the attribute (FIELDS_READ_PDL=0).
 __device__ __forceinline__ void wait_for_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -2265,7 +2267,10 @@ int fields_step_block(const struct fields_step_args* g, void* stream) {
     p.in_b = g->in_b; p.par = g->par; p.out_b = g->out_b;
     p.read_eps = g->read_eps; p.ff_eps = g->ff_eps; p.M = g->rows; p.D = D; p.C = C; p.H = H;
     Stream st = reinterpret_cast<Stream>(stream);
+    // the first product waits where a parameter may still be on its way; it lets the second in afterwards
+    p.wait_first = !g->settled;
     int rc = launch_step<EpiIn>(g->xb, g->in_w, 5 * C, D, C / 8, p, st);
+    p.wait_first = 0;
     const bool narrow = (g->rows + kStepRows - 1) / kStepRows * ((D + 63) / 64) * 8 <= 148;
     if (!rc) rc = narrow ? launch_step<EpiOut<4>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st)
                          : launch_step<EpiOut<8>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st);

@@ -231,8 +231,7 @@ class FieldStack {
         return true;
     }
 
-    // Weights in the order of the fused step. Its first kernel reads them before it waits for the kernel
-    // ahead of it, so a kernel that waits for this one has to stand between the two (step()'s copy of x).
+    // Weights in the order of the fused step.
     void step_layout(void* st) {
         const Api& f = api();
         const int64_t D = D_, C = D / 2;
@@ -266,6 +265,7 @@ class FieldStack {
         g.x = fp(x); g.y = fp(y); g.xb = vp(xb); g.yb = vp(yb); g.read = vp(read); g.gate = vp(gate); g.act = vp(act);
         g.read_sq = fp(read_sq); g.y_sq = fp(y_sq);
         g.rows = (int)N; g.dim = D_; g.hidden = H_;
+        g.settled = 1;  // step()'s copy of x stands between a layout and the first block, and waits for it
         for (size_t i = 0; i < blocks_.size(); ++i) {
             const Block& b = blocks_[i];
             g.state = fp(states[i]);

@@ -525,7 +525,9 @@ int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, fl
  * fields_step_block: x [M, D] in (the block's input; xb its bfloat16 copy), y [M, D] out (may be x) and
  *   xb its copy; state [M, 2C] advances in place. out_w16, w3_16 and par as fields_stack_layout leaves
  *   them. Scratch: yb [M, D], read [M, 4C], gate [M, D], act [M, H] bfloat16, read_sq [C / 8, M],
- *   y_sq [D / 8, M].
+ *   y_sq [D / 8, M]. The products load their weights, in_b, par and out_b ahead of the kernel before them on the
+ *   stream if settled is non-zero: these were then complete, in stream order, before the kernel (or copy) that
+ *   this call follows. 0: nothing is read ahead of what the call follows (a layout, say).
  */
 struct fields_step_weights {
     const float *write_w, *write_b, *gate_w, *gate_b, *w12, *ff_norm_w;
@@ -541,7 +543,7 @@ struct fields_step_args {
     const void *in_w, *out_w16, *w12_w, *w3_16;
     const float *in_b, *par, *out_b;
     float read_eps, ff_eps;
-    int rows, dim, hidden;
+    int rows, dim, hidden, settled;
 };
 int fields_step_w12_rows(int hidden);
 int fields_step_layout(const struct fields_step_weights *weights, void *stream);
