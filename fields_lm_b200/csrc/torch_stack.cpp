@@ -10,6 +10,7 @@
 // it). Parameters without a count (inference tensors) are laid out for every step.
 #include "torch_gemm.h"
 
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/ops/addmm_cuda_dispatch.h>
 #include <ATen/ops/mm_cuda_dispatch.h>
 #include <torch/csrc/utils/pybind.h>
@@ -39,6 +40,89 @@ struct Block {
     // rows of `in` and w12 in the order of the fused step, its biases (made by the first step after a layout)
     Tensor step_in, step_w12, step_b;
     float* f(int i) const { return fp(src[i].t); }
+};
+
+// The copies of a plan lie in memory of the stream that first laid them out (home), and every later call may be
+// on another: a call waits for the layout, a layout for the calls on other streams, and the memory goes back only
+// behind all of them. On one stream this costs an event per layout. One thread issues at a time.
+class CopyUses {
+  public:
+    using Stream = c10::cuda::CUDAStream;
+
+    // One call that uses (or, `writes`, lays out) the copies on the current stream of `device`.
+    class Call {
+      public:
+        Call(CopyUses& u, c10::Device device, bool writes)
+            : u_(u), lock_(u.mu_), stream_(c10::cuda::getCurrentCUDAStream(device.index())), writes_(writes) {
+            if (!u.home_) u.home_ = stream_;
+            if (u.laid_on_ && *u.laid_on_ != stream_) u.laid_.block(stream_);
+            if (writes) u.wait_for_uses(stream_);
+        }
+        // (not on the way out of an exception alone: what was issued before it is a use as well)
+        ~Call() {
+            try {
+                if (writes_) laid_out();
+                else if (stream_ != *u_.home_ || external(stream_)) u_.used_on(stream_);
+            } catch (...) {
+            }
+        }
+        Call(const Call&) = delete;
+        // what a reading call has laid out on the way
+        void laid_out() {
+            if (captured(stream_)) return;  // (a plan of its own, used on this stream only)
+            u_.laid_.record(stream_);
+            u_.laid_on_ = stream_;
+        }
+
+      private:
+        CopyUses& u_;
+        std::lock_guard<std::recursive_mutex> lock_;
+        Stream stream_;
+        bool writes_;
+    };
+
+    CopyUses() = default;
+    CopyUses(const CopyUses&) = delete;
+    ~CopyUses() {
+        try {
+            if (home_ && !captured(*home_)) {
+                if (laid_on_ && *laid_on_ != *home_) laid_.block(*home_);
+                wait_for_uses(*home_);
+            }
+        } catch (...) {
+        }
+    }
+
+  private:
+    struct Use {
+        Stream stream;
+        at::cuda::CUDAEvent last;
+    };
+    static bool captured(Stream s) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(s.stream(), &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+    }
+    // another library's stream, which may be gone when a later call would record on it
+    static bool external(Stream s) { return s.id() != 0 && !(s.id() & 1); }
+    void used_on(Stream s) {
+        if (captured(s)) return;
+        for (Use& u : uses_)
+            if (u.stream == s) return u.last.record(s);
+        uses_.push_back(Use{s, at::cuda::CUDAEvent()});
+        uses_.back().last.record(s);
+    }
+    void wait_for_uses(Stream s) {
+        if (captured(s)) return;
+        if (*home_ != s && !external(*home_) && !captured(*home_)) used_on(*home_);
+        for (Use& u : uses_)
+            if (u.stream != s) u.last.block(s);
+        uses_.clear();
+    }
+
+    std::recursive_mutex mu_;
+    std::optional<Stream> home_, laid_on_;
+    at::cuda::CUDAEvent laid_;
+    std::vector<Use> uses_;  // last uses on streams other than home since all of them were waited for
 };
 
 class FieldStack {
@@ -84,8 +168,9 @@ class FieldStack {
     // itself, from the weights of the moment it runs, into memory of its own.
     std::unique_ptr<FieldStack> fresh() const {
         auto other = std::make_unique<FieldStack>(*this);
+        other->uses_ = std::make_shared<CopyUses>();
         for (Block& b : other->blocks_) b.in_w = b.in_b = b.in_t = b.out_t = b.w12_t = b.w3_t = b.par = b.step_in = b.step_w12 = b.step_b = Tensor();
-        other->head_w_ = other->head_b_ = Tensor();
+        other->head_ = other->head_w_ = other->head_b_ = Tensor();
         other->laid_out_ = other->step_laid_out_ = false;
         return other;
     }
@@ -100,7 +185,9 @@ class FieldStack {
     void layout() {
         const c10::Device dev = blocks_[0].src[0].t.device();
         const c10::cuda::CUDAGuard guard(dev);
+        const CopyUses::Call call(*uses_, dev, true);
         const int64_t D = D_, C = D / 2, H = H_;
+        laid_out_ = step_laid_out_ = false;
         std::vector<fields_stack_weights> all;
         for (Block& b : blocks_) {
             for (Source& s : b.src) s.copied();
@@ -125,8 +212,17 @@ class FieldStack {
         check(api().fields_stack_layout(all.data(), (int)all.size(), stream_of(blocks_[0].in_w)), "fields_stack_layout");
         if (!tail_.empty()) {
             for (Source& s : tail_) s.copied();
-            head_w_ = tail_[1].t.detach().to(at::kBFloat16).t();
-            if (tail_.size() > 2) head_b_ = tail_[2].t.detach().to(at::kBFloat16);
+            const at::NoGradGuard no_grad;
+            auto copy = [&](Tensor& to, const Tensor& from) {
+                if (!to.defined()) {
+                    const c10::InferenceMode off(false);  // written again in whatever mode the next layout has
+                    to = empty(from.sizes(), at::kBFloat16, dev);
+                }
+                to.copy_(from);
+            };
+            copy(head_, tail_[1].t);
+            head_w_ = head_.t();
+            if (tail_.size() > 2) copy(head_b_, tail_[2].t);
         }
         laid_out_ = true;
         step_laid_out_ = false;
@@ -139,6 +235,7 @@ class FieldStack {
         const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
+        const CopyUses::Call call(*uses_, dev, false);
         void* st = stream_of(x);
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
                      read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
@@ -187,13 +284,17 @@ class FieldStack {
             aligned = aligned && reinterpret_cast<uintptr_t>(s.data_ptr()) % 16 == 0;
         }
         const c10::cuda::CUDAGuard guard(x.device());
+        CopyUses::Call call(*uses_, x.device(), false);
         if (!aligned)
             for (Tensor& s : own) s = s.clone();
         // Four launches per block while its products have tiles (128 rows x 64 features) few enough that K
         // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 600 us at 16 rows and 670 at 256
         // against 763 and 768 with library products, but 986 against 787 at 384.
         const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
-        if (fused && !step_laid_out_) step_layout(stream_of(x));
+        if (fused && !step_laid_out_) {
+            step_layout(stream_of(x));
+            call.laid_out();
+        }
         const Tensor xb = empty({N, D}, at::kBFloat16, x.device()), y = empty({N, D}, at::kFloat, x.device());
         check(api().fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, stream_of(x)),
               "fields_stack_close_ff");
@@ -317,11 +418,12 @@ class FieldStack {
     std::vector<std::pair<py::object, int64_t>> sizes_;                  // dicts and the sizes they have to have
     std::vector<std::pair<py::object, py::object>> classes_;             // and the `forward` they have to have
     std::vector<Source> tail_;  // final norm weight, head weight[, head bias]; may be empty
-    Tensor head_w_, head_b_;
+    Tensor head_, head_w_, head_b_;
     double tail_eps_;
     bool usable_;
     int D_ = 0, H_ = 0;
     bool laid_out_ = false, step_laid_out_ = false;
+    std::shared_ptr<CopyUses> uses_ = std::make_shared<CopyUses>();  // destroyed before the copies above
 };
 
 void add_stack(PyObject* module) {

@@ -194,3 +194,69 @@ def test_activations_that_are_not_aligned():
     model.emb.__class__ = Shifted
     got, _ = _run(model, tokens, 5, True)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_calls_on_other_streams_wait_for_the_copies():
+    """A step on a stream that does not wait for the one of the layout, a layout on one that does not wait for the one
+    of a step, and a decoder that goes away while its last call is pending."""
+    torch.manual_seed(6)
+    model = LM(256, 4, 704).cuda()
+    tokens = torch.randint(0, 97, (8, 12), device="cuda")
+    _, ref = _run(model, tokens, 12, True)
+    kept = [s.clone() for s in ref.states]
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = ref.step(tokens[:, 0])
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        dec = FieldStackDecoder(model)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            dec._native_stack(model.emb(tokens))  # (making the plan waits for the GPU)
+            states = [s.clone() for s in kept]
+            torch.cuda.synchronize()
+            with torch.cuda.stream(a):
+                torch.cuda._sleep(20_000_000)
+                dec.prefill(tokens)
+            dec.states = states
+            with torch.cuda.stream(b):
+                got = dec.step(tokens[:, 0])
+            with torch.cuda.stream(a):
+                torch.cuda._sleep(20_000_000)
+                dec.states = [s.clone() for s in kept]
+                again = dec.step(tokens[:, 0])
+            with torch.cuda.stream(b):
+                other = dec.prefill(tokens)
+                dec.states = None
+            del dec
+            with torch.cuda.stream(a):
+                junk = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(64)]
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and torch.equal(again, want) and not bool(other.isnan().any())
+        del junk
+
+
+def test_threads_share_a_decoder():
+    import threading
+    torch.manual_seed(7)
+    model = LM(128, 3, 352).cuda()
+    batches = [torch.randint(0, 97, (4, 9 + i), device="cuda") for i in range(4)]
+    want = [_run(model, t, t.shape[1], True)[0][0] for t in batches]
+    dec, bad = FieldStackDecoder(model), []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()), torch.autocast("cuda", dtype=torch.bfloat16):
+                for _ in range(30):
+                    got = dec.prefill(batches[i])
+                    torch.cuda.current_stream().synchronize()
+                    assert _rel(got, want[i]) < 1e-6
+        except BaseException as e:  # noqa: BLE001
+            bad.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
