@@ -4,6 +4,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -16,7 +17,9 @@
 #include <atomic>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/fields_read.h"
@@ -104,40 +107,106 @@ inline bool all_aligned(std::initializer_list<const void*> ptrs, uintptr_t bytes
     return any % bytes == 0;
 }
 
-// The workspace of one forward or backward pass on the current stream.
-//
-// One is kept per stream (fields_read_use_kept), for the last few streams, up to a size: that saves an
-// allocation and a fill launch per pass, about 4 us of host time and 2 us on the GPU. It is held
-// (locked) while a pass is issued, because a pass may be two launches. Passes that are captured into a
-// graph and larger ones get one of their own, as does every pass where the library refuses.
-class PassWorkspace {
+// The kept workspaces of the torch layer: one per stream (fields_read_use_kept), for the last few streams, up to a
+// size. A workspace is 256 bytes and three times a half (two that take turns, and the partial rows), so at most
+// 8 x 96 MiB in all. When the allocator runs short on a device (less than an eighth of it left) it takes back
+// those that no pass is being issued on; the next pass on such a stream makes its own again.
+class KeptWorkspaces {
   public:
-    PassWorkspace(size_t need, const Tensor& on) {
-        const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(on.device().index());
-        // (torch's own streams: another library's may be destroyed while work is pending)
-        const bool own_stream = stream.id() == 0 || (stream.id() & 1);
-        if (need <= kMostBytes && own_stream &&
-            c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
-            kept_ = entry(on.device().index(), stream.id());
-            lock_ = std::unique_lock<std::mutex>(kept_->mu);
-            if (kept_->state.half_bytes < need || !kept_->ws.defined()) {
-                // (either call may throw: the entry changes when both are done)
-                size_t half = std::max(kLeastBytes, kept_->state.half_bytes);
-                while (half < need) half *= 2;
-                Tensor ws = empty({(int64_t)(256 + 3 * half)}, at::kByte, on.device());
-                C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0xFF, 256 + 2 * half, stream.stream()));
-                kept_->ws = std::move(ws);
-                kept_->state = fields_kept{half, {0, 0}, 0};
-            }
-            // the last step that can fail: a registration without a pass would be taken by the thread's next one
-            if (api().fields_read_use_kept(&kept_->state) != FIELDS_OK) {
-                lock_.unlock();
-                kept_.reset();
+    struct Entry {
+        int device;
+        int64_t stream;
+        std::mutex mu;
+        std::atomic<bool> busy{false};  // while `ws` must not be taken: by one who holds `mu`, or by release()
+        Tensor ws;
+        fields_kept state{};
+    };
+    // An entry held while a pass is issued on it (a pass may be two launches).
+    class Hold {
+      public:
+        Hold(int device, std::optional<int64_t> stream) {
+            if (!stream) return;
+            e_ = entry(device, *stream);
+            lock_ = std::unique_lock<std::mutex>(e_->mu);
+            while (e_->busy.exchange(true)) std::this_thread::yield();
+        }
+        ~Hold() { drop(); }
+        Hold(const Hold&) = delete;
+        void drop() {
+            if (!e_) return;
+            e_->busy = false;
+            lock_.unlock();
+            e_.reset();
+        }
+        explicit operator bool() const { return e_ != nullptr; }
+        Entry* operator->() const { return e_.get(); }
+
+      private:
+        std::shared_ptr<Entry> e_;
+        std::unique_lock<std::mutex> lock_;  // released before e_
+    };
+
+    // Called by the allocator of the current device, with its lock held, when it has no block for a request.
+    static bool release() {
+        int device = 0;
+        size_t left = 0, total = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaMemGetInfo(&left, &total) != cudaSuccess) return false;
+        const double limit = c10::cuda::CUDACachingAllocator::getMemoryFraction((c10::DeviceIndex)device) * (double)total;
+        const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats((c10::DeviceIndex)device);
+        const auto reserved = (double)stats.reserved_bytes[(size_t)c10::CachingAllocator::StatType::AGGREGATE].current;
+        if (std::min((double)left, limit - reserved) > (double)total / 8) return false;
+        const std::unique_lock<std::mutex> guard(mu(), std::try_to_lock);  // (its holder may wait for the allocator)
+        if (!guard) return false;
+        bool any = false;
+        for (const auto& e : list()) {
+            if (e->device != device || e->busy.exchange(true)) continue;
+            any = any || e->ws.defined();
+            e->ws = Tensor();
+            e->busy = false;
+        }
+        return any;
+    }
+
+  private:
+    static constexpr size_t kStreams = 8;
+    // (never destroyed: the allocator may be gone by the time a process ends)
+    static std::vector<std::shared_ptr<Entry>>& list() {
+        static auto* all = new std::vector<std::shared_ptr<Entry>>();  // most recently used first
+        return *all;
+    }
+    static std::mutex& mu() {
+        static auto* m = new std::mutex();
+        return *m;
+    }
+    static std::shared_ptr<Entry> entry(int device, int64_t stream) {
+        const std::lock_guard<std::mutex> guard(mu());
+        auto& all = list();
+        for (size_t i = 0; i < all.size(); ++i) {
+            if (all[i]->device == device && all[i]->stream == stream) {
+                if (i) std::rotate(all.begin(), all.begin() + i, all.begin() + i + 1);
+                return all.front();
             }
         }
+        if (all.size() == kStreams) all.pop_back();
+        auto e = std::make_shared<Entry>();
+        e->device = device;
+        e->stream = stream;
+        all.insert(all.begin(), e);
+        return e;
+    }
+};
+
+// The workspace of one forward or backward pass on the current stream: a kept one, which saves an allocation
+// and a fill launch per pass, about 4 us of host time and 2 us on the GPU. Passes that are captured into a
+// graph and larger ones get one of their own, as does every pass where the library refuses or where there is
+// memory for the pass but not for a kept workspace.
+class PassWorkspace {
+  public:
+    PassWorkspace(size_t need, const Tensor& on) : kept_(on.device().index(), keep_for(need, on)) {
+        if (kept_ && !ready(need, on)) kept_.drop();
         if (!kept_) {
             own_ = workspace(need, on.device());
-            api().fields_read_use_kept(nullptr);  // nor one that a caller of the library has left
+            api().fields_read_use_kept(nullptr);  // one that a caller of the library may have left
         }
         ptr_ = kept_ ? kept_->ws.data_ptr() : own_.data_ptr();
     }
@@ -156,35 +225,36 @@ class PassWorkspace {
 
   private:
     static constexpr size_t kLeastBytes = 1 << 20, kMostBytes = 32 << 20;  // of a half
-    static constexpr size_t kStreams = 8;
-    struct Entry {
-        int device;
-        int64_t stream;
-        std::mutex mu;
-        Tensor ws;
-        fields_kept state{};
-    };
-    static std::shared_ptr<Entry> entry(int device, int64_t stream) {
-        // most recently used first; never destroyed (the allocator may be gone by the time a process ends)
-        static auto* list = new std::vector<std::shared_ptr<Entry>>();
-        static auto* mu = new std::mutex();
-        const std::lock_guard<std::mutex> guard(*mu);
-        for (size_t i = 0; i < list->size(); ++i) {
-            if ((*list)[i]->device == device && (*list)[i]->stream == stream) {
-                if (i) std::rotate(list->begin(), list->begin() + i, list->begin() + i + 1);
-                return list->front();
+    // The current stream, if a pass of this size keeps its workspace there.
+    static std::optional<int64_t> keep_for(size_t need, const Tensor& on) {
+        const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(on.device().index());
+        // (torch's own streams: another library's may be destroyed while work is pending)
+        if (need > kMostBytes || (stream.id() != 0 && !(stream.id() & 1)) ||
+            c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+            return std::nullopt;
+        return stream.id();
+    }
+    // Whether the entry has a workspace for the pass and the library takes it.
+    bool ready(size_t need, const Tensor& on) {
+        if (kept_->state.half_bytes < need || !kept_->ws.defined()) {
+            size_t half = std::max(kLeastBytes, kept_->state.half_bytes);
+            while (half < need) half *= 2;
+            Tensor ws;
+            try {
+                ws = empty({(int64_t)(256 + 3 * half)}, at::kByte, on.device());
+            } catch (const c10::OutOfMemoryError&) {
+                return false;
             }
+            C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0xFF, 256 + 2 * half, static_cast<cudaStream_t>(stream_of(on))));
+            // (the entry changes when nothing can fail any more)
+            kept_->ws = std::move(ws);
+            kept_->state = fields_kept{half, {0, 0}, 0};
         }
-        if (list->size() == kStreams) list->pop_back();
-        auto e = std::make_shared<Entry>();
-        e->device = device;
-        e->stream = stream;
-        list->insert(list->begin(), e);
-        return e;
+        // the last step: a registration without a pass would be taken by the thread's next one
+        return api().fields_read_use_kept(&kept_->state) == FIELDS_OK;
     }
 
-    std::shared_ptr<Entry> kept_;
-    std::unique_lock<std::mutex> lock_;  // released before kept_
+    KeptWorkspaces::Hold kept_;
     Tensor own_;
     void* ptr_;
     bool done_ = false;

@@ -19,6 +19,18 @@ namespace fields_torch {
 void add_stack(PyObject* module);                                                 // torch_stack.cpp
 PyObject* py_fused_mixer(PyObject*, PyObject* const* args, Py_ssize_t n);  // torch_mixer.cpp
 
+class ReleaseKept : public c10::FreeMemoryCallback {
+  public:
+    bool Execute() override { return KeptWorkspaces::release(); }
+};
+static void register_release() {
+    auto* registry = c10::FreeCudaMemoryCallbacksRegistry();
+    if (!registry->Has("fields_kept_workspaces"))
+        registry->Register(
+            "fields_kept_workspaces", [] { return std::unique_ptr<c10::FreeMemoryCallback>(new ReleaseKept()); }, "",
+            c10::REGISTRY_DEFAULT);
+}
+
 struct Dims {
     int B, L, C;
 };
@@ -429,6 +441,7 @@ PyMODINIT_FUNC PyInit_libfields_torch(void) {
     PyObject* m = PyModule_Create(&fields_torch::g_module);
     if (!m) return nullptr;
     try {
+        fields_torch::register_release();
         fields_torch::add_stack(m);
     } catch (const std::exception& e) {
         PyErr_SetString(PyExc_ImportError, e.what());

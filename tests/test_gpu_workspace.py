@@ -128,28 +128,74 @@ def test_odd_width_on_a_workspace_of_its_own(B, L, C):
         assert rel_err(g.cpu().numpy(), np.asarray(w)) < FP32_TOL
 
 
+def _limit(room):
+    """Lets this process reserve `room` more bytes than it has."""
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / total)
+
+
+def _take_back():
+    """Leaves no workspace kept by earlier passes."""
+    torch.cuda.synchronize()
+    try:
+        _limit(0)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            torch.empty(8 << 30, dtype=torch.uint8, device="cuda")
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    torch.cuda.empty_cache()
+
+
 def test_a_failed_allocation_leaves_nothing_behind():
-    """A pass that gets no memory for its kept workspace (96 MiB here), then one on a workspace of its own (above
-    the most that is kept) and the first one again."""
+    """A pass without memory for a kept workspace (96 MiB here) but for its own (28 MB), one without memory for
+    either, then one on a workspace of its own (above the most that is kept) and the first one again."""
     few, many = _case(1, 300_000, 4, 1), _case(1, 360_000, 4, 2)
     par = [t.detach() for t in few[0][1:]]
     small, large = few[0][0].detach(), many[0][0].detach()
+    host = [p.cpu().numpy() for p in par]
+    want = {id(t): field_oracle.forward(t.cpu().numpy(), *host)[0] for t in (small, large)}
     stream = torch.cuda.Stream()
+    _take_back()
+    with torch.cuda.stream(stream):
+        try:
+            _limit(70 << 20)
+            got = [(small, fused_field_read(small, *par).cpu())]
+            torch.cuda.empty_cache()
+            _limit(30 << 20)
+            with pytest.raises(torch.cuda.OutOfMemoryError):
+                fused_field_read(small, *par)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        got += [(t, fused_field_read(t, *par).cpu()) for t in (large, small, large, small)]
+    for t, g in got:
+        assert rel_err(g.numpy(), want[id(t)]) < FP32_TOL
+
+
+def test_kept_workspaces_are_given_back():
+    """What other streams keep is there for an allocation that needs it, and the passes after it are right."""
+    leaves, grad = _case(1, 300_000, 4, 3)
+    par, raw = [t.detach() for t in leaves[1:]], leaves[0].detach()
+    want = torch.from_numpy(field_oracle.forward(raw.cpu().numpy(), *[p.cpu().numpy() for p in par])[0])
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    _take_back()
+    before = torch.cuda.memory_allocated()
+    for s in streams:
+        with torch.cuda.stream(s):
+            fused_field_read(raw, *par)
     torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated() - before
+    assert held > 300 << 20
     torch.cuda.empty_cache()
-    total = torch.cuda.get_device_properties(0).total_memory
-    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (70 << 20)) / total)
     try:
-        with torch.cuda.stream(stream), pytest.raises(torch.cuda.OutOfMemoryError):
-            fused_field_read(small, *par)
+        _limit(100 << 20)
+        big = torch.empty(held, dtype=torch.uint8, device="cuda")
+        del big
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
-    with torch.cuda.stream(stream):
-        got = [fused_field_read(t, *par) for t in (large, small, large, small)]
-    torch.cuda.synchronize()
-    host = [p.cpu().numpy() for p in par]
-    for g, t in zip(got, (large, small, large, small)):
-        assert rel_err(g.cpu().numpy(), field_oracle.forward(t.cpu().numpy(), *host)[0]) < FP32_TOL
+    assert torch.cuda.memory_allocated() < before + held // 2
+    for s in streams:
+        with torch.cuda.stream(s):
+            assert rel_err(fused_field_read(raw, *par).cpu().numpy(), want.numpy()) < FP32_TOL
 
 
 @pytest.mark.parametrize("which", range(4))
