@@ -34,18 +34,17 @@ using torch::autograd::variable_list;
 // ---------------------------------------------------------------------------------------------
 // The library's entry points, looked up in the build that bind() names.
 // ---------------------------------------------------------------------------------------------
-#define FIELDS_API(X)                                                                             \
-    X(fields_status_string) X(fields_last_cuda_error) X(fields_read_workspace_bytes)              \
-    X(fields_read_forward) X(fields_read_backward) X(fields_read_state_rows)                      \
-    X(fields_read_backward_from_states) X(fields_read_forward_bf16)                               \
-    X(fields_read_forward_bf16_stats) X(fields_read_backward_bf16)                                \
-    X(fields_read_norm_grad_combine) X(fields_read_step) X(fields_read_step_bf16)                 \
-    X(fields_scan_workspace_bytes) X(fields_scan_forward) X(fields_scan_backward)                 \
-    X(fields_stack_layout) X(fields_stack_step_norm) X(fields_stack_close_mixer)                  \
-    X(fields_stack_swiglu) X(fields_stack_close_ff) X(fields_read_forward_bf16_rows)              \
-    X(fields_read_backward_bf16_rows) X(fields_mixer_grad_rows) X(fields_mixer_grad_scratch_bytes) \
-    X(fields_mixer_open_grad) X(fields_mixer_close_grad) X(fields_step_w12_rows)                  \
-    X(fields_step_layout) X(fields_step_block) X(fields_read_use_kept) X(fields_read_forward_rows)
+#define FIELDS_API(X)                                                                               \
+    X(fields_status_string) X(fields_last_cuda_error) X(fields_read_workspace_bytes)                \
+    X(fields_read_forward) X(fields_read_backward) X(fields_read_backward_from_states)              \
+    X(fields_read_forward_bf16) X(fields_read_forward_bf16_stats) X(fields_read_backward_bf16)      \
+    X(fields_read_norm_grad_combine) X(fields_read_step) X(fields_read_step_bf16)                   \
+    X(fields_scan_forward) X(fields_scan_backward) X(fields_stack_layout)                           \
+    X(fields_stack_step_norm) X(fields_stack_close_mixer) X(fields_stack_swiglu)                    \
+    X(fields_stack_close_ff) X(fields_read_forward_bf16_rows) X(fields_read_backward_bf16_rows)     \
+    X(fields_mixer_grad_rows) X(fields_mixer_grad_scratch_bytes) X(fields_mixer_open_grad)          \
+    X(fields_mixer_close_grad) X(fields_step_w12_rows) X(fields_step_layout) X(fields_step_block)   \
+    X(fields_read_use_kept) X(fields_read_forward_rows)
 
 struct Api {
 #define X(name) decltype(&::name) name;
