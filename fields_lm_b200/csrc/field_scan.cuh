@@ -81,12 +81,13 @@ struct ScanWalk {
         at.chan_ok = at.c < s.C;
         const int pos = k * s.Q + rank;  // in walking order; tiles past the end have no steps
         at.tile = BWD ? s.NT - 1 - pos : pos;
-        at.t0 = at.tile * kScanTile + (thread >> 5) * kScanSteps;
+        at.t0 = (int)((unsigned)at.tile * kScanTile + (unsigned)(thread >> 5) * kScanSteps);
         return at;
     }
-    // (a step outside the sequence is the identity in either direction)
+    // (a step outside the sequence is the identity in either direction; unsigned, because the tiles that fill the
+    // last super-tile may lie beyond 2^31 steps)
     FL_HD static bool inside(const ScanShape& s, const At& at, int j) {
-        return at.chan_ok && at.tile >= 0 && at.t0 + j < s.L;
+        return at.chan_ok && (unsigned)at.t0 + (unsigned)j < (unsigned)s.L;
     }
     FL_HD static int warp_at(int pos) { return BWD ? kScanWarps - 1 - pos : pos; }
 
@@ -100,7 +101,7 @@ struct ScanWalk {
             st.a[j] = in ? ap[j * s.a_step] : 1.0f;
             st.x[j] = in ? p.x[row + (size_t)j * s.C] : 0.0f;
             if constexpr (BWD) {
-                if (at.t0 + j > 0) st.prev[j] = in ? p.states[row + (size_t)j * s.C - s.C] : 0.0f;
+                if ((unsigned)at.t0 + (unsigned)j > 0) st.prev[j] = in ? p.states[row + (size_t)j * s.C - s.C] : 0.0f;
                 else st.prev[j] = in && p.first ? p.first[(size_t)at.b * s.C + at.c] : 0.0f;
             }
         }

@@ -1342,7 +1342,7 @@ static ScanShape make_scan_shape(int B, int L, int C, long long a_batch, long lo
                                  int a_chan) {
     ScanShape s{};
     s.B = B; s.L = L; s.C = C;
-    s.NT = (L + kScanTile - 1) / kScanTile;
+    s.NT = (int)(((long long)L + kScanTile - 1) / kScanTile);
     s.CG = (C + 31) / 32;
     s.a_batch = a_batch; s.a_step = a_step; s.a_chan = a_chan;
 #ifdef FIELDS_HOST_EMU

@@ -104,3 +104,52 @@ def test_empty_and_argument_errors():
                                  1, 0, 4, None)
     assert rc == 0
     np.testing.assert_array_equal(sout, sin)
+
+
+def test_scan_tiles_of_the_longest_sequences(tmp_path):
+    """Steps of the tiles around the end of a sequence of almost 2^31 steps: those of the sequence, once, in both
+    directions (the index arithmetic of the kernels, compiled for the host)."""
+    import subprocess
+    from pathlib import Path
+    root = Path(__file__).resolve().parent.parent
+    program = r"""
+#include "field_scan.cuh"
+#include <cstdio>
+using namespace fields;
+template <bool BWD> static int check(int L) {
+    using W = ScanWalk<BWD>;
+    ScanShape s{};
+    s.B = 1; s.L = L; s.C = 1; s.CG = 1; s.Q = 16;
+    s.NT = (int)(((long long)L + kScanTile - 1) / kScanTile);
+    s.K = (s.NT + s.Q - 1) / s.Q;
+    long long first = 0, seen = 0;
+    const int from = s.K - 2;  // the last two super-tiles in walking order, and one that does not exist
+    for (int k = from; k <= s.K; ++k)
+        for (int rank = 0; rank < s.Q; ++rank)
+            for (int warp = 0; warp < kScanWarps; ++warp) {
+                const typename W::At at = W::where(s, 0, rank, k, warp * 32);
+                for (int j = 0; j < kScanSteps; ++j) {
+                    if (!W::inside(s, at, j)) continue;
+                    const long long t = (long long)at.t0 + j;
+                    if (t < 0 || t >= L) return 1;
+                    first += t;
+                    ++seen;
+                }
+            }
+    const long long lo = BWD ? 0 : (long long)from * s.Q * kScanTile;
+    const long long hi = BWD ? (long long)(s.NT - (long long)from * s.Q) * kScanTile : L;  // [lo, hi)
+    return !(seen == hi - lo && first == (lo + hi - 1) * (hi - lo) / 2);
+}
+int main() {
+    const int lengths[] = {2147483647, 2147483647 - 63, 2147483647 - 127, 2147483647 - 2048, 2147483647 - 5000, 100000};
+    for (int L : lengths)
+        if (check<false>(L) || check<true>(L)) { std::printf("%d\n", L); return 1; }
+    return 0;
+}
+"""
+    source, exe = tmp_path / "tiles.cpp", tmp_path / "tiles"
+    source.write_text(program)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-ftrapv", "-DFIELDS_HOST_EMU", "-Wno-unknown-pragmas",
+                    f"-I{root / 'fields_lm_b200' / 'csrc'}", "-o", str(exe), str(source)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, (out.returncode, out.stdout)
