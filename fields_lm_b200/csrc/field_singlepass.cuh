@@ -114,9 +114,9 @@ FL_HD SpTile sp_decode(const SpShape& s, unsigned ticket) {
 // the raw bits, half as much, and evaluates the gates a second time. (One reciprocal for the three gates,
 // four special-function operations per channel instead of six, gained 4 % at 1 x 65,536 x 512 and nothing at
 // 8 x 2,048; its state was 1.9e-7 from 64-bit arithmetic instead of 1.3e-7, and a gate that is masked with -inf did
-// not close.) Forward, workspace fill included: 48.1 -> 44.1 us at 8 x 2,048 x 512 against the staged form
-// below, 185 -> 157 us at 1 x 65,536. Blocks of four warps overlap their phases better than blocks of eight; holding
-// tickets and staging the next tile in shared memory (an earlier form) came to 43.0 us.
+// not close.) With the workspace fill, launched alone on a cold L2: 48.1 -> 44.1 us at 8 x 2,048 x 512 and 185 -> 157
+// at 1 x 65,536 against an earlier form that held tickets and staged the next tile in shared memory. Blocks of
+// four warps overlap their phases better than blocks of eight.
 // ROWS: also writes the state after every kStateRowEvery-th step, what a backward pass from state rows keeps.
 template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false, bool ROWS = false>
 struct FwdSinglePass {

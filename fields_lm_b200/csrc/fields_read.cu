@@ -643,13 +643,15 @@ static Algo algo_from_env() { return kAlgoAuto; }
 // registers with 24-step tiles: 96). At 1 x 65,536 x 512 189 -> 183 us against the earlier two blocks of
 // eight warps and 48-step tiles, at 1 x 16,384 54.2 -> 51.8, at 2 x 3,001 x 384 20.6 -> 19.5, equal at
 // 8 x 2,048. From eight rounds of blocks on, where the last one weighs little, 40-step tiles are a little
-// faster in spite of a few spilled registers: 183 -> 179 us at 1 x 65,536, 175 -> 171 at 4 x 16,384.
+// faster in spite of a few spilled registers: 184 -> 179 us at 1 x 65,536, 173 -> 169 at 4 x 16,384.
 using FwdSp0 = FwdSinglePass<9, 4, 3>;
 using FwdSpDeep = FwdSinglePass<10, 4, 3>;
 static long long tiles_of(int B, int L, int C, int steps) {
     return (long long)B * ((C + kGroup - 1) / kGroup) * ((L + steps - 1) / steps);
 }
-// Tensors without 128-bit access (F32Any), forward and backward: the same kernels with four 32-bit accesses.
+// Tensors without 128-bit access (F32Any), forward and backward: the same kernels with four 32-bit accesses. Eight steps
+// per warp against six (a tile below what the workspace is counted for): 127 / 143 us at 1 x 30,000 x 513, 44.9 / 47.0
+// at 8 x 2,048 x 333, 12.5 / 12.0 at 3 x 777 x 333; blocks of six and eight warps 13.2 to 15.7 at the last.
 using FwdSpAny = FwdSinglePass<8, 4, 3, F32Any>;
 using FwdSpRows = FwdSinglePass<9, 4, 3, float, false, true>;  // also writes state rows
 #ifdef FIELDS_ALL_VARIANTS
@@ -670,15 +672,9 @@ using BwdSp2 = BwdRecompute<8, 4, 1, 3, 2>;   // 73 KB per block, 12 warps per S
 using BwdSp3 = BwdTileResident<4, 4, 3>;      // tile 16, 68 KB per block, 12 warps per SM
 #endif
 //   bfloat16 raw / read / grad_read / grad_raw (bits as uint16_t); state and arithmetic stay fp32
-// The forward in two tile shapes: blocks of four warps (tile 40) overlap their phases better, blocks of
-// eight (tile 80) look back over half as many tiles. 36.2 / 37.6 us at 8 x 2,048 x 512 (1,640 small
-// tiles), 43.2 / 41.4 at 1 x 16,384, 150 / 142 at 1 x 65,536, 129 / 128 at 8 x 8,192. The second
-// needs tiles enough that a part-filled last round costs little: the line is at 3,500 small tiles.
-static bool deep_tiles(int B, int L, int C) {
-    return tiles_of(B, L, C, 40) >= 3500;
-}
-template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;
-template <bool STATS> using FwdSpBf16Deep = FwdSinglePass<10, 8, 2, uint16_t, STATS>;  // STATS: per-token sums of squares too
+// The forward: blocks of four warps. (Blocks of eight, 80 steps, look back over half as many tiles, but at 8 x 2,048 x 512
+// they take 38.9 us against 37.7, at 8 x 8,192 140 against 135, at 4 x 16,384 142 against 138, and as long at 1 x 65,536.)
+template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;  // STATS: per-token sums of squares too
 // bfloat16 ring cells are half the size, so a 64-step tile (4 warps x 16 steps) still leaves room for
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
 // 16-byte cells) on 8 x 2,048 tokens.
@@ -1533,14 +1529,9 @@ template <bool STATS>
 static int run_forward_bf16(const void* raw, long long pitch, const float* tr, const float* ti, const float* gamma,
                             const float* state_in, void* read, float* sumsq, float* state_out, void* workspace,
                             int B, int L, int C, void* stream) {
-    const auto* z = static_cast<const uint16_t*>(raw);
-    auto* out = static_cast<uint16_t*>(read);
-    Stream st = reinterpret_cast<Stream>(stream);
-    if (deep_tiles(B, L, C))
-        return run_forward_single_pass<FwdSpBf16Deep<STATS>, uint16_t>(z, tr, ti, gamma, state_in, out, state_out,
-                                                                       workspace, B, L, C, st, sumsq, pitch);
-    return run_forward_single_pass<FwdSpBf16<STATS>, uint16_t>(z, tr, ti, gamma, state_in, out, state_out,
-                                                               workspace, B, L, C, st, sumsq, pitch);
+    return run_forward_single_pass<FwdSpBf16<STATS>, uint16_t>(static_cast<const uint16_t*>(raw), tr, ti, gamma, state_in,
+                                                               static_cast<uint16_t*>(read), state_out, workspace, B, L, C,
+                                                               reinterpret_cast<Stream>(stream), sumsq, pitch);
 }
 
 extern "C" {
