@@ -43,7 +43,7 @@ FP32_TOL, BF16_TOL = 1e-5, 2e-2
 KERNEL_LAUNCHES_PER_STEP = 5   # forward: fill + kernel; backward: fill + kernel + parameter-gradient reduce
 FALLBACK_HBM_GBS = 6650.0
 # dram__bytes_read.sum + dram__bytes_write.sum per step from the ncu capture of this workload
-# (forward 102.2 + 134.2 MB, backward 323.3 + 100.7 MB; writes still in L2 at kernel end counted in full)
+# (forward 103.1 + 134.2 MB, backward 322.4 + 100.7 MB; writes still in L2 at kernel end counted in full)
 NCU_DRAM_BYTES_PER_STEP = 660.4e6
 LONG_L = 65536
 

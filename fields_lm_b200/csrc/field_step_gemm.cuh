@@ -9,10 +9,8 @@
 //
 // A step of a few hundred rows is bound by the 25 MB of weights per block of d_model 1,024 (3.9 us at the
 // copy bandwidth) and, far above that, by latency: as library products with elementwise kernels between
-// them a block took nine launches and 35 us of kernels. Here it is four of about 8.7 us each: 256 rows
-// through 18 blocks 768 -> 675 us, eight blocks of d_model 256 372 -> 230 us. What a kernel's time is made of
-// (us, 256 rows): set-up 1.4, operands and product 2 to 4, exchange 1.2 to 2.5, epilogue 0.7 to 1.6. What is
-// done about it:
+// them a block took nine launches. Here it is four, of about 9.4 us each in a row of them (10.8 to 12.3 alone
+// and on a cold cache): 256 rows through 18 blocks 763 -> 680 us, 16 rows 745 -> 620. What is done about it:
 //   - the RMS norms become a per-row scale of the product that follows (their weights are folded into the
 //     bfloat16 copies), so a norm needs only partial sums of squares per row, which the
 //     producing epilogue leaves in a small table;
@@ -209,7 +207,7 @@ struct EpiIn {  // slice: eight channels' z_r | z_i | z_v, then sixteen gate fea
 // EpiOut and EpiFf come with tiles of 64 and of 32 features (and EpiUv with two of its slices for the same row
 // counts). Where 64 leave so few tiles that K would be split
 // over clusters of eight (up to 128 rows at d_model 1,024), 32 with clusters of four are faster: a kernel's
-// clusters of eight took up to 14 us to get started (18 blocks, 16 rows: 661 -> 571 us; 128 rows: 681 -> 548).
+// clusters of eight took up to 14 us to get started (18 blocks, 16 rows: 736 -> 620 us; 128 rows: 730 -> 589).
 template <int SLICES>
 struct EpiOut {  // slice: eight features
     static constexpr int kSlice = 8, kSlices = SLICES, kStages = 7, kConst = 8;

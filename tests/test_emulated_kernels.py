@@ -72,7 +72,7 @@ def test_scalar_path_equals_vector_path():
     raw = rng.standard_normal((B, L, 3 * C)).astype(np.float32)
     a, sa = emu.forward(raw, tr, ti, gm)
     b, sb = emu.forward(raw, tr, ti, gm, misalign=True)
-    # the scalar path is the three-phase kernels: same arithmetic, different association
+    # the same kernels with 32-bit accesses and another tile: same arithmetic, different association
     assert rel_err(a, b) < 1e-6
     assert rel_err(sa, sb) < 1e-6
 

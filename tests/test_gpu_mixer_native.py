@@ -64,7 +64,7 @@ def test_forward_at_the_edges_of_the_tiles(L):
 
 
 def test_bf16_forward_with_long_tiles():
-    """3,500 tiles of 40 steps and more: blocks of eight warps."""
+    """Some thousand tiles of 40 steps in three channel groups."""
     B, L, C = 2, 35_003, 260
     torch.manual_seed(0)
     raw = (0.577 * torch.randn(B, L, 3 * C, device="cuda")).bfloat16()

@@ -75,7 +75,7 @@ def test_noalloc_forward_allocates_nothing_and_covers_the_scalar_kernels():
     """The property the entry point exists for: after the first call on a device (which asks
     for the address of the built-in buffer), a call changes neither the driver's free memory
     nor the caching allocator's books. Also a channel count that is not a multiple of four
-    (the three-phase scalar kernels on the shared buffer), and the per-device address on a
+    (the kernels with 32-bit accesses on the shared buffer), and the per-device address on a
     second GPU where the box has one."""
     from fields_lm_b200 import _lib
     lib = _lib.load()
