@@ -59,6 +59,7 @@ SYMBOLS = {
     "fields_mixer_epilogue_backward": (_I, [_P] * 11 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
     "fields_step_w12_rows": (_I, [_I]),
     "fields_step_layout": (_I, [_P, _P]),
+    "fields_step_stack": (_I, [_P, _I, _P, _P]),
     "fields_step_block": (_I, [_P, _P]),
     "fields_read_forward_bf16_rows": (_I, [_P, _LL] + [_P] * 8 + [_SZ, _I, _I, _I, _P]),
     "fields_read_backward_bf16_rows": (_I, [_P, _LL] + [_P] * 6 + [_LL] + [_P] * 4 + [_SZ, _I, _I, _I, _P]),

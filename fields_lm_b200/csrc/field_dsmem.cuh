@@ -24,28 +24,44 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+template <bool PEERS>
 __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
     unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if constexpr (PEERS)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return done != 0;
 }
 // Waits for a phase, with a bound (a try suspends for a while by itself, so 2^20 of them are a second
 // or more). `dead` is the thread's record that a wait has run out: it is set then, and later waits
-// give up at once, so a kernel always terminates.
-__device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool& dead) {
+// give up at once, so a kernel always terminates. Acquires at cluster scope; mbar_wait_local, for barriers
+// that only this block and its own copies arrive on, at block scope.
+template <bool PEERS>
+__device__ __forceinline__ void mbar_wait_scope(unsigned bar, unsigned parity, bool& dead) {
     unsigned tries = 0;
-    while (!mbar_try(bar, parity)) {
+    while (!mbar_try<PEERS>(bar, parity)) {
         if (dead || ++tries >= (1u << 20)) {
             dead = true;
             return;
         }
     }
+}
+__device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool& dead) { mbar_wait_scope<true>(bar, parity, dead); }
+__device__ __forceinline__ void mbar_wait_local(unsigned bar, unsigned parity, bool& dead) {
+    mbar_wait_scope<false>(bar, parity, dead);
 }
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;

@@ -24,6 +24,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -2193,84 +2194,176 @@ static bool operand_map(CUtensorMap* map, const void* base, long long rows, int 
     if (!encode) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    const cuuint32_t box[2] = {kStepKBlock, (cuuint32_t)box_rows}, ones[2] = {1, 1};
+    const cuuint32_t box[2] = {kStepKBox, (cuuint32_t)box_rows}, ones[2] = {1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, ones,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// One product of the step: A [M, K] activations, B [n_rows, K] weights, `slices` column slices.
-template <class Epi>
-static int launch_step(const void* a, const void* b, int n_rows, int K, int slices, StepBlockParams p, Stream st) {
-    using T = StepTile<Epi>;
-    p.k_blocks = (K + kStepKBlock - 1) / kStepKBlock;
-    p.tiles_n = (slices + Epi::kSlices - 1) / Epi::kSlices;
-    const int tiles = p.tiles_n * ((p.M + kStepRows - 1) / kStepRows);
-    // K over as many blocks as share the GPU in one round, every one of them with a part of K
-    p.S = 1;
-    for (int S = 2; S <= Epi::kSlices && tiles * S <= 148; S *= 2)
-        if ((S - 1) * ((p.k_blocks + S - 1) / S) < p.k_blocks) p.S = S;
-    CUtensorMap a_map, b_map;
-    if (!operand_map(&a_map, a, p.M, K, kStepRows) || !operand_map(&b_map, b, n_rows, K, T::kNT))
-        return FIELDS_ERR_UNSUPPORTED;
+// How a launch of step_stack covers the GPU: `clusters` are resident at once.
+template <bool NARROW>
+static int step_phases(StepStackParams& p, int clusters) {
+    using T = StepShape<NARROW>;
+    p.groups = p.row_tiles < clusters ? p.row_tiles : clusters;
+    const int most = clusters / p.groups, blocks = most * kStepCluster;
+    const int K[kStepPhases] = {p.D, 4 * p.C, p.D, p.H};
+    const int cols[kStepPhases] = {5 * p.C, p.D, fields_step_w12_rows(p.H), p.D};
+    const int split[kStepPhases] = {T::In::kMaxSplit, T::Out::kMaxSplit, T::Uv::kMaxSplit, T::Ff::kMaxSplit};
+    p.group_clusters = 1;
+    for (int i = 0; i < kStepPhases; ++i) {
+        StepPhase& h = p.phase[i];
+        h.tiles_n = (cols[i] + T::nt(i) - 1) / T::nt(i);
+        h.k_blocks = (K[i] + kStepKBlock - 1) / kStepKBlock;
+        h.S = 1;  // K over as many blocks as there are, every one of them with a part of K
+        for (int S = 2; S <= split[i] && h.tiles_n * S <= blocks; S *= 2)
+            if ((S - 1) * ((h.k_blocks + S - 1) / S) < h.k_blocks) h.S = S;
+        h.per = (h.k_blocks + h.S - 1) / h.S;
+        const int subs = kStepCluster / h.S, want = (h.tiles_n + subs - 1) / subs;
+        h.iters = (want + most - 1) / most;
+        if (p.group_clusters < (want < most ? want : most)) p.group_clusters = want < most ? want : most;
+    }
+    for (StepPhase& h : p.phase) {
+        const int per = p.group_clusters * (kStepCluster / h.S);
+        h.iters = (h.tiles_n + per - 1) / per;
+    }
+    return FIELDS_OK;
+}
+
+// Clusters of step_stack that the device holds at once.
+template <bool NARROW>
+static int step_clusters(cudaLaunchConfig_t cfg, int* clusters) {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    const int rc = check_cuda(cudaGetDevice(&dev));
+    if (rc) return rc;
+    if (dev < 0 || dev >= 64) return FIELDS_ERR_UNSUPPORTED;
+    *clusters = known[dev].load();
+    if (*clusters > 0) return FIELDS_OK;
+    cfg.gridDim = dim3(kStepCluster);
+    const int rc2 = check_cuda(cudaOccupancyMaxActiveClusters(clusters, step_stack<NARROW>, &cfg));
+    if (rc2) return rc2;
+    if (*clusters < 1) return FIELDS_ERR_UNSUPPORTED;
+    known[dev].store(*clusters);
+    return FIELDS_OK;
+}
+
+// Phases [first, last) of the blocks in p: as one cooperative launch (p.sync), or one phase by itself.
+template <bool NARROW>
+static int launch_step(StepStackParams& p, bool cooperative, Stream st) {
+    using T = StepShape<NARROW>;
     static bool ready[64] = {};
-    const int rc = allow_shared_memory(step_gemm<Epi>, T::kSmemBytes, ready);
+    int rc = allow_shared_memory(step_stack<NARROW>, T::kSmemBytes, ready);
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * p.S));
     cfg.blockDim = dim3(kStepThreads);
     cfg.dynamicSmemBytes = T::kSmemBytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (dependent_launch_enabled()) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (p.S > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = (unsigned)p.S;
-        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
-        ++n;
-    }
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kStepCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = n;
-    return check_cuda(cudaLaunchKernelEx(&cfg, step_gemm<Epi>, a_map, b_map, p));
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    rc = step_clusters<NARROW>(cfg, &clusters);
+    if (!rc) rc = step_phases<NARROW>(p, clusters);
+    if (rc) return rc;
+    if (cooperative) {
+        attr[1].id = cudaLaunchAttributeCooperative;
+        attr[1].val.cooperative = 1;
+        cfg.numAttrs = 2;
+    } else if (dependent_launch_enabled()) {
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    }
+    cfg.gridDim = dim3((unsigned)(p.groups * p.group_clusters * kStepCluster));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, step_stack<NARROW>, p);
+    if (cooperative && e == cudaErrorCooperativeLaunchTooLarge) {
+        (void)cudaGetLastError();
+        return FIELDS_ERR_UNSUPPORTED;
+    }
+    return check_cuda(e);
+}
+
+template <bool NARROW>
+static int run_step(const struct fields_step_args* g, int count, unsigned* sync, Stream st) {
+    using T = StepShape<NARROW>;
+    auto h = [](void* q) { return static_cast<uint16_t*>(q); };
+    StepStackParams p;
+    std::memset(&p, 0, sizeof(p));
+    const int M = g->rows, D = g->dim, C = D / 2, H = g->hidden;
+    p.gate = h(g->gate); p.read = h(g->read); p.yb = h(g->yb); p.act = h(g->act); p.xb = h(g->xb);
+    p.y = g->y; p.read_sq = g->read_sq; p.y_sq = g->y_sq;
+    p.M = M; p.D = D; p.C = C; p.H = H;
+    p.row_tiles = (M + kStepRows - 1) / kStepRows;
+    p.a_rows = M < kStepRows ? (M + 7) / 8 * 8 : kStepRows;
+    const void* a[kStepPhases] = {g->xb, g->read, g->yb, g->act};
+    const int K[kStepPhases] = {D, 4 * C, D, H};
+    const int rows[kStepPhases] = {5 * C, D, fields_step_w12_rows(H), D};
+    for (int i = 0; i < kStepPhases; ++i)
+        if (!operand_map(&p.a[i], a[i], M, K[i], p.a_rows)) return FIELDS_ERR_UNSUPPORTED;
+    for (int at = 0; at < count; at += kStepMaxBlocks) {
+        const int n = count - at < kStepMaxBlocks ? count - at : kStepMaxBlocks;
+        for (int j = 0; j < n; ++j) {
+            const struct fields_step_args& q = g[at + j];
+            StepWeights& w = p.block[j];
+            w.x = q.x; w.in_b = q.in_b; w.par = q.par; w.out_b = q.out_b; w.state = q.state;
+            w.read_eps = q.read_eps; w.ff_eps = q.ff_eps;
+            const void* b[kStepPhases] = {q.in_w, q.out_w16, q.w12_w, q.w3_16};
+            for (int i = 0; i < kStepPhases; ++i)
+                if (!operand_map(&w.b[i], b[i], rows[i], K[i], T::box(i))) return FIELDS_ERR_UNSUPPORTED;
+        }
+        int rc = FIELDS_ERR_UNSUPPORTED;
+        if (sync) {
+            p.sync = sync;
+            p.first = 0;
+            p.last = n * kStepPhases;
+            rc = check_cuda(cudaMemsetAsync(sync, 0, kStepSyncBytes, st));
+            if (!rc) rc = launch_step<NARROW>(p, true, st);
+        }
+        if (rc == FIELDS_ERR_UNSUPPORTED) {  // one launch per phase: none of them waits for another
+            p.sync = nullptr;
+            rc = FIELDS_OK;
+            for (int i = 0; i < n * kStepPhases && !rc; ++i) {
+                p.first = i;
+                p.last = i + 1;
+                rc = launch_step<NARROW>(p, false, st);
+            }
+        }
+        if (rc) return rc;
+    }
+    return FIELDS_OK;
 }
 
 extern "C" {
 
-int fields_step_block(const struct fields_step_args* g, void* stream) {
-    if (!g || g->rows < 0) return FIELDS_ERR_ARGUMENT;
-    if (g->rows == 0) return FIELDS_OK;
-    const void* all[] = {g->x, g->state, g->y, g->xb, g->yb, g->read, g->gate, g->act, g->read_sq, g->y_sq, g->in_w,
-                         g->out_w16, g->w12_w, g->w3_16, g->in_b, g->par, g->out_b};
-    for (const void* q : all)
-        if (!q) return FIELDS_ERR_ARGUMENT;
-    if (!step_sizes(g->dim, g->hidden) || g->rows > 512) return FIELDS_ERR_UNSUPPORTED;
-    for (const void* q : all)
-        if (!aligned16(q)) return FIELDS_ERR_UNSUPPORTED;
-    const int D = g->dim, C = D / 2, H = g->hidden;
-    auto h = [](void* q) { return static_cast<uint16_t*>(q); };
-    StepBlockParams p{};
-    p.x = g->x; p.gate = h(g->gate); p.read = h(g->read); p.state = g->state; p.y = g->y; p.yb = h(g->yb);
-    p.act = h(g->act); p.out = g->y; p.xb = h(g->xb); p.read_sq = g->read_sq; p.y_sq = g->y_sq;
-    p.in_b = g->in_b; p.par = g->par; p.out_b = g->out_b;
-    p.read_eps = g->read_eps; p.ff_eps = g->ff_eps; p.M = g->rows; p.D = D; p.C = C; p.H = H;
-    Stream st = reinterpret_cast<Stream>(stream);
-    // the first product waits where a parameter may still be on its way; it lets the second in afterwards
-    p.wait_first = !g->settled;
-    int rc = launch_step<EpiIn>(g->xb, g->in_w, 5 * C, D, C / 8, p, st);
-    p.wait_first = 0;
-    const bool narrow = (g->rows + kStepRows - 1) / kStepRows * ((D + 63) / 64) * 8 <= 148;
-    if (!rc) rc = narrow ? launch_step<EpiOut<4>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st)
-                         : launch_step<EpiOut<8>>(g->read, g->out_w16, D, 2 * D, D / 8, p, st);
-    if (!rc) rc = narrow ? launch_step<EpiUv<2>>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st)
-                         : launch_step<EpiUv<4>>(g->yb, g->w12_w, fields_step_w12_rows(H), D, (H + 19) / 20, p, st);
-    if (!rc) rc = narrow ? launch_step<EpiFf<4>>(g->act, g->w3_16, D, H, D / 8, p, st)
-                         : launch_step<EpiFf<8>>(g->act, g->w3_16, D, H, D / 8, p, st);
-    return rc;
+int fields_step_stack(const struct fields_step_args* g, int count, void* sync, void* stream) {
+    if (!g || count < 0 || g->rows < 0) return FIELDS_ERR_ARGUMENT;
+    if (g->rows == 0 || count == 0) return FIELDS_OK;
+    for (int i = 0; i < count; ++i) {
+        const struct fields_step_args& q = g[i];
+        const void* all[] = {q.x, q.state, q.y, q.xb, q.yb, q.read, q.gate, q.act, q.read_sq, q.y_sq, q.in_w,
+                             q.out_w16, q.w12_w, q.w3_16, q.in_b, q.par, q.out_b};
+        for (const void* v : all)
+            if (!v) return FIELDS_ERR_ARGUMENT;
+        if (!step_sizes(q.dim, q.hidden) || q.rows > 512) return FIELDS_ERR_UNSUPPORTED;
+        for (const void* v : all)
+            if (!aligned16(v)) return FIELDS_ERR_UNSUPPORTED;
+        // one block goes on from the other
+        if (q.y != g->y || q.xb != g->xb || q.yb != g->yb || q.read != g->read || q.gate != g->gate || q.act != g->act ||
+            q.read_sq != g->read_sq || q.y_sq != g->y_sq || q.rows != g->rows || q.dim != g->dim ||
+            q.hidden != g->hidden || (i > 0 && q.x != g->y))
+            return FIELDS_ERR_ARGUMENT;
+    }
+    if (sync && !aligned16(sync)) return FIELDS_ERR_UNSUPPORTED;
+    const bool narrow = (g->rows + kStepRows - 1) / kStepRows * ((g->dim + 63) / 64) * 8 <= 148;
+    return narrow ? run_step<true>(g, count, static_cast<unsigned*>(sync), reinterpret_cast<Stream>(stream))
+                  : run_step<false>(g, count, static_cast<unsigned*>(sync), reinterpret_cast<Stream>(stream));
 }
+
+int fields_step_block(const struct fields_step_args* g, void* stream) { return fields_step_stack(g, 1, nullptr, stream); }
+
 #endif  // FIELDS_HOST_EMU
 
 }  // extern "C"

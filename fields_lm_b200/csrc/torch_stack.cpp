@@ -288,9 +288,9 @@ class FieldStack {
         CopyUses::Call call(*uses_, x.device(), false);
         if (!aligned)
             for (Tensor& s : own) s = s.clone();
-        // Four launches per block while its products have tiles (128 rows x 64 features) few enough that K
-        // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 620 us at 16 rows and 680 at 256
-        // against 745 and 763 with library products, but 1,002 against 776 at 384.
+        // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
+        // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
+        // against 745 and 763 with library products, but 815 against 776 at 384.
         const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
         if (fused && !step_laid_out_) {
             step_layout(stream_of(x));
@@ -354,7 +354,7 @@ class FieldStack {
         step_laid_out_ = true;
     }
 
-    // The blocks of a step, each a chain of four products with fused epilogues (field_step_gemm.cuh).
+    // The blocks of a step in one launch, each a chain of four products with fused epilogues (field_step_gemm.cuh).
     void step_fused(const Tensor& x, const std::vector<Tensor>& states, const Tensor& xb, const Tensor& y) {
         const Api& f = api();
         const int64_t N = x.size(0), D = D_, C = D / 2, H = H_;
@@ -362,21 +362,23 @@ class FieldStack {
         void* st = stream_of(x);
         const Tensor yb = empty({N, D}, at::kBFloat16, dev), read = empty({N, 4 * C}, at::kBFloat16, dev),
                      gate = empty({N, D}, at::kBFloat16, dev), act = empty({N, H}, at::kBFloat16, dev),
-                     read_sq = empty({C / 8, N}, at::kFloat, dev), y_sq = empty({D / 8, N}, at::kFloat, dev);
+                     read_sq = empty({C / 8, N}, at::kFloat, dev), y_sq = empty({D / 8, N}, at::kFloat, dev),
+                     sync = empty({512}, at::kByte, dev);
+        std::vector<fields_step_args> all;
         fields_step_args g{};
         g.x = fp(x); g.y = fp(y); g.xb = vp(xb); g.yb = vp(yb); g.read = vp(read); g.gate = vp(gate); g.act = vp(act);
         g.read_sq = fp(read_sq); g.y_sq = fp(y_sq);
         g.rows = (int)N; g.dim = D_; g.hidden = H_;
-        g.settled = 1;  // step()'s copy of x stands between a layout and the first block, and waits for it
         for (size_t i = 0; i < blocks_.size(); ++i) {
             const Block& b = blocks_[i];
             g.state = fp(states[i]);
             g.in_w = vp(b.step_in); g.out_w16 = vp(b.out_t); g.w12_w = vp(b.step_w12); g.w3_16 = vp(b.w3_t);
             g.in_b = fp(b.step_b); g.par = fp(b.par); g.out_b = b.f(Block::kOutB);
             g.read_eps = (float)b.read_eps; g.ff_eps = (float)b.ff_eps;
-            check(f.fields_step_block(&g, st), "fields_step_block");
+            all.push_back(g);
             g.x = g.y;
         }
+        check(f.fields_step_stack(all.data(), (int)all.size(), vp(sync), st), "fields_step_stack");
     }
 
     // The same with library products, for what the fused step does not take.

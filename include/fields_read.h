@@ -516,18 +516,21 @@ int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, fl
                           float norm_eps, long long N, int D, void *stream);
 
 /*
- * The single-token step of a block as four launches, each a tensor-core product whose epilogue goes on to
- * the operand of the next (D = dim, C = D / 2, H = hidden; D % 16 == 0, D <= 4096, H % 8 == 0, up to
+ * The single-token step of a stack of blocks: per block four tensor-core products, each of whose epilogues goes on
+ * to the operand of the next (D = dim, C = D / 2, H = hidden; D % 16 == 0, D <= 4096, H % 8 == 0, up to
  * 512 rows; tensors dense and 16-byte aligned; FIELDS_ERR_UNSUPPORTED otherwise).
  *
  * fields_step_layout: the rows of [write | gate] and of w12 diag(ff_norm) in the column order of the
  *   products: in_w [5C, D] and w12_w [fields_step_w12_rows(H), D] bfloat16, in_b [5C].
- * fields_step_block: x [M, D] in (the block's input; xb its bfloat16 copy), y [M, D] out (may be x) and
- *   xb its copy; state [M, 2C] advances in place. out_w16, w3_16 and par as fields_stack_layout leaves
- *   them. Scratch: yb [M, D], read [M, 4C], gate [M, D], act [M, H] bfloat16, read_sq [C / 8, M],
- *   y_sq [D / 8, M]. The products load their weights, in_b, par and out_b ahead of the kernel before them on the
- *   stream if settled is non-zero: these were then complete, in stream order, before the kernel (or copy) that
- *   this call follows. 0: nothing is read ahead of what the call follows (a layout, say).
+ * fields_step_stack: `count` blocks, each going on from the one before (x of a block is y of the one before it;
+ *   everything but x, state, the weights and the epsilons is the same for all). x [M, D] in (the block's input;
+ *   xb its bfloat16 copy), y [M, D] out (may be x) and xb its copy; state [M, 2C] advances in place. out_w16, w3_16
+ *   and par as fields_stack_layout leaves them. Scratch: yb [M, D], read [M, 4C], gate [M, D], act [M, H] bfloat16,
+ *   read_sq [C / 8, M], y_sq [D / 8, M], sync 512 bytes. One cooperative launch per 24 blocks, whose waits for
+ *   one another are bounded (NaN results if one runs out); with sync NULL, or where the device holds no such launch, one
+ *   launch per product.
+ * fields_step_block: one block, one launch per product.
+ * `settled` is not used any more: nothing is read ahead of what a call follows.
  */
 struct fields_step_weights {
     const float *write_w, *write_b, *gate_w, *gate_b, *w12, *ff_norm_w;
@@ -547,6 +550,7 @@ struct fields_step_args {
 };
 int fields_step_w12_rows(int hidden);
 int fields_step_layout(const struct fields_step_weights *weights, void *stream);
+int fields_step_stack(const struct fields_step_args *blocks, int count, void *sync, void *stream);
 int fields_step_block(const struct fields_step_args *args, void *stream);
 
 /*

@@ -1,4 +1,4 @@
-"""fields_step_block through the C ABI, directly behind the layouts that it needs (GPU)."""
+"""fields_step_block and fields_step_stack through the C ABI (GPU)."""
 import ctypes
 
 import pytest
@@ -63,3 +63,39 @@ def test_step_block_waits_for_the_layout_it_follows(M, D, H):
         got, want = block(False), block(True)
         assert all(torch.equal(g, w) for g, w in zip(got, want))
         assert not bool(got[0].isnan().any())
+
+
+# rows at the edges of a row tile and of the share of a row tile that a block of a cluster finishes, up to four row
+# tiles; widths with few and many column tiles; more blocks than one launch takes
+@pytest.mark.parametrize("M,D,H,blocks", [(1, 64, 8, 26), (3, 272, 360, 2), (127, 16, 24, 3), (129, 1024, 2528, 2),
+                                          (200, 512, 1344, 3), (257, 256, 704, 2), (512, 1024, 704, 2), (5, 2048, 96, 2)])
+def test_step_stack_is_its_phases_one_by_one(M, D, H, blocks):
+    """One launch whose blocks wait for one another computes bit for bit what a launch per product does."""
+    lib, C = _lib.load(), D // 2
+    torch.manual_seed(M + D)
+
+    def bf16(*shape):
+        return (torch.randn(shape, device="cuda") / shape[-1] ** 0.5).bfloat16()
+
+    weights = [dict(in_w=bf16(5 * C, D), out_w16=bf16(D, 2 * D), w12_w=bf16(lib.fields_step_w12_rows(H), D), w3_16=bf16(D, H),
+                    in_b=torch.randn(5 * C, device="cuda"), par=torch.rand(3, C, device="cuda"),
+                    out_b=torch.randn(D, device="cuda")) for _ in range(blocks)]
+    x0, state0 = torch.randn(M, D, device="cuda"), torch.randn(blocks, M, D, device="cuda")
+
+    def run(one_launch):
+        x, state = x0.clone(), state0.clone()
+        scratch = dict(y=torch.empty_like(x), xb=x.bfloat16(), yb=bf16(M, D), read=bf16(M, 2 * D), gate=bf16(M, D), act=bf16(M, H),
+                       read_sq=torch.empty(C // 8, M, device="cuda"), y_sq=torch.empty(D // 8, M, device="cuda"))
+        args = (StepArgs * blocks)()
+        for i, w in enumerate(weights):
+            given = {n: t.data_ptr() for n, t in {**scratch, **w}.items()}
+            given.update(x=(x if i == 0 else scratch["y"]).data_ptr(), state=state[i].data_ptr())
+            args[i] = StepArgs(*[given[n] for n, _ in StepArgs._fields_[:17]], 1e-6, 1e-5, M, D, H, 0)
+        sync = torch.empty(512, dtype=torch.uint8, device="cuda")
+        stream = torch.cuda.current_stream().cuda_stream
+        assert lib.fields_step_stack(args, blocks, sync.data_ptr() if one_launch else None, stream) == 0
+        torch.cuda.synchronize()
+        return scratch["y"], scratch["xb"], state
+
+    got, want = run(True), run(False)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and not bool(want[0].isnan().any())
