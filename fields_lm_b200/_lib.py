@@ -59,6 +59,8 @@ SYMBOLS = {
     "fields_mixer_epilogue_backward": (_I, [_P] * 11 + [ctypes.c_float, _I, ctypes.c_longlong, _I, _P]),
     "fields_step_w12_rows": (_I, [_I]),
     "fields_step_layout": (_I, [_P, _P]),
+    "fields_product": (_I, [_P, _I, _P]),
+    "fields_transpose_bf16": (_I, [_P, _I, _P]),
     "fields_step_stack": (_I, [_P, _I, _P, _P]),
     "fields_step_block": (_I, [_P, _P]),
     "fields_read_forward_bf16_rows": (_I, [_P, _LL] + [_P] * 8 + [_SZ, _I, _I, _I, _P]),
@@ -69,6 +71,7 @@ SYMBOLS = {
                                                                        _I, _P]),
     "fields_mixer_close_grad": (_I, [_P, _LL, _I, _P]),
     "fields_stack_layout": (_I, [_P, _I, _P]),
+    "fields_stack_layout_parts": (_I, [_P, _P, _I, _I, _P]),
     "fields_stack_step_norm": (_I, [_P, _LL, _P, _P, _P, ctypes.c_float, _LL, _I, _P]),
     "fields_stack_close_mixer": (_I, [_P, _P, _P, _LL, _P, _I] + [_P] * 5 +
                                  [ctypes.c_float, _I, ctypes.c_float, _LL, _I, _P]),

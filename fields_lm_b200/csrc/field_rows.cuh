@@ -322,6 +322,7 @@ struct LayoutPiece {
     const float* scale;
     long long n;
     int cols;
+    int hidden;  // w12 in the order of the fused step and product: rows 16 j ... are u of eight features, then v of the same
 };
 constexpr int kLayoutPieces = 8;
 constexpr int kLayoutChunk = kRowThreads * 4 * 4;  // elements per block: four loads of four per thread
@@ -367,8 +368,13 @@ __global__ void __launch_bounds__(kRowThreads) layout_block(const __grid_constan
     Vec<4> v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const long long i = i0 + j * kRowThreads * 4;
-        v[j] = i < q.n && q.src ? vec_load_stream<4>(q.src + i) : vec_fill<4>(0.0f);
+        long long i = i0 + j * kRowThreads * 4;
+        const bool inside = i < q.n && q.src;
+        if (q.hidden) {
+            const int r = (int)(i / q.cols), h = r / 16 * 8 + r % 8;
+            i += (long long)((r % 16 < 8 ? h : q.hidden + h) - r) * q.cols;
+        }
+        v[j] = inside ? vec_load_stream<4>(q.src + i) : vec_fill<4>(0.0f);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -380,6 +386,36 @@ __global__ void __launch_bounds__(kRowThreads) layout_block(const __grid_constan
             for (int e = 0; e < 4; ++e) v[j].v[e] *= s.v[e];
         }
         store_bf16x4(q.dst + i, v[j]);
+    }
+}
+
+// out [cols, rows] = in [rows, cols] transposed, bfloat16: 64 x 64 through shared memory, two matrices in a launch.
+struct TransposePart {
+    const uint16_t* in;
+    uint16_t* out;
+    int rows, cols, tiles_c, tiles;
+};
+struct TransposeParams {
+    TransposePart part[2];
+};
+__global__ void __launch_bounds__(kRowThreads) transpose_bf16(const TransposeParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ uint16_t tile[64][66];
+    const int second = (int)blockIdx.x >= p.part[0].tiles;
+    const TransposePart& q = p.part[second];
+    const int t = (int)blockIdx.x - (second ? p.part[0].tiles : 0);
+    const int r0 = t / q.tiles_c * 64, c0 = t % q.tiles_c * 64, x = threadIdx.x % 32 * 2;
+    for (int y = threadIdx.x / 32; y < 64; y += kRowThreads / 32) {
+        if (r0 + y >= q.rows || c0 + x >= q.cols) continue;  // (an even number of columns)
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(q.in + (size_t)(r0 + y) * q.cols + c0 + x);
+        tile[y][x] = (uint16_t)w;
+        tile[y][x + 1] = (uint16_t)(w >> 16);
+    }
+    __syncthreads();
+    for (int y = threadIdx.x / 32; y < 64; y += kRowThreads / 32) {
+        if (c0 + y >= q.cols || r0 + x >= q.rows) continue;  // (and of rows)
+        *reinterpret_cast<uint32_t*>(q.out + (size_t)(c0 + y) * q.rows + r0 + x) =
+            (uint32_t)tile[x][y] | (uint32_t)tile[x + 1][y] << 16;
     }
 }
 

@@ -19,6 +19,7 @@
 #include "field_rows.cuh"
 #include "field_mixer_grad.cuh"
 #include "field_step_gemm.cuh"
+#include "field_product.cuh"
 
 #include "../../include/fields_read.h"
 
@@ -170,11 +171,9 @@ static thread_local const char* g_last_error = "no error";
 // programmatic-serialization attribute and waits until the kernel before it on the stream has
 // completed and its writes are visible. The launch itself (grid set-up, block scheduling) then
 // overlaps the end of the previous kernel instead of following it. Because every kernel waits, the
-// completion order of the stream is kept along the whole chain. All but one wait before they
+// completion order of the stream is kept along the whole chain. They wait before they
 // touch any memory and do not signal early: letting the next grid take SM slots while this one
-// still ran its last blocks was measured and was slower for the recurrence. step_gemm does both: it
-// lets the next kernel in at its start and reads parameters ahead of its own wait, which its
-// caller has to allow (settled, in fields_step_args). The instruction does nothing in a kernel launched
+// still ran its last blocks was measured and was slower for the recurrence. The instruction does nothing in a kernel launched
 // without the attribute (FIELDS_READ_PDL=0).
 __device__ __forceinline__ void wait_for_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1889,11 +1888,15 @@ int fields_read_norm_grad_combine(const void* grad_read, const void* read, const
 }  // extern "C"
 
 // The layout of one block; the number of thread blocks it takes in *blocks.
-static int layout_params(const struct fields_stack_weights* w, LayoutParams& p, long long* blocks) {
+static int layout_params(const struct fields_stack_weights* w, const float* ff_norm_w, int parts, LayoutParams& p,
+                         long long* blocks) {
     if (!w || w->dim <= 0 || w->hidden < 0) return FIELDS_ERR_ARGUMENT;
+    const bool rest = parts & FIELDS_LAYOUT_REST, w12 = parts & (FIELDS_LAYOUT_W12 | FIELDS_LAYOUT_W12_STEP),
+               step = parts & FIELDS_LAYOUT_W12_STEP;
+    if (step && (!ff_norm_w || !aligned16(ff_norm_w))) return ff_norm_w ? FIELDS_ERR_UNSUPPORTED : FIELDS_ERR_ARGUMENT;
     if (!w->write_w || !w->write_b || !w->gate_w || !w->out_w || !w->read_norm_w || !w->radius_logit ||
         !w->theta || !w->in_w || !w->in_b || !w->out_w16 || !w->par ||
-        (w->hidden && (!w->w12 || !w->w3 || !w->w12_16 || !w->w3_16)))
+        (w->hidden && (!w->w3 || !w->w3_16 || (w12 && (!w->w12 || !w->w12_16)))))
         return FIELDS_ERR_ARGUMENT;
     const long long D = w->dim, H = w->hidden, C = D / 2;
     const void* all[] = {w->write_w, w->write_b, w->gate_w, w->out_w, w->read_norm_w, w->w12, w->w3,
@@ -1906,34 +1909,45 @@ static int layout_params(const struct fields_stack_weights* w, LayoutParams& p, 
     p.piece[1] = {w->gate_w, in_w + 3 * C * D, nullptr, D * D, (int)D};
     p.piece[2] = {w->write_b, static_cast<uint16_t*>(w->in_b), nullptr, 3 * C, (int)(3 * C)};
     p.piece[3] = {w->out_w, static_cast<uint16_t*>(w->out_w16), w->read_norm_w, D * 2 * D, (int)(2 * D)};
-    p.piece[4] = {w->w12, static_cast<uint16_t*>(w->w12_16), nullptr, 2 * H * D, (int)D};
+    p.piece[4] = {w->w12, static_cast<uint16_t*>(w->w12_16), step ? ff_norm_w : nullptr, 2 * H * D, (int)D, step ? (int)H : 0};
     p.piece[5] = {w->w3, static_cast<uint16_t*>(w->w3_16), nullptr, D * H, (int)H};
     p.piece[6] = {nullptr, static_cast<uint16_t*>(w->in_b) + 3 * C, nullptr, D, (int)D};
     p.radius_logit = w->radius_logit; p.theta = w->theta; p.par = w->par; p.C = (int)C;
     p.piece[7] = {nullptr, nullptr, nullptr, 0, 4};
+    for (int k = 0; k < kLayoutPieces; ++k)
+        if (!(k == 4 ? w12 : rest)) p.piece[k].n = 0;
     long long at = 0;
     for (int k = 0; k < kLayoutPieces; ++k) {
         p.first[k] = at;
         at += (p.piece[k].n + kLayoutChunk - 1) / kLayoutChunk;
     }
     p.first[kLayoutPieces] = at;
-    *blocks = at + (C + kRowThreads - 1) / kRowThreads;
+    *blocks = at + (rest ? (C + kRowThreads - 1) / kRowThreads : 0);
     return *blocks > 0x7fffffffLL ? FIELDS_ERR_UNSUPPORTED : FIELDS_OK;
 }
 
 extern "C" {
 
 int fields_stack_layout(const struct fields_stack_weights* w, int count, void* stream) {
-    if (!w || count <= 0) return FIELDS_ERR_ARGUMENT;
+    return fields_stack_layout_parts(w, nullptr, count, FIELDS_LAYOUT_REST | FIELDS_LAYOUT_W12, stream);
+}
+
+int fields_stack_layout_parts(const struct fields_stack_weights* w, const float* const* ff_norm_w, int count, int parts,
+                              void* stream) {
+    const int both = FIELDS_LAYOUT_W12 | FIELDS_LAYOUT_W12_STEP;
+    if (!w || count <= 0 || parts <= 0 || (parts & ~(FIELDS_LAYOUT_REST | both)) || (parts & both) == both ||
+        ((parts & FIELDS_LAYOUT_W12_STEP) && !ff_norm_w))
+        return FIELDS_ERR_ARGUMENT;
     for (int i = 0; i < count; i += kLayoutBlocks) {
         LayoutBatch batch{};
         const int n = count - i < kLayoutBlocks ? count - i : kLayoutBlocks;
         long long blocks = 0;
         for (int k = 0; k < n; ++k) {
             if (w[i + k].dim != w[0].dim || w[i + k].hidden != w[0].hidden) return FIELDS_ERR_ARGUMENT;
-            const int rc = layout_params(&w[i + k], batch.block[k], &blocks);
+            const int rc = layout_params(&w[i + k], ff_norm_w ? ff_norm_w[i + k] : nullptr, parts, batch.block[k], &blocks);
             if (rc) return rc;
         }
+        if (blocks == 0) continue;
         const int rc = launch_grid<LayoutBatch>(layout_block, dim3((unsigned)blocks, (unsigned)n), kRowThreads,
                                                 reinterpret_cast<Stream>(stream), batch);
         if (rc) return rc;
@@ -2200,6 +2214,51 @@ static bool operand_map(CUtensorMap* map, const void* base, long long rows, int 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <class Epi, int NT>
+static int launch_product(const struct fields_product_args& g, ProductParams p, Stream st) {
+    using T = ProductShape<NT>;
+    p.k_blocks = (g.depth + T::kBox - 1) / T::kBox;
+    p.tiles_n = (p.N + NT - 1) / NT;
+    p.tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * p.tiles_n;
+    CUtensorMap a_map, b_map;
+    if (!operand_map(&a_map, g.a, p.M, g.depth, kProductRows) || !operand_map(&b_map, g.b, p.N, g.depth, NT / 2))
+        return FIELDS_ERR_UNSUPPORTED;
+    static bool ready[64] = {};
+    int rc = allow_shared_memory(pair_product<Epi, NT>, T::kSmemBytes, ready);
+    if (rc) return rc;
+    int dev = 0, sms = 0;
+    rc = check_cuda(cudaGetDevice(&dev));
+    if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (rc) return rc;
+    p.pairs = p.tiles < sms / 2 ? (int)p.tiles : sms > 1 ? sms / 2 : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p.pairs * 2);
+    cfg.blockDim = dim3(32 * (kProductWarps + 2));
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent_launch_enabled() ? 2 : 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, pair_product<Epi, NT>, a_map, b_map, p));
+}
+
+// Tiles of 256 or of 128 columns: by the rounds of tiles that a pair takes, each as long as its columns and about 64 more
+// (loads and a wave's end; 2,048 rows: 2,560 columns of depth 1,024 16.9 and 15.3 us, 1,024 of depth 2,528 21.4 and 14.4; 8,192
+// rows: 32.1 and 35.9, 41.7 and 47.2).
+template <class Epi>
+static int run_product(const struct fields_product_args& g, const ProductParams& p, Stream st) {
+    auto rounds = [&](int nt) {
+        const long long tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * ((p.N + nt - 1) / nt);
+        return (tiles + 73) / 74 * (nt + 64);
+    };
+    return rounds(128) < rounds(256) ? launch_product<Epi, 128>(g, p, st) : launch_product<Epi, 256>(g, p, st);
+}
+
 // How a launch of step_stack covers the GPU: `clusters` are resident at once.
 template <bool NARROW>
 static int step_phases(StepStackParams& p, int clusters) {
@@ -2337,6 +2396,61 @@ static int run_step(const struct fields_step_args* g, int count, unsigned* sync,
 }
 
 extern "C" {
+
+int fields_transpose_bf16(const struct fields_transpose* parts, int count, void* stream) {
+    if (!parts || count < 1 || count > 2) return FIELDS_ERR_ARGUMENT;
+    TransposeParams p{};
+    long long tiles = 0;
+    for (int i = 0; i < count; ++i) {
+        const struct fields_transpose& q = parts[i];
+        if (!q.in || !q.out || q.rows <= 0 || q.cols <= 0) return FIELDS_ERR_ARGUMENT;
+        if (q.rows % 2 || q.cols % 2 || (reinterpret_cast<uintptr_t>(q.in) | reinterpret_cast<uintptr_t>(q.out)) % 4)
+            return FIELDS_ERR_UNSUPPORTED;
+        const long long across = (q.cols + 63) / 64, n = (q.rows + 63) / 64 * across;
+        tiles += n;
+        if (tiles > 0x7fffffffLL) return FIELDS_ERR_UNSUPPORTED;
+        p.part[i] = {static_cast<const uint16_t*>(q.in), static_cast<uint16_t*>(q.out), q.rows, q.cols, (int)across, (int)n};
+    }
+    return launch_on<TransposeParams>(transpose_bf16, (unsigned)tiles, kRowThreads, 0, reinterpret_cast<Stream>(stream), p);
+}
+
+int fields_product(const struct fields_product_args* g, int kind, void* stream) {
+    if (!g || g->rows < 0 || g->cols <= 0 || g->depth <= 0) return FIELDS_ERR_ARGUMENT;
+    if (g->rows == 0) return FIELDS_OK;
+    if (!g->a || !g->b) return FIELDS_ERR_ARGUMENT;
+    if (g->cols % 4 || g->depth % 8 || g->rows > 0x7fffff00LL || !aligned16(g->a) || !aligned16(g->b) || !aligned16(g->x) ||
+        !aligned16(g->y) || !aligned16(g->bias) || !aligned16(g->gate_bias) || !aligned8(g->bias16) || !aligned8(g->gate) ||
+        !aligned8(g->read) || !aligned8(g->h) || !aligned8(g->acc) || g->gate_pitch % 4 || g->h_pitch % 4)
+        return FIELDS_ERR_UNSUPPORTED;
+    ProductParams p{};
+    auto h = [](const void* q) { return static_cast<const uint16_t*>(q); };
+    p.M = g->rows; p.N = g->cols;
+    p.x = g->x; p.bias16 = h(g->bias16); p.bias = g->bias; p.gate_bias = g->gate_bias; p.gate = h(g->gate);
+    p.gate_pitch = g->gate_pitch; p.sums = g->sums; p.entries = g->entries;
+    p.inv_features = g->features > 0 ? 1.0f / (float)g->features : 0.0f; p.eps = g->eps;
+    p.row = g->row; p.read = h(g->read); p.y = g->y; p.h = static_cast<uint16_t*>(g->h); p.h_pitch = g->h_pitch;
+    p.sums_out = g->sums_out; p.acc = static_cast<uint16_t*>(g->acc);
+    Stream st = reinterpret_cast<Stream>(stream);
+    switch (kind) {
+        case FIELDS_PRODUCT_BIAS:
+            if (!p.bias16 || !p.h) return FIELDS_ERR_ARGUMENT;
+            return run_product<ProductBias>(*g, p, st);
+        case FIELDS_PRODUCT_GATE:
+            if (!p.x || !p.bias || !p.gate_bias || !p.gate || !p.sums || p.entries <= 0 || g->features <= 0 || !p.y)
+                return FIELDS_ERR_ARGUMENT;
+            return run_product<ProductGate>(*g, p, st);
+        case FIELDS_PRODUCT_SWIGLU:
+            if (!p.sums || p.entries <= 0 || g->features <= 0 || !p.h || p.N % 16) return FIELDS_ERR_ARGUMENT;
+            return run_product<ProductSwiglu>(*g, p, st);
+        case FIELDS_PRODUCT_RESIDUAL:
+            if (!p.x || !p.y) return FIELDS_ERR_ARGUMENT;
+            return run_product<ProductResidual>(*g, p, st);
+        case FIELDS_PRODUCT_NORM_GRAD:
+            if (!p.read || !p.row || !p.h) return FIELDS_ERR_ARGUMENT;
+            return run_product<ProductNormGrad>(*g, p, st);
+    }
+    return FIELDS_ERR_ARGUMENT;
+}
 
 int fields_step_stack(const struct fields_step_args* g, int count, void* sync, void* stream) {
     if (!g || count < 0 || g->rows < 0) return FIELDS_ERR_ARGUMENT;

@@ -10,6 +10,16 @@
 
 namespace fields_torch {
 
+// Whether products with fused epilogues (field_product.cuh) take the place of the library's with row kernels between
+// them; `least` rows where the GPU is the limit. Prefill of eight blocks, 128 to 8,192 rows: d_model 512 436 to 854 us and 256
+// 346 to 512 against 500 to 946 and 497 to 559 (the host's launches bound the library's). Wider models: their tiles of 256
+// rows leave much of the GPU idle when there are few; d_model 1,024, 1,024 rows 693 us against 622, 2,048 798 against
+// 820, 4,096 1,135 against 1,217, 8,192 1,905 against 2,087.
+constexpr int64_t kPrefillRows = 2048;
+// The mixer's backward pass has two weights to transpose (12 us) for 18 us at 4,096 rows, some 50 at 16,384.
+constexpr int64_t kMixerRows = 6144;
+inline bool fused_products(int64_t rows, int64_t dim, int64_t least) { return dim <= 512 || rows >= least; }
+
 // A bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any; rows as stored are
 // `pitch` elements apart (0: dense).
 struct Operand {

@@ -1,9 +1,10 @@
 // A stack of Field blocks at inference under bfloat16 autocast: the prefill of a batch of prompts and the
 // single-token step, block by block in native code.
 //
-// Per block five matrix products (library calls) and four kernels of this library between them
-// (field_rows.cuh) instead of the ~48 launches that the block's modules make; the bfloat16 copies of
-// the weights that autocast makes on every call are laid out once per prefill and kept for the steps
+// Per block of a prefill the recurrence and four products with fused epilogues (field_product.cuh), or, for few rows of a
+// wide model, library products and row kernels (field_rows.cuh); a step is one launch (field_step_gemm.cuh).
+// A block's modules make some 48 launches. The bfloat16 copies of the weights that autocast makes on
+// every call are laid out once per prefill and kept for the steps
 // that follow it. The owner (FieldStackDecoder) asks current() before a step: the copies are used
 // only while every module, parameter and hook is what it was and no parameter has been written to, as far as
 // torch counts it (a write through `.data` or by another library is not counted; the next prefill sees
@@ -171,7 +172,7 @@ class FieldStack {
         other->uses_ = std::make_shared<CopyUses>();
         for (Block& b : other->blocks_) b.in_w = b.in_b = b.in_t = b.out_t = b.w12_t = b.w3_t = b.par = b.step_in = b.step_w12 = b.step_b = Tensor();
         other->head_ = other->head_w_ = other->head_b_ = Tensor();
-        other->laid_out_ = other->step_laid_out_ = false;
+        other->laid_out_ = other->step_laid_out_ = other->w12_laid_out_ = other->step_w12_laid_out_ = false;
         return other;
     }
 
@@ -188,7 +189,7 @@ class FieldStack {
         const c10::cuda::CUDAGuard guard(dev);
         const CopyUses::Call call(*uses_, dev, true);
         const int64_t D = D_, C = D / 2, H = H_;
-        laid_out_ = step_laid_out_ = false;
+        laid_out_ = step_laid_out_ = w12_laid_out_ = step_w12_laid_out_ = false;
         std::vector<fields_stack_weights> all;
         for (Block& b : blocks_) {
             for (Source& s : b.src) s.copied();
@@ -197,20 +198,14 @@ class FieldStack {
                 b.in_b = empty({3 * C + D}, at::kBFloat16, dev);
                 b.in_t = b.in_w.t();
                 b.out_t = empty({D, 2 * D}, at::kBFloat16, dev).t();
-                b.w12_t = empty({2 * H, D}, at::kBFloat16, dev).t();
                 b.w3_t = empty({D, H}, at::kBFloat16, dev).t();
                 b.par = empty({3, C}, at::kFloat, dev);
             }
-            fields_stack_weights w{};
-            w.write_w = b.f(Block::kWriteW); w.write_b = b.f(Block::kWriteB); w.gate_w = b.f(Block::kGateW);
-            w.out_w = b.f(Block::kOutW); w.read_norm_w = b.f(Block::kReadNorm); w.w12 = b.f(Block::kW12);
-            w.w3 = b.f(Block::kW3); w.radius_logit = b.f(Block::kRadius); w.theta = b.f(Block::kTheta);
-            w.in_w = vp(b.in_w); w.in_b = vp(b.in_b); w.out_w16 = vp(b.out_t); w.w12_16 = vp(b.w12_t);
-            w.w3_16 = vp(b.w3_t); w.par = fp(b.par);
-            w.dim = D_; w.hidden = H_;
+            const fields_stack_weights w = weights_of(b);
             all.push_back(w);
         }
-        check(api().fields_stack_layout(all.data(), (int)all.size(), stream_of(blocks_[0].in_w)), "fields_stack_layout");
+        check(api().fields_stack_layout_parts(all.data(), nullptr, (int)all.size(), FIELDS_LAYOUT_REST, stream_of(blocks_[0].in_w)),
+              "fields_stack_layout_parts");
         if (!tail_.empty()) {
             for (Source& s : tail_) s.copied();
             const at::NoGradGuard no_grad;
@@ -226,7 +221,6 @@ class FieldStack {
             if (tail_.size() > 2) copy(head_b_, tail_[2].t);
         }
         laid_out_ = true;
-        step_laid_out_ = false;
     }
 
     // x [B, L, D] fp32 -> the stack's output [B, L, D] and every block's end state [B, D].
@@ -236,34 +230,64 @@ class FieldStack {
         const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
-        const CopyUses::Call call(*uses_, dev, false);
+        CopyUses::Call call(*uses_, dev, false);
         void* st = stream_of(x);
+        const bool products = fused_products(N, D, kPrefillRows);
+        if (need_w12(products, st)) call.laid_out();
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
                      read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         const size_t ws_bytes = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
-        Tensor acc = empty({N, D}, at::kBFloat16, dev), u = empty({N, W}, at::kBFloat16, dev),
-               uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev);
+        Tensor u = empty({N, W}, at::kBFloat16, dev), act = empty({N, H_}, at::kBFloat16, dev), acc, uv, y_sq;
+        if (products) {
+            y_sq = empty({N, (D + 31) / 32}, at::kFloat, dev);
+        } else {
+            acc = empty({N, D}, at::kBFloat16, dev);
+            uv = empty({N, 2 * (int64_t)H_}, at::kBFloat16, dev);
+        }
         std::vector<Tensor> states;
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, st),
               "fields_stack_close_ff");
         const float* in = fp(x);
         for (const Block& b : blocks_) {
-            at::cuda::addmm_out(u, b.in_b, xb, b.in_t, 1, 1);
+            fields_product_args q{};
+            q.rows = N;
+            if (products) {
+                q.a = vp(xb); q.b = vp(b.in_w); q.cols = (int)W; q.depth = D_;
+                q.bias16 = vp(b.in_b); q.h = vp(u); q.h_pitch = W;
+                check(f.fields_product(&q, FIELDS_PRODUCT_BIAS, st), "fields_product");
+            } else {
+                at::cuda::addmm_out(u, b.in_b, xb, b.in_t, 1, 1);
+            }
             const Tensor state = empty({B, D}, at::kFloat, dev);
             PassWorkspace ws(ws_bytes, u);
             float* par = fp(b.par);
             ws.check(f.fields_read_forward_bf16_rows(vp(u), W, par, par + C, par + 2 * C, nullptr, vp(read), fp(groups),
                                                   fp(state), ws.ptr(), ws_bytes, (int)B, (int)L, (int)C, st),
                   "fields_read_forward_bf16_rows");
-            product(acc, plain(read), transposed(b.out_t), N, D, 2 * D);
             const void* gate = static_cast<at::BFloat16*>(vp(u)) + 3 * C;
-            check(f.fields_stack_close_mixer(in, vp(acc), gate, W, fp(groups), (int)G,
-                                             b.f(Block::kOutB), b.f(Block::kGateB), b.f(Block::kFfNorm), fp(y),
-                                             vp(xb), (float)b.read_eps, 2 * D_, (float)b.ff_eps, N, D_, st),
-                  "fields_stack_close_mixer");
-            feed_forward(b, xb, uv, act, acc, N, st);
-            check(f.fields_stack_close_ff(fp(y), vp(acc), nullptr, fp(y), vp(xb), 0.0f, N, D_, st),
-                  "fields_stack_close_ff");
+            if (products) {
+                q.a = vp(read); q.b = vp(b.out_t); q.cols = D_; q.depth = 2 * D_;
+                q.x = in; q.bias = b.f(Block::kOutB); q.gate_bias = b.f(Block::kGateB); q.gate = gate; q.gate_pitch = W;
+                q.sums = fp(groups); q.entries = (int)G; q.features = 2 * D_; q.eps = (float)b.read_eps;
+                q.y = fp(y); q.h = vp(xb); q.h_pitch = D; q.sums_out = fp(y_sq);
+                check(f.fields_product(&q, FIELDS_PRODUCT_GATE, st), "fields_product");
+                q.a = vp(xb); q.b = vp(b.step_w12); q.cols = 2 * H_; q.depth = D_;
+                q.sums = fp(y_sq); q.entries = (int)((D + 31) / 32); q.features = D_; q.eps = (float)b.ff_eps;
+                q.h = vp(act); q.h_pitch = H_;
+                check(f.fields_product(&q, FIELDS_PRODUCT_SWIGLU, st), "fields_product");
+                q.a = vp(act); q.b = vp(b.w3_t); q.cols = D_; q.depth = H_;
+                q.x = fp(y); q.h = vp(xb); q.h_pitch = D;
+                check(f.fields_product(&q, FIELDS_PRODUCT_RESIDUAL, st), "fields_product");
+            } else {
+                product(acc, plain(read), transposed(b.out_t), N, D, 2 * D);
+                check(f.fields_stack_close_mixer(in, vp(acc), gate, W, fp(groups), (int)G,
+                                                 b.f(Block::kOutB), b.f(Block::kGateB), b.f(Block::kFfNorm), fp(y),
+                                                 vp(xb), (float)b.read_eps, 2 * D_, (float)b.ff_eps, N, D_, st),
+                      "fields_stack_close_mixer");
+                feed_forward(b, xb, uv, act, acc, N, st);
+                check(f.fields_stack_close_ff(fp(y), vp(acc), nullptr, fp(y), vp(xb), 0.0f, N, D_, st),
+                      "fields_stack_close_ff");
+            }
             in = fp(y);
             states.push_back(state);
         }
@@ -296,6 +320,7 @@ class FieldStack {
             step_layout(stream_of(x));
             call.laid_out();
         }
+        if (!fused && need_w12(false, stream_of(x))) call.laid_out();
         const Tensor xb = empty({N, D}, at::kBFloat16, x.device()), y = empty({N, D}, at::kFloat, x.device());
         check(api().fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, stream_of(x)),
               "fields_stack_close_ff");
@@ -341,9 +366,9 @@ class FieldStack {
         for (Block& b : blocks_) {
             if (!b.step_in.defined()) {
                 b.step_in = empty({5 * C, D}, at::kBFloat16, dev);
-                b.step_w12 = empty({f.fields_step_w12_rows(H_), D}, at::kBFloat16, dev);
                 b.step_b = empty({5 * C}, at::kFloat, dev);
             }
+            if (!b.step_w12.defined()) b.step_w12 = empty({f.fields_step_w12_rows(H_), D}, at::kBFloat16, dev);
             fields_step_weights w{};
             w.write_w = b.f(Block::kWriteW); w.write_b = b.f(Block::kWriteB); w.gate_w = b.f(Block::kGateW);
             w.gate_b = b.f(Block::kGateB); w.w12 = b.f(Block::kW12); w.ff_norm_w = b.f(Block::kFfNorm);
@@ -351,7 +376,40 @@ class FieldStack {
             w.dim = D_; w.hidden = H_;
             check(f.fields_step_layout(&w, st), "fields_step_layout");
         }
-        step_laid_out_ = true;
+        step_laid_out_ = step_w12_laid_out_ = true;
+    }
+
+    fields_stack_weights weights_of(const Block& b) const {
+        fields_stack_weights w{};
+        w.write_w = b.f(Block::kWriteW); w.write_b = b.f(Block::kWriteB); w.gate_w = b.f(Block::kGateW);
+        w.out_w = b.f(Block::kOutW); w.read_norm_w = b.f(Block::kReadNorm); w.w12 = b.f(Block::kW12);
+        w.w3 = b.f(Block::kW3); w.radius_logit = b.f(Block::kRadius); w.theta = b.f(Block::kTheta);
+        w.in_w = vp(b.in_w); w.in_b = vp(b.in_b); w.out_w16 = vp(b.out_t); w.w3_16 = vp(b.w3_t); w.par = fp(b.par);
+        w.dim = D_; w.hidden = H_;
+        return w;
+    }
+
+    // w12 as the library's products take it, or in the order of the fused products and of the step: whichever a call
+    // needs first lays it out. Whether it did.
+    bool need_w12(bool step, void* st) {
+        bool& laid_out = step ? step_w12_laid_out_ : w12_laid_out_;
+        if (laid_out) return false;
+        const c10::Device dev = blocks_[0].in_w.device();
+        std::vector<fields_stack_weights> all;
+        std::vector<const float*> norms;
+        for (Block& b : blocks_) {
+            Tensor& to = step ? b.step_w12 : b.w12_t;
+            if (!to.defined())
+                to = step ? empty({api().fields_step_w12_rows(H_), D_}, at::kBFloat16, dev)
+                          : empty({2 * (int64_t)H_, D_}, at::kBFloat16, dev).t();
+            all.push_back(weights_of(b));
+            all.back().w12_16 = vp(to);
+            norms.push_back(b.f(Block::kFfNorm));
+        }
+        check(api().fields_stack_layout_parts(all.data(), norms.data(), (int)all.size(),
+                                              step ? FIELDS_LAYOUT_W12_STEP : FIELDS_LAYOUT_W12, st),
+              "fields_stack_layout_parts");
+        return laid_out = true;
     }
 
     // The blocks of a step in one launch, each a chain of four products with fused epilogues (field_step_gemm.cuh).
@@ -425,7 +483,7 @@ class FieldStack {
     double tail_eps_;
     bool usable_;
     int D_ = 0, H_ = 0;
-    bool laid_out_ = false, step_laid_out_ = false;
+    bool laid_out_ = false, step_laid_out_ = false, w12_laid_out_ = false, step_w12_laid_out_ = false;
     std::shared_ptr<CopyUses> uses_ = std::make_shared<CopyUses>();  // destroyed before the copies above
 };
 

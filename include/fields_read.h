@@ -505,6 +505,12 @@ struct fields_stack_weights {
     int dim, hidden;
 };
 int fields_stack_layout(const struct fields_stack_weights *weights, int count, void *stream);
+/* fields_stack_layout in parts, OR-ed: w12 as it is, or (one of the two) in the order and with the norm weights of
+ * fields_step_layout (ff_norm_w[i] of block i; w12_16 [2H, D]), and everything else. Pointers of w12 and ff_norm_w may be
+ * NULL where the part does not need them. */
+enum { FIELDS_LAYOUT_REST = 1, FIELDS_LAYOUT_W12 = 2, FIELDS_LAYOUT_W12_STEP = 4 };
+int fields_stack_layout_parts(const struct fields_stack_weights *weights, const float *const *ff_norm_w, int count, int parts,
+                              void *stream);
 int fields_stack_step_norm(const void *raw, long long raw_stride, const float *par, float *state,
                            void *out, float eps, long long N, int C, void *stream);
 int fields_stack_close_mixer(const float *x, const void *acc, const void *gate, long long gate_stride,
@@ -552,6 +558,47 @@ int fields_step_w12_rows(int hidden);
 int fields_step_layout(const struct fields_step_weights *weights, void *stream);
 int fields_step_stack(const struct fields_step_args *blocks, int count, void *sync, void *stream);
 int fields_step_block(const struct fields_step_args *args, void *stream);
+
+/*
+ * out = a @ b^T on the tensor cores, a [rows, depth] and b [cols, depth] bfloat16, fp32 accumulation, and what follows it
+ * (tensors dense unless a pitch, in elements, is given; cols and depth multiples of 8, a, b and fp32 tensors 16-byte
+ * aligned, bfloat16 ones 8-byte, pitches multiples of 4):
+ *   FIELDS_PRODUCT_BIAS       h = out + bias16
+ *   FIELDS_PRODUCT_GATE       y = x + (out r + bias) sigmoid(gate + gate_bias), r of a row rsqrt(its `entries` values in
+ *                             sums / features + eps); if given, h = y, acc = out, and sums_out [rows, ceil(cols / 32)]
+ *                             parts of the rows' sums of squares of y. y may be x.
+ *   FIELDS_PRODUCT_SWIGLU     h [., cols / 2] = silu(u r) (v r): columns 16 j ... 16 j + 7 of out are u of eight features,
+ *                             the next eight are v of the same (fields_step_layout's w12_w). cols a multiple of 16.
+ *   FIELDS_PRODUCT_RESIDUAL   y = x + out, and h = y if given. y may be x.
+ *   FIELDS_PRODUCT_NORM_GRAD  h = out + 2 row read, `row` one factor per row
+ */
+enum {
+    FIELDS_PRODUCT_BIAS,
+    FIELDS_PRODUCT_GATE,
+    FIELDS_PRODUCT_SWIGLU,
+    FIELDS_PRODUCT_RESIDUAL,
+    FIELDS_PRODUCT_NORM_GRAD
+};
+struct fields_product_args {
+    const void *a, *b;
+    long long rows;
+    int cols, depth;
+    const float *x, *bias, *gate_bias, *sums, *row;
+    const void *bias16, *gate, *read;
+    long long gate_pitch, h_pitch;
+    int entries, features;
+    float eps;
+    float *y, *sums_out;
+    void *h, *acc;
+};
+int fields_product(const struct fields_product_args *args, int kind, void *stream);
+/* out [cols, rows] = in [rows, cols] transposed, bfloat16, for one matrix or two (4-byte aligned, even extents). */
+struct fields_transpose {
+    const void *in;
+    void *out;
+    int rows, cols;
+};
+int fields_transpose_bf16(const struct fields_transpose *parts, int count, void *stream);
 
 /*
  * fields_read_forward_bf16(_stats) and fields_read_backward_bf16 on rows that lie raw_pitch (and

@@ -1,0 +1,138 @@
+"""fields_product, the products with fused epilogues (csrc/field_product.cuh), and the layouts of their weights, through the
+C ABI against the same formulas in 64 bits (GPU)."""
+import ctypes
+
+import pytest
+import torch
+
+from fields_lm_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+P, LL, I, F = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_float
+BIAS, GATE, SWIGLU, RESIDUAL, NORM_GRAD = range(5)
+
+
+class Args(ctypes.Structure):
+    _fields_ = [("a", P), ("b", P), ("rows", LL), ("cols", I), ("depth", I), ("x", P), ("bias", P), ("gate_bias", P), ("sums", P),
+                ("row", P), ("bias16", P), ("gate", P), ("read", P), ("gate_pitch", LL), ("h_pitch", LL), ("entries", I),
+                ("features", I), ("eps", F), ("y", P), ("sums_out", P), ("h", P), ("acc", P)]
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+# one row; rows, columns and depth around the edges of a warp's piece, of a block's tile and of a k-block; one tile and
+# several rounds of tiles, of 128 and of 256 columns
+@pytest.mark.parametrize("kind", range(5))
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (31, 48, 72), (129, 144, 64), (257, 272, 1000), (300, 1024, 2528), (4100, 5056, 1024),
+                                   (12000, 1040, 200), (20000, 256, 136)])
+def test_product(kind, M, N, K):
+    torch.manual_seed(M + N + kind)
+    dev, pitch = "cuda", N + 8
+
+    def rand(*shape):
+        return torch.randn(*shape, device=dev)
+
+    def halves(width):  # rows of a wider matrix
+        return torch.full((M, pitch), float("nan"), device=dev, dtype=torch.bfloat16)[:, :width]
+
+    t = dict(a=rand(M, K).bfloat16(), b=(rand(N, K) / K ** 0.5).bfloat16())
+    d = {}
+    out = t["a"].double() @ t["b"].double().T
+    entries, features, eps = {31: 4, 257: 32, 4100: 36}.get(M, 3), 100, 1e-3
+    sums = rand(M, entries).square() * 30
+    rstd = torch.rsqrt(sums.double().sum(1, keepdim=True) / features + eps)
+    if kind == BIAS:
+        t.update(bias16=rand(N).bfloat16(), h=halves(N))
+        d["h"] = out + t["bias16"].double()
+    if kind == GATE:
+        x = rand(M, N)
+        gate = halves(N).copy_(rand(M, N))
+        t.update(x=x.clone(), bias=rand(N), gate_bias=rand(N), gate=gate, sums=sums, h=halves(N),
+                 acc=torch.empty(M, N, device=dev, dtype=torch.bfloat16), sums_out=torch.empty(M, (N + 31) // 32, device=dev))
+        t["y"] = t["x"]  # in place
+        y = x.double() + (out * rstd + t["bias"].double()) * torch.sigmoid(gate.double() + t["gate_bias"].double())
+        d.update(y=y, h=y, acc=out)
+    if kind == SWIGLU:
+        t.update(sums=sums, h=halves(N // 2))
+        uv = (out * rstd).view(M, N // 16, 2, 8)
+        d["h"] = torch.nn.functional.silu(uv[:, :, 0]).mul(uv[:, :, 1]).reshape(M, N // 2)
+    if kind == RESIDUAL:
+        t.update(x=rand(M, N), y=torch.empty(M, N, device=dev), h=halves(N))
+        d["y"] = d["h"] = t["x"].double() + out
+    if kind == NORM_GRAD:
+        t.update(read=rand(M, N).bfloat16(), row=rand(M), h=halves(N))
+        d["h"] = out + 2 * t["row"].double()[:, None] * t["read"].double()
+    args = Args(rows=M, cols=N, depth=K, gate_pitch=pitch, h_pitch=pitch, entries=entries, features=features, eps=eps,
+                **{k: v.data_ptr() for k, v in t.items()})
+    assert _lib.load().fields_product(ctypes.byref(args), kind, _stream()) == 0
+    torch.cuda.synchronize()
+    for name, want in d.items():
+        # one rounding to bfloat16 is 2^-9 of each value; fp32 sums of K products err by less than 1e-5 in the norm
+        err = float((t[name].double() - want).norm() / want.norm())
+        assert err < (2 ** -8 if t[name].dtype == torch.bfloat16 else 1e-5), (name, err)
+    if kind == GATE:
+        want = d["y"].square().sum(1)
+        assert float(((t["sums_out"].double().sum(1) - want).abs() / want).max()) < 1e-4
+    if "h" in t:  # nothing beside the columns
+        whole = torch.as_strided(t["h"], (M, pitch), (pitch, 1))
+        assert bool(whole[:, t["h"].shape[1]:].isnan().all())
+
+
+def test_refusals():
+    lib, a = _lib.load(), torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16)
+    ok = dict(a=a.data_ptr(), b=a.data_ptr(), rows=8, cols=16, depth=16, bias16=a.data_ptr(), h=a.data_ptr(), h_pitch=64)
+    assert lib.fields_product(None, BIAS, _stream()) == 1
+    for bad, rc in ((dict(b=None), 1), (dict(cols=0), 1), (dict(h=None), 1), (dict(depth=12), 2), (dict(a=a.data_ptr() + 2), 2),
+                    (dict(h_pitch=63), 2)):
+        assert (lib.fields_product(ctypes.byref(Args(**{**ok, **bad})), BIAS, _stream()) != 0) == bool(rc), bad
+    assert lib.fields_product(ctypes.byref(Args(**ok)), 5, _stream()) != 0
+    assert lib.fields_product(ctypes.byref(Args(**{**ok, "rows": 0})), BIAS, _stream()) == 0
+
+
+class Transpose(ctypes.Structure):
+    _fields_ = [("in_", P), ("out", P), ("rows", I), ("cols", I)]
+
+
+@pytest.mark.parametrize("shapes", [[(2, 2)], [(62, 64), (66, 130)], [(1024, 2048), (2560, 1024)], [(16, 40)]])
+def test_transpose(shapes):
+    ins = [torch.randn(s, device="cuda").bfloat16() for s in shapes]
+    outs = [torch.zeros(s[::-1], device="cuda", dtype=torch.bfloat16) for s in shapes]
+    parts = (Transpose * len(ins))(*[Transpose(i.data_ptr(), o.data_ptr(), *i.shape) for i, o in zip(ins, outs)])
+    assert _lib.load().fields_transpose_bf16(parts, len(ins), _stream()) == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, i.T) for i, o in zip(ins, outs))
+
+
+@pytest.mark.parametrize("D,H", [(16, 8), (64, 40), (1024, 2528)])
+def test_w12_in_parts(D, H):
+    """w12 by itself, as it is and in the order of the fused products, which is that of the step."""
+    from test_gpu_step_block import StackWeights, StepWeights
+    lib, C = _lib.load(), D // 2
+    torch.manual_seed(D)
+    rows = lib.fields_step_w12_rows(H)
+    f32 = {n: torch.randn(s, device="cuda") for n, s in dict(
+        write_w=(3 * C, D), write_b=(3 * C,), gate_w=(D, D), gate_b=(D,), out_w=(D, 2 * D), read_norm_w=(2 * D,),
+        w12=(2 * H, D), w3=(D, H), radius_logit=(C,), theta=(C,), par=(3, C), norm=(D,), in_b32=(5 * C,)).items()}
+    b16 = {n: torch.zeros(s, device="cuda", dtype=torch.bfloat16) for n, s in dict(
+        in_w=(5 * C, D), in_b=(5 * C,), out_w16=(D, 2 * D), w3_16=(D, H), plain=(2 * H, D), order=(2 * H, D), step=(rows, D),
+        step_in=(5 * C, D)).items()}
+    a = {n: t.data_ptr() for n, t in {**f32, **b16}.items()}
+
+    def weights(w12_16):
+        return StackWeights(a["write_w"], a["write_b"], a["gate_w"], a["out_w"], a["read_norm_w"], a["w12"], a["w3"],
+                            a["radius_logit"], a["theta"], a["in_w"], a["in_b"], a["out_w16"], w12_16, a["w3_16"], a["par"], D, H)
+
+    norms = (P * 1)(a["norm"])
+    assert lib.fields_stack_layout_parts(ctypes.byref(weights(None)), None, 1, 1, _stream()) == 0
+    assert lib.fields_stack_layout_parts(ctypes.byref(weights(a["plain"])), None, 1, 2, _stream()) == 0
+    assert lib.fields_stack_layout_parts(ctypes.byref(weights(a["order"])), norms, 1, 4, _stream()) == 0
+    step = StepWeights(a["write_w"], a["write_b"], a["gate_w"], a["gate_b"], a["w12"], a["norm"], a["step_in"], a["step"], a["in_b32"],
+                       D, H)
+    assert lib.fields_step_layout(ctypes.byref(step), _stream()) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(b16["plain"], f32["w12"].bfloat16()) and torch.equal(b16["w3_16"], f32["w3"].bfloat16())
+    assert torch.equal(b16["order"], b16["step"][:2 * H])
+    u, v = (f32["w12"] * f32["norm"]).bfloat16().view(2, H // 8, 8, D)
+    assert torch.equal(b16["order"].view(H // 8, 2, 8, D), torch.stack([u, v], 1))
