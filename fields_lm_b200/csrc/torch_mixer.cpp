@@ -2,9 +2,10 @@
 //
 // As a composition of torch operations the mixer's forward + backward made 76 launches and was bound
 // by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is three matrix
-// products forward and four backward (library calls; the two projections of x are one product over
+// products forward and four backward (the two projections of x are one product over
 // [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
-// field_mixer_grad.cuh between them. Weight gradients come out of the products in fp32.
+// field_mixer_grad.cuh between them. With rows enough the first product and the gradients of read and x have
+// fused epilogues (field_product.cuh); the others are library calls. Weight gradients come out of the products in fp32.
 #include "torch_gemm.h"
 
 #include <ATen/ops/addmm_cuda_dispatch.h>
@@ -54,7 +55,14 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, (int)D, st),
               "fields_stack_close_ff");
         Tensor u = empty({N, W}, at::kBFloat16, dev);
-        at::cuda::addmm_out(u, in_b, xb, in_w.t(), 1, 1);
+        if (fused_products(N, D)) {
+            fields_product_args q{};
+            q.a = vp(xb); q.b = vp(in_w); q.rows = N; q.cols = (int)W; q.depth = (int)D;
+            q.bias16 = vp(in_b); q.h = vp(u); q.h_pitch = W;
+            check(f.fields_product(&q, FIELDS_PRODUCT_BIAS, st), "fields_product");
+        } else {
+            at::cuda::addmm_out(u, in_b, xb, in_w.t(), 1, 1);
+        }
         const Tensor read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         {
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
@@ -105,11 +113,28 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         auto need = [&](int i) { return ctx->needs_input_grad(i); };
         const bool recurrence = need(kX) || need(kWriteW) || need(kWriteB) || need(kRadius) || need(kTheta);
         float* p = fp(par);
+        // The products of the gradients of read and x have epilogues where there are rows enough; their weights then lie
+        // the other way round.
+        const bool fused = fused_products(N, D);
+        Tensor out16_t, in_w_t;
+        if (fused && recurrence) {
+            out16_t = empty({2 * D, D}, at::kBFloat16, dev);
+            if (need(kX)) in_w_t = empty({D, W}, at::kBFloat16, dev);
+            const fields_transpose parts[2] = {{vp(out16), vp(out16_t), (int)D, (int)(2 * D)}, {vp(in_w), vp(in_w_t), (int)W, (int)D}};
+            check(f.fields_transpose_bf16(parts, need(kX) ? 2 : 1, st), "fields_transpose_bf16");
+        }
         if (recurrence) {
             const Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
-            product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
-            check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
-                  "fields_read_norm_grad_combine");
+            if (fused) {
+                fields_product_args q{};
+                q.a = vp(grad_acc); q.b = vp(out16_t); q.rows = N; q.cols = (int)(2 * D); q.depth = (int)D;
+                q.read = vp(read); q.row = grad_sumsq; q.h = vp(grad_read); q.h_pitch = 2 * D;
+                check(f.fields_product(&q, FIELDS_PRODUCT_NORM_GRAD, st), "fields_product");
+            } else {
+                product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
+                check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
+                      "fields_read_norm_grad_combine");
+            }
             const size_t n = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_BACKWARD);
             PassWorkspace ws(n, u);
             ws.check(f.fields_read_backward_bf16_rows(vp(u), W, p, p + C, p + 2 * C, vp(read), vp(grad_read), vp(grad_u), W,
@@ -123,11 +148,18 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         }
         Tensor grad_x;
         if (need(kX)) {
-            Tensor back = empty({N, D}, at::kBFloat16, dev);
-            product(back, plain(grad_u), plain(in_w), N, D, W);
             grad_x = f32s({B, L, D});
-            check(f.fields_stack_close_ff(fp(gy), vp(back), nullptr, fp(grad_x), nullptr, 0.0f, N, (int)D, st),
-                  "fields_stack_close_ff");
+            if (fused && reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 == 0) {
+                fields_product_args q{};
+                q.a = vp(grad_u); q.b = vp(in_w_t); q.rows = N; q.cols = (int)D; q.depth = (int)W;
+                q.x = fp(gy); q.y = fp(grad_x);
+                check(f.fields_product(&q, FIELDS_PRODUCT_RESIDUAL, st), "fields_product");
+            } else {
+                Tensor back = empty({N, D}, at::kBFloat16, dev);
+                product(back, plain(grad_u), plain(in_w), N, D, W);
+                check(f.fields_stack_close_ff(fp(gy), vp(back), nullptr, fp(grad_x), nullptr, 0.0f, N, (int)D, st),
+                      "fields_stack_close_ff");
+            }
         }
         Tensor grad_write_w, grad_gate_w;  // (one product over both where both are wanted)
         if (need(kWriteW) || need(kGateW)) {
@@ -159,6 +191,8 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
     }
 
   private:
+    // (widths whose rows TMA can address)
+    static bool fused_products(int64_t N, int64_t D) { return D % 16 == 0 && fields_torch::fused_products(N, D, kMixerRows); }
     // the gate columns of [raw | gate]
     static void* gate_of(const Tensor& u, int64_t C) { return static_cast<at::BFloat16*>(vp(u)) + 3 * C; }
 };
