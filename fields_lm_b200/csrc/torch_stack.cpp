@@ -314,7 +314,7 @@ class FieldStack {
             for (Tensor& s : own) s = s.clone();
         // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
         // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
-        // against 745 and 763 with library products, but 815 against 776 at 384.
+        // against 745 and 763 with library products. (384 rows as four launches per block 1,002 against 776.)
         const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
         if (fused && !step_laid_out_) {
             step_layout(stream_of(x));
