@@ -2418,6 +2418,9 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
     if (!g || g->rows < 0 || g->cols <= 0 || g->depth <= 0) return FIELDS_ERR_ARGUMENT;
     if (g->rows == 0) return FIELDS_OK;
     if (!g->a || !g->b) return FIELDS_ERR_ARGUMENT;
+    constexpr int kWidest = 1 << 26;  // 32 rows of a tensor are addressed with 32 bits
+    if (g->cols > kWidest || g->gate_pitch > kWidest || g->h_pitch > kWidest || g->gate_pitch < 0 || g->h_pitch < 0)
+        return FIELDS_ERR_UNSUPPORTED;
     if (g->cols % 4 || g->depth % 8 || g->rows > 0x7fffff00LL || !aligned16(g->a) || !aligned16(g->b) || !aligned16(g->x) ||
         !aligned16(g->y) || !aligned16(g->bias) || !aligned16(g->gate_bias) || !aligned8(g->bias16) || !aligned8(g->gate) ||
         !aligned8(g->read) || !aligned8(g->h) || !aligned8(g->acc) || g->gate_pitch % 4 || g->h_pitch % 4)
