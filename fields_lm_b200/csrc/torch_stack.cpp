@@ -16,6 +16,8 @@
 #include <ATen/ops/mm_cuda_dispatch.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <array>
+
 namespace fields_torch {
 
 namespace py = pybind11;
@@ -43,14 +45,15 @@ struct Block {
     float* f(int i) const { return fp(src[i].t); }
 };
 
-// The copies of a plan lie in memory of the stream that first laid them out (home), and every later call may be
-// on another: a call waits for the layout, a layout for the calls on other streams, and the memory goes back only
-// behind all of them. On one stream this costs an event per layout. One thread issues at a time.
+// Copies that are allocated together lie in memory of the stream that first laid them out (home), and every later call
+// may be on another: a call waits for the layout, a layout for the calls on other streams, and the memory goes back
+// only behind all of them. On one stream this costs an event per layout. One thread issues at a time. Copies that calls
+// lay out on the way have a home of their own each: the stream of the call that first needed them.
 class CopyUses {
   public:
     using Stream = c10::cuda::CUDAStream;
 
-    // One call that uses (or, `writes`, lays out) the copies on the current stream of `device`.
+    // One call that uses (or, `writes`, lays out and may then use) the copies on the current stream of `device`.
     class Call {
       public:
         Call(CopyUses& u, c10::Device device, bool writes)
@@ -63,13 +66,14 @@ class CopyUses {
         ~Call() {
             try {
                 if (writes_) laid_out();
-                else if (stream_ != *u_.home_ || external(stream_)) u_.used_on(stream_);
+                if (stream_ != *u_.home_ || external(stream_)) u_.used_on(stream_);
             } catch (...) {
             }
         }
         Call(const Call&) = delete;
-        // what a reading call has laid out on the way
+        // The layout has been issued: calls on other streams wait for nothing behind it.
         void laid_out() {
+            writes_ = false;
             if (captured(stream_)) return;  // (a plan of its own, used on this stream only)
             u_.laid_.record(stream_);
             u_.laid_on_ = stream_;
@@ -162,17 +166,16 @@ class FieldStack {
 
     // ... and whether the copies of the parameters are up to date.
     bool current() const {
-        return laid_out_ && same_model() && every_source([](const Source& s) { return s.current(); });
+        return copies_[kBase].laid_out && same_model() && every_source([](const Source& s) { return s.current(); });
     }
 
     // The same plan without copies, for a graph that is being captured: its copies are laid out by the graph
     // itself, from the weights of the moment it runs, into memory of its own.
     std::unique_ptr<FieldStack> fresh() const {
         auto other = std::make_unique<FieldStack>(*this);
-        other->uses_ = std::make_shared<CopyUses>();
+        for (Copies& c : other->copies_) c = Copies();
         for (Block& b : other->blocks_) b.in_w = b.in_b = b.in_t = b.out_t = b.w12_t = b.w3_t = b.par = b.step_in = b.step_w12 = b.step_b = Tensor();
         other->head_ = other->head_w_ = other->head_b_ = Tensor();
-        other->laid_out_ = other->step_laid_out_ = other->w12_laid_out_ = other->step_w12_laid_out_ = false;
         return other;
     }
 
@@ -187,9 +190,9 @@ class FieldStack {
     void layout() {
         const c10::Device dev = blocks_[0].src[0].t.device();
         const c10::cuda::CUDAGuard guard(dev);
-        const CopyUses::Call call(*uses_, dev, true);
+        const CopyUses::Call call(*copies_[kBase].uses, dev, true);
         const int64_t D = D_, C = D / 2, H = H_;
-        laid_out_ = step_laid_out_ = w12_laid_out_ = step_w12_laid_out_ = false;
+        for (Copies& c : copies_) c.laid_out = false;
         std::vector<fields_stack_weights> all;
         for (Block& b : blocks_) {
             for (Source& s : b.src) s.copied();
@@ -220,7 +223,7 @@ class FieldStack {
             head_w_ = head_.t();
             if (tail_.size() > 2) copy(head_b_, tail_[2].t);
         }
-        laid_out_ = true;
+        copies_[kBase].laid_out = true;
     }
 
     // x [B, L, D] fp32 -> the stack's output [B, L, D] and every block's end state [B, D].
@@ -230,10 +233,11 @@ class FieldStack {
         const int64_t B = x.size(0), L = x.size(1), N = B * L, D = D_, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
-        CopyUses::Call call(*uses_, dev, false);
+        const CopyUses::Call call(*copies_[kBase].uses, dev, false);
         void* st = stream_of(x);
         const bool products = fused_products(N, D, kPrefillRows);
-        if (need_w12(products, st)) call.laid_out();
+        std::optional<CopyUses::Call> w12_call;
+        need_w12(products, w12_call, st);
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
                      read = empty({N, 4 * C}, at::kBFloat16, dev), groups = empty({N, G}, at::kFloat, dev);
         const size_t ws_bytes = f.fields_read_workspace_bytes((int)B, (int)L, (int)C, FIELDS_PASS_FORWARD);
@@ -309,18 +313,16 @@ class FieldStack {
             aligned = aligned && reinterpret_cast<uintptr_t>(s.data_ptr()) % 16 == 0;
         }
         const c10::cuda::CUDAGuard guard(x.device());
-        CopyUses::Call call(*uses_, x.device(), false);
+        const CopyUses::Call call(*copies_[kBase].uses, x.device(), false);
+        std::optional<CopyUses::Call> w12_call, in_call;
         if (!aligned)
             for (Tensor& s : own) s = s.clone();
         // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
         // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
         // against 745 and 763 with library products. (384 rows as four launches per block 1,002 against 776.)
         const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
-        if (fused && !step_laid_out_) {
-            step_layout(stream_of(x));
-            call.laid_out();
-        }
-        if (!fused && need_w12(false, stream_of(x))) call.laid_out();
+        if (fused) step_layout(w12_call, in_call, stream_of(x));
+        else need_w12(false, w12_call, stream_of(x));
         const Tensor xb = empty({N, D}, at::kBFloat16, x.device()), y = empty({N, D}, at::kFloat, x.device());
         check(api().fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, D_, stream_of(x)),
               "fields_stack_close_ff");
@@ -359,8 +361,14 @@ class FieldStack {
     }
 
     // Weights in the order of the fused step.
-    void step_layout(void* st) {
+    void step_layout(std::optional<CopyUses::Call>& w12_call, std::optional<CopyUses::Call>& in_call, void* st) {
         const Api& f = api();
+        if (use(kStepIn, in_call)) {
+            use(kOrdered, w12_call);
+            return;
+        }
+        copies_[kOrdered].laid_out = false;  // (laid out again)
+        use(kOrdered, w12_call);
         const int64_t D = D_, C = D / 2;
         const c10::Device dev = blocks_[0].in_w.device();
         for (Block& b : blocks_) {
@@ -376,7 +384,8 @@ class FieldStack {
             w.dim = D_; w.hidden = H_;
             check(f.fields_step_layout(&w, st), "fields_step_layout");
         }
-        step_laid_out_ = step_w12_laid_out_ = true;
+        laid_out(kOrdered, *w12_call);
+        laid_out(kStepIn, *in_call);
     }
 
     fields_stack_weights weights_of(const Block& b) const {
@@ -389,11 +398,21 @@ class FieldStack {
         return w;
     }
 
+    // Opens a call on copies that may have to be laid out first; whether they need not be.
+    bool use(int which, std::optional<CopyUses::Call>& call) {
+        call.emplace(*copies_[which].uses, blocks_[0].in_w.device(), !copies_[which].laid_out);
+        return copies_[which].laid_out;
+    }
+    void laid_out(int which, CopyUses::Call& call) {
+        call.laid_out();
+        copies_[which].laid_out = true;
+    }
+
     // w12 as the library's products take it, or in the order of the fused products and of the step: whichever a call
-    // needs first lays it out. Whether it did.
-    bool need_w12(bool step, void* st) {
-        bool& laid_out = step ? step_w12_laid_out_ : w12_laid_out_;
-        if (laid_out) return false;
+    // needs first lays it out.
+    void need_w12(bool step, std::optional<CopyUses::Call>& call, void* st) {
+        const int which = step ? kOrdered : kPlain;
+        if (use(which, call)) return;
         const c10::Device dev = blocks_[0].in_w.device();
         std::vector<fields_stack_weights> all;
         std::vector<const float*> norms;
@@ -409,7 +428,7 @@ class FieldStack {
         check(api().fields_stack_layout_parts(all.data(), norms.data(), (int)all.size(),
                                               step ? FIELDS_LAYOUT_W12_STEP : FIELDS_LAYOUT_W12, st),
               "fields_stack_layout_parts");
-        return laid_out = true;
+        laid_out(which, *call);
     }
 
     // The blocks of a step in one launch, each a chain of four products with fused epilogues (field_step_gemm.cuh).
@@ -483,8 +502,13 @@ class FieldStack {
     double tail_eps_;
     bool usable_;
     int D_ = 0, H_ = 0;
-    bool laid_out_ = false, step_laid_out_ = false, w12_laid_out_ = false, step_w12_laid_out_ = false;
-    std::shared_ptr<CopyUses> uses_ = std::make_shared<CopyUses>();  // destroyed before the copies above
+    // in_w, in_b, out_t, w3_t, par and the head; w12_t; step_w12; step_in and step_b. A call takes kBase first.
+    enum { kBase, kPlain, kOrdered, kStepIn, kCopies };
+    struct Copies {
+        std::shared_ptr<CopyUses> uses = std::make_shared<CopyUses>();
+        bool laid_out = false;
+    };
+    std::array<Copies, kCopies> copies_;  // destroyed before the copies above
 };
 
 void add_stack(PyObject* module) {

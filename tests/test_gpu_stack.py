@@ -235,6 +235,51 @@ def test_calls_on_other_streams_wait_for_the_copies():
         del junk
 
 
+# (rows of the first call and of the late one, which needs weights in another order: the fused step, the step with library
+# products, the prefill with fused products behind one with library products and the other way round)
+@pytest.mark.parametrize("dim,hidden,B,first,late", [(256, 704, 8, 12, "step"), (64, 40, 513, 2, "step"), (1024, 704, 2, 3, 1024),
+                                                     (1024, 704, 2, 1024, 3)])
+def test_copies_made_on_the_way_outlive_their_calls(dim, hidden, B, first, late):
+    """Copies that a call on b was the first to need are read by a pending call on a when the decoder goes away; what b
+    allocates next does not get their memory before that call is done."""
+    torch.manual_seed(8)
+    model = LM(dim, 2, hidden).cuda()
+    tokens = torch.randint(0, 97, (B, 1024 if dim == 1024 else 12), device="cuda")
+    kept = [torch.randn(B, dim, device="cuda") for _ in model.blocks]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def call(dec):
+        if late != "step":
+            return dec.prefill(tokens[:, :late])
+        dec.states = [s.clone() for s in kept]
+        return dec.step(tokens[:, 0])
+
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ref = FieldStackDecoder(model)
+        ref.prefill(tokens[:, :first])
+        want = call(ref)
+        for _ in range(3):
+            dec = FieldStackDecoder(model)
+            dec._native_stack(model.emb(tokens))
+            torch.cuda.synchronize()
+            with torch.cuda.stream(a):
+                dec.prefill(tokens[:, :first])
+            torch.cuda.synchronize()
+            with torch.cuda.stream(b):
+                call(dec)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(a):
+                torch.cuda._sleep(20_000_000)
+                got = call(dec)
+            del dec
+            with torch.cuda.stream(b):  # (of the sizes of the copies)
+                junk = [torch.full((rows, dim), float("nan"), device="cuda", dtype=torch.bfloat16)
+                        for rows in (2 * hidden, (hidden + 19) // 20 * 40, 5 * dim // 2) for _ in range(8)]
+            torch.cuda.synchronize()
+            assert torch.equal(got, want)
+            del junk
+
+
 def test_threads_share_a_decoder():
     import threading
     torch.manual_seed(7)
