@@ -2170,8 +2170,8 @@ int fields_step_w12_rows(int hidden) { return hidden > 0 ? (hidden + 19) / 20 * 
 static bool step_sizes(int D, int H) { return D > 0 && D % 16 == 0 && D <= 4096 && H > 0 && H % 8 == 0; }
 
 int fields_step_layout(const struct fields_step_weights* w, void* stream) {
-    if (!w || !w->write_w || !w->write_b || !w->gate_w || !w->gate_b || !w->w12 || !w->ff_norm_w || !w->in_w ||
-        !w->w12_w || !w->in_b)
+    if (!w || !w->write_w || !w->write_b || !w->gate_w || !w->gate_b || !w->in_w || !w->in_b ||
+        (w->w12_w && (!w->w12 || !w->ff_norm_w)) || (!w->w12_w && w->w12))
         return FIELDS_ERR_ARGUMENT;
     if (!step_sizes(w->dim, w->hidden) || !aligned16(w->write_w) || !aligned16(w->gate_w) || !aligned16(w->w12) ||
         !aligned16(w->ff_norm_w) || !aligned16(w->in_w) || !aligned16(w->w12_w))
@@ -2179,8 +2179,8 @@ int fields_step_layout(const struct fields_step_weights* w, void* stream) {
     const int D = w->dim, C = D / 2;
     StepLayoutParams p{w->write_w, w->write_b, w->gate_w, w->gate_b, w->w12, w->ff_norm_w,
                        static_cast<uint16_t*>(w->in_w), static_cast<uint16_t*>(w->w12_w), w->in_b, D, C, w->hidden};
-    return launch_on<StepLayoutParams>(step_layout, (unsigned)(5 * C + fields_step_w12_rows(w->hidden)), kRowThreads, 0,
-                                       reinterpret_cast<Stream>(stream), p);
+    return launch_on<StepLayoutParams>(step_layout, (unsigned)(5 * C + (w->w12_w ? fields_step_w12_rows(w->hidden) : 0)),
+                                       kRowThreads, 0, reinterpret_cast<Stream>(stream), p);
 }
 
 }  // extern "C"

@@ -360,15 +360,12 @@ class FieldStack {
         return true;
     }
 
-    // Weights in the order of the fused step.
+    // Weights in the order of the fused step. (w12 may be there already, from a prefill with fused products. The rows that its
+    // buffer has beyond those of w12 reach no column that is stored.)
     void step_layout(std::optional<CopyUses::Call>& w12_call, std::optional<CopyUses::Call>& in_call, void* st) {
         const Api& f = api();
-        if (use(kStepIn, in_call)) {
-            use(kOrdered, w12_call);
-            return;
-        }
-        copies_[kOrdered].laid_out = false;  // (laid out again)
-        use(kOrdered, w12_call);
+        need_w12(true, w12_call, st);
+        if (use(kStepIn, in_call)) return;
         const int64_t D = D_, C = D / 2;
         const c10::Device dev = blocks_[0].in_w.device();
         for (Block& b : blocks_) {
@@ -376,15 +373,13 @@ class FieldStack {
                 b.step_in = empty({5 * C, D}, at::kBFloat16, dev);
                 b.step_b = empty({5 * C}, at::kFloat, dev);
             }
-            if (!b.step_w12.defined()) b.step_w12 = empty({f.fields_step_w12_rows(H_), D}, at::kBFloat16, dev);
             fields_step_weights w{};
             w.write_w = b.f(Block::kWriteW); w.write_b = b.f(Block::kWriteB); w.gate_w = b.f(Block::kGateW);
-            w.gate_b = b.f(Block::kGateB); w.w12 = b.f(Block::kW12); w.ff_norm_w = b.f(Block::kFfNorm);
-            w.in_w = vp(b.step_in); w.w12_w = vp(b.step_w12); w.in_b = fp(b.step_b);
+            w.gate_b = b.f(Block::kGateB);
+            w.in_w = vp(b.step_in); w.in_b = fp(b.step_b);
             w.dim = D_; w.hidden = H_;
             check(f.fields_step_layout(&w, st), "fields_step_layout");
         }
-        laid_out(kOrdered, *w12_call);
         laid_out(kStepIn, *in_call);
     }
 

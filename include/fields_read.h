@@ -527,7 +527,8 @@ int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, fl
  * 512 rows; tensors dense and 16-byte aligned; FIELDS_ERR_UNSUPPORTED otherwise).
  *
  * fields_step_layout: the rows of [write | gate] and of w12 diag(ff_norm) in the column order of the
- *   products: in_w [5C, D] and w12_w [fields_step_w12_rows(H), D] bfloat16, in_b [5C].
+ *   products: in_w [5C, D] and w12_w [fields_step_w12_rows(H), D] bfloat16, in_b [5C]. With w12 and w12_w NULL
+ *   all but w12 (fields_stack_layout_parts lays out w12 in this order as well).
  * fields_step_stack: `count` blocks, each going on from the one before (x of a block is y of the one before it;
  *   everything but x, state, the weights and the epsilons is the same for all). x [M, D] in (the block's input;
  *   xb its bfloat16 copy), y [M, D] out (may be x) and xb its copy; state [M, 2C] advances in place. out_w16, w3_16

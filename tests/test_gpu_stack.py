@@ -280,6 +280,21 @@ def test_copies_made_on_the_way_outlive_their_calls(dim, hidden, B, first, late)
             del junk
 
 
+def test_first_step_leaves_the_w12_of_the_prefill():
+    """A prefill with fused products has laid out w12 in the order of the step: the step does not write it again (a call on
+    another stream may be reading it), so a write that torch does not count is not seen."""
+    torch.manual_seed(9)
+    model = LM(64, 2, 40).cuda()
+    tokens = torch.randint(0, 97, (3, 6), device="cuda")
+    _, ref = _run(model, tokens, 6, True)
+    _, dec = _run(model, tokens, 6, True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = ref.step(tokens[:, 0])
+        for b in model.blocks:
+            b.ff.w12.weight.data.mul_(-3.0)
+        assert torch.equal(dec.step(tokens[:, 0]), want)
+
+
 def test_threads_share_a_decoder():
     import threading
     torch.manual_seed(7)
