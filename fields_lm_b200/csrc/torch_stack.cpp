@@ -185,15 +185,16 @@ class FieldStack {
     // Whether step() goes on to the logits.
     bool has_head() const { return !tail_.empty(); }
 
-    // Makes the bfloat16 copies (once per prefill: 0.21 ms for 18 blocks of d_model 1,024; 0.45 GB, and another
-    // 0.28 GB in the order of the fused step, whose layout takes 0.18 ms, from the first such step on).
-    void layout() {
+    // Makes the bfloat16 copies for a prefill of `prefill_rows` rows and the steps of `step_rows` rows that may follow it, or
+    // (0 rows of prefill) for a step. Once per prefill: 0.21 ms for 18 blocks of d_model 1,024, 0.45 GB. What only
+    // a fused step reads is made by the first one: 0.09 GB, and 0.19 GB of w12 in its order where the prefill took
+    // library products.
+    void layout(int64_t prefill_rows, int64_t step_rows) {
         const c10::Device dev = blocks_[0].src[0].t.device();
         const c10::cuda::CUDAGuard guard(dev);
         const CopyUses::Call call(*copies_[kBase].uses, dev, true);
         const int64_t D = D_, C = D / 2, H = H_;
         for (Copies& c : copies_) c.laid_out = false;
-        std::vector<fields_stack_weights> all;
         for (Block& b : blocks_) {
             for (Source& s : b.src) s.copied();
             if (!b.in_w.defined()) {
@@ -204,11 +205,20 @@ class FieldStack {
                 b.w3_t = empty({D, H}, at::kBFloat16, dev).t();
                 b.par = empty({3, C}, at::kFloat, dev);
             }
-            const fields_stack_weights w = weights_of(b);
-            all.push_back(w);
         }
-        check(api().fields_stack_layout_parts(all.data(), nullptr, (int)all.size(), FIELDS_LAYOUT_REST, stream_of(blocks_[0].in_w)),
-              "fields_stack_layout_parts");
+        void* st = stream_of(blocks_[0].in_w);
+        bool need[kCopies] = {};  // the orders of w12
+        if (prefill_rows > 0) need[fused_products(prefill_rows, D_, kPrefillRows) ? kOrdered : kPlain] = true;
+        if (prefill_rows == 0 || !fused_step(step_rows)) need[fused_step(step_rows) ? kOrdered : kPlain] = true;
+        int parts = FIELDS_LAYOUT_REST;
+        for (int which : {kOrdered, kPlain}) {
+            if (!need[which]) continue;
+            std::optional<CopyUses::Call> w12_call;
+            use(which, w12_call);
+            lay_out(parts | part_of_w12(which), st);
+            laid_out(which, *w12_call);
+            parts = 0;
+        }
         if (!tail_.empty()) {
             for (Source& s : tail_) s.copied();
             const at::NoGradGuard no_grad;
@@ -317,10 +327,7 @@ class FieldStack {
         std::optional<CopyUses::Call> w12_call, in_call;
         if (!aligned)
             for (Tensor& s : own) s = s.clone();
-        // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
-        // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
-        // against 745 and 763 with library products. (384 rows as four launches per block 1,002 against 776.)
-        const bool fused = D % 16 == 0 && H_ % 8 == 0 && N <= 512 && (N + 127) / 128 * ((D + 63) / 64) <= 32;
+        const bool fused = fused_step(N);
         if (fused) step_layout(w12_call, in_call, stream_of(x));
         else need_w12(false, w12_call, stream_of(x));
         const Tensor xb = empty({N, D}, at::kBFloat16, x.device()), y = empty({N, D}, at::kFloat, x.device());
@@ -341,6 +348,13 @@ class FieldStack {
     }
 
   private:
+    // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
+    // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
+    // against 745 and 763 with library products. (384 rows as four launches per block 1,002 against 776.)
+    bool fused_step(int64_t rows) const {
+        return D_ % 16 == 0 && H_ % 8 == 0 && rows <= 512 && (rows + 127) / 128 * ((D_ + 63) / 64) <= 32;
+    }
+
     // The embedding's output as the kernels take it: a width of another model is refused, as nn.Linear does.
     Tensor activations(const Tensor& x, int64_t dims) const {
         const c10::Device dev = blocks_[0].src[0].t.device();
@@ -403,26 +417,31 @@ class FieldStack {
         copies_[which].laid_out = true;
     }
 
+    static int part_of_w12(int which) { return which == kOrdered ? FIELDS_LAYOUT_W12_STEP : FIELDS_LAYOUT_W12; }
+    // `parts` of all blocks, w12 among them in one of its orders.
+    void lay_out(int parts, void* st) {
+        const c10::Device dev = blocks_[0].in_w.device();
+        std::vector<fields_stack_weights> all;
+        std::vector<const float*> norms;
+        for (Block& b : blocks_) {
+            const bool ordered = parts & FIELDS_LAYOUT_W12_STEP;
+            Tensor& to = ordered ? b.step_w12 : b.w12_t;
+            if (!to.defined())
+                to = ordered ? empty({api().fields_step_w12_rows(H_), D_}, at::kBFloat16, dev)
+                             : empty({2 * (int64_t)H_, D_}, at::kBFloat16, dev).t();
+            all.push_back(weights_of(b));
+            all.back().w12_16 = vp(to);
+            norms.push_back(b.f(Block::kFfNorm));
+        }
+        check(api().fields_stack_layout_parts(all.data(), norms.data(), (int)all.size(), parts, st), "fields_stack_layout_parts");
+    }
+
     // w12 as the library's products take it, or in the order of the fused products and of the step: whichever a call
     // needs first lays it out.
     void need_w12(bool step, std::optional<CopyUses::Call>& call, void* st) {
         const int which = step ? kOrdered : kPlain;
         if (use(which, call)) return;
-        const c10::Device dev = blocks_[0].in_w.device();
-        std::vector<fields_stack_weights> all;
-        std::vector<const float*> norms;
-        for (Block& b : blocks_) {
-            Tensor& to = step ? b.step_w12 : b.w12_t;
-            if (!to.defined())
-                to = step ? empty({api().fields_step_w12_rows(H_), D_}, at::kBFloat16, dev)
-                          : empty({2 * (int64_t)H_, D_}, at::kBFloat16, dev).t();
-            all.push_back(weights_of(b));
-            all.back().w12_16 = vp(to);
-            norms.push_back(b.f(Block::kFfNorm));
-        }
-        check(api().fields_stack_layout_parts(all.data(), norms.data(), (int)all.size(),
-                                              step ? FIELDS_LAYOUT_W12_STEP : FIELDS_LAYOUT_W12, st),
-              "fields_stack_layout_parts");
+        lay_out(part_of_w12(which), st);
         laid_out(which, *call);
     }
 
@@ -518,7 +537,9 @@ void add_stack(PyObject* module) {
         .def("same_model", &FieldStack::same_model)
         .def("current", &FieldStack::current)
         .def("fresh", &FieldStack::fresh)
-        .def("layout", torch::wrap_pybind_function_no_gil([](FieldStack& s) { s.layout(); }))
+        .def("layout", torch::wrap_pybind_function_no_gil([](FieldStack& s, int64_t prefill_rows, int64_t step_rows) {
+                           s.layout(prefill_rows, step_rows);
+                       }))
         .def("prefill", torch::wrap_pybind_function_no_gil([](FieldStack& s, const Tensor& x) { return s.prefill(x); }))
         .def("step", torch::wrap_pybind_function_no_gil(
                          [](FieldStack& s, const Tensor& x, const std::vector<Tensor>& st) { return s.step(x, st); }));

@@ -84,14 +84,15 @@ class FieldStackDecoder:
         follow use the same copies until a parameter changes: an in-place write as torch counts
         it (``load_state_dict``, an optimizer, ``copy_`` under ``no_grad``) or another tensor in
         its place. A write that torch does not count, through ``.data`` or into the memory by
-        other means, is seen by the next prefill only. Inference tensors, which have no count, are
-        laid out for every step."""
+        other means, is seen by the next prefill; of what only the steps read (biases, and weights in an
+        order of theirs, which the first step lays out) by a step as well. Inference tensors, which
+        have no count, are laid out for every step."""
         from .mixer import block_prefill
         x = self.model.emb(tokens)
         if self._bf16_products(x) and x.dim() == 3:
             stack = self._native_stack(x)
             if stack is not None:
-                stack.layout()
+                stack.layout(x.shape[0] * x.shape[1], x.shape[0])
                 x, self.states = stack.prefill(x)
                 return self.model.lm_head(self.model.final_norm(x[:, -1] if last_only else x))
         states = []
@@ -116,7 +117,7 @@ class FieldStackDecoder:
                     or torch.cuda.is_current_stream_capturing()):
                 stack = self._native_stack(x)
                 if stack is not None:
-                    stack.layout()
+                    stack.layout(0, x.shape[0])
             if stack is not None:
                 out = stack.step(x, self.states)
                 return out if stack.has_head else self.model.lm_head(self.model.final_norm(out))

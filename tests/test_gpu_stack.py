@@ -295,6 +295,20 @@ def test_first_step_leaves_the_w12_of_the_prefill():
         assert torch.equal(dec.step(tokens[:, 0]), want)
 
 
+def test_library_step_uses_the_weights_of_the_prefill():
+    """... and so does the step with library products behind a prefill with fused ones."""
+    torch.manual_seed(10)
+    model = LM(64, 2, 40).cuda()
+    tokens = torch.randint(0, 97, (513, 3), device="cuda")
+    _, ref = _run(model, tokens, 3, True)
+    _, dec = _run(model, tokens, 3, True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = ref.step(tokens[:, 0])
+        for b in model.blocks:
+            b.ff.w12.weight.data.mul_(-3.0)
+        assert torch.equal(dec.step(tokens[:, 0]), want)
+
+
 def test_threads_share_a_decoder():
     import threading
     torch.manual_seed(7)
