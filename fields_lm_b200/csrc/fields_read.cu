@@ -2419,19 +2419,23 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
     if (g->rows == 0) return FIELDS_OK;
     if (!g->a || !g->b) return FIELDS_ERR_ARGUMENT;
     constexpr int kWidest = 1 << 26;  // 32 rows of a tensor are addressed with 32 bits
-    if (g->cols > kWidest || g->gate_pitch > kWidest || g->h_pitch > kWidest || g->gate_pitch < 0 || g->h_pitch < 0)
+    const int h_cols = kind == FIELDS_PRODUCT_SWIGLU ? g->cols / 2 : g->cols;
+    const long long gate_pitch = g->gate_pitch ? g->gate_pitch : g->cols, h_pitch = g->h_pitch ? g->h_pitch : h_cols;
+    if ((kind == FIELDS_PRODUCT_GATE && gate_pitch < g->cols) || (g->h && h_pitch < h_cols))
+        return FIELDS_ERR_ARGUMENT;  // rows would overlap
+    if (g->cols > kWidest || gate_pitch > kWidest || h_pitch > kWidest || gate_pitch < 0 || h_pitch < 0)
         return FIELDS_ERR_UNSUPPORTED;
     if (g->cols % 4 || g->depth % 8 || g->rows > 0x7fffff00LL || !aligned16(g->a) || !aligned16(g->b) || !aligned16(g->x) ||
         !aligned16(g->y) || !aligned16(g->bias) || !aligned16(g->gate_bias) || !aligned8(g->bias16) || !aligned8(g->gate) ||
-        !aligned8(g->read) || !aligned8(g->h) || !aligned8(g->acc) || g->gate_pitch % 4 || g->h_pitch % 4)
+        !aligned8(g->read) || !aligned8(g->h) || !aligned8(g->acc) || gate_pitch % 4 || h_pitch % 4)
         return FIELDS_ERR_UNSUPPORTED;
     ProductParams p{};
     auto h = [](const void* q) { return static_cast<const uint16_t*>(q); };
     p.M = g->rows; p.N = g->cols;
     p.x = g->x; p.bias16 = h(g->bias16); p.bias = g->bias; p.gate_bias = g->gate_bias; p.gate = h(g->gate);
-    p.gate_pitch = g->gate_pitch; p.sums = g->sums; p.entries = g->entries;
+    p.gate_pitch = gate_pitch; p.sums = g->sums; p.entries = g->entries;
     p.inv_features = g->features > 0 ? 1.0f / (float)g->features : 0.0f; p.eps = g->eps;
-    p.row = g->row; p.read = h(g->read); p.y = g->y; p.h = static_cast<uint16_t*>(g->h); p.h_pitch = g->h_pitch;
+    p.row = g->row; p.read = h(g->read); p.y = g->y; p.h = static_cast<uint16_t*>(g->h); p.h_pitch = h_pitch;
     p.sums_out = g->sums_out; p.acc = static_cast<uint16_t*>(g->acc);
     Stream st = reinterpret_cast<Stream>(stream);
     switch (kind) {

@@ -562,7 +562,7 @@ int fields_step_block(const struct fields_step_args *args, void *stream);
 
 /*
  * out = a @ b^T on the tensor cores, a [rows, depth] and b [cols, depth] bfloat16, fp32 accumulation, and what follows it
- * (tensors dense unless a pitch, in elements, is given; cols and depth multiples of 8, a, b and fp32 tensors 16-byte
+ * (tensors dense unless a pitch, in elements and no less than the columns, is given; cols and depth multiples of 8, a, b and fp32 tensors 16-byte
  * aligned, bfloat16 ones 8-byte, pitches multiples of 4):
  *   FIELDS_PRODUCT_BIAS       h = out + bias16
  *   FIELDS_PRODUCT_GATE       y = x + (out r + bias) sigmoid(gate + gate_bias), r of a row rsqrt(its `entries` values in

@@ -91,6 +91,37 @@ def test_refusals():
     assert lib.fields_product(ctypes.byref(Args(**{**ok, "rows": 0})), BIAS, _stream()) == 0
 
 
+@pytest.mark.parametrize("kind", [BIAS, GATE, SWIGLU])
+def test_pitches(kind):
+    """None is dense; one that makes rows overlap or that 32 bits do not address is refused."""
+    M, N, K, lib = 5, 32, 16, _lib.load()
+    torch.manual_seed(kind)
+    width = N // 2 if kind == SWIGLU else N
+
+    def rand(*shape):
+        return torch.randn(*shape, device="cuda")
+
+    t = dict(a=rand(M, K).bfloat16(), b=rand(N, K).bfloat16(), bias16=rand(N).bfloat16(), x=rand(M, N), bias=rand(N),
+             gate_bias=rand(N), gate=rand(M, N).bfloat16(), sums=rand(M, 3).square())
+
+    def call(**pitches):
+        h, y = torch.full((M, width), float("nan"), device="cuda", dtype=torch.bfloat16), torch.empty(M, N, device="cuda")
+        args = Args(rows=M, cols=N, depth=K, entries=3, features=10, eps=1e-3, h=h.data_ptr(), y=y.data_ptr(),
+                    **{k: v.data_ptr() for k, v in t.items()}, **pitches)
+        rc = lib.fields_product(ctypes.byref(args), kind, _stream())
+        torch.cuda.synchronize()
+        return rc, h
+
+    (rc, got), (rc2, want) = call(), call(gate_pitch=N, h_pitch=width)
+    assert rc == rc2 == 0 and torch.equal(got, want) and not bool(want.isnan().any())
+    refused = [dict(h_pitch=width - 4), dict(h_pitch=4), dict(h_pitch=-width), dict(h_pitch=(1 << 26) + 4)]
+    if kind == GATE:
+        refused += [dict(gate_pitch=N - 4), dict(gate_pitch=-N), dict(gate_pitch=(1 << 26) + 4)]
+    for pitches in refused:
+        rc, h = call(**pitches)
+        assert rc != 0 and bool(h.isnan().all()), pitches
+
+
 class Transpose(ctypes.Structure):
     _fields_ = [("in_", P), ("out", P), ("rows", I), ("cols", I)]
 
