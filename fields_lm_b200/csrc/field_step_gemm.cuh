@@ -11,7 +11,7 @@
 // 3.9 us at the copy bandwidth, its products 4 us. A phase takes 6 to 8 us (256 rows: 3,000 cycles from the last
 // tile of one phase to the first load of the next, 4,200 until the product is done, 7 in the 160-column
 // product, 1,800 for the exchange of partial sums, 1,200 to 4,000 for the epilogue, 1,400 until it is
-// published). As four launches per block, each with its own set-up, weights first loaded then, a phase took 8 to 9.4:
+// published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 take 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
 // 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
@@ -59,10 +59,6 @@ __device__ __forceinline__ void tma_load2(unsigned dst, const CUtensorMap* map, 
 __device__ __forceinline__ void send4(unsigned dst, float x, float y, float z, float w, unsigned bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
                  "f"(x), "f"(y), "f"(z), "f"(w), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void send1(unsigned dst, float x, unsigned bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(x), "r"(bar)
                  : "memory");
 }
 // Shared-memory descriptor of a K-major operand with the 128-byte swizzle: rows of 128 bytes, groups

@@ -19,6 +19,7 @@
 #include "field_rows.cuh"
 #include "field_mixer_grad.cuh"
 #include "field_step_gemm.cuh"
+#include "field_step_phase.cuh"
 #include "field_product.cuh"
 
 #include "../../include/fields_read.h"
@@ -171,9 +172,11 @@ static thread_local const char* g_last_error = "no error";
 // programmatic-serialization attribute and waits until the kernel before it on the stream has
 // completed and its writes are visible. The launch itself (grid set-up, block scheduling) then
 // overlaps the end of the previous kernel instead of following it. Because every kernel waits, the
-// completion order of the stream is kept along the whole chain. They wait before they
+// completion order of the stream is kept along the whole chain. All but one wait before they
 // touch any memory and do not signal early: letting the next grid take SM slots while this one
-// still ran its last blocks was measured and was slower for the recurrence. The instruction does nothing in a kernel launched
+// still ran its last blocks was measured and was slower for the recurrence. step_phase does both: it lets the next kernel
+// in at its start and reads parameters ahead of its own wait, which its caller has to allow (settled, in
+// fields_step_args). The instruction does nothing in a kernel launched
 // without the attribute (FIELDS_READ_PDL=0).
 __device__ __forceinline__ void wait_for_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2345,6 +2348,72 @@ static int launch_step(StepStackParams& p, bool cooperative, Stream st) {
     return check_cuda(e);
 }
 
+// Whether the narrow tiles leave less of the GPU without one.
+static bool step_narrow(int rows, int dim) { return (rows + kStepRows - 1) / kStepRows * ((dim + 63) / 64) * 8 <= 148; }
+
+// One product of a block: A [M, K] activations, B [n_rows, K] weights, `slices` column slices.
+template <class Epi>
+static int launch_phase(const void* a, const void* b, int n_rows, int K, int slices, PhaseParams p, Stream st) {
+    using T = PhaseTile<Epi>;
+    p.k_blocks = (K + kStepKBox - 1) / kStepKBox;
+    p.tiles_n = (slices + Epi::kSlices - 1) / Epi::kSlices;
+    const int tiles = p.tiles_n * ((p.M + kStepRows - 1) / kStepRows);
+    // K over as many blocks as share the GPU in one round, every one of them with a part of K (clusters of four or more
+    // do not find room for 144 blocks: 384 features, 384 rows took 250 us instead of 215 for eight blocks)
+    p.S = 1;
+    for (int S = 2; S <= Epi::kMaxSplit && tiles * S <= (S > 2 ? 132 : 148); S *= 2)
+        if ((S - 1) * ((p.k_blocks + S - 1) / S) < p.k_blocks) p.S = S;
+    CUtensorMap a_map, b_map;
+    if (!operand_map(&a_map, a, p.M, K, kStepRows) || !operand_map(&b_map, b, n_rows, K, T::kNT))
+        return FIELDS_ERR_UNSUPPORTED;
+    static bool ready[64] = {};
+    const int rc = allow_shared_memory(step_phase<Epi>, T::kSmemBytes, ready);
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * p.S));
+    cfg.blockDim = dim3(kPhaseThreads);
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (dependent_launch_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.S > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)p.S;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return check_cuda(cudaLaunchKernelEx(&cfg, step_phase<Epi>, a_map, b_map, p));
+}
+
+// A block as four launches.
+static int step_block(const struct fields_step_args& g, Stream st) {
+    const int D = g.dim, C = D / 2, H = g.hidden;
+    auto h = [](void* q) { return static_cast<uint16_t*>(q); };
+    PhaseParams p{};
+    p.x = g.x; p.gate = h(g.gate); p.read = h(g.read); p.state = g.state; p.y = g.y; p.yb = h(g.yb);
+    p.act = h(g.act); p.xb = h(g.xb); p.read_sq = g.read_sq; p.y_sq = g.y_sq;
+    p.in_b = g.in_b; p.par = g.par; p.out_b = g.out_b;
+    p.read_eps = g.read_eps; p.ff_eps = g.ff_eps; p.M = g.rows; p.D = D; p.C = C; p.H = H;
+    // the first product waits where a parameter may still be on its way; it lets the second in afterwards
+    p.wait_first = !g.settled;
+    int rc = launch_phase<PhaseIn>(g.xb, g.in_w, 5 * C, D, C / 8, p, st);
+    p.wait_first = 0;
+    const bool narrow = step_narrow(g.rows, D);
+    if (!rc) rc = narrow ? launch_phase<PhaseOut<4>>(g.read, g.out_w16, D, 2 * D, D / 8, p, st)
+                         : launch_phase<PhaseOut<8>>(g.read, g.out_w16, D, 2 * D, D / 8, p, st);
+    if (!rc) rc = narrow ? launch_phase<PhaseUv<5>>(g.yb, g.w12_w, fields_step_w12_rows(H), D, H / 8, p, st)
+                         : launch_phase<PhaseUv<10>>(g.yb, g.w12_w, fields_step_w12_rows(H), D, H / 8, p, st);
+    if (!rc) rc = narrow ? launch_phase<PhaseFf<4>>(g.act, g.w3_16, D, H, D / 8, p, st)
+                         : launch_phase<PhaseFf<8>>(g.act, g.w3_16, D, H, D / 8, p, st);
+    return rc;
+}
+
 template <bool NARROW>
 static int run_step(const struct fields_step_args* g, int count, unsigned* sync, Stream st) {
     using T = StepShape<NARROW>;
@@ -2380,9 +2449,11 @@ static int run_step(const struct fields_step_args* g, int count, unsigned* sync,
             p.last = n * kStepPhases;
             rc = check_cuda(cudaMemsetAsync(sync, 0, kStepSyncBytes, st));
             if (!rc) rc = launch_step<NARROW>(p, true, st);
-        }
-        if (rc == FIELDS_ERR_UNSUPPORTED) {  // one launch per phase: none of them waits for another
-            p.sync = nullptr;
+            if (rc == FIELDS_ERR_UNSUPPORTED) {  // no such launch on this device
+                rc = FIELDS_OK;
+                for (int i = 0; i < n && !rc; ++i) rc = step_block(g[at + i], st);
+            }
+        } else {  // one launch per phase: none of them waits for another
             rc = FIELDS_OK;
             for (int i = 0; i < n * kStepPhases && !rc; ++i) {
                 p.first = i;
@@ -2392,6 +2463,17 @@ static int run_step(const struct fields_step_args* g, int count, unsigned* sync,
         }
         if (rc) return rc;
     }
+    return FIELDS_OK;
+}
+
+static int step_arguments(const struct fields_step_args& q) {
+    const void* all[] = {q.x, q.state, q.y, q.xb, q.yb, q.read, q.gate, q.act, q.read_sq, q.y_sq, q.in_w,
+                         q.out_w16, q.w12_w, q.w3_16, q.in_b, q.par, q.out_b};
+    for (const void* v : all)
+        if (!v) return FIELDS_ERR_ARGUMENT;
+    if (!step_sizes(q.dim, q.hidden) || q.rows > 512) return FIELDS_ERR_UNSUPPORTED;
+    for (const void* v : all)
+        if (!aligned16(v)) return FIELDS_ERR_UNSUPPORTED;
     return FIELDS_OK;
 }
 
@@ -2464,13 +2546,8 @@ int fields_step_stack(const struct fields_step_args* g, int count, void* sync, v
     if (g->rows == 0 || count == 0) return FIELDS_OK;
     for (int i = 0; i < count; ++i) {
         const struct fields_step_args& q = g[i];
-        const void* all[] = {q.x, q.state, q.y, q.xb, q.yb, q.read, q.gate, q.act, q.read_sq, q.y_sq, q.in_w,
-                             q.out_w16, q.w12_w, q.w3_16, q.in_b, q.par, q.out_b};
-        for (const void* v : all)
-            if (!v) return FIELDS_ERR_ARGUMENT;
-        if (!step_sizes(q.dim, q.hidden) || q.rows > 512) return FIELDS_ERR_UNSUPPORTED;
-        for (const void* v : all)
-            if (!aligned16(v)) return FIELDS_ERR_UNSUPPORTED;
+        const int rc = step_arguments(q);
+        if (rc) return rc;
         // one block goes on from the other
         if (q.y != g->y || q.xb != g->xb || q.yb != g->yb || q.read != g->read || q.gate != g->gate || q.act != g->act ||
             q.read_sq != g->read_sq || q.y_sq != g->y_sq || q.rows != g->rows || q.dim != g->dim ||
@@ -2478,12 +2555,16 @@ int fields_step_stack(const struct fields_step_args* g, int count, void* sync, v
             return FIELDS_ERR_ARGUMENT;
     }
     if (sync && !aligned16(sync)) return FIELDS_ERR_UNSUPPORTED;
-    const bool narrow = (g->rows + kStepRows - 1) / kStepRows * ((g->dim + 63) / 64) * 8 <= 148;
-    return narrow ? run_step<true>(g, count, static_cast<unsigned*>(sync), reinterpret_cast<Stream>(stream))
+    return step_narrow(g->rows, g->dim) ? run_step<true>(g, count, static_cast<unsigned*>(sync), reinterpret_cast<Stream>(stream))
                   : run_step<false>(g, count, static_cast<unsigned*>(sync), reinterpret_cast<Stream>(stream));
 }
 
-int fields_step_block(const struct fields_step_args* g, void* stream) { return fields_step_stack(g, 1, nullptr, stream); }
+int fields_step_block(const struct fields_step_args* g, void* stream) {
+    if (!g || g->rows < 0) return FIELDS_ERR_ARGUMENT;
+    if (g->rows == 0) return FIELDS_OK;
+    const int rc = step_arguments(*g);
+    return rc ? rc : step_block(*g, reinterpret_cast<Stream>(stream));
+}
 
 #endif  // FIELDS_HOST_EMU
 

@@ -44,6 +44,7 @@ using torch::autograd::variable_list;
     X(fields_stack_close_ff) X(fields_read_forward_bf16_rows) X(fields_read_backward_bf16_rows)     \
     X(fields_mixer_grad_rows) X(fields_mixer_grad_scratch_bytes) X(fields_mixer_open_grad)          \
     X(fields_mixer_close_grad) X(fields_step_w12_rows) X(fields_step_layout) X(fields_step_stack)   \
+    X(fields_step_block)                                                                            \
     X(fields_read_use_kept) X(fields_read_forward_rows)
 
 struct Api {

@@ -355,6 +355,15 @@ class FieldStack {
         return D_ % 16 == 0 && H_ % 8 == 0 && rows <= 512 && (rows + 127) / 128 * ((D_ + 63) / 64) <= 32;
     }
 
+    // Whether its blocks are one launch or four launches each. Eight blocks, us as one and as four each: d_model 256 168 and 151
+    // at 16 rows, 181 and 162 at 128, 195 and 176 at 512; 384 172 and 179, 198 and 195, 214 and 216 at 384 rows; 512 175 and
+    // 193, 187 and 204, 197 and 196 at 256 rows, 224 and 224 at 512; 640 237 and 223 at 256 rows, 282 and 326 at 512; 768
+    // 190 and 220, 242 and 245 at 256. Of the narrow ones 96 to 224 at up to 64 rows (128: 159 and 164 at one row, 159 and 166
+    // at 64; 224: 167 and 186, 173 and 188), not 64 (167 and 150 at 64 rows).
+    bool step_in_one_launch(int64_t rows) const {
+        return D_ >= (rows <= 128 ? 384 : rows <= 256 ? 704 : 512) || (rows <= 64 && D_ > 64 && D_ < 256);
+    }
+
     // The embedding's output as the kernels take it: a width of another model is refused, as nn.Linear does.
     Tensor activations(const Tensor& x, int64_t dims) const {
         const c10::Device dev = blocks_[0].src[0].t.device();
@@ -460,6 +469,7 @@ class FieldStack {
         g.x = fp(x); g.y = fp(y); g.xb = vp(xb); g.yb = vp(yb); g.read = vp(read); g.gate = vp(gate); g.act = vp(act);
         g.read_sq = fp(read_sq); g.y_sq = fp(y_sq);
         g.rows = (int)N; g.dim = D_; g.hidden = H_;
+        g.settled = 1;  // step()'s copy of x stands between a layout and the first block, and waits for it
         for (size_t i = 0; i < blocks_.size(); ++i) {
             const Block& b = blocks_[i];
             g.state = fp(states[i]);
@@ -468,6 +478,10 @@ class FieldStack {
             g.read_eps = (float)b.read_eps; g.ff_eps = (float)b.ff_eps;
             all.push_back(g);
             g.x = g.y;
+        }
+        if (!step_in_one_launch(N)) {
+            for (const fields_step_args& block : all) check(f.fields_step_block(&block, st), "fields_step_block");
+            return;
         }
         check(f.fields_step_stack(all.data(), (int)all.size(), vp(sync), st), "fields_step_stack");
     }

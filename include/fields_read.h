@@ -534,10 +534,12 @@ int fields_stack_close_ff(const float *x, const void *f, const float *norm_w, fl
  *   xb its bfloat16 copy), y [M, D] out (may be x) and xb its copy; state [M, 2C] advances in place. out_w16, w3_16
  *   and par as fields_stack_layout leaves them. Scratch: yb [M, D], read [M, 4C], gate [M, D], act [M, H] bfloat16,
  *   read_sq [C / 8, M], y_sq [D / 8, M], sync 512 bytes. One cooperative launch per 24 blocks, whose waits for
- *   one another are bounded (NaN results if one runs out); with sync NULL, or where the device holds no such launch, one
- *   launch per product.
- * fields_step_block: one block, one launch per product.
- * `settled` is not used any more: nothing is read ahead of what a call follows.
+ *   one another are bounded (NaN results if one runs out); with sync NULL one launch
+ *   per product of the same kernel (and the same results bit for bit), where the device holds no such launch
+ *   fields_step_block for each block.
+ * fields_step_block: one block, as four launches. They load their weights, in_b, par and out_b ahead of the kernel
+ *   before them on the stream if settled is non-zero: these were then complete, in stream order, before the kernel
+ *   (or copy) that this call follows. 0: nothing is read ahead of what the call follows (a layout, say).
  */
 struct fields_step_weights {
     const float *write_w, *write_b, *gate_w, *gate_b, *w12, *ff_norm_w;

@@ -99,3 +99,41 @@ def test_step_stack_is_its_phases_one_by_one(M, D, H, blocks):
 
     got, want = run(True), run(False)
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and not bool(want[0].isnan().any())
+
+
+# one row; rows and widths at the edges of a tile; K in one part, in as many as a cluster has blocks, and in fewer than fit
+# the GPU (384 rows); feed-forward widths that leave part of a tile; wide and narrow tiles
+@pytest.mark.parametrize("M,D,H", [(1, 16, 8), (3, 272, 360), (128, 48, 24), (127, 64, 176), (384, 384, 960), (129, 1024, 2528),
+                                   (512, 256, 704), (5, 2048, 96), (300, 768, 72)])
+def test_step_block_is_the_step_of_a_stack(M, D, H):
+    """Four launches with sums in an order of their own: the state to fp32 rounding, what lies behind bfloat16
+    intermediates to theirs."""
+    lib, C = _lib.load(), D // 2
+    torch.manual_seed(M + D)
+
+    def bf16(*shape):
+        return (torch.randn(shape, device="cuda") / shape[-1] ** 0.5).bfloat16()
+
+    w = dict(in_w=bf16(5 * C, D), out_w16=bf16(D, 2 * D), w12_w=bf16(lib.fields_step_w12_rows(H), D), w3_16=bf16(D, H),
+             in_b=torch.randn(5 * C, device="cuda"), par=torch.rand(3, C, device="cuda"), out_b=torch.randn(D, device="cuda"))
+    x0, state0 = torch.randn(M, D, device="cuda"), torch.randn(M, D, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(call):
+        t = dict(w, x=x0, state=state0.clone(), y=torch.empty_like(x0), xb=x0.bfloat16(), yb=bf16(M, D), read=bf16(M, 2 * D),
+                 gate=bf16(M, D), act=bf16(M, H), read_sq=torch.empty(C // 8, M, device="cuda"),
+                 y_sq=torch.empty(D // 8, M, device="cuda"))
+        args = StepArgs(*[t[n].data_ptr() for n, _ in StepArgs._fields_[:17]], 1e-6, 1e-5, M, D, H, 0)
+        assert call(ctypes.byref(args)) == 0
+        torch.cuda.synchronize()
+        return t
+
+    got = run(lambda a: lib.fields_step_block(a, stream))
+    want = run(lambda a: lib.fields_step_stack(a, 1, None, stream))
+    # fp32 sums of 2,048 products at most err by 2,048 2^-24 of their absolute sum at the very most. Two roundings to bfloat16
+    # of nearly the same value are at most neighbours, 2^-7 of it apart; act and y are computed from such values.
+    for name, bound in (("state", 2 ** -13), ("read", 2 ** -7), ("gate", 2 ** -7), ("yb", 2 ** -7), ("act", 2 ** -6), ("y", 2 ** -7),
+                        ("xb", 2 ** -6)):
+        assert torch.isfinite(want[name]).all()
+        err = float((got[name].float() - want[name].float()).abs().max())
+        assert err <= bound * float(want[name].float().abs().max()), name
