@@ -11,14 +11,24 @@
 namespace fields_torch {
 
 // Whether products with fused epilogues (field_product.cuh) take the place of the library's with row kernels between
-// them; `least` rows where the GPU is the limit. Prefill of eight blocks, 128 to 8,192 rows: d_model 512 436 to 854 us and 256
-// 346 to 512 against 500 to 946 and 497 to 559 (the host's launches bound the library's). Wider models: their tiles of 256
-// rows leave much of the GPU idle when there are few; d_model 1,024, 1,024 rows 693 us against 622, 2,048 798 against
-// 820, 4,096 1,135 against 1,217, 8,192 1,905 against 2,087.
-constexpr int64_t kPrefillRows = 2048;
-// The mixer's backward pass has two weights to transpose (12 us) for 18 us at 4,096 rows, some 50 at 16,384.
-constexpr int64_t kMixerRows = 6144;
-inline bool fused_products(int64_t rows, int64_t dim, int64_t least) { return dim <= 512 || rows >= least; }
+// them, us against the library's. Prefill of eight blocks, 128 to 8,192 rows: d_model 512 397 to 847 and 256 337 to 507
+// against 490 to 938 and 491 to 548 (the host's launches bound the library's). Wider models from `least` rows on: their
+// tiles of 256 rows leave much of the GPU idle when there are few; d_model 1,024, 1,024 rows 693 against 622, 2,048 793 against
+// 812, 4,096 1,151 against 1,207, 8,192 1,993 against 2,179; 600 at 2,048 rows 608 and 734, 768 611 and 627, 1,536 1,341 and
+// 1,364. Up to `widest`: all column tiles follow one another for each 256 rows, and beyond it the weights of a product no
+// longer stay in L2 meanwhile. Two blocks, 2,048 and 8,192 rows: d_model 2,048 535 and 1,536 against 541 and 1,631, 2,560 874 and
+// 2,649 against 747 and 2,552, 4,096 2,178 and 6,924 against 1,827 and 6,080.
+struct ProductRule {
+    int64_t least, widest;
+};
+constexpr ProductRule kPrefillProducts{2048, 2048};
+// The mixer's backward pass has two weights to transpose (12 us at d_model 1,024) for 18 us at 4,096 rows, some 50 at 16,384:
+// d_model 1,024 at 6,144 rows 285 against 295, 640 219 against 240, 2,048 750 against 763; at 6,144 and 8,192 rows 3,072 1,641 and
+// 2,127 against 1,617 and 2,149, 4,096 2,927 and 3,728 against 2,785 and 3,580.
+constexpr ProductRule kMixerProducts{6144, 3072};
+inline bool fused_products(int64_t rows, int64_t dim, ProductRule rule) {
+    return dim <= 512 || (rows >= rule.least && dim <= rule.widest);
+}
 
 // A bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any; rows as stored are
 // `pitch` elements apart (0: dense).

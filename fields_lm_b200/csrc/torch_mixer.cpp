@@ -192,7 +192,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
 
   private:
     // (widths whose rows TMA can address)
-    static bool fused_products(int64_t N, int64_t D) { return D % 16 == 0 && fields_torch::fused_products(N, D, kMixerRows); }
+    static bool fused_products(int64_t N, int64_t D) { return D % 16 == 0 && fields_torch::fused_products(N, D, kMixerProducts); }
     // the gate columns of [raw | gate]
     static void* gate_of(const Tensor& u, int64_t C) { return static_cast<at::BFloat16*>(vp(u)) + 3 * C; }
 };

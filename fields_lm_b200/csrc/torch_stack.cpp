@@ -208,7 +208,7 @@ class FieldStack {
         }
         void* st = stream_of(blocks_[0].in_w);
         bool need[kCopies] = {};  // the orders of w12
-        if (prefill_rows > 0) need[fused_products(prefill_rows, D_, kPrefillRows) ? kOrdered : kPlain] = true;
+        if (prefill_rows > 0) need[fused_products(prefill_rows, D_, kPrefillProducts) ? kOrdered : kPlain] = true;
         if (prefill_rows == 0 || !fused_step(step_rows)) need[fused_step(step_rows) ? kOrdered : kPlain] = true;
         int parts = FIELDS_LAYOUT_REST;
         for (int which : {kOrdered, kPlain}) {
@@ -245,7 +245,7 @@ class FieldStack {
         const c10::cuda::CUDAGuard guard(dev);
         const CopyUses::Call call(*copies_[kBase].uses, dev, false);
         void* st = stream_of(x);
-        const bool products = fused_products(N, D, kPrefillRows);
+        const bool products = fused_products(N, D, kPrefillProducts);
         std::optional<CopyUses::Call> w12_call;
         need_w12(products, w12_call, st);
         const Tensor xb = empty({N, D}, at::kBFloat16, dev), y = empty({B, L, D}, at::kFloat, dev),
