@@ -48,6 +48,37 @@ def test_native_mixer_matches_the_composed_one(dim, B, L):
         assert rel_err(got[name].float().cpu().numpy(), want[name].float().cpu().numpy()) < BF16_TOL, name
 
 
+# rows from which the products of a wide mixer have fused epilogues, at the edge of a tile and a ragged number; the last
+# width for which they have
+@pytest.mark.parametrize("dim,B,L", [(1024, 7, 1003), (1040, 1, 6145), (3072, 3, 2048)])
+@pytest.mark.parametrize("x_grad", [True, False])
+def test_mixer_with_fused_products(dim, B, L, x_grad):
+    """... where x needs a gradient, and where it does not, which leaves one weight to transpose."""
+    torch.manual_seed(dim)
+    m = mirror.IndependentVacancyField(dim).cuda()
+    with torch.no_grad():
+        m.read_norm.weight.add_(0.2 * torch.randn(2 * dim, device="cuda"))
+    x = torch.randn(B, L, dim, device="cuda", requires_grad=x_grad)
+    gy = torch.randn(B, L, dim, device="cuda")
+    params, keep = dict(m.named_parameters()), mixer._native_mixer
+
+    def run(native):
+        mixer._native_mixer = keep if native else lambda *a: None
+        try:
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = mixer.fused_mixer_forward(m, x)
+        finally:
+            mixer._native_mixer = keep
+        assert ("FusedMixer" in y.grad_fn.name()) == native
+        return [y.detach(), *torch.autograd.grad(y, ([x] if x_grad else []) + list(params.values()), gy)]
+
+    for name, got, want in zip(["y"] + (["x"] if x_grad else []) + list(params), run(True), run(False)):
+        assert got.shape == want.shape and got.dtype == want.dtype, name
+        assert float((got - want).norm() / want.norm()) < BF16_TOL, name
+        rows = want.flatten(0, -2) if want.dim() > 1 else want[None]  # (no row of a tile is off by itself)
+        assert float(((got.view_as(rows) if rows.dim() > 1 else got) - rows).norm(dim=-1).max()) < BF16_TOL * float(rows.norm(dim=-1).max()), name
+
+
 @pytest.mark.parametrize("L", [8, 9, 10, 35, 36, 37, 39, 40, 41, 79, 80, 81])
 def test_forward_at_the_edges_of_the_tiles(L):
     rng = np.random.default_rng(L)

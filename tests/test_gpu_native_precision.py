@@ -91,3 +91,11 @@ def test_prefill_and_step(dim, hidden, layers, B, L):
         assert _err(a, want) < FACTOR * _err(b, want)
     a, b, want = (torch.cat(list(s)) for s in (native[1].states, modules[1].states, states))
     assert _err(a, want) < FACTOR * _err(b, want)
+
+
+def test_mixer_with_fused_products():
+    test_mixer(640, 8, 800)
+
+
+def test_prefill_with_fused_products():
+    test_prefill_and_step(1024, 2528, 4, 8, 256)

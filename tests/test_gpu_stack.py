@@ -309,6 +309,28 @@ def test_library_step_uses_the_weights_of_the_prefill():
         assert torch.equal(dec.step(tokens[:, 0]), want)
 
 
+# (the step as four launches per block, as one, and with library products)
+@pytest.mark.parametrize("dim,B", [(64, 3), (384, 3), (64, 520)])
+def test_nan_stays_in_its_sequence(dim, B):
+    """A NaN embedding: NaN logits from that token on in its sequence and nowhere else, through the prefill and a step; so
+    does a NaN in a state."""
+    torch.manual_seed(11)
+    model = LM(dim, 2, 40).cuda()
+    with torch.no_grad():
+        model.emb.weight[5] = float("nan")
+    tokens = torch.randint(6, 97, (B, 9), device="cuda")
+    tokens[1, 4] = 5
+    dec = FieldStackDecoder(model)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        logits = dec.prefill(tokens, last_only=False)
+        assert dec._stack is not None
+        bad = logits.isnan()
+        assert bool(bad[1, 4:].all()) and int(bad.sum()) == bad[1, 4:].numel()
+        dec.states[0][2, 7] = float("nan")
+        bad = dec.step(tokens[:, 0]).isnan()
+    assert bool(bad[1:3].all()) and int(bad.sum()) == bad[1:3].numel()
+
+
 def test_threads_share_a_decoder():
     import threading
     torch.manual_seed(7)
