@@ -8,10 +8,10 @@
 //   EpiFf   f = act @ w3^T                  -> x' = y + f, bf16 copy
 //
 // A step of a few hundred rows is bound by latency: the 25 MB of weights of a block of d_model 1,024 take
-// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 6 to 8 us (256 rows: 3,000 cycles from the last
-// tile of one phase to the first load of the next, 4,200 until the product is done, 7 in the 160-column
-// product, 1,800 for the exchange of partial sums, 1,200 to 4,000 for the epilogue, 1,400 until it is
-// published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
+// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 6 to 8 us (256 rows: 2,400 to 3,000
+// cycles from the last tile of one phase to the first load of the next, 1,700 until its operands are there, 3,100 to 4,100
+// until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
+// 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 take 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
 // 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
@@ -78,24 +78,18 @@ __device__ __forceinline__ void step_mma(unsigned d, unsigned long long a, unsig
 __device__ __forceinline__ void step_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Eight or four columns of the thread's lane; the values are there after tmem_wait().
+// Eight columns of the thread's lane, or a multiple of eight; the values are there after tmem_wait().
 __device__ __forceinline__ void tmem_load8(unsigned addr, unsigned* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(addr)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_load4(unsigned addr, unsigned* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr)
-                 : "memory");
-}
 template <int N>
 __device__ __forceinline__ void tmem_load(unsigned addr, unsigned* r) {
+    static_assert(N % 8 == 0, "columns");
 #pragma unroll
-    for (int k = 0; k + 8 <= N; k += 8) tmem_load8(addr + k, r + k);
-    if constexpr (N % 8) tmem_load4(addr + N / 8 * 8, r + N / 8 * 8);
+    for (int k = 0; k < N; k += 8) tmem_load8(addr + k, r + k);
 }
 __device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Everything the four epilogues touch.

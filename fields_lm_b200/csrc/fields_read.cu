@@ -2218,7 +2218,7 @@ static bool operand_map(CUtensorMap* map, const void* base, long long rows, int 
 }
 
 template <class Epi, int NT>
-static int launch_product(const struct fields_product_args& g, ProductParams p, Stream st) {
+static int launch_product(const struct fields_product_args& g, ProductParams p, int pairs, Stream st) {
     using T = ProductShape<NT>;
     p.k_blocks = (g.depth + T::kBox - 1) / T::kBox;
     p.tiles_n = (p.N + NT - 1) / NT;
@@ -2227,13 +2227,9 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     if (!operand_map(&a_map, g.a, p.M, g.depth, kProductRows) || !operand_map(&b_map, g.b, p.N, g.depth, NT / 2))
         return FIELDS_ERR_UNSUPPORTED;
     static bool ready[64] = {};
-    int rc = allow_shared_memory(pair_product<Epi, NT>, T::kSmemBytes, ready);
+    const int rc = allow_shared_memory(pair_product<Epi, NT>, T::kSmemBytes, ready);
     if (rc) return rc;
-    int dev = 0, sms = 0;
-    rc = check_cuda(cudaGetDevice(&dev));
-    if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (rc) return rc;
-    p.pairs = p.tiles < sms / 2 ? (int)p.tiles : sms > 1 ? sms / 2 : 1;
+    p.pairs = p.tiles < pairs ? (int)p.tiles : pairs;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)p.pairs * 2);
     cfg.blockDim = dim3(32 * (kProductWarps + 2));
@@ -2255,16 +2251,21 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
 // rows: 32.1 and 35.9, 41.7 and 47.2).
 template <class Epi>
 static int run_product(const struct fields_product_args& g, const ProductParams& p, Stream st) {
+    int dev = 0, sms = 0;
+    int rc = check_cuda(cudaGetDevice(&dev));
+    if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (rc) return rc;
+    const int pairs = sms > 1 ? sms / 2 : 1;
     auto rounds = [&](int nt) {
         const long long tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * ((p.N + nt - 1) / nt);
-        return (tiles + 73) / 74 * (nt + 64);
+        return (tiles + pairs - 1) / pairs * (nt + 64);
     };
-    return rounds(128) < rounds(256) ? launch_product<Epi, 128>(g, p, st) : launch_product<Epi, 256>(g, p, st);
+    return rounds(128) < rounds(256) ? launch_product<Epi, 128>(g, p, pairs, st) : launch_product<Epi, 256>(g, p, pairs, st);
 }
 
 // How a launch of step_stack covers the GPU: `clusters` are resident at once.
 template <bool NARROW>
-static int step_phases(StepStackParams& p, int clusters) {
+static void step_phases(StepStackParams& p, int clusters) {
     using T = StepShape<NARROW>;
     p.groups = p.row_tiles < clusters ? p.row_tiles : clusters;
     const int most = clusters / p.groups, blocks = most * kStepCluster;
@@ -2281,14 +2282,12 @@ static int step_phases(StepStackParams& p, int clusters) {
             if ((S - 1) * ((h.k_blocks + S - 1) / S) < h.k_blocks) h.S = S;
         h.per = (h.k_blocks + h.S - 1) / h.S;
         const int subs = kStepCluster / h.S, want = (h.tiles_n + subs - 1) / subs;
-        h.iters = (want + most - 1) / most;
         if (p.group_clusters < (want < most ? want : most)) p.group_clusters = want < most ? want : most;
     }
     for (StepPhase& h : p.phase) {
         const int per = p.group_clusters * (kStepCluster / h.S);
         h.iters = (h.tiles_n + per - 1) / per;
     }
-    return FIELDS_OK;
 }
 
 // Clusters of step_stack that the device holds at once.
@@ -2328,8 +2327,8 @@ static int launch_step(StepStackParams& p, bool cooperative, Stream st) {
     cfg.numAttrs = 1;
     int clusters = 0;
     rc = step_clusters<NARROW>(cfg, &clusters);
-    if (!rc) rc = step_phases<NARROW>(p, clusters);
     if (rc) return rc;
+    step_phases<NARROW>(p, clusters);
     if (cooperative) {
         attr[1].id = cudaLaunchAttributeCooperative;
         attr[1].val.cooperative = 1;
