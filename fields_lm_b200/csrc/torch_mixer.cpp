@@ -1,7 +1,7 @@
 // The fused Field mixer (bfloat16 boundary, norm behind the output projection) as one autograd node.
 //
 // As a composition of torch operations the mixer's forward + backward made 76 launches and was bound
-// by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is three matrix
+// by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is two matrix
 // products forward and four backward (the two projections of x are one product over
 // [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
 // field_mixer_grad.cuh between them. With rows enough the first product and the gradients of read and x have
