@@ -309,8 +309,10 @@ __global__ void __launch_bounds__(kPhaseThreads, 1)
         for (int i = 0; i < kStages && i < count; ++i) load_a(i);
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(T::kNT >> 3) << 17) |
                                ((unsigned)(kStepRows >> 4) << 24);
+        int issued = kStages < count ? kStages : count;
         for (int i = 0; i < count; ++i) {
             mbar_wait(full + (i % kStages) * 8, (i / kStages) & 1, dead);
+            if (dead) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned long long a = step_desc(stage_a(i)), b = step_desc(stage_a(i) + T::kABytes);
 #pragma unroll
@@ -321,11 +323,19 @@ __global__ void __launch_bounds__(kPhaseThreads, 1)
             const int j = i - 1 + kStages;
             if (i > 0 && j < count) {
                 mbar_wait(empty + ((i - 1) % kStages) * 8, ((i - 1) / kStages) & 1, dead);
+                if (dead) break;
                 load_b(j);
                 load_a(j);
+                ++issued;
             }
         }
-        step_commit(done);
+        if (!dead) {
+            step_commit(done);
+        } else {  // what is still on its way arrives before the block leaves
+            bool late = false;
+            for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
+                mbar_wait(full + (i % kStages) * 8, (i / kStages) & 1, late);
+        }
     } else if (row_ok) {
 #pragma unroll
         for (int q = 0; q < kAhead; ++q)
@@ -340,7 +350,9 @@ __global__ void __launch_bounds__(kPhaseThreads, 1)
     if (warp < 4) {
         const unsigned lane_addr = tmem + ((unsigned)(warp * 32) << 16);
         if constexpr (Epi::kScaled) shares[rank * kStepRows + tid] = share;
-        for (int d = 1; d < S; ++d) {  // the other blocks' columns, each block starting with its neighbour
+        // the other blocks' columns, each block starting with its neighbour (after a wait that ran out nothing is sent: theirs
+        // run out as well)
+        for (int d = 1; d < S && !__any_sync(0xffffffffu, dead); ++d) {
             const int j = (rank + d) % S, src = rank > j ? rank - 1 : rank;
             const unsigned bar = peer_addr(got, j);
             const unsigned at = peer_addr(smem_addr(recv) + (unsigned)((src * own * kSlice / 4 * kStepRows + tid) * 16), j);
@@ -395,6 +407,8 @@ __global__ void __launch_bounds__(kPhaseThreads, 1)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kColumns) : "memory");
     }
+    // (a block that has given up stays until the others have left: they may still send to it)
+    if (S > 1 && dead) asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
 }
 
 }  // namespace fields
