@@ -770,6 +770,46 @@ struct BwdSinglePass {
         return smem + kSumFloats + kCarryFloats +
                ((size_t)(stage * kCells + idx) * kThreads + thread) * kCellFloats;
     }
+    // The second sweep's inputs on their way into the ring: batches of U2 steps, the next one ends just before `t`. (Rows
+    // descend; the pointers may step below the tile after the last batch and are not dereferenced then.)
+    struct Second {
+        const IO *z, *g, *r;  // rows t - 1 of raw and grad_read, t - 2 of read
+        int t;
+        FL_HD Second(const Params& p, const SpTile& tl, int c0, int t_) : t(t_) {
+            const ptrdiff_t first = (ptrdiff_t)tl.b * p.s.L + t_ - 1;
+            z = p.raw + first * p.s.zp + c0;
+            g = p.grad_read + first * 4 * p.s.C + c0;
+            r = p.read + (first - 1) * 4 * p.s.C + c0;
+        }
+        FL_HD void issue(const SpShape& s, float* smem, int thread, int nch, int tbeg, int stage) {
+            const int C = s.C;
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int tu = t - 1 - u;
+                if (tu >= tbeg) {
+                    const IO* zrow = z - (ptrdiff_t)u * s.zp;
+                    const IO* grow = g - (ptrdiff_t)u * 4 * C;
+                    async_copy4(cell_at(smem, stage, u * 9 + 0, thread), zrow, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 1, thread), zrow + C, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 2, thread), zrow + 2 * C, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 3, thread), grow, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 4, thread), grow + C, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 5, thread), grow + 2 * C, nch);
+                    async_copy4(cell_at(smem, stage, u * 9 + 6, thread), grow + 3 * C, nch);
+                    if (tu > 0) {
+                        const IO* prow = r - (ptrdiff_t)u * 4 * C;
+                        async_copy4(cell_at(smem, stage, u * 9 + 7, thread), prow, nch);
+                        async_copy4(cell_at(smem, stage, u * 9 + 8, thread), prow + C, nch);
+                    }
+                }
+            }
+            t -= U2;
+            z -= (ptrdiff_t)U2 * s.zp;
+            g -= (ptrdiff_t)U2 * 4 * C;
+            r -= (ptrdiff_t)U2 * 4 * C;
+            async_commit();
+        }
+    };
     // Warms L2 with the first-sweep inputs (z_v, grad_read) of the tile this block takes next.
     FL_HD static void prefetch(const Params& p, int tile, int thread) {
         const SpShape& s = p.s;
@@ -889,6 +929,15 @@ struct BwdSinglePass {
                     }
                 }
             }
+            // The first batches of the second sweep: under the look-back nothing else is in flight (forward + backward
+            // 127.5 -> 125.8 us at 8 x 2,048 x 512, 137.0 -> 135.4 at 1 x 16,384, 93.7 -> 92.9 with bfloat16 rows).
+            if constexpr (ASYNC) {
+                if (chan_ok) {
+                    Second in(p, tl, c0, tend);
+#pragma unroll
+                    for (int j = 0; j < STAGES - 1; ++j) in.issue(s, smem, thread, nch, tbeg, j);
+                }
+            }
             vec_store<4>(sum_at(smem, slot, 0) + lane * 4, join2(m[0].ar, m[1].ar));
             vec_store<4>(sum_at(smem, slot, 1) + lane * 4, join2(m[0].ai, m[1].ai));
             vec_store<4>(sum_at(smem, slot, 2) + lane * 4, join2(m[0].br, m[1].br));
@@ -943,46 +992,12 @@ struct BwdSinglePass {
                 const IO* gbase = p.grad_read + ((size_t)tl.b * s.L) * 4 * C + c0;
                 const IO* rbase = p.read + ((size_t)tl.b * s.L) * 4 * C + c0;
                 IO* obase = p.grad_raw + ((size_t)tl.b * s.L) * s.gp + c0;
-                int t_issue = tend;
-                const IO* zq = zbase + (ptrdiff_t)(tend - 1) * s.zp;
-                const IO* gq = gbase + (ptrdiff_t)(tend - 1) * 4 * C;
-                const IO* rq = rbase + (ptrdiff_t)(tend - 2) * 4 * C;  // row of s_{t-1}
-                auto issue2 = [&](int, int stage) {
-#pragma unroll
-                    for (int u = 0; u < U2; ++u) {
-                        const int t = t_issue - 1 - u;
-                        if (t >= tbeg) {
-                            const IO* zrow = zq - (ptrdiff_t)u * s.zp;
-                            const IO* grow = gq - (ptrdiff_t)u * 4 * C;
-                            async_copy4(cell_at(smem, stage, u * 9 + 0, thread), zrow, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 1, thread), zrow + C, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 2, thread), zrow + 2 * C, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 3, thread), grow, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 4, thread), grow + C, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 5, thread), grow + 2 * C, nch);
-                            async_copy4(cell_at(smem, stage, u * 9 + 6, thread), grow + 3 * C, nch);
-                            if (t > 0) {
-                                const IO* prow = rq - (ptrdiff_t)u * 4 * C;
-                                async_copy4(cell_at(smem, stage, u * 9 + 7, thread), prow, nch);
-                                async_copy4(cell_at(smem, stage, u * 9 + 8, thread), prow + C, nch);
-                            }
-                        }
-                    }
-                    t_issue -= U2;
-                    zq -= (ptrdiff_t)U2 * s.zp;
-                    gq -= (ptrdiff_t)U2 * 4 * C;
-                    rq -= (ptrdiff_t)U2 * 4 * C;
-                    async_commit();
-                };
-                if constexpr (ASYNC) {
-#pragma unroll
-                    for (int j = 0; j < STAGES - 1; ++j) issue2(tend - j * U2, j);
-                }
+                Second in(p, tl, c0, tend - (ASYNC ? STAGES - 1 : 0) * U2);  // (the first batches: see phase 0)
                 int stage = 0;
                 for (int t0 = tend; t0 > tbeg; t0 -= U2, stage = stage + 1 == STAGES ? 0 : stage + 1) {
                     Vec<4> zr[U2], zi[U2], zv[U2], ur[U2], ui[U2], gr[U2], gi[U2], pr[U2], pi[U2];
                     if constexpr (ASYNC) {
-                        issue2(t0 - (STAGES - 1) * U2, stage == 0 ? STAGES - 1 : stage - 1);
+                        in.issue(s, smem, thread, nch, tbeg, stage == 0 ? STAGES - 1 : stage - 1);
                         async_wait_pending<STAGES - 1>();
 #pragma unroll
                         for (int u = 0; u < U2; ++u) {
@@ -1140,6 +1155,28 @@ struct BwdRecompute {
         async_copy4(cell_at(smem, stage, u * 7 + 6, thread), grow + 3 * C);
     }
 
+    // The second sweep's batches of U steps on their way into the ring, the next one just before `t`. (Rows descend; the
+    // pointers may step below the tile after the last batch.)
+    struct Second {
+        const IO *z, *g;  // rows t - 1
+        int t;
+        FL_HD Second(const Params& p, const SpTile& tl, int c0, int t_) : t(t_) {
+            const ptrdiff_t first = (ptrdiff_t)tl.b * p.s.L + t_ - 1;
+            z = p.raw + first * 3 * p.s.C + c0;
+            g = p.grad_read + first * 4 * p.s.C + c0;
+        }
+        FL_HD void issue(const SpShape& s, float* smem, int thread, int tbeg, int stage) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t - 1 - u >= tbeg)
+                    issue_step(smem, stage, u, thread, z - (ptrdiff_t)u * 3 * s.C, g - (ptrdiff_t)u * 4 * s.C, s.C);
+            t -= U;
+            z -= (ptrdiff_t)U * 3 * s.C;
+            g -= (ptrdiff_t)U * 4 * s.C;
+            async_commit();
+        }
+    };
+
     FL_HD static void finish(const Params& p, int block, int thread, float* smem) {
         if (p.grad_par[0]) fold_partial_rows(p, sp_decode(p.s, (unsigned)block).cg, thread, reinterpret_cast<int*>(carry_at(smem, 0, 0)));
     }
@@ -1226,6 +1263,10 @@ struct BwdRecompute {
                         }
                     }
                 }
+                // the first batches of the second sweep: under the look-back nothing else is in flight
+                Second in(p, tl, c0, tend);
+#pragma unroll
+                for (int j = 0; j < STAGES - 1; ++j) in.issue(s, smem, thread, tbeg, j);
             }
             vec_store<4>(sum_at(smem, slot, 0) + lane * 4, join2(m[0].ar, m[1].ar));
             vec_store<4>(sum_at(smem, slot, 1) + lane * 4, join2(m[0].ai, m[1].ai));
@@ -1278,26 +1319,10 @@ struct BwdRecompute {
                 const Vec<4> ci4 = vec_load<4>(carry_at(smem, slot, 1) + lane * 4);
                 F2 cr[2] = {lo2(cr4), hi2(cr4)}, ci[2] = {lo2(ci4), hi2(ci4)};
                 IO* obase = p.grad_raw + ((size_t)tl.b * s.L) * 3 * C + c0;
-                // rows descend; the pointers may step below the tile after the last batch
-                int t_issue = tend;
-                const IO* zq = p.raw + ((size_t)tl.b * s.L) * 3 * C + c0 + (ptrdiff_t)(tend - 1) * 3 * C;
-                const IO* gq = p.grad_read + ((size_t)tl.b * s.L) * 4 * C + c0 + (ptrdiff_t)(tend - 1) * 4 * C;
-                auto issue = [&](int stage) {
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-                        if (t_issue - 1 - u >= tbeg)
-                            issue_step(smem, stage, u, thread, zq - (ptrdiff_t)u * 3 * C,
-                                       gq - (ptrdiff_t)u * 4 * C, C);
-                    t_issue -= U;
-                    zq -= (ptrdiff_t)U * 3 * C;
-                    gq -= (ptrdiff_t)U * 4 * C;
-                    async_commit();
-                };
-#pragma unroll
-                for (int j = 0; j < STAGES - 1; ++j) issue(j);
+                Second in(p, tl, c0, tend - (STAGES - 1) * U);  // (the first batches: see phase 0)
                 int stage = 0;
                 for (int t0 = tend; t0 > tbeg; t0 -= U, stage = stage + 1 == STAGES ? 0 : stage + 1) {
-                    issue(stage == 0 ? STAGES - 1 : stage - 1);
+                    in.issue(s, smem, thread, tbeg, stage == 0 ? STAGES - 1 : stage - 1);
                     async_wait_pending<STAGES - 1>();
 #pragma unroll
                     for (int u = 0; u < U; ++u) {

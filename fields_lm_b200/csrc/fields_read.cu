@@ -680,8 +680,9 @@ using BwdSp3 = BwdTileResident<4, 4, 3>;      // tile 16, 68 KB per block, 12 wa
 template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;  // STATS: per-token sums of squares too
 // bfloat16 ring cells are half the size, so a 64-step tile (4 warps x 16 steps) still leaves room for
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
-// 16-byte cells) on 8 x 2,048 tokens.
-using BwdSpBf16 = BwdSinglePass<16, 4, 2, 1, 3, true, 3, uint16_t>;
+// 16-byte cells) on 8 x 2,048 tokens. (The bound of 128 registers keeps the fourth block: without it the second sweep's early
+// batches take 138.)
+using BwdSpBf16 = BwdSinglePass<16, 4, 2, 1, 4, true, 3, uint16_t>;
 // Smallest time tile of any instantiation above, for the workspace bound (the run functions assert it). The
 // bound also decides which extents fields_read_forward_noalloc takes.
 constexpr int kSpMinTile = 32;
