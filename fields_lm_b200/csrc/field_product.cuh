@@ -10,11 +10,19 @@
 //
 // As library products with row kernels between them a Field block wrote and read every product's result once
 // more: of a prefill of 8 x 1,024 tokens through 18 blocks of d_model 1,024 (4.93 ms) 3.05 ms were products and
-// 1.0 ms the row kernels. Now 4.57. Alone, 8,192 rows, products of the library and, with what follows, these (us): bias,
-// 2,560 columns of depth 1,024, 33 and 32; SwiGLU, 5,056 of 1,024, 66 (+ 19 for the row kernel) and 56; residual,
-// 1,024 of 2,528, 33 (+ 14) and 42; gate, 1,024 of 2,048, 27 (+ 21) and 46; gradient of the norm, 2,048 of 1,024, 30 (+ 18)
-// and 35. Products run at 1.3 to 1.5 PFLOP/s; the epilogues with fp32 inputs and outputs are bound by the latency
-// of HBM under load (3,000 cycles) and the 24 to 32 KB that a block's registers keep in flight.
+// 1.0 ms the row kernels. Then 4.45, and now 4.20. Alone, 8,192 rows, products of the library and, with what follows, these
+// (us): bias, 2,560 columns of depth 1,024, 33 and 35; SwiGLU, 5,056 of 1,024, 66 (+ 19 for the row kernel) and 61; residual,
+// 1,024 of 2,528, 33 (+ 14) and 43; gate, 1,024 of 2,048, 27 (+ 21) and 42; 16,384 rows: gate 51 (+ 37) and 74, gradient of the
+// norm, 2,048 of 1,024, 59 (+ 36) and 56.
+//
+// What bounds them. Products of many tiles the tensor cores, at the clock that power leaves (1.4 to 1.5 GHz in a prefill).
+// Those of two tiles a pair (1,024 columns, 8,192 rows) one tile's products, the other's, of which the epilogue of the first is
+// in the shadow, and the epilogue of the second: in cycles for the gate 22,500, 23,000 and 13,500, for the residual 24,500, 26,000
+// and 7,500. What the epilogue's own cycles go to, gate, per tile: arithmetic 7,000 (4,000 of them special functions), waiting
+// for the inputs 8,000 (2,000 in the last tile), for the buffer to be read and the stores to be issued 5,500.
+// With every access to global memory by the epilogue's lanes (rows of 64 or 128 bytes, through shared memory to turn
+// them) the gate took 24,000 and 20,000 cycles, the residual 15,000 and 11,500, SwiGLU 8,700 of a tile's 8,200 of products
+// (50, 45 and 65 us): the loads and stores were issued at the rate of the addresses that they touch, not waited for.
 //
 // A pair of thread blocks (cluster of two, cta_group::2) computes tiles of 256 x NT: each block holds 128 rows of a
 // and NT / 2 rows of b, so that an operand byte fetched from L2 serves twice the products of a single block.
@@ -33,6 +41,7 @@ namespace fields {
 
 constexpr int kProductWarps = 8;     // of the epilogue; loads and products: a warp each
 constexpr int kProductRows = 128;     // of a block; a tile is twice as high
+constexpr int kProductColumns = 128;  // of a tile that a warp of the epilogue does, at the most
 
 struct ProductParams {
     long long M;
@@ -40,47 +49,100 @@ struct ProductParams {
     int tiles_n, pairs;
     long long tiles;
     // (what an epilogue does not use is null)
-    const float* x;          // [M, N]
     const uint16_t* bias16;  // [N]
     const float *bias, *gate_bias;  // [N]
-    const uint16_t* gate;    // rows of gate_pitch
-    long long gate_pitch;
     const float* sums;       // [M, entries] sums of squares behind rstd = rsqrt(sum * inv_features + eps)
     int entries;
     float inv_features, eps;
     const float* row;        // [M] factor of a row
-    const uint16_t* read;    // [M, N]
-    float* y;                // [M, N] (may be x)
-    uint16_t* h;             // [M, N], or rows of h_pitch
-    long long h_pitch;
     float* sums_out;         // [M, ceil(N / 32)]: a warp's columns in the first of their entries, zero in the other
+    // The bfloat16 tensors beside the matrix, for rows that TMA does not address (`direct`), and h and acc where both
+    // are wanted: in16 is gate or read, h the output.
+    int direct;
+    const uint16_t* in16;
+    long long in_pitch;
+    uint16_t* h;
+    long long h_pitch;
     uint16_t* acc;           // [M, N]
+    int has_h, has_acc;      // whether h, and whether acc, is wanted at all
+};
+// Operands, and the tensors of the epilogue in boxes of 32 rows: x and y fp32, in16 gate or read, out16 h (or acc where no h is
+// wanted).
+struct alignas(64) ProductMaps {
+    CUtensorMap a, b, x, y, in16, out16;
 };
 
-// Tensors from the first row and column of a warp's part of a tile on.
-struct ProductBase {
-    const float* x;
-    float* y;
-    uint16_t *h, *acc;
-    const uint16_t *gate, *read;
-};
-
-// A lane's four columns of a row. Column holds what they need whatever the row (`col` counts in the matrix), Loaded what
-// they need of the row, `factor` is a value of the row; run() does the rest and returns their sum of squares. Offsets
-// count from the ProductBase: `at` in [M, N], `gate_at` and `h_at` in the tensors with a pitch. A piece is kPiece columns.
-struct ProductBias {
-    static constexpr int kPiece = 32;
-    static constexpr bool kSums = false, kSwiglu = false;
-    using Column = Vec<4>;
-    struct Loaded {};
-    __device__ static Column column(const ProductParams& p, int col) { return load4(p.bias16 + col); }
-    __device__ static float factor(const ProductParams&, long long) { return 1.0f; }
-    __device__ static void load(const ProductBase&, int, int, Loaded&) {}
-    __device__ static float run(const ProductBase& b, int, int h_at, Vec<4> v, float, const Column& bias, const Loaded&) {
+// A row's part of a 16-byte unit in a box of 32 rows as TMA writes it with the swizzle of that row length: eight neighbouring
+// rows' units of one column lie in different banks, so a lane per row reads and writes them at full rate.
+template <int ROW_BYTES>
+__device__ __forceinline__ unsigned product_unit(int row, int u) {
+    static_assert(ROW_BYTES == 128 || ROW_BYTES == 64, "swizzles");
+    return (unsigned)(row * ROW_BYTES + ((u ^ (ROW_BYTES == 128 ? row & 7 : row >> 1 & 3)) << 4));
+}
+__device__ __forceinline__ uint4 lds16(unsigned addr) {
+    uint4 r;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(addr) : "memory");
+    return r;
+}
+__device__ __forceinline__ void sts16(unsigned addr, const uint4& v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// Eight bfloat16 values of a row in global memory that may lie on 8 bytes only, the second four where they exist.
+__device__ __forceinline__ uint4 load_halves(const uint16_t* p, bool second) {
+    const uint2 a = *reinterpret_cast<const uint2*>(p);
+    const uint2 b = second ? *reinterpret_cast<const uint2*>(p + 4) : make_uint2(0u, 0u);
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store_halves(uint16_t* p, const uint4& v, bool second) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(v.x, v.y);
+    if (second) *reinterpret_cast<uint2*>(p + 4) = make_uint2(v.z, v.w);
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+    uint4 r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.x) : "f"(v[1]), "f"(v[0]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.y) : "f"(v[3]), "f"(v[2]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.z) : "f"(v[5]), "f"(v[4]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.w) : "f"(v[7]), "f"(v[6]));
+    return r;
+}
+__device__ __forceinline__ void unpack8(const uint4& w, float* v) {
+    const Vec<4> a = bf16x4_unpack(w.x, w.y), b = bf16x4_unpack(w.z, w.w);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v.v[k] += bias.v[k];
-        store_bf16x4(b.h + h_at, v);
-        return 0.0f;
+    for (int k = 0; k < 4; ++k) { v[k] = a.v[k]; v[4 + k] = b.v[k]; }
+}
+__device__ __forceinline__ uint4 float_bits(const float* v) {
+    return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+}
+__device__ __forceinline__ void bits_float(const uint4& w, float* v) {
+    v[0] = __uint_as_float(w.x); v[1] = __uint_as_float(w.y); v[2] = __uint_as_float(w.z); v[3] = __uint_as_float(w.w);
+}
+
+// An epilogue. run() does eight columns of a row, `at` counted in the warp's: of the product in v, of fp32 input in x (then
+// output), of bfloat16 input in `in`. Leaves fp32 output in x, bfloat16 output in v.
+//   kF32     fp32 input and output      kIn   bfloat16 input      kChunk   columns between two exchanges with memory
+//   keep     constants of four columns of a tile, by the lane of those columns, `to` its place in shared memory
+struct ProductBias {
+    static constexpr bool kDependents = false;
+    static constexpr int kChunk = 64;
+    static constexpr bool kF32 = false, kIn = false, kScaled = false, kSums = false, kSwiglu = false, kAcc = false;
+    __device__ static float factor(const ProductParams&, long long) { return 1.0f; }
+    // A lane keeps four columns' biases, and all take them from there: a load of the same address by all lanes is as slow as
+    // any (5,000 cycles of a tile's epilogue against 3,300).
+    using Kept = uint2;
+    static constexpr int kConstants = 0;
+    __device__ static Kept keep(const ProductParams& p, int col, bool here, float*) {
+        return here ? *reinterpret_cast<const uint2*>(p.bias16 + col) : make_uint2(0u, 0u);
+    }
+    __device__ static void run(const Kept& kept, const float*, int at, float* v, float*, const float*, float, F2&) {
+        uint4 w;
+        w.x = __shfl_sync(0xffffffffu, kept.x, at / 4);
+        w.y = __shfl_sync(0xffffffffu, kept.y, at / 4);
+        w.z = __shfl_sync(0xffffffffu, kept.x, at / 4 + 1);
+        w.w = __shfl_sync(0xffffffffu, kept.y, at / 4 + 1);
+        float b[8];
+        unpack8(w, b);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] += b[k];
     }
 };
 // rsqrt of the mean of a row's squares. (The loads of a row go out together: one by one, 32 entries took longer than the
@@ -103,93 +165,98 @@ __device__ __forceinline__ float product_rstd(const ProductParams& p, long long 
     return rsqrtf(sum * p.inv_features + p.eps);
 }
 struct ProductGate {
-    static constexpr int kPiece = 16;  // (two pieces' inputs are in registers)
-    static constexpr bool kSums = true, kSwiglu = false;
-    struct Column {
-        Vec<4> b, gb;
-    };
-    struct Loaded {
-        Vec<4> x;
-        uint2 gate;
-    };
-    __device__ static Column column(const ProductParams& p, int col) { return Column{load4(p.bias + col), load4(p.gate_bias + col)}; }
+    static constexpr bool kDependents = true;
+    static constexpr int kChunk = 32;
+    static constexpr bool kF32 = true, kIn = true, kSums = true, kSwiglu = false, kAcc = true;
     __device__ static float factor(const ProductParams& p, long long row) { return product_rstd(p, row); }
-    __device__ static void load(const ProductBase& b, int at, int gate_at, Loaded& l) {
-        l.x = load4(b.x + at);
-        l.gate = *reinterpret_cast<const uint2*>(b.gate + gate_at);
+    // Both biases of a warp's columns wait in shared memory (loaded by all lanes from the same address where they are needed,
+    // arithmetic took 11,500 cycles of a tile instead of 7,700).
+    struct Kept {};
+    static constexpr int kConstants = 2;  // floats per column
+    __device__ static Kept keep(const ProductParams& p, int col, bool here, float* to) {
+        const Vec<4> b = here ? load4(p.bias + col) : vec_fill<4>(0.0f), gb = here ? load4(p.gate_bias + col) : vec_fill<4>(0.0f);
+        vec_store<4>(to, b);
+        vec_store<4>(to + kProductColumns, gb);
+        return {};
     }
-    __device__ static float run(const ProductBase& b, int at, int h_at, Vec<4> v, float rstd, const Column& c, const Loaded& l) {
-        if (b.acc) store_bf16x4(b.acc + at, v);
-        const Vec<4> gate = bf16x4_unpack(l.gate.x, l.gate.y);
-        float sq = 0.0f;
+    __device__ static void run(const Kept&, const float* constants, int at, float* v, float* x, const float* in, float rstd, F2& sq) {
+        const F2* b = reinterpret_cast<const F2*>(constants + at);
+        const F2* gb = reinterpret_cast<const F2*>(constants + kProductColumns + at);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            v.v[k] = l.x.v[k] + (v.v[k] * rstd + c.b.v[k]) * sigmoidf_fast(gate.v[k] + c.gb.v[k]);
-            sq += v.v[k] * v.v[k];
+        for (int k = 0; k < 8; k += 2) {
+            const F2 g = sigmoid2(add2(F2{in[k], in[k + 1]}, gb[k / 2]));
+            const F2 y = fma2(fma2(F2{v[k], v[k + 1]}, splat2(rstd), b[k / 2]), g, F2{x[k], x[k + 1]});
+            sq = fma2(y, y, sq);
+            x[k] = v[k] = y.x;
+            x[k + 1] = v[k + 1] = y.y;
         }
-        vec_store<4>(b.y + at, v);
-        if (b.h) store_bf16x4(b.h + h_at, v);
-        return sq;
     }
 };
 struct ProductSwiglu {
-    static constexpr int kPiece = 32;
-    static constexpr bool kSums = false, kSwiglu = true;
-    struct Column {};
-    struct Loaded {};
+    static constexpr bool kDependents = true;
+    static constexpr int kChunk = 64;
+    static constexpr bool kF32 = false, kIn = false, kSums = false, kSwiglu = true, kAcc = false;
+    struct Kept {};
+    static constexpr int kConstants = 0;
+    __device__ static Kept keep(const ProductParams&, int, bool, float*) { return {}; }
     __device__ static float factor(const ProductParams& p, long long row) { return product_rstd(p, row); }
+    // (sixteen columns: u of eight features, then v of the same)
+    __device__ static void run(float* v, float rstd) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float us = v[k] * rstd;
+            v[k] = us * sigmoidf_fast(us) * (v[8 + k] * rstd);
+        }
+    }
 };
 struct ProductResidual {
-    static constexpr int kPiece = 32;
-    static constexpr bool kSums = false, kSwiglu = false;
-    struct Column {};
-    struct Loaded {
-        Vec<4> x;
-    };
-    __device__ static Column column(const ProductParams&, int) { return {}; }
+    static constexpr bool kDependents = true;
+    static constexpr int kChunk = 32;
+    static constexpr bool kF32 = true, kIn = false, kSums = false, kSwiglu = false, kAcc = false;
+    struct Kept {};
+    static constexpr int kConstants = 0;
+    __device__ static Kept keep(const ProductParams&, int, bool, float*) { return {}; }
     __device__ static float factor(const ProductParams&, long long) { return 1.0f; }
-    __device__ static void load(const ProductBase& b, int at, int, Loaded& l) { l.x = load4(b.x + at); }
-    __device__ static float run(const ProductBase& b, int at, int h_at, Vec<4> v, float, const Column&, const Loaded& l) {
+    __device__ static void run(const Kept&, const float*, int, float* v, float* x, const float*, float, F2&) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v.v[k] += l.x.v[k];
-        vec_store<4>(b.y + at, v);
-        if (b.h) store_bf16x4(b.h + h_at, v);
-        return 0.0f;
+        for (int k = 0; k < 8; ++k) v[k] = x[k] += v[k];
     }
 };
 struct ProductNormGrad {
-    static constexpr int kPiece = 32;
-    static constexpr bool kSums = false, kSwiglu = false;
-    struct Column {};
-    struct Loaded {
-        uint2 r;
-    };
-    __device__ static Column column(const ProductParams&, int) { return {}; }
+    static constexpr bool kDependents = false;
+    static constexpr int kChunk = 64;
+    static constexpr bool kF32 = false, kIn = true, kSums = false, kSwiglu = false, kAcc = false;
+    struct Kept {};
+    static constexpr int kConstants = 0;
+    __device__ static Kept keep(const ProductParams&, int, bool, float*) { return {}; }
     __device__ static float factor(const ProductParams& p, long long row) { return 2.0f * p.row[row]; }
-    __device__ static void load(const ProductBase& b, int at, int, Loaded& l) { l.r = *reinterpret_cast<const uint2*>(b.read + at); }
-    __device__ static float run(const ProductBase& b, int, int h_at, Vec<4> v, float c, const Column&, const Loaded& l) {
-        const Vec<4> r = bf16x4_unpack(l.r.x, l.r.y);
+    __device__ static void run(const Kept&, const float*, int, float* v, float*, const float* in, float c, F2&) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v.v[k] += c * r.v[k];
-        store_bf16x4(b.h + h_at, v);
-        return 0.0f;
+        for (int k = 0; k < 8; ++k) v[k] += c * in[k];
     }
 };
 
-template <int NT>
+template <class Epi, int NT>
 struct ProductShape {
     static constexpr int kBox = 64;  // of K
     static constexpr int kABytes = kProductRows * kBox * 2, kBBytes = NT / 2 * kBox * 2, kStageBytes = kABytes + kBBytes;
-    // As many stages as there is space for beside 32 rows x 256 columns of pieces: under load a copy takes some 3,000
-    // cycles to arrive, the products of a stage 512. With five stages instead of six the products of a tile of depth
-    // 2,528 took 26,000 cycles instead of 20,900, with four those of depth 2,048 29,000 instead of 17,000.
-    static constexpr int kPiecesBytes = 32 * 1024;
-    static constexpr int kStages = (227 * 1024 - 1024 - 256 - kPiecesBytes) / kStageBytes;
-    static constexpr int kBars = 2 * kStages + 4;
-    static constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + kPiecesBytes + kBars * 8 + 16;
-    static constexpr unsigned kColumns = 2 * NT;  // of tensor memory
+    // A warp's share of a tile: 32 rows x kColumns, in chunks that pass through a buffer of its own: fp32 rows of 128 bytes and
+    // behind them bfloat16 rows of kHalfRow bytes.
+    static constexpr int kColumns = NT / (kProductWarps / 4), kChunk = Epi::kChunk, kChunks = kColumns / kChunk;
+    static constexpr int kHalfColumns = Epi::kSwiglu ? kChunk / 2 : kChunk, kHalfRow = kHalfColumns * 2;
+    static constexpr int kF32Bytes = Epi::kF32 ? 32 * 128 : 0, kBufferBytes = kF32Bytes + 32 * kHalfRow;
+    // As many stages as there is space for beside the buffers. (The loop of products alone, 8,192 x 1,024: depth 2,048 28.4 us
+    // with six stages, 29.1 with five, 32.4 with four; depth 2,528 35.2, 36.5 and 41.9. Five stages beside buffers for h as well or
+    // six with h through the buffer of y, after it, are the same, 47 us.)
+    static constexpr int kConstBytes = Epi::kConstants * kProductColumns * 4;  // of a warp
+    static constexpr int kStages = (227 * 1024 - 1024 - 512 - kProductWarps * (kBufferBytes + kConstBytes)) / kStageBytes;
+    static constexpr int kLoads = Epi::kF32 || Epi::kIn ? kProductWarps * kChunks : 0;  // barriers of the inputs
+    static constexpr int kBars = 2 * kStages + 4 + kLoads;
+    static constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + kProductWarps * (kBufferBytes + kConstBytes) + kBars * 8 + 16;
+    static constexpr unsigned kTmem = 2 * NT;  // columns of tensor memory
     static_assert(kSmemBytes <= 227 * 1024, "shared memory of an SM");
     static_assert(NT == 256 || NT == 128, "tiles the tensor cores and the epilogue's warps take");
+    static_assert((kChunks - 1) * kProductWarps * kBufferBytes <= kStages * kStageBytes, "the last tile's inputs go where operands were");
 };
 
 // A load whose bytes count on a barrier of either block of the pair.
@@ -227,162 +294,212 @@ __device__ __forceinline__ void tmem_load32(unsigned addr, unsigned* r) {
         : "memory");
 }
 
-__device__ __forceinline__ Vec<4> vec_of(const float4& a) { return Vec<4>{{a.x, a.y, a.z, a.w}}; }
+__device__ __forceinline__ void tma_store2(const CUtensorMap* map, unsigned src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y),
+                 "r"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// A tile's share of one warp: 32 rows x NT / 2 columns of its block, a piece at a time. A lane has a row of
-// the product, and accesses to global memory want lanes along the rows, so a piece passes through shared memory.
-// What it needs besides is loaded into registers under the piece before it, that of the first under the product. (The
-// pieces are a loop, two at a time for the registers' sake: unrolled they are up to 77 KB of code, run at the rate at
-// which it is fetched. Loads of the next piece between the stores of this one made every row wait for all of them:
-// their scoreboards are shared.)
+// An epilogue warp: 32 rows x kColumns of every tile of its block. A lane has a row, as tensor memory gives it; what the row
+// needs from global memory comes, and what it leaves goes, by TMA through the warp's buffer in shared memory, the outputs in the
+// place of the inputs.
 template <class Epi, int NT>
-struct ProductTile {
-    using T = ProductShape<NT>;
-    static constexpr int kPiece = Epi::kPiece, kColumns = NT / (kProductWarps / 4), kPieces = kColumns / kPiece;
-    static constexpr int kUnits = kPiece / 4, kRows = 32 / kUnits;  // units of four columns; rows of a warp-wide access
-    static_assert(kPieces % 2 == 0, "pieces go in pairs");
-    struct Inputs {  // of a lane: its unit of kUnits rows
-        typename Epi::Column column;
-        typename Epi::Loaded row[kUnits];
-    };
+struct ProductWarp {
+    using T = ProductShape<Epi, NT>;
+    static constexpr int kChunks = T::kChunks;
+    static constexpr bool kLoads = Epi::kF32 || Epi::kIn;
     const ProductParams& p;
-    char* piece;
-    long long row0;
-    int col0, lane, rows;
-    ProductBase base;
-    float factor = 1.0f;  // of row0 + lane
-    float sq[kUnits];
-    Inputs even, odd;
+    const ProductMaps& maps;
+    unsigned own, ring, bars;  // the buffer; where the last tile's other chunks go; this warp's barriers, one per chunk
+    float* constants;          // of the tile's columns
+    int warp, lane;
+    bool leader, dead = false;
+    unsigned parity = 0;       // of the first barrier
 
-    __device__ ProductTile(const ProductParams& p, char* piece, long long row0, int col0)
-        : p(p), piece(piece), row0(row0), col0(col0), lane(threadIdx.x & 31),
-          rows(p.M - row0 < 32 ? (int)(p.M - row0) : 32) {
-        const long long at = row0 * p.N + col0;
-        base.x = p.x + at;
-        base.y = p.y + at;
-        base.read = p.read + at;
-        base.acc = p.acc ? p.acc + at : nullptr;
-        base.h = p.h ? p.h + row0 * p.h_pitch + (Epi::kSwiglu ? col0 / 2 : col0) : nullptr;
-        base.gate = p.gate + row0 * p.gate_pitch + col0;
-        load(0, even);
-        if (lane < rows) factor = Epi::factor(p, row0 + lane);
+    __device__ unsigned buffer(int c, bool last) const {
+        return last && c > 0 ? ring + (unsigned)(((c - 1) * kProductWarps + warp) * T::kBufferBytes) : own;
     }
-    __device__ int row_of(int i) const { return i * kRows + lane / kUnits; }
-    __device__ int col_of(int k) const { return k * kPiece + lane % kUnits * 4; }
-    __device__ void load(int k, Inputs& to) const {
-        if constexpr (!Epi::kSwiglu) {
-            const int col = col_of(k);
-            if (k >= kPieces || col0 + col >= p.N) return;
-            to.column = Epi::column(p, col0 + col);
-#pragma unroll
-            for (int i = 0; i < kUnits; ++i)
-                if (row_of(i) < rows) Epi::load(base, row_of(i) * p.N + col, row_of(i) * (int)p.gate_pitch + col, to.row[i]);
-        }
+    // Inputs of the 32 rows from row0 on and the chunk's columns from col on.
+    __device__ void load(unsigned buf, unsigned bar, long long row0, int col) const {
+        if (!leader || dead) return;
+        const bool in = Epi::kIn && !p.direct;
+        const int bytes = T::kF32Bytes + (in ? 32 * T::kHalfRow : 0);
+        if (bytes == 0) return;
+        mbar_expect(bar, (unsigned)bytes);
+        if constexpr (Epi::kF32) tma_load2(buf, &maps.x, col, (int)row0, bar);
+        if (in) tma_load2(buf + T::kF32Bytes, &maps.in16, col, (int)row0, bar);
     }
-    // 16 bytes of a row of the piece, permuted so that neither a lane per row nor lanes along the rows meet in a bank
-    __device__ float4* unit(int row, int u) const {
-        const int turn = kUnits == 8 ? row & 7 : row >> 1 & 3;
-        return reinterpret_cast<float4*>(piece + row * (kPiece * 4) + (u ^ turn) * 16);
-    }
-    // tmem: the warp's lanes and first column; released: where to say that they have been read
-    __device__ void one(int k, unsigned tmem, unsigned released, bool dead, const Inputs& use, Inputs& next) {
-        load(k + 1, next);
-        unsigned v[kPiece];
+    __device__ void buffer_read() const {  // what was sent from the buffer has left it
+        if (leader) bulk_wait_read();
         __syncwarp();
-        if constexpr (kPiece == 32) tmem_load32(tmem + (unsigned)(k * kPiece), v);
-        else tmem_load<kPiece>(tmem + (unsigned)(k * kPiece), v);
-        tmem_wait();
-        if (k + 1 == kPieces) {
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            // (at block scope: at cluster scope it waits for the warp's stores, 2,500 cycles, and orders nothing but
-            // tensor memory)
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(released) : "memory");
+    }
+    // 32 columns of the row, `k` of the chunk on, which begins at the warp's column `c0` and the matrix's column `col0`. (Loads,
+    // arithmetic and stores one after the other: in turns for eight columns the loads' latency was waited for four times,
+    // 7,700 cycles of a tile's gate against 6,700.)
+    __device__ void part(const typename Epi::Kept& kept, int k, unsigned buf, float* v, int row, bool in_rows, int c0, int col0,
+                         float factor, F2& sq) const {
+        constexpr int kUnits = Epi::kSwiglu ? 2 : 4, kWide = Epi::kSwiglu ? 16 : 8;  // units of eight bfloat16 columns
+        const int cols = Epi::kSwiglu ? p.N / 2 : p.N, hk = Epi::kSwiglu ? k / 2 : k, hcol = Epi::kSwiglu ? (col0 + k) / 2 : col0 + k;
+        auto half_at = [&](int j) { return buf + T::kF32Bytes + product_unit<T::kHalfRow>(lane, hk / 8 + j); };
+        auto inside = [&](int j) { return in_rows && hcol + 8 * j < cols; };
+        auto second = [&](int j) { return hcol + 8 * j + 4 < cols; };
+        float x[Epi::kF32 ? 32 : 1];
+        uint4 in[Epi::kIn ? kUnits : 1], acc[Epi::kAcc ? kUnits : 1];
+        if constexpr (Epi::kF32) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bits_float(lds16(buf + product_unit<128>(lane, k / 4 + j)), x + 4 * j);
         }
-        if (dead) {
+        if constexpr (Epi::kIn) {
 #pragma unroll
-            for (int i = 0; i < kPiece; ++i) v[i] = ~0u;  // NaN
+            for (int j = 0; j < kUnits; ++j) {
+                in[j] = make_uint4(0u, 0u, 0u, 0u);
+                if (!p.direct) in[j] = lds16(half_at(j));
+                else if (inside(j)) in[j] = load_halves(p.in16 + (long long)row * p.in_pitch + hcol + 8 * j, second(j));
+            }
         }
 #pragma unroll
-        for (int i = 0; i < kUnits; ++i)
-            *unit(lane, i) = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                         __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-        __syncwarp();
-        if constexpr (Epi::kSwiglu) {
-            // columns: u of eight features, v of the same; a lane takes four features of a row
-            const int j = lane % 4, at = j / 2 * 4 + j % 2, f = k * (kPiece / 2) + j * 4;
+        for (int j = 0; j < kUnits; ++j) {
+            float* w = v + j * kWide;
+            if constexpr (Epi::kSwiglu) {
+                Epi::run(w, factor);
+            } else {
+                float u[8];
+                if constexpr (Epi::kIn) unpack8(in[j], u);
+                if constexpr (Epi::kAcc) acc[j] = pack8(w);
+                Epi::run(kept, constants, c0 + k + 8 * j, w, x + (Epi::kF32 ? 8 * j : 0), u, factor, sq);
+            }
+        }
+        if constexpr (Epi::kF32) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int rl = i * 8 + lane / 4;
-                const float rs = __shfl_sync(0xffffffffu, factor, rl);
-                const Vec<4> u = vec_of(*unit(rl, at)), w = vec_of(*unit(rl, at + 2));
-                Vec<4> a;
+            for (int j = 0; j < 8; ++j) sts16(buf + product_unit<128>(lane, k / 4 + j), float_bits(x + 4 * j));
+        }
+        if constexpr (Epi::kAcc) {
+            if (p.has_acc) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float us = u.v[e] * rs;
-                    a.v[e] = us * sigmoidf_fast(us) * (w.v[e] * rs);
+                for (int j = 0; j < kUnits; ++j) {
+                    if (!p.direct && !p.has_h) sts16(half_at(j), acc[j]);
+                    else if (inside(j)) store_halves(p.acc + (long long)row * p.N + hcol + 8 * j, acc[j], second(j));
                 }
-                if (rl < rows && col0 / 2 + f < p.N / 2) store_bf16x4(base.h + rl * (int)p.h_pitch + f, a);
             }
-        } else {
-            const int col = col_of(k);
-            Vec<4> a[kUnits];
+        }
+        if (p.has_h) {
 #pragma unroll
-            for (int i = 0; i < kUnits; ++i) a[i] = vec_of(*unit(row_of(i), lane % kUnits));
-#pragma unroll
-            for (int i = 0; i < kUnits; ++i) {
-                const float f = __shfl_sync(0xffffffffu, factor, row_of(i));
-                if (row_of(i) < rows && col0 + col < p.N)
-                    sq[i] += Epi::run(base, row_of(i) * p.N + col, row_of(i) * (int)p.h_pitch + col, a[i], f, use.column, use.row[i]);
+            for (int j = 0; j < kUnits; ++j) {
+                const uint4 t = pack8(v + j * kWide);
+                if (!p.direct) sts16(half_at(j), t);
+                else if (inside(j)) store_halves(p.h + (long long)row * p.h_pitch + hcol + 8 * j, t, second(j));
             }
         }
     }
-    __device__ void finish(unsigned tmem, unsigned released, bool dead) {
+    // A tile: tmem is the warp's lanes and first column, acc_full is done where the product is, released where to say that
+    // it has been read.
+    __device__ void tile(long long row0, int col0, bool last, unsigned tmem, unsigned acc_full, unsigned acc_parity, unsigned released) {
+        const int left = p.M - row0 < 32 ? (int)(p.M - row0) : 32, row = (int)row0 + lane;
+        const bool in_rows = lane < left, any = left > 0 && col0 < p.N;
+        if (kLoads) {
+            buffer_read();
+            if (any) load(own, bars, row0, col0);
+        }
+        const float factor = in_rows ? Epi::factor(p, row) : 1.0f;
+        const typename Epi::Kept kept =
+            Epi::keep(p, col0 + lane * 4, lane * 4 < T::kColumns && col0 + lane * 4 < p.N, constants + lane * 4);
+        F2 sq = splat2(0.0f);
+        mbar_wait_local(acc_full, acc_parity, dead);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // (all operands of the last tile have been read: there is space for the inputs of its other chunks)
+        last = last && !__any_sync(0xffffffffu, dead);
+        if (kLoads && last)
 #pragma unroll
-        for (int i = 0; i < kUnits; ++i) sq[i] = 0.0f;
+            for (int c = 1; c < kChunks; ++c)
+                if (any && col0 + c * T::kChunk < p.N) load(buffer(c, true), bars + c * 8, row0, col0 + c * T::kChunk);
 #pragma unroll 1
-        for (int k = 0; k < kPieces; k += 2) {
-            one(k, tmem, released, dead, even, odd);
-            one(k + 1, tmem, released, dead, odd, even);
+        for (int c = 0; c < kChunks; ++c) {
+            const int col = col0 + c * T::kChunk;
+            const bool here = any && col < p.N;
+            const unsigned buf = buffer(c, last);
+            if (!kLoads) {
+                if (here) buffer_read();
+            } else if (c > 0 && !last && here) {
+                buffer_read();
+                load(own, bars, row0, col);
+            }
+            if (here && kLoads && (Epi::kF32 || !p.direct)) {
+                if (last && c > 0) {
+                    mbar_wait_local(bars + c * 8, 0, dead);
+                } else {
+                    mbar_wait_local(bars, parity, dead);
+                    parity ^= 1;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < T::kChunk; k += 32) {
+                unsigned v[32];
+                tmem_load32(tmem + (unsigned)(c * T::kChunk + k), v);
+                tmem_wait();
+                if (c + 1 == kChunks && k + 32 == T::kChunk) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    // (at block scope: at cluster scope it waits for the warp's stores, 2,500 cycles, and orders nothing but
+                    // tensor memory)
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(released) : "memory");
+                }
+                float f[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) f[i] = dead ? nanf("") : __uint_as_float(v[i]);
+                if (here) part(kept, k, buf, f, row, in_rows, c * T::kChunk, col, factor, sq);
+                __syncwarp();
+            }
+            if (here) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (leader) {
+                    if constexpr (Epi::kF32) tma_store2(&maps.y, buf, col, (int)row0);
+                    if (!p.direct && (p.has_h || p.has_acc))
+                        tma_store2(&maps.out16, buf + T::kF32Bytes, Epi::kSwiglu ? col / 2 : col, (int)row0);
+                    bulk_commit();
+                }
+            }
         }
         if constexpr (Epi::kSums) {
-            if (!p.sums_out) return;
-            const int entries = (p.N + 31) / 32, at = col0 / 32 + lane % kUnits;
+            const int entries = (p.N + 31) / 32;
+            if (p.sums_out && in_rows)
 #pragma unroll
-            for (int i = 0; i < kUnits; ++i) {
-#pragma unroll
-                for (int off = kUnits / 2; off > 0; off >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], off);
-                if (lane % kUnits < kColumns / 32 && row_of(i) < rows && at < entries)
-                    p.sums_out[(row0 + row_of(i)) * entries + at] = lane % kUnits ? 0.0f : sq[i];
-            }
+                for (int i = 0; i < T::kColumns / 32; ++i)
+                    if (col0 / 32 + i < entries) p.sums_out[(long long)row * entries + col0 / 32 + i] = i ? 0.0f : sq.x + sq.y;
         }
     }
 };
 
 template <class Epi, int NT>
 __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
-    pair_product(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
-                 const __grid_constant__ ProductParams p) {
-    using T = ProductShape<NT>;
+    pair_product(const __grid_constant__ ProductMaps maps, const __grid_constant__ ProductParams p) {
+    using T = ProductShape<Epi, NT>;
     extern __shared__ __align__(1024) char product_smem[];
     char* ring = product_smem + (1024 - (smem_addr(product_smem) & 1023)) % 1024;
-    char* pieces = ring + T::kStages * T::kStageBytes;
-    char* tail = pieces + T::kPiecesBytes;
+    char* buffers = ring + T::kStages * T::kStageBytes;
+    char* constants = buffers + kProductWarps * T::kBufferBytes;
+    char* tail = constants + kProductWarps * T::kConstBytes;
     // loads have landed (both blocks', on the first block's barriers); stage free, accumulator full (each block's own);
-    // accumulator free (the first block's)
+    // accumulator free (the first block's); inputs of the epilogue have landed
     const unsigned full = smem_addr(tail), empty = full + T::kStages * 8, acc_full = empty + T::kStages * 8,
-                   acc_free = acc_full + 16;
+                   acc_free = acc_full + 16, loaded = acc_free + 16;
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(tail + T::kBars * 8);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), rank = (int)cluster_rank();
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2 * T::kStages + 2; ++i) mbar_init(full + i * 8, 1);
         for (int i = 0; i < 2; ++i) mbar_init(acc_free + i * 8, 2 * kProductWarps);
+        for (int i = 0; i < T::kLoads; ++i) mbar_init(loaded + i * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kProductWarps) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
-                     "r"(T::kColumns)
+                     "r"(T::kTmem)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -392,22 +509,28 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Every block runs from the start: those of the next kernel take the places of the first that end, and set themselves up
+    // (prefill of 4 x 500 tokens through 8 blocks of d_model 512 494 -> 472 us, of 8 x 1,024 through 18 of 1,024 4,258 -> 4,219).
+    // Where the next kernel is a product, that is where it reads h: the blocks of a recurrence or of a row kernel then lie on
+    // few SMs (mixer of 8 x 2,048 567 -> 584 us with all products, 546 -> 551 with those two).
+    if (Epi::kDependents && p.has_h) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const long long first = blockIdx.x / 2;
     bool dead = false;
-    static_assert(kProductWarps * 32 * Epi::kPiece * 4 <= T::kPiecesBytes, "space for the pieces");
     if (warp < kProductWarps) {
-        const unsigned lanes = tmem + ((unsigned)(warp % 4 * 32) << 16) + (unsigned)(warp / 4 * ProductTile<Epi, NT>::kColumns);
+        ProductWarp<Epi, NT> w{p, maps, smem_addr(buffers + warp * T::kBufferBytes), smem_addr(ring),
+                               loaded + (unsigned)(T::kLoads ? warp * T::kChunks * 8 : 0),
+                               reinterpret_cast<float*>(constants + warp * T::kConstBytes), warp, (int)threadIdx.x & 31, elect_one()};
+        const unsigned lanes = tmem + ((unsigned)(warp % 4 * 32) << 16) + (unsigned)(warp / 4 * T::kColumns);
         unsigned n = 0;
         for (long long t = first; t < p.tiles; t += p.pairs, ++n) {
             const unsigned buf = n & 1;
-            ProductTile<Epi, NT> tile(p, pieces + warp * (32 * Epi::kPiece * 4), t / p.tiles_n * (2 * kProductRows) + rank * kProductRows + warp % 4 * 32,
-                                      (int)(t % p.tiles_n) * NT + warp / 4 * ProductTile<Epi, NT>::kColumns);
-            mbar_wait_local(acc_full + buf * 8, n / 2 & 1, dead);
-            __syncwarp();
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tile.finish(lanes + buf * NT, peer_addr(acc_free + buf * 8, 0), dead);
+            w.tile(t / p.tiles_n * (2 * kProductRows) + rank * kProductRows + warp % 4 * 32,
+                   (int)(t % p.tiles_n) * NT + warp / 4 * T::kColumns, t + p.pairs >= p.tiles, lanes + buf * NT, acc_full + buf * 8,
+                   n / 2 & 1, peer_addr(acc_free + buf * 8, 0));
         }
+        if (w.leader) bulk_wait_all();
+        dead = w.dead;
     } else if (warp == kProductWarps) {
         if (elect_one()) {
             StepRing<T::kStages> r;
@@ -419,8 +542,8 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
                     if (dead) break;
                     if (rank == 0) mbar_expect(full + r.slot * 8, 2 * T::kStageBytes);
                     const unsigned bar = peer_addr(full + r.slot * 8, 0), at = smem_addr(ring + r.slot * T::kStageBytes);
-                    tma_load2_pair(at, &a_map, i * T::kBox, m0, bar);
-                    tma_load2_pair(at + T::kABytes, &b_map, i * T::kBox, n0, bar);
+                    tma_load2_pair(at, &maps.a, i * T::kBox, m0, bar);
+                    tma_load2_pair(at + T::kABytes, &maps.b, i * T::kBox, n0, bar);
                     r.next();
                 }
             }
@@ -462,7 +585,7 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
     cluster_sync_all();  // no arrivals at a block that has left
     if (warp == kProductWarps) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kColumns) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kTmem) : "memory");
     }
 }
 

@@ -2218,15 +2218,36 @@ static bool operand_map(CUtensorMap* map, const void* base, long long rows, int 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A matrix of fp32 or bfloat16 in boxes of 32 rows x box_cols columns, of 128 or 64 bytes, with the swizzle of that length.
+static bool box_map(CUtensorMap* map, const void* base, long long rows, int cols, long long pitch, int box_cols, bool f32) {
+    const EncodeTiled encode = encode_tiled();
+    if (!encode) return false;
+    const int size = f32 ? 4 : 2;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch * size};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, 32}, ones[2] = {1, 1};
+    return encode(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
+                  strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  box_cols * size == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <class Epi, int NT>
 static int launch_product(const struct fields_product_args& g, ProductParams p, int pairs, Stream st) {
-    using T = ProductShape<NT>;
+    using T = ProductShape<Epi, NT>;
     p.k_blocks = (g.depth + T::kBox - 1) / T::kBox;
     p.tiles_n = (p.N + NT - 1) / NT;
     p.tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * p.tiles_n;
-    CUtensorMap a_map, b_map;
-    if (!operand_map(&a_map, g.a, p.M, g.depth, kProductRows) || !operand_map(&b_map, g.b, p.N, g.depth, NT / 2))
-        return FIELDS_ERR_UNSUPPORTED;
+    ProductMaps maps;
+    std::memset(&maps, 0, sizeof(maps));
+    bool ok = operand_map(&maps.a, g.a, p.M, g.depth, kProductRows) && operand_map(&maps.b, g.b, p.N, g.depth, NT / 2);
+    if (Epi::kF32) ok = ok && box_map(&maps.x, g.x, p.M, p.N, p.N, T::kChunk, true) && box_map(&maps.y, g.y, p.M, p.N, p.N, T::kChunk, true);
+    if (!p.direct) {
+        if (Epi::kIn) ok = ok && box_map(&maps.in16, p.in16, p.M, p.N, p.in_pitch, T::kHalfColumns, false);
+        if (p.has_h) ok = ok && box_map(&maps.out16, p.h, p.M, Epi::kSwiglu ? p.N / 2 : p.N, p.h_pitch, T::kHalfColumns, false);
+        else if (p.has_acc) ok = ok && box_map(&maps.out16, p.acc, p.M, p.N, p.N, T::kHalfColumns, false);
+    }
+    if (!ok) return FIELDS_ERR_UNSUPPORTED;
     static bool ready[64] = {};
     const int rc = allow_shared_memory(pair_product<Epi, NT>, T::kSmemBytes, ready);
     if (rc) return rc;
@@ -2244,7 +2265,7 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = dependent_launch_enabled() ? 2 : 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, pair_product<Epi, NT>, a_map, b_map, p));
+    return check_cuda(cudaLaunchKernelEx(&cfg, pair_product<Epi, NT>, maps, p));
 }
 
 // Tiles of 256 or of 128 columns: by the rounds of tiles that a pair takes, each as long as its columns and about 64 more
@@ -2514,28 +2535,33 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
     ProductParams p{};
     auto h = [](const void* q) { return static_cast<const uint16_t*>(q); };
     p.M = g->rows; p.N = g->cols;
-    p.x = g->x; p.bias16 = h(g->bias16); p.bias = g->bias; p.gate_bias = g->gate_bias; p.gate = h(g->gate);
-    p.gate_pitch = gate_pitch; p.sums = g->sums; p.entries = g->entries;
+    const bool gated = kind == FIELDS_PRODUCT_GATE;
+    p.bias16 = h(g->bias16); p.bias = g->bias; p.gate_bias = g->gate_bias;
+    p.sums = g->sums; p.entries = g->entries;
     p.inv_features = g->features > 0 ? 1.0f / (float)g->features : 0.0f; p.eps = g->eps;
-    p.row = g->row; p.read = h(g->read); p.y = g->y; p.h = static_cast<uint16_t*>(g->h); p.h_pitch = h_pitch;
-    p.sums_out = g->sums_out; p.acc = static_cast<uint16_t*>(g->acc);
+    p.row = g->row; p.sums_out = g->sums_out;
+    p.in16 = h(gated ? g->gate : g->read); p.in_pitch = gated ? gate_pitch : p.N;
+    p.h = static_cast<uint16_t*>(g->h); p.h_pitch = h_pitch; p.acc = static_cast<uint16_t*>(g->acc);
+    p.has_h = p.h != nullptr; p.has_acc = gated && p.acc;
+    p.direct = !aligned16(p.in16) || p.in_pitch % 8 || (p.has_h && (!aligned16(p.h) || h_pitch % 8)) ||
+               (p.has_acc && !p.has_h && (!aligned16(p.acc) || p.N % 8));
     Stream st = reinterpret_cast<Stream>(stream);
     switch (kind) {
         case FIELDS_PRODUCT_BIAS:
             if (!p.bias16 || !p.h) return FIELDS_ERR_ARGUMENT;
             return run_product<ProductBias>(*g, p, st);
         case FIELDS_PRODUCT_GATE:
-            if (!p.x || !p.bias || !p.gate_bias || !p.gate || !p.sums || p.entries <= 0 || g->features <= 0 || !p.y)
+            if (!g->x || !p.bias || !p.gate_bias || !p.in16 || !p.sums || p.entries <= 0 || g->features <= 0 || !g->y)
                 return FIELDS_ERR_ARGUMENT;
             return run_product<ProductGate>(*g, p, st);
         case FIELDS_PRODUCT_SWIGLU:
             if (!p.sums || p.entries <= 0 || g->features <= 0 || !p.h || p.N % 16) return FIELDS_ERR_ARGUMENT;
             return run_product<ProductSwiglu>(*g, p, st);
         case FIELDS_PRODUCT_RESIDUAL:
-            if (!p.x || !p.y) return FIELDS_ERR_ARGUMENT;
+            if (!g->x || !g->y) return FIELDS_ERR_ARGUMENT;
             return run_product<ProductResidual>(*g, p, st);
         case FIELDS_PRODUCT_NORM_GRAD:
-            if (!p.read || !p.row || !p.h) return FIELDS_ERR_ARGUMENT;
+            if (!p.in16 || !p.row || !p.h) return FIELDS_ERR_ARGUMENT;
             return run_product<ProductNormGrad>(*g, p, st);
     }
     return FIELDS_ERR_ARGUMENT;

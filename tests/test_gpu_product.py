@@ -125,6 +125,51 @@ def test_pitches(kind):
         assert rc != 0 and bool(h.isnan().all()), pitches
 
 
+# one row, the edges of a warp's 32 rows and of its 32 or 64 columns, several tiles of a pair
+@pytest.mark.parametrize("kind", range(5))
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (33, 80, 72), (97, 272, 200), (12000, 1040, 72)])
+def test_rows_that_tma_does_not_address(kind, M, N, K):
+    """bfloat16 rows that lie on 8 bytes only give the same bits as aligned ones; so do N - 4 columns, and acc without h."""
+    torch.manual_seed(M + kind)
+    lib = _lib.load()
+
+    def rand(*shape):
+        return torch.randn(*shape, device="cuda")
+
+    whole = dict(a=rand(M, K).bfloat16(), b=rand(N, K).bfloat16(), bias16=rand(N).bfloat16(), x=rand(M, N), bias=rand(N),
+                 gate_bias=rand(N), gate=rand(M, N).bfloat16(), sums=rand(M, 3).square(), read=rand(M, N).bfloat16(), row=rand(M))
+
+    def call(n, shift, h=True):
+        width = n // 2 if kind == SWIGLU else n
+        t = {k: v[:, :n].contiguous() if k in ("x", "read") else v for k, v in whole.items()}
+        pitch = n + 8 + shift
+
+        def halves(cols):  # rows `shift` elements off 16 bytes
+            return torch.full((M * pitch + 8,), float("nan"), device="cuda", dtype=torch.bfloat16)[shift:shift + M * pitch].view(
+                M, pitch)[:, :cols]
+
+        t["gate"] = halves(n).copy_(whole["gate"][:, :n])
+        out = dict(y=rand(M, n), acc=torch.full((M, n), float("nan"), device="cuda", dtype=torch.bfloat16),
+                   sums_out=torch.zeros(M, (n + 31) // 32, device="cuda"), h=halves(width) if h else None)
+        args = Args(rows=M, cols=n, depth=K, entries=3, features=10, eps=1e-3, gate_pitch=pitch, h_pitch=pitch,
+                    **{k: v.data_ptr() for k, v in {**t, **out}.items() if v is not None})
+        assert lib.fields_product(ctypes.byref(args), kind, _stream()) == 0
+        torch.cuda.synchronize()
+        names = {GATE: ("y", "acc", "h"), RESIDUAL: ("y", "h")}.get(kind, ("h",))
+        return {k: out[k] for k in names if out[k] is not None}, out["sums_out"]
+
+    want, sums = call(N, 0)
+    assert not any(bool(v.isnan().any()) for v in want.values())
+    got, got_sums = call(N, 4)
+    assert all(torch.equal(got[k], want[k]) for k in want) and torch.equal(got_sums, sums)
+    if kind != SWIGLU:  # (of u and v in turn no four columns can go)
+        got, _ = call(N - 4, 0)
+        assert all(torch.equal(got[k], want[k][:, :N - 4]) for k in want)
+    if kind in (GATE, RESIDUAL):
+        got, _ = call(N, 0, h=False)
+        assert all(torch.equal(got[k], want[k]) for k in got)
+
+
 class Transpose(ctypes.Structure):
     _fields_ = [("in_", P), ("out", P), ("rows", I), ("cols", I)]
 
