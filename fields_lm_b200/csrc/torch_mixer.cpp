@@ -4,7 +4,7 @@
 // by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is two matrix
 // products forward and four backward (the two projections of x are one product over
 // [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
-// field_mixer_grad.cuh between them. With rows enough the first product and the gradients of read and x have
+// field_mixer_grad.cuh between them. With rows enough the products of the forward pass and the gradients of read and x have
 // fused epilogues (field_product.cuh); the others are library calls. Weight gradients come out of the products in fp32.
 #include "torch_gemm.h"
 
@@ -55,7 +55,8 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         check(f.fields_stack_close_ff(fp(x), nullptr, nullptr, nullptr, vp(xb), 0.0f, N, (int)D, st),
               "fields_stack_close_ff");
         Tensor u = empty({N, W}, at::kBFloat16, dev);
-        if (fused_products(N, D)) {
+        const bool fused = fused_products(N, D);
+        if (fused) {
             fields_product_args q{};
             q.a = vp(xb); q.b = vp(in_w); q.rows = N; q.cols = (int)W; q.depth = (int)D;
             q.bias16 = vp(in_b); q.h = vp(u); q.h_pitch = W;
@@ -73,11 +74,20 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
                   "fields_read_forward_bf16_rows");
         }
         Tensor acc = empty({N, D}, at::kBFloat16, dev);
-        product(acc, plain(read), transposed(out16), N, D, 2 * D);
         const Tensor y = empty({B, L, D}, at::kFloat, dev);
-        check(f.fields_stack_close_mixer(fp(x), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
-                                         nullptr, fp(y), nullptr, (float)eps, (int)(2 * D), 0.0f, N, (int)D, st),
-              "fields_stack_close_mixer");
+        if (fused) {  // (74 us at 16,384 rows of 1,024; the library's product and the row kernel 51 + 41)
+            fields_product_args q{};
+            q.a = vp(read); q.b = vp(out16); q.rows = N; q.cols = (int)D; q.depth = (int)(2 * D);
+            q.x = fp(x); q.bias = fp(out_b); q.gate_bias = fp(gate_b); q.gate = gate_of(u, C); q.gate_pitch = W;
+            q.sums = fp(groups); q.entries = (int)G; q.features = (int)(2 * D); q.eps = (float)eps;
+            q.y = fp(y); q.acc = vp(acc);
+            check(f.fields_product(&q, FIELDS_PRODUCT_GATE, st), "fields_product");
+        } else {
+            product(acc, plain(read), transposed(out16), N, D, 2 * D);
+            check(f.fields_stack_close_mixer(fp(x), vp(acc), gate_of(u, C), W, fp(groups), (int)G, fp(out_b), fp(gate_b),
+                                             nullptr, fp(y), nullptr, (float)eps, (int)(2 * D), 0.0f, N, (int)D, st),
+                  "fields_stack_close_mixer");
+        }
         ctx->save_for_backward({xb, u, read, groups, acc, in_w, out16, par, radius, theta, norm_w, out_w, out_b, gate_b});
         ctx->saved_data["eps"] = eps;
         ctx->saved_data["length"] = L;
