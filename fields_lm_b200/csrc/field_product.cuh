@@ -1,5 +1,6 @@
 // Matrix products of thousands of rows with everything that follows them elementwise as their epilogue:
-//   out = a @ b^T, a [M, K] activations, b [N, K] weights, both bfloat16 with K contiguous, fp32 accumulation.
+//   out = a @ b^T, a [M, K] activations, b [N, K] weights, both bfloat16 with K contiguous, fp32 accumulation (or out = a @ b,
+//   b [K, N]).
 //
 //   ProductBias      u = out + bias                                      in bfloat16
 //   ProductGate      y = x + (out rstd + b) sigmoid(gate + b_g)          fp32, and what the caller asks for of: its
@@ -475,7 +476,17 @@ struct ProductWarp {
     }
 };
 
-template <class Epi, int NT>
+// Shared-memory descriptor of b as it lies in memory with K as its rows: 64 columns of N are 128 bytes of a row of K, with the
+// 128-byte swizzle; groups of eight rows 1,024 bytes apart, the next 64 columns behind the k-block's rows.
+__device__ __forceinline__ unsigned long long depth_desc(unsigned addr) {
+    constexpr unsigned long long kNext64 = 64 * 128 >> 4;
+    return (unsigned long long)((addr & 0x3FFFFu) >> 4) | (kNext64 << 16) | ((unsigned long long)(1024 >> 4) << 32) | (1ull << 46) |
+           (2ull << 61);
+}
+
+// BY_DEPTH: b is [K, N], N contiguous, a weight as the forward pass has it. (The mixer's two had been transposed by a launch of
+// their own, 11 us: 558 -> 549 us at 8 x 2,048 x 1,024. The products are as fast either way.)
+template <class Epi, int NT, bool BY_DEPTH>
 __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
     pair_product(const __grid_constant__ ProductMaps maps, const __grid_constant__ ProductParams p) {
     using T = ProductShape<Epi, NT>;
@@ -543,7 +554,13 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
                     if (rank == 0) mbar_expect(full + r.slot * 8, 2 * T::kStageBytes);
                     const unsigned bar = peer_addr(full + r.slot * 8, 0), at = smem_addr(ring + r.slot * T::kStageBytes);
                     tma_load2_pair(at, &maps.a, i * T::kBox, m0, bar);
-                    tma_load2_pair(at + T::kABytes, &maps.b, i * T::kBox, n0, bar);
+                    if constexpr (BY_DEPTH) {
+#pragma unroll
+                        for (int g = 0; g < NT / 128; ++g)
+                            tma_load2_pair(at + T::kABytes + g * (T::kBox * 128), &maps.b, n0 + g * 64, i * T::kBox, bar);
+                    } else {
+                        tma_load2_pair(at + T::kABytes, &maps.b, i * T::kBox, n0, bar);
+                    }
                     r.next();
                 }
             }
@@ -551,8 +568,9 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
     } else if (rank == 0) {
         if (elect_one()) {
             StepRing<T::kStages> r;
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) |
+            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)BY_DEPTH << 16) | ((unsigned)(NT >> 3) << 17) |
                                    ((unsigned)(2 * kProductRows >> 4) << 24);
+            constexpr unsigned kNextK = BY_DEPTH ? 16 * 128 >> 4 : 16 * 2 >> 4;  // 16 of K further in b
             unsigned n = 0;
             for (long long t = first; t < p.tiles; t += p.pairs, ++n) {
                 const unsigned buf = n & 1;
@@ -565,10 +583,12 @@ __global__ void __launch_bounds__(32 * (kProductWarps + 2), 1)
                     if (dead) break;
                     r.next();
                     here = i + 1 < p.k_blocks && mbar_try<false>(full + r.slot * 8, r.parity);
-                    const unsigned long long a = step_desc(smem_addr(ring + slot * T::kStageBytes)), b = a + (T::kABytes >> 4);
+                    const unsigned at = smem_addr(ring + slot * T::kStageBytes);
+                    const unsigned long long a = step_desc(at),
+                                             b = BY_DEPTH ? depth_desc(at + T::kABytes) : step_desc(at + T::kABytes);
 #pragma unroll
                     for (int k = 0; k < T::kBox / 16; ++k)
-                        pair_mma(tmem + buf * NT, a + 2 * k, b + 2 * k, idesc, i > 0 || k > 0);
+                        pair_mma(tmem + buf * NT, a + 2 * k, b + kNextK * k, idesc, i > 0 || k > 0);
                     pair_commit(empty + slot * 8);
                 }
                 if (dead) break;

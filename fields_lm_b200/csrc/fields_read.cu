@@ -2232,7 +2232,7 @@ static bool box_map(CUtensorMap* map, const void* base, long long rows, int cols
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <class Epi, int NT>
+template <class Epi, int NT, bool BY_DEPTH>
 static int launch_product(const struct fields_product_args& g, ProductParams p, int pairs, Stream st) {
     using T = ProductShape<Epi, NT>;
     p.k_blocks = (g.depth + T::kBox - 1) / T::kBox;
@@ -2240,7 +2240,8 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     p.tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * p.tiles_n;
     ProductMaps maps;
     std::memset(&maps, 0, sizeof(maps));
-    bool ok = operand_map(&maps.a, g.a, p.M, g.depth, kProductRows) && operand_map(&maps.b, g.b, p.N, g.depth, NT / 2);
+    bool ok = operand_map(&maps.a, g.a, p.M, g.depth, kProductRows) &&
+              (BY_DEPTH ? operand_map(&maps.b, g.b, g.depth, p.N, T::kBox) : operand_map(&maps.b, g.b, p.N, g.depth, NT / 2));
     if (Epi::kF32) ok = ok && box_map(&maps.x, g.x, p.M, p.N, p.N, T::kChunk, true) && box_map(&maps.y, g.y, p.M, p.N, p.N, T::kChunk, true);
     if (!p.direct) {
         if (Epi::kIn) ok = ok && box_map(&maps.in16, p.in16, p.M, p.N, p.in_pitch, T::kHalfColumns, false);
@@ -2249,7 +2250,7 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     }
     if (!ok) return FIELDS_ERR_UNSUPPORTED;
     static bool ready[64] = {};
-    const int rc = allow_shared_memory(pair_product<Epi, NT>, T::kSmemBytes, ready);
+    const int rc = allow_shared_memory(pair_product<Epi, NT, BY_DEPTH>, T::kSmemBytes, ready);
     if (rc) return rc;
     p.pairs = p.tiles < pairs ? (int)p.tiles : pairs;
     cudaLaunchConfig_t cfg = {};
@@ -2265,13 +2266,13 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = dependent_launch_enabled() ? 2 : 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, pair_product<Epi, NT>, maps, p));
+    return check_cuda(cudaLaunchKernelEx(&cfg, pair_product<Epi, NT, BY_DEPTH>, maps, p));
 }
 
 // Tiles of 256 or of 128 columns: by the rounds of tiles that a pair takes, each as long as its columns and about 64 more
 // (loads and a wave's end; 2,048 rows: 2,560 columns of depth 1,024 16.9 and 15.3 us, 1,024 of depth 2,528 21.4 and 14.4; 8,192
 // rows: 32.1 and 35.9, 41.7 and 47.2).
-template <class Epi>
+template <class Epi, bool BY_DEPTH = false>
 static int run_product(const struct fields_product_args& g, const ProductParams& p, Stream st) {
     int dev = 0, sms = 0;
     int rc = check_cuda(cudaGetDevice(&dev));
@@ -2282,7 +2283,8 @@ static int run_product(const struct fields_product_args& g, const ProductParams&
         const long long tiles = (p.M + 2 * kProductRows - 1) / (2 * kProductRows) * ((p.N + nt - 1) / nt);
         return (tiles + pairs - 1) / pairs * (nt + 64);
     };
-    return rounds(128) < rounds(256) ? launch_product<Epi, 128>(g, p, pairs, st) : launch_product<Epi, 256>(g, p, pairs, st);
+    return rounds(128) < rounds(256) ? launch_product<Epi, 128, BY_DEPTH>(g, p, pairs, st)
+                                     : launch_product<Epi, 256, BY_DEPTH>(g, p, pairs, st);
 }
 
 // How a launch of step_stack covers the GPU: `clusters` are resident at once.
@@ -2518,6 +2520,11 @@ int fields_transpose_bf16(const struct fields_transpose* parts, int count, void*
 }
 
 int fields_product(const struct fields_product_args* g, int kind, void* stream) {
+    const bool by_depth = kind >= 0 && (kind & FIELDS_PRODUCT_BY_DEPTH);
+    if (by_depth) {
+        kind -= FIELDS_PRODUCT_BY_DEPTH;
+        if (kind != FIELDS_PRODUCT_RESIDUAL && kind != FIELDS_PRODUCT_NORM_GRAD) return FIELDS_ERR_ARGUMENT;
+    }
     if (!g || g->rows < 0 || g->cols <= 0 || g->depth <= 0) return FIELDS_ERR_ARGUMENT;
     if (g->rows == 0) return FIELDS_OK;
     if (!g->a || !g->b) return FIELDS_ERR_ARGUMENT;
@@ -2528,7 +2535,7 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
         return FIELDS_ERR_ARGUMENT;  // rows would overlap
     if (g->cols > kWidest || gate_pitch > kWidest || h_pitch > kWidest || gate_pitch < 0 || h_pitch < 0)
         return FIELDS_ERR_UNSUPPORTED;
-    if (g->cols % 4 || g->depth % 8 || g->rows > 0x7fffff00LL || !aligned16(g->a) || !aligned16(g->b) || !aligned16(g->x) ||
+    if (g->cols % (by_depth ? 8 : 4) || g->depth % 8 || g->rows > 0x7fffff00LL || !aligned16(g->a) || !aligned16(g->b) || !aligned16(g->x) ||
         !aligned16(g->y) || !aligned16(g->bias) || !aligned16(g->gate_bias) || !aligned8(g->bias16) || !aligned8(g->gate) ||
         !aligned8(g->read) || !aligned8(g->h) || !aligned8(g->acc) || gate_pitch % 4 || h_pitch % 4)
         return FIELDS_ERR_UNSUPPORTED;
@@ -2559,10 +2566,10 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
             return run_product<ProductSwiglu>(*g, p, st);
         case FIELDS_PRODUCT_RESIDUAL:
             if (!g->x || !g->y) return FIELDS_ERR_ARGUMENT;
-            return run_product<ProductResidual>(*g, p, st);
+            return by_depth ? run_product<ProductResidual, true>(*g, p, st) : run_product<ProductResidual>(*g, p, st);
         case FIELDS_PRODUCT_NORM_GRAD:
             if (!p.in16 || !p.row || !p.h) return FIELDS_ERR_ARGUMENT;
-            return run_product<ProductNormGrad>(*g, p, st);
+            return by_depth ? run_product<ProductNormGrad, true>(*g, p, st) : run_product<ProductNormGrad>(*g, p, st);
     }
     return FIELDS_ERR_ARGUMENT;
 }

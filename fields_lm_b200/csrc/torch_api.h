@@ -39,7 +39,7 @@ using torch::autograd::variable_list;
     X(fields_read_forward) X(fields_read_backward) X(fields_read_backward_from_states)              \
     X(fields_read_forward_bf16) X(fields_read_forward_bf16_stats) X(fields_read_backward_bf16)      \
     X(fields_read_norm_grad_combine) X(fields_read_step) X(fields_read_step_bf16)                   \
-    X(fields_scan_forward) X(fields_scan_backward) X(fields_stack_layout) X(fields_stack_layout_parts) X(fields_product) X(fields_transpose_bf16)                           \
+    X(fields_scan_forward) X(fields_scan_backward) X(fields_stack_layout) X(fields_stack_layout_parts) X(fields_product)                                                    \
     X(fields_stack_step_norm) X(fields_stack_close_mixer) X(fields_stack_swiglu)                    \
     X(fields_stack_close_ff) X(fields_read_forward_bf16_rows) X(fields_read_backward_bf16_rows)     \
     X(fields_mixer_grad_rows) X(fields_mixer_grad_scratch_bytes) X(fields_mixer_open_grad)          \

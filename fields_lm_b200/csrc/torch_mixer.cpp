@@ -123,23 +123,15 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         auto need = [&](int i) { return ctx->needs_input_grad(i); };
         const bool recurrence = need(kX) || need(kWriteW) || need(kWriteB) || need(kRadius) || need(kTheta);
         float* p = fp(par);
-        // The products of the gradients of read and x have epilogues where there are rows enough; their weights then lie
-        // the other way round.
+        // The products of the gradients of read and x have epilogues where there are rows enough.
         const bool fused = fused_products(N, D);
-        Tensor out16_t, in_w_t;
-        if (fused && recurrence) {
-            out16_t = empty({2 * D, D}, at::kBFloat16, dev);
-            if (need(kX)) in_w_t = empty({D, W}, at::kBFloat16, dev);
-            const fields_transpose parts[2] = {{vp(out16), vp(out16_t), (int)D, (int)(2 * D)}, {vp(in_w), vp(in_w_t), (int)W, (int)D}};
-            check(f.fields_transpose_bf16(parts, need(kX) ? 2 : 1, st), "fields_transpose_bf16");
-        }
         if (recurrence) {
             const Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
             if (fused) {
                 fields_product_args q{};
-                q.a = vp(grad_acc); q.b = vp(out16_t); q.rows = N; q.cols = (int)(2 * D); q.depth = (int)D;
+                q.a = vp(grad_acc); q.b = vp(out16); q.rows = N; q.cols = (int)(2 * D); q.depth = (int)D;
                 q.read = vp(read); q.row = grad_sumsq; q.h = vp(grad_read); q.h_pitch = 2 * D;
-                check(f.fields_product(&q, FIELDS_PRODUCT_NORM_GRAD, st), "fields_product");
+                check(f.fields_product(&q, FIELDS_PRODUCT_NORM_GRAD + FIELDS_PRODUCT_BY_DEPTH, st), "fields_product");
             } else {
                 product(grad_read, plain(grad_acc), plain(out16), N, 2 * D, D);
                 check(f.fields_read_norm_grad_combine(vp(grad_read), vp(read), grad_sumsq, vp(grad_read), N, (int)(4 * C), st),
@@ -161,9 +153,9 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
             grad_x = f32s({B, L, D});
             if (fused && reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 == 0) {
                 fields_product_args q{};
-                q.a = vp(grad_u); q.b = vp(in_w_t); q.rows = N; q.cols = (int)D; q.depth = (int)W;
+                q.a = vp(grad_u); q.b = vp(in_w); q.rows = N; q.cols = (int)D; q.depth = (int)W;
                 q.x = fp(gy); q.y = fp(grad_x);
-                check(f.fields_product(&q, FIELDS_PRODUCT_RESIDUAL, st), "fields_product");
+                check(f.fields_product(&q, FIELDS_PRODUCT_RESIDUAL + FIELDS_PRODUCT_BY_DEPTH, st), "fields_product");
             } else {
                 Tensor back = empty({N, D}, at::kBFloat16, dev);
                 product(back, plain(grad_u), plain(in_w), N, D, W);

@@ -574,13 +574,15 @@ int fields_step_block(const struct fields_step_args *args, void *stream);
  *                             the next eight are v of the same (fields_step_layout's w12_w). cols a multiple of 16.
  *   FIELDS_PRODUCT_RESIDUAL   y = x + out, and h = y if given. y may be x.
  *   FIELDS_PRODUCT_NORM_GRAD  h = out + 2 row read, `row` one factor per row
+ * With FIELDS_PRODUCT_BY_DEPTH added to one of the last two b is [depth, cols] (cols a multiple of 8): out = a @ b.
  */
 enum {
     FIELDS_PRODUCT_BIAS,
     FIELDS_PRODUCT_GATE,
     FIELDS_PRODUCT_SWIGLU,
     FIELDS_PRODUCT_RESIDUAL,
-    FIELDS_PRODUCT_NORM_GRAD
+    FIELDS_PRODUCT_NORM_GRAD,
+    FIELDS_PRODUCT_BY_DEPTH = 16
 };
 struct fields_product_args {
     const void *a, *b;

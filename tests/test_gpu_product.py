@@ -170,6 +170,35 @@ def test_rows_that_tma_does_not_address(kind, M, N, K):
         assert all(torch.equal(got[k], want[k]) for k in got)
 
 
+# columns and depth around the edges of 64 (a box of the weights), of both tile widths; several tiles of a pair
+@pytest.mark.parametrize("kind", [RESIDUAL, NORM_GRAD])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (130, 72, 64), (257, 200, 136), (300, 1024, 2528), (16000, 272, 72), (9000, 1024, 200)])
+def test_weights_by_depth(kind, M, N, K):
+    torch.manual_seed(M + kind)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(K, N, device="cuda") / K ** 0.5).bfloat16()
+    x, row = torch.randn(M, N, device="cuda"), torch.randn(M, device="cuda")
+    read, h = torch.randn(M, N, device="cuda").bfloat16(), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    y = torch.empty(M, N, device="cuda")
+    args = Args(rows=M, cols=N, depth=K, **{k: v.data_ptr() for k, v in dict(a=a, b=b, x=x, row=row, read=read, h=h, y=y).items()})
+    assert _lib.load().fields_product(ctypes.byref(args), kind + 16, _stream()) == 0
+    torch.cuda.synchronize()
+    want = a.double() @ b.double() + (x.double() if kind == RESIDUAL else 2 * row.double()[:, None] * read.double())
+    for got in (h, y) if kind == RESIDUAL else (h,):
+        # (as above: a rounding to bfloat16, and fp32 sums of K products)
+        bound = 1e-4 * want.square().mean().sqrt() + (2 ** -8 * want.abs() if got is h else 0)
+        assert bool(((got.double() - want).abs() <= bound).all())
+
+
+def test_weights_by_depth_refusals():
+    lib, a = _lib.load(), torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16)
+    args = Args(rows=8, cols=12, depth=16, **{k: a.data_ptr() for k in ("a", "b", "x", "y", "bias16", "h", "read", "row")})
+    assert lib.fields_product(ctypes.byref(args), RESIDUAL, _stream()) == 0
+    assert lib.fields_product(ctypes.byref(args), RESIDUAL + 16, _stream()) != 0  # rows of 24 bytes
+    args.cols = 16
+    for kind in (BIAS, GATE, SWIGLU):
+        assert lib.fields_product(ctypes.byref(args), kind + 16, _stream()) != 0
+
+
 class Transpose(ctypes.Structure):
     _fields_ = [("in_", P), ("out", P), ("rows", I), ("cols", I)]
 
