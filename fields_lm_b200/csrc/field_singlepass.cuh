@@ -109,16 +109,18 @@ FL_HD SpTile sp_decode(const SpShape& s, unsigned ticket) {
 // IO = float, or uint16_t for bfloat16 raw / read (the state, the maps and all arithmetic stay fp32).
 //
 // What bounds it: a tile lives about 10 us (its loads, the look-back, its stores), so bandwidth is the
-// tile state that an SM holds divided by that. fp32 keeps a step's gate values in registers between the
-// two halves, 12 bytes per channel and step (the raw values are as large). bfloat16 keeps
-// the raw bits, half as much, and evaluates the gates a second time. (One reciprocal for the three gates,
-// four special-function operations per channel instead of six, gained 4 % at 1 x 65,536 x 512 and nothing at
-// 8 x 2,048; its state was 1.9e-7 from 64-bit arithmetic instead of 1.3e-7, and a gate that is masked with -inf did
-// not close.) With the workspace fill, launched alone on a cold L2: 48.1 -> 44.1 us at 8 x 2,048 x 512 and 185 -> 157
-// at 1 x 65,536 against an earlier form that held tickets and staged the next tile in shared memory. Blocks of
+// tile state that an SM holds divided by that. A step's gate values, 12 bytes per channel and step, are kept
+// between the two halves, in registers and, of the first PARKED steps of a warp, in shared memory, in cells of the thread's own.
+// Of fp32 rows all are in registers: parked, a third more tiles per SM at once were 5 to 10 % slower (46.9 -> 50.0 us at
+// 8 x 2,048 x 512, 178 -> 194 at 1 x 65,536). bfloat16 rows take half the memory traffic and are bound by the arithmetic:
+// six of ten steps parked against raw bits in registers and the gates evaluated twice 39.0 -> 33.3 us at 8 x 2,048 x 512,
+// 153 -> 135 at 1 x 65,536, 139 -> 121 at 4 x 16,384, 23.8 -> 20.4 at 8 x 1,024, with statistics 41.0 -> 35.2 and 24.8 -> 21.8
+// (eight steps, four parked: 34.0, 150, 128 and 20.3; none parked, three blocks per SM: 36.1, 148, 129 and 21.4). One
+// reciprocal for the three gates (four special-function operations per channel instead of six) was not taken: its state was
+// 1.9e-7 from 64-bit arithmetic instead of 1.3e-7, and a gate that is masked with -inf did not close. Blocks of
 // four warps overlap their phases better than blocks of eight.
 // ROWS: also writes the state after every kStateRowEvery-th step, what a backward pass from state rows keeps.
-template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false, bool ROWS = false>
+template <int TS, int WARPS, int MIN_BLOCKS, typename IO = float, bool STATS = false, bool ROWS = false, int PARKED = 0>
 struct FwdSinglePass {
     using Params = SpFwdParamsT<IO>;
     static constexpr int kThreads = 32 * WARPS;
@@ -130,30 +132,53 @@ struct FwdSinglePass {
     // per warp: product of keep, Re B, Im B; later the lane partials of the statistics
     static constexpr int kMapFloats = WARPS * 3 * kGroup;
     static constexpr int kSumFloats = STATS && kTile * kStatRow > kMapFloats ? (kTile * kStatRow + 3) / 4 * 4 : kMapFloats;
-    static constexpr bool kPacked = sizeof(IO) == 2;  // hold the raw bits, evaluate the gates twice
+    static constexpr bool kHalf = sizeof(IO) == 2;
+    static constexpr int kHeld = TS - PARKED;  // steps in registers
     static constexpr int kCarryFloats = WARPS * 2 * kGroup;
-    static constexpr int kSmemFloats = kSumFloats + kCarryFloats;
+    static constexpr int kSmemFloats = kSumFloats + kCarryFloats + PARKED * 3 * kThreads * 4;
+    static_assert(PARKED < TS && (kHalf || PARKED == 0), "fp32 rows are loaded to where the gate values go");
     static constexpr int kClaimAfter = 2;  // the next tile is claimed after the look-back phase
     FL_HD static constexpr bool barrier_after(int ph) { return ph != 1; }
 
     struct State {
-        // float: raw on load, then gamma*v*inj and vacancy; bfloat16: the raw bits of four channels
-        F2 br[kPacked ? 1 : TS][2], bi[kPacked ? 1 : TS][2], vac[kPacked ? 1 : TS][2];
-        Bits4 raw[kPacked ? TS : 1][3];
+        F2 br[kHeld][2], bi[kHeld][2], vac[kHeld][2];  // gamma*v*inj and vacancy (of fp32 rows, first the raw values)
     };
 
-    FL_HD static void take(State& st, int u, int plane, const IO* src, int nch) {
-        if constexpr (kPacked) {
-            st.raw[u][plane] = load_bits4(src);
-        } else {
-            const Vec<4> z = io_load4_stream(src, nch);
-            F2(&d)[2] = plane == 0 ? st.br[u] : plane == 1 ? st.bi[u] : st.vac[u];
-            d[0] = lo2(z); d[1] = hi2(z);
+    FL_HD static float* cell_at(float* smem, int u, int plane, int thread) {
+        return smem + kSumFloats + kCarryFloats + ((u * 3 + plane) * kThreads + thread) * 4;
+    }
+    // The gate values of step u (a constant once the loops are unrolled).
+    FL_HD static void hold(State& st, float* smem, int thread, int u, const F2 (&g)[3][2]) {
+        if (u < PARKED) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) vec_store<4>(cell_at(smem, u, q, thread), join2(g[q][0], g[q][1]));
+            return;
+        }
+        const int k = u < PARKED ? 0 : u - PARKED;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            st.br[k][h] = g[0][h];
+            st.bi[k][h] = g[1][h];
+            st.vac[k][h] = g[2][h];
         }
     }
-    FL_HD static Gate2 gate(const State& st, int u, int h) {
-        if constexpr (kPacked) return make_gate2(st.raw[u][0].pair(h), st.raw[u][1].pair(h), st.raw[u][2].pair(h));
-        else return make_gate2(st.br[u][h], st.bi[u][h], st.vac[u][h]);
+    FL_HD static void held(const State& st, float* smem, int thread, int u, F2 (&g)[3][2]) {
+        if (u < PARKED) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const Vec<4> z = vec_load<4>(cell_at(smem, u, q, thread));
+                g[q][0] = lo2(z);
+                g[q][1] = hi2(z);
+            }
+            return;
+        }
+        const int k = u < PARKED ? 0 : u - PARKED;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            g[0][h] = st.br[k][h];
+            g[1][h] = st.bi[k][h];
+            g[2][h] = st.vac[k][h];
+        }
     }
 
     // Steps of warp w of the tile that lie inside the sequence.
@@ -197,13 +222,22 @@ struct FwdSinglePass {
             F2 Br[2] = {splat2(0.0f), splat2(0.0f)}, Bi[2] = {splat2(0.0f), splat2(0.0f)};
             if (chan_ok) {
                 // (only bfloat16 rows may be columns of a wider matrix)
-                const size_t pitch = kPacked ? (size_t)s.zp : (size_t)3 * C;
+                const size_t pitch = kHalf ? (size_t)s.zp : (size_t)3 * C;
                 const IO* row = p.raw + ((size_t)tl.b * s.L + tw) * pitch + c0;
+                Bits4 bits[kHalf ? TS : 1][3];
 #pragma unroll
                 for (int u = 0; u < TS; ++u) {
                     if (tw + u < s.L) {
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) take(st, u, q, row + (size_t)q * C, nch);
+                        for (int q = 0; q < 3; ++q) {
+                            if constexpr (kHalf) {
+                                bits[u][q] = load_bits4(row + (size_t)q * C);
+                            } else {
+                                const Vec<4> z = io_load4_stream(row + (size_t)q * C, nch);
+                                F2(&d)[2] = q == 0 ? st.br[u] : q == 1 ? st.bi[u] : st.vac[u];
+                                d[0] = lo2(z); d[1] = hi2(z);
+                            }
+                        }
                     }
                     row += pitch;
                 }
@@ -215,22 +249,25 @@ struct FwdSinglePass {
 #pragma unroll
                 for (int u = 0; u < TS; ++u) {
                     if (tw + u < s.L) {
+                        F2 kept[3][2];
+                        if constexpr (!kHalf) held(st, smem, thread, u, kept);
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            const Gate2 g = gate(st, u, h);
+                            Gate2 g;
+                            if constexpr (kHalf) g = make_gate2(bits[u][0].pair(h), bits[u][1].pair(h), bits[u][2].pair(h));
+                            else g = make_gate2(kept[0][h], kept[1][h], kept[2][h]);
                             const F2 bs = mul2(gm[h], g.vac);
                             const F2 br = mul2(bs, g.inj_r), bi = mul2(bs, g.inj_i);
-                            if constexpr (!kPacked) {
-                                st.br[u][h] = br;
-                                st.bi[u][h] = bi;
-                                st.vac[u][h] = g.vac;
-                            }
+                            kept[0][h] = br;
+                            kept[1][h] = bi;
+                            kept[2][h] = g.vac;
                             prod[h] = mul2(prod[h], g.keep);
                             const F2 mr = fma2(lr[h], Br[h], mul2(nli[h], Bi[h]));
                             const F2 mi = fma2(lr[h], Bi[h], mul2(li[h], Br[h]));
                             Br[h] = fma2(g.keep, mr, br);
                             Bi[h] = fma2(g.keep, mi, bi);
                         }
+                        hold(st, smem, thread, u, kept);
                     }
                 }
             }
@@ -307,8 +344,7 @@ struct FwdSinglePass {
             }
             const Vec<4> lr4 = par_load4<IO>(p.tr + c0, nch);
             const Vec<4> li4 = par_load4<IO>(p.ti + c0, nch);
-            const Vec<4> gm4 = kPacked ? par_load4<IO>(p.gamma + c0, nch) : lr4;
-            const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)}, gm[2] = {lo2(gm4), hi2(gm4)};
+            const F2 lr[2] = {lo2(lr4), hi2(lr4)}, li[2] = {lo2(li4), hi2(li4)};
             const F2 nli[2] = {mul2(li[0], splat2(-1.0f)), mul2(li[1], splat2(-1.0f))};
             const Vec<4> sr4 = vec_load<4>(carry_at(smem, warp, 0) + lane * 4);
             const Vec<4> si4 = vec_load<4>(carry_at(smem, warp, 1) + lane * 4);
@@ -317,26 +353,17 @@ struct FwdSinglePass {
 #pragma unroll
             for (int u = 0; u < TS; ++u) {
                 if (tw + u < s.L) {
-                    F2 dr[2], di[2], sq = splat2(0.0f);
+                    F2 dr[2], di[2], sq = splat2(0.0f), kept[3][2];
+                    held(st, smem, thread, u, kept);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const F2 mr = fma2(lr[h], sr[h], mul2(nli[h], si[h]));
                         const F2 mi = fma2(lr[h], si[h], mul2(li[h], sr[h]));
-                        F2 v, keep, br, bi;
-                        if constexpr (kPacked) {
-                            const Gate2 g = gate(st, u, h);
-                            const F2 bs = mul2(gm[h], g.vac);
-                            v = g.vac; keep = g.keep;
-                            br = mul2(bs, g.inj_r); bi = mul2(bs, g.inj_i);
-                        } else {
-                            v = st.vac[u][h];
-                            keep = fma2(v, splat2(-1.0f), splat2(1.0f));
-                            br = st.br[u][h]; bi = st.bi[u][h];
-                        }
+                        const F2 v = kept[2][h], keep = fma2(v, splat2(-1.0f), splat2(1.0f));
                         dr[h] = mul2(v, mr);
                         di[h] = mul2(v, mi);
-                        sr[h] = fma2(keep, mr, br);
-                        si[h] = fma2(keep, mi, bi);
+                        sr[h] = fma2(keep, mr, kept[0][h]);
+                        si[h] = fma2(keep, mi, kept[1][h]);
                         if constexpr (STATS)
                             sq = fma2(sr[h], sr[h], fma2(si[h], si[h], fma2(dr[h], dr[h], fma2(di[h], di[h], sq))));
                     }

@@ -675,9 +675,8 @@ using BwdSp2 = BwdRecompute<8, 4, 1, 3, 2>;   // 73 KB per block, 12 warps per S
 using BwdSp3 = BwdTileResident<4, 4, 3>;      // tile 16, 68 KB per block, 12 warps per SM
 #endif
 //   bfloat16 raw / read / grad_read / grad_raw (bits as uint16_t); state and arithmetic stay fp32
-// The forward: blocks of four warps. (Blocks of eight, 80 steps, look back over half as many tiles, but at 8 x 2,048 x 512
-// they take 38.9 us against 37.7, at 8 x 8,192 140 against 135, at 4 x 16,384 142 against 138, and as long at 1 x 65,536.)
-template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS>;  // STATS: per-token sums of squares too
+// The forward: blocks of four warps, four to an SM, ten steps per warp of which six wait in shared memory (figures at FwdSinglePass).
+template <bool STATS> using FwdSpBf16 = FwdSinglePass<10, 4, 4, uint16_t, STATS, false, 6>;  // STATS: per-token sums of squares too
 // bfloat16 ring cells are half the size, so a 64-step tile (4 warps x 16 steps) still leaves room for
 // four blocks per SM; measured 54.9 us against 59.7 us for the 32-step tile (and 71.5 us with
 // 16-byte cells) on 8 x 2,048 tokens. (The bound of 128 registers keeps the fourth block: without it the second sweep's early
