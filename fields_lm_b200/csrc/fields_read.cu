@@ -2113,7 +2113,7 @@ int fields_mixer_open_grad(const float* grad_y, const void* acc, const void* gat
     if (D <= 4 * kRowThreads) {
         int threads = (D / 4 + 31) / 32 * 32;
         if (threads < kGradRowsMax) threads = kGradRowsMax;  // one thread per row at the end
-        return launch_on<OpenGradParams>(open_grad<1, 4>, (unsigned)blocks, (unsigned)threads, 0, st, p);
+        return launch_on<OpenGradParams>(open_grad<1, 2>, (unsigned)blocks, (unsigned)threads, 0, st, p);
     }
     return launch_on<OpenGradParams>(open_grad<4, 1>, (unsigned)blocks, kRowThreads, 0, st, p);
 }
