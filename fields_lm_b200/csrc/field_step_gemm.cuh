@@ -12,8 +12,9 @@
 // cycles from the last tile of one phase to the first load of the next, 1,700 until its operands are there, 3,100 to 4,100
 // until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
-// 18 blocks of d_model 1,024 take 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
-// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256. What is done about it:
+// 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
+// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with one addition per block to a phase's count 407 at 1 row
+// and 584 at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
@@ -330,14 +331,14 @@ struct StepStackParams {
     StepPhase phase[kStepPhases];
     uint16_t *gate, *read, *yb, *act, *xb;
     float *y, *read_sq, *y_sq;
-    unsigned* sync;  // finished eighths of tiles (a warp's) of each row tile, 32 words apart, or null: one phase alone
+    unsigned* sync;  // finished parts of tiles (a block's) of each row tile, 32 words apart, or null: one phase alone
     int M, D, C, H;
     int a_rows;                            // rows of a box of activations
     int row_tiles, groups, group_clusters; // clusters of a group serve the same row tiles
     int first, last;                       // phases of this launch, counted over the blocks of the stack
 };
 
-// Waits until `count` eighths of tiles are finished, with a bound (2^22 polls are seconds).
+// Waits until `count` parts of tiles are finished, with a bound (2^22 polls are seconds).
 __device__ __forceinline__ void wait_for_tiles(const unsigned* p, unsigned count, bool& dead) {
     for (unsigned tries = 0; !dead; ++tries) {
         unsigned v;
@@ -523,15 +524,14 @@ __device__ __forceinline__ void step_epilogue(const StepStackParams& p, const St
             // (what was stored is read by TMA loads of other blocks, and the space of the block's own sums is written by its
             // own next ones)
             asm volatile("fence.proxy.async;" ::: "memory");
-            if (p.sync) {
-                __syncwarp();
-                if ((tid & 31) == 0)
-                    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.sync + row_tile * 32) : "memory");
-            }
         }
         epilogue_sync();
         if (tid == 0) {
             if (tile >= 0) mbar_arrive(c.tmem_free);
+            // One addition per block: with one per warp, up to 1,152 to the same word and as many waits for the stores before
+            // them, 18 blocks of d_model 1,024 took 426 us at 1 row, 491 at 100 and 596 at 256, now 404, 467 and 578. (Polls
+            // without acquire and a fence behind the last: 437, 501 and 610; two polls in flight: 443, 507 and 614.)
+            if (p.sync && tile >= 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.sync + row_tile * 32) : "memory");
             for (int j = 0; j < kStepCluster; ++j)
                 if (j != c.rank) mbar_arrive_at(peer_addr(c.freed + (n.iters % 2 * kStepCluster + c.rank) * 8, j));
         }
@@ -577,7 +577,7 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
                     wait_for_tiles(p.sync + m * 32, target, dead);
                     if (dead) *c.dead = 1;
                 }
-                target += (unsigned)(h.tiles_n * h.S) * 8;
+                target += (unsigned)(h.tiles_n * h.S);
                 mbar_arrive(c.ready);
             }
             for (int it = 0; it < iters; ++it) {
