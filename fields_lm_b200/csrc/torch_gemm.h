@@ -11,23 +11,25 @@
 namespace fields_torch {
 
 // Whether products with fused epilogues (field_product.cuh) take the place of the library's with row kernels between
-// them, us against the library's. Prefill of eight blocks, 128 to 8,192 rows: d_model 512 397 to 847 and 256 337 to 507
-// against 490 to 938 and 491 to 548 (the host's launches bound the library's). Wider models from `least` rows on: their
-// tiles of 256 rows leave much of the GPU idle when there are few; d_model 1,024, 1,024 rows 693 against 622, 2,048 793 against
-// 812, 4,096 1,151 against 1,207, 8,192 1,993 against 2,179; 600 at 2,048 rows 608 and 734, 768 611 and 627, 1,536 1,341 and
-// 1,364. Up to `widest`: all column tiles follow one another for each 256 rows, and beyond it the weights of a product no
-// longer stay in L2 meanwhile. Two blocks, 2,048 and 8,192 rows: d_model 2,048 535 and 1,536 against 541 and 1,631, 2,560 874 and
-// 2,649 against 747 and 2,552, 4,096 2,178 and 6,924 against 1,827 and 6,080.
+// them: up to `narrow` always, where the host's launches bound the library's; up to `widest` from `least` rows on, as their
+// tiles of 256 rows leave much of the GPU idle when there are few.
 struct ProductRule {
-    int64_t least, widest;
+    int64_t narrow, least, widest;
 };
-constexpr ProductRule kPrefillProducts{2048, 2048};
-// The mixer's backward pass has two weights to transpose (12 us at d_model 1,024) for 18 us at 4,096 rows, some 50 at 16,384:
-// d_model 1,024 at 6,144 rows 285 against 295, 640 219 against 240, 2,048 750 against 763; at 6,144 and 8,192 rows 3,072 1,641 and
-// 2,127 against 1,617 and 2,149, 4,096 2,927 and 3,728 against 2,785 and 3,580.
-constexpr ProductRule kMixerProducts{6144, 3072};
+// Prefill, us against the library's. Eight blocks: d_model 256 438 to 355 against 524 and 512 374 to 461 against 527 (128 to
+// 2,048 rows); 640 424 at 256 rows, 453 at 1,024 and 506 at 2,048 against 506, 510 and 545; 768 469, 497 and 561 against 512, 514
+// and 607 (544 and 531 at 1,536); 1,024 562, 585 and 648 at 256, 512 and 1,024 rows against 514, 520 and 601, but 673 against 703 at
+// 1,536 and 752 against 792 at 2,048. Two blocks: 1,536 304 against 318 at 1,536 rows, 2,048 511 and 1,512 against 534 and 1,646 at 2,048
+// and 8,192. Wider: all column tiles follow one another for each 256 rows, and the weights of a product no
+// longer stay in L2 meanwhile: 2,560 854 and 1,354 against 741 and 1,343 at 2,048 and 4,096 rows, 3,072 3,697 against 3,474 at 8,192,
+// 4,096 6,460 against 6,003.
+constexpr ProductRule kPrefillProducts{768, 1536, 2048};
+// Mixer, forward and backward: 640 to 2,048 wide 202 to 297 against 244 to 337 from 512 to 2,048 rows, 2,048 869 against 936 at 8,192; 2,560
+// 495 against 479 at 2,048 rows, but 726 against 753 at 4,096, 3,072 968 and 1,931 against 1,048 and 2,018 at 4,096 and 8,192, 4,096 1,750 and
+// 3,378 against 1,813 and 3,398.
+constexpr ProductRule kMixerProducts{2048, 4096, 4096};
 inline bool fused_products(int64_t rows, int64_t dim, ProductRule rule) {
-    return dim <= 512 || (rows >= rule.least && dim <= rule.widest);
+    return dim <= rule.narrow || (rows >= rule.least && dim <= rule.widest);
 }
 
 // A bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any; rows as stored are
