@@ -13,8 +13,8 @@
 // until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
-// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with one addition per block to a phase's count 407 at 1 row
-// and 584 at 256. What is done about it:
+// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps 366 at 1
+// row and 530 at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
@@ -426,8 +426,10 @@ __device__ __forceinline__ void step_epilogue(const StepStackParams& p, const St
         }
         if (n.iters > 0) {  // the peers have read what was sent to them in the iteration before
             const unsigned last = n.iters - 1;
-            for (int j = 0; j < kStepCluster; ++j)
-                if (j != c.rank) mbar_wait(c.freed + (last % 2 * kStepCluster + j) * 8, last / 2 & 1, n.dead);
+            const int j = tid & 31;
+            bool late = n.dead;
+            if (j < kStepCluster && j != c.rank) mbar_wait(c.freed + (last % 2 * kStepCluster + j) * 8, last / 2 & 1, late);
+            n.dead = __any_sync(0xffffffffu, late);
         }
         if (it == 0) {
             mbar_wait_local(c.ready, n.phases++ & 1, n.dead);
@@ -521,22 +523,25 @@ __device__ __forceinline__ void step_epilogue(const StepStackParams& p, const St
                 finish(u, fetched[0]);
             }
             ++n.items;
-            // (what was stored is read by TMA loads of other blocks, and the space of the block's own sums is written by its
-            // own next ones)
-            asm volatile("fence.proxy.async;" ::: "memory");
+            // (the space of the block's own sums is written by its next loads)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         epilogue_sync();
         if (tid == 0) {
             if (tile >= 0) mbar_arrive(c.tmem_free);
             // One addition per block: with one per warp, up to 1,152 to the same word and as many waits for the stores before
-            // them, 18 blocks of d_model 1,024 took 426 us at 1 row, 491 at 100 and 596 at 256, now 404, 467 and 578. (Polls
-            // without acquire and a fence behind the last: 437, 501 and 610; two polls in flight: 443, 507 and 614.)
+            // them, 18 blocks of d_model 1,024 took 426 us at 1 row, 491 at 100 and 596 at 256; 404, 467 and 578 with one, and 363,
+            // 409 and 525 with the arrivals at the peers, 300 cycles each behind the addition's 1,000, by other warps and the proxy
+            // fence for what is stored by the reader. (Polls without acquire and a fence behind the last: 33 us more; two polls in
+            // flight: 35; polls that begin 800 to 2,400 cycles later: the same; two warps that do nothing but this: 15 at 1 row.)
             if (p.sync && tile >= 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.sync + row_tile * 32) : "memory");
-            for (int j = 0; j < kStepCluster; ++j)
-                if (j != c.rank) mbar_arrive_at(peer_addr(c.freed + (n.iters % 2 * kStepCluster + c.rank) * 8, j));
         }
+        if (tid >= 32 && tid % 32 == 0 && tid < 32 * (1 + kStepCluster)) {  // a warp per peer
+            const int j = tid / 32 - 1;
+            if (j != c.rank) mbar_arrive_at(peer_addr(c.freed + (n.iters % 2 * kStepCluster + c.rank) * 8, j));
+        }
+        if (tid == 32 * 5 && it + 1 == h.iters) mbar_arrive(c.left);
     }
-    if (tid == 0) mbar_arrive(c.left);
 }
 
 // The three single threads that feed the tensor cores walk the same phases, tiles and k-blocks. They are elected
@@ -576,6 +581,7 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
                 if (p.sync && q > p.first) {
                     wait_for_tiles(p.sync + m * 32, target, dead);
                     if (dead) *c.dead = 1;
+                    asm volatile("fence.proxy.async.global;" ::: "memory");  // (stored by lanes, read by TMA)
                 }
                 target += (unsigned)(h.tiles_n * h.S);
                 mbar_arrive(c.ready);
