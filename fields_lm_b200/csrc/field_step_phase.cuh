@@ -2,11 +2,10 @@
 // order: each is a matrix product on the tensor cores (tcgen05.mma, operands by TMA, accumulator in tensor memory)
 // whose epilogue goes on to the operand of the next.
 //
-// For single blocks, for devices that do not hold the cooperative launch of a stack, and for stacks of narrow blocks: there a
-// phase has a few tiles, whose K cannot be split, so that a thread block finishes 128 rows by itself, and that and the
-// hand-over through global memory cost more than a launch that was let in ahead. Eight blocks: d_model 64 at 128 rows 150 us,
-// as one launch 195; 256 at 16 and 512 rows 151 and 176, as one launch 168 and 192; 384 at 16 rows 179 and 172; 1,024 at 16
-// rows 269 and 198. What is done about a launch:
+// For single blocks, for devices that do not hold the cooperative launch of a stack, and for stacks of d_model 64 at 65 to 256
+// rows: there a phase is one tile, whose K cannot be split, so that a thread block finishes 128 rows by itself, and that and the
+// hand-over through global memory cost more than a launch that was let in ahead. Eight blocks: d_model 64 at 128 rows 162 us,
+// as one launch 173; 128 175 and 165, 256 at 16 and 512 rows 173 and 149, 187 and 159. What is done about a launch:
 //   - the next kernel is let in at the start (dependent launch) and loads its weights before it waits for
 //     this one, as far as SMs are free for it;
 //   - K is split over a cluster of S blocks; each then owns 1/S of the tile's columns, to which the others send

@@ -348,21 +348,22 @@ class FieldStack {
     }
 
   private:
-    // The blocks as one launch while their products have tiles (128 rows x 64 features) few enough that K
-    // can be split to fill the GPU once: 18 blocks of d_model 1,024 take 471 us at 16 rows and 602 at 256
-    // against 745 and 763 with library products. (384 rows as four launches per block 1,002 against 776.)
+    // Fused products instead of the library's while those of the step have tiles (128 rows x 64 features) few enough. us per step
+    // against library products: eight blocks of d_model 576 264 and 355 at 512 rows, 1,024 250 and 350 at 256 rows, 316 and 358 at 257,
+    // 322 and 355 at 512 (64 tiles), 1,280 360 and 395 at 384, but 604 and 441 at 400 (80); four blocks of 2,048 258 and 260 at
+    // 256 rows. Wider ones while there are up to 64 rows: 2,560 255 and 284 at 1 row, 269 and 276 at 64, 297 and 289 at 128; 3,072 293
+    // and 366, 311 and 323, 340 and 332; 4,096 389 and 512, 412 and 449.
     bool fused_step(int64_t rows) const {
-        return D_ % 16 == 0 && H_ % 8 == 0 && rows <= 512 && (rows + 127) / 128 * ((D_ + 63) / 64) <= 32;
+        return D_ % 16 == 0 && H_ % 8 == 0 && rows <= 512 && (rows + 127) / 128 * ((D_ + 63) / 64) <= 64 &&
+               (D_ <= 2048 || rows <= 64);
     }
 
-    // Whether its blocks are one launch or four launches each. Eight blocks, us as one and as four each: d_model 256 168 and 151
-    // at 16 rows, 181 and 162 at 128, 195 and 176 at 512; 384 172 and 179, 198 and 195, 214 and 216 at 384 rows; 512 175 and
-    // 193, 187 and 204, 197 and 196 at 256 rows, 224 and 224 at 512; 640 237 and 223 at 256 rows, 282 and 326 at 512; 768
-    // 190 and 220, 242 and 245 at 256. Of the narrow ones 96 to 224 at up to 64 rows (128: 159 and 164 at one row, 159 and 166
-    // at 64; 224: 167 and 186, 173 and 188), not 64 (167 and 150 at 64 rows).
-    bool step_in_one_launch(int64_t rows) const {
-        return D_ >= (rows <= 128 ? 384 : rows <= 256 ? 704 : 512) || (rows <= 64 && D_ > 64 && D_ < 256);
-    }
+    // Whether its blocks are one launch or four launches each. Eight blocks, us as one and as four each: d_model 64 113 and 147 at one
+    // row, 130 and 151 at 64, 148 and 150 at 65, but 173 and 162 at 128 and 174 and 170 at 256, where a phase is one tile of which
+    // a thread block finishes 128 rows by itself; 176 and 177 at 512. Wider ones always: 128 117 and 164 at one row, 165 and 175 at 128,
+    // 168 and 196 at 512; 256 130 and 165, 156 and 175, 159 and 187; 512 142 and 211, 164 and 216, 210 and 239; 768 158 and 235,
+    // 187 and 242 and, at 256 rows, 226 and 262.
+    bool step_in_one_launch(int64_t rows) const { return D_ > 64 || rows <= 64 || rows > 256; }
 
     // The embedding's output as the kernels take it: a width of another model is refused, as nn.Linear does.
     Tensor activations(const Tensor& x, int64_t dims) const {

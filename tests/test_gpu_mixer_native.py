@@ -50,6 +50,12 @@ def test_native_mixer_matches_the_composed_one(dim, B, L):
 
 # rows from which the products of a wide mixer have fused epilogues, at the edge of a tile and a ragged number; the last
 # width for which they have
+# where fused and library products take turns
+@pytest.mark.parametrize("dim,B,L", [(2048, 1, 3), (2056, 1, 40), (2064, 1, 4095), (2064, 1, 4096), (1024, 1, 129)])
+def test_edges_of_the_rule(dim, B, L):
+    test_native_mixer_matches_the_composed_one(dim, B, L)
+
+
 @pytest.mark.parametrize("dim,B,L", [(1024, 7, 1003), (1040, 1, 6145), (3072, 3, 2048)])
 @pytest.mark.parametrize("x_grad", [True, False])
 def test_mixer_with_fused_products(dim, B, L, x_grad):
