@@ -13,8 +13,8 @@
 // until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
-// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps 366 at 1
-// row and 530 at 256. What is done about it:
+// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps and the
+// partial sums loaded together 328 at 1 row and 486 at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
@@ -495,7 +495,11 @@ __device__ __forceinline__ void step_epilogue(const StepStackParams& p, const St
                     for (int k = 0; k < kSlice; k += 4) {
                         const int line = (k / 4 * kSlices + s) * pitch + rl;
                         float4 w = reinterpret_cast<const float4*>(c.a)[line];
-                        for (int src = 0; src < S - 1; ++src) {
+                        // (of constant length: as a loop over S - 1 every source was waited for before the next one's load
+                        // went out; 18 blocks of d_model 1,024 525 us instead of 486 at 256 rows, 367 and 328 at 1)
+#pragma unroll
+                        for (int src = 0; src < Epi::kMaxSplit - 1; ++src) {
+                            if (src >= S - 1) continue;
                             const float4 o = reinterpret_cast<const float4*>(c.recv)[src * (kColumns / 4) * pitch + line];
                             w.x += o.x; w.y += o.y; w.z += o.z; w.w += o.w;
                         }
