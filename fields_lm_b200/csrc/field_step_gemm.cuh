@@ -14,7 +14,7 @@
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
 // 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps and the
-// partial sums loaded together 328 at 1 row and 486 at 256. What is done about it:
+// partial sums loaded together 319 at 1 row and 476 at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
@@ -579,9 +579,15 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
             const int ph = q % kStepPhases, parts = T::parts(ph), box = T::box(ph);
             const StepPhase& h = p.phase[ph];
             const int r = c.rank % h.S, count = step_k(h, r), k0 = r * h.per, iters = h.iters;
+            const int first_tile = step_tile(p, h, c, 0);
             if constexpr (ROLE == kStepActivations) {
                 if (phases > 0) mbar_wait_local(c.left, (phases - 1) & 1, dead);
                 ++phases;
+                // What does not depend on the phase before is done ahead of the wait for it (with the products' wait for weights
+                // ahead of that for activations 487 -> 476 us for 18 blocks of d_model 1,024 at 256 rows, 327 -> 319 at 1).
+                if (first_tile >= 0 && !dead)
+                    for (int i = 0; i < count && i < T::kAStages; ++i)
+                        mbar_expect(c.a_full + (ar.slot + i) % T::kAStages * 8, (unsigned)p.a_rows * 128 * kStepKBoxes);
                 if (p.sync && q > p.first) {
                     wait_for_tiles(p.sync + m * 32, target, dead);
                     if (dead) *c.dead = 1;
@@ -591,7 +597,7 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
                 mbar_arrive(c.ready);
             }
             for (int it = 0; it < iters; ++it) {
-                const int tile = step_tile(p, h, c, it);
+                const int tile = it == 0 ? first_tile : step_tile(p, h, c, it);
                 if (tile < 0) continue;
                 if constexpr (ROLE == kStepWeights) {
                     const CUtensorMap* map = &p.block[q / kStepPhases].b[ph];
@@ -617,7 +623,7 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
                     for (int i = 0; i < count; ++i) {
                         if (i >= T::kAStages) mbar_wait_local(c.a_empty + ar.slot * 8, ar.parity ^ 1, dead);
                         if (dead) continue;
-                        mbar_expect(c.a_full + ar.slot * 8, bytes);
+                        if (it > 0 || i >= T::kAStages) mbar_expect(c.a_full + ar.slot * 8, bytes);
 #pragma unroll
                         for (int x = 0; x < kStepKBoxes; ++x)
                             tma_load2(smem_addr(c.a + ar.slot * T::kABytes + x * T::kABox), map,
@@ -639,8 +645,8 @@ __device__ __forceinline__ void step_feed(const StepStackParams& p, const StepCt
                         for (int part = 0; part < parts; ++part) {
                             const unsigned as = ar.slot, bs = br.slot;
                             if (!here) {
+                                mbar_wait_local(c.b_full + bs * 8, br.parity, dead);  // (there long before)
                                 if (part == 0) mbar_wait_local(c.a_full + as * 8, ar.parity, dead);
-                                mbar_wait_local(c.b_full + bs * 8, br.parity, dead);
                             }
                             if (dead) continue;
                             const bool last_part = part + 1 == parts;
