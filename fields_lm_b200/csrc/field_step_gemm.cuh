@@ -14,7 +14,7 @@
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
 // 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
 // 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps and the
-// partial sums loaded together 319 at 1 row and 476 at 256. What is done about it:
+// partial sums loaded together 312 at 1 row and 471 at 256. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
@@ -453,18 +453,20 @@ __device__ __forceinline__ void step_epilogue(const StepStackParams& p, const St
                 }
             }
             if (tid == 0 && S > 1 && !n.dead) mbar_expect(c.got, (unsigned)((S - 1) * mine * kColumns * 4));
+            // (where the sums go is worked out under the product: 476 -> 471 us for 18 blocks of d_model 1,024 at 256 rows, 318 ->
+            // 312 at 1)
+            constexpr int kHalf = kColumns / 2;
+            const int row = tid % kStepRows, to = row / per, rl = row - to * per, col0 = tid / kStepRows * kHalf;
+            const int src = r > to ? r - 1 : r;
+            float4* own = reinterpret_cast<float4*>(c.a) + rl;
+            const unsigned peer = first + (row < rows ? to : r), bar = peer_addr(c.got, peer);
+            const unsigned at = peer_addr(smem_addr(c.recv) + (unsigned)((src * (kColumns / 4) * pitch + rl) * 16), peer);
+            const unsigned lane_addr = c.tmem + ((unsigned)(row & ~31) << 16) + (unsigned)col0;
             mbar_wait_local(c.done, n.items & 1, n.dead);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             {   // the product's rows to the blocks that finish them; two warps share a quarter of the lanes
-                constexpr int kHalf = kColumns / 2;
-                const int row = tid % kStepRows, to = row / per, rl = row - to * per, col0 = tid / kStepRows * kHalf;
                 const bool send = row < rows && to != r && !n.dead;  // (nothing after a wait that ran out)
-                const int src = r > to ? r - 1 : r;
-                float4* own = reinterpret_cast<float4*>(c.a) + rl;
-                const unsigned peer = first + (row < rows ? to : r), bar = peer_addr(c.got, peer);
-                const unsigned at = peer_addr(smem_addr(c.recv) + (unsigned)((src * (kColumns / 4) * pitch + rl) * 16), peer);
-                const unsigned lane_addr = c.tmem + ((unsigned)(row & ~31) << 16) + (unsigned)col0;
                 constexpr int kStep = kHalf % 16 == 0 ? 16 : 8;
 #pragma unroll
                 for (int k0 = 0; k0 < kHalf; k0 += kStep) {
