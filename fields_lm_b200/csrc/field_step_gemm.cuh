@@ -8,7 +8,7 @@
 //   EpiFf   f = act @ w3^T                  -> x' = y + f, bf16 copy
 //
 // A step of a few hundred rows is bound by latency: the 25 MB of weights of a block of d_model 1,024 take
-// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 6 to 8 us (256 rows: 2,400 to 3,000
+// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 4.3 to 6.5 us, in its first form 6 to 8 (256 rows: 2,400 to 3,000
 // cycles from the last tile of one phase to the first load of the next, 1,700 until its operands are there, 3,100 to 4,100
 // until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
 // 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
