@@ -337,7 +337,7 @@ FL_HD F2 fma2(const F2& a, const F2& b, const F2& c) {
     const float2 r = __ffma2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
     return F2{r.x, r.y};
 #else
-    return F2{a.x * b.x + c.x, a.y * b.y + c.y};
+    return F2{std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)};
 #endif
 }
 

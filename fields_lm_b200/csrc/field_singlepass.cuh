@@ -141,7 +141,7 @@ struct FwdSinglePass {
     FL_HD static constexpr bool barrier_after(int ph) { return ph != 1; }
 
     struct State {
-        F2 br[kHeld][2], bi[kHeld][2], vac[kHeld][2];  // gamma*v*inj and vacancy (of fp32 rows, first the raw values)
+        F2 br[kHeld][2], bi[kHeld][2], sig[kHeld][2];  // gamma*v*inj and sigmoid(z_v) (of fp32 rows, first the raw values)
     };
 
     FL_HD static float* cell_at(float* smem, int u, int plane, int thread) {
@@ -159,7 +159,7 @@ struct FwdSinglePass {
         for (int h = 0; h < 2; ++h) {
             st.br[k][h] = g[0][h];
             st.bi[k][h] = g[1][h];
-            st.vac[k][h] = g[2][h];
+            st.sig[k][h] = g[2][h];
         }
     }
     FL_HD static void held(const State& st, float* smem, int thread, int u, F2 (&g)[3][2]) {
@@ -177,7 +177,7 @@ struct FwdSinglePass {
         for (int h = 0; h < 2; ++h) {
             g[0][h] = st.br[k][h];
             g[1][h] = st.bi[k][h];
-            g[2][h] = st.vac[k][h];
+            g[2][h] = st.sig[k][h];
         }
     }
 
@@ -234,7 +234,7 @@ struct FwdSinglePass {
                                 bits[u][q] = load_bits4(row + (size_t)q * C);
                             } else {
                                 const Vec<4> z = io_load4_stream(row + (size_t)q * C, nch);
-                                F2(&d)[2] = q == 0 ? st.br[u] : q == 1 ? st.bi[u] : st.vac[u];
+                                F2(&d)[2] = q == 0 ? st.br[u] : q == 1 ? st.bi[u] : st.sig[u];
                                 d[0] = lo2(z); d[1] = hi2(z);
                             }
                         }
@@ -260,7 +260,7 @@ struct FwdSinglePass {
                             const F2 br = mul2(bs, g.inj_r), bi = mul2(bs, g.inj_i);
                             kept[0][h] = br;
                             kept[1][h] = bi;
-                            kept[2][h] = g.vac;
+                            kept[2][h] = g.sig;
                             prod[h] = mul2(prod[h], g.keep);
                             const F2 mr = fma2(lr[h], Br[h], mul2(nli[h], Bi[h]));
                             const F2 mi = fma2(lr[h], Bi[h], mul2(li[h], Br[h]));
@@ -359,7 +359,9 @@ struct FwdSinglePass {
                     for (int h = 0; h < 2; ++h) {
                         const F2 mr = fma2(lr[h], sr[h], mul2(nli[h], si[h]));
                         const F2 mi = fma2(lr[h], si[h], mul2(li[h], sr[h]));
-                        const F2 v = kept[2][h], keep = fma2(v, splat2(-1.0f), splat2(1.0f));
+                        // (1 - v would round twice: an open gate's keep was off by 3e-7 of itself a step, and not the one in
+                        // the maps between tiles)
+                        const F2 v = mul2(kept[2][h], splat2(kVacMax)), keep = fma2(kept[2][h], splat2(-kVacMax), splat2(1.0f));
                         dr[h] = mul2(v, mr);
                         di[h] = mul2(v, mi);
                         sr[h] = fma2(keep, mr, kept[0][h]);

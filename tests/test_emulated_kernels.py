@@ -400,6 +400,34 @@ def test_forward_with_norm_statistics(monkeypatch, B, L, C, order):
     assert rel_err(sumsq, want) < FP32_TOL
 
 
+def test_open_gates_of_the_bf16_forward():
+    """The recurrence inside a tile takes 1 - 0.9 sigmoid with one rounding, as the maps between tiles do: a state that only
+    decays, lambda = 1, at the open gate (z_v from 3 to 8) where a second rounding would change most."""
+    k = np.float32(0.9)
+    z = (np.arange(3 * 64, 8 * 64, dtype=np.float32) / 64)
+    z = _unbits(_bits(z))
+    e = np.exp2(np.float32(-1.4426950408889634) * z)
+    low, high = (np.float32(1) + np.nextafter(e, np.float32(to)) for to in (0, 1))
+    sig = np.float32(1) / (np.float32(1) + e)
+    once = np.float32(1 - k.astype(np.float64) * sig.astype(np.float64))
+    twice = np.float32(1) - k * sig
+    apart = np.where(low == high, np.abs(twice.astype(np.float64) - once) / once, 0)  # (an ulp of the exponential is not seen)
+    at = int(apart.argmax())
+    assert apart[at] > 2.2e-7
+    L, C = 10, 4  # steps of one warp
+    raw = np.zeros((1, L, 3 * C), np.float32)
+    raw[:, 0, :C], raw[:, :, 2 * C:] = 1.0, z[at]
+    one, zero = np.ones(C, np.float32), np.zeros(C, np.float32)
+    _, sumsq = emu.forward_bf16_stats(_bits(raw), one, zero, one)
+    vac = float(k) * float(sig[at])
+    # from the second step on each is that before it, squared twice the relative error: a rounding of keep and of the product
+    # per step, three in the squares and their sum
+    got = np.asarray(sumsq, np.float64)[0, 1:, 0]
+    want = got[0] * (1 - vac) ** (2.0 * np.arange(L - 1))
+    bound = 2.0 ** -24 * (4 * np.arange(L - 1) + 6)
+    assert (np.abs(got / want - 1) <= bound).all(), np.abs(got / want - 1) / bound
+
+
 def test_bf16_boundary_refuses_odd_channel_counts():
     raw_b = np.zeros((1, 4, 21), np.uint16)
     p = np.ones(7, np.float32)

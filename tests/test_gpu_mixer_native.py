@@ -166,6 +166,35 @@ def test_state_of_the_bf16_forward_is_as_accurate_as_the_fp32_one():
     assert err[0] < 1.15 * err[1], err  # (1.3e-7 both; 1.9e-7 with one reciprocal shared by the three gates)
 
 
+def test_open_gates_of_the_bf16_forward():
+    """The recurrence inside a tile takes the keep factor of the maps between tiles: a state that only decays (lambda = 1),
+    in the sums of squares of ten steps against the end states of one and of ten."""
+    from fields_lm_b200 import _lib
+    lib, B, L, C = _lib.load(), 320, 10, 4
+    raw = torch.zeros(B, L, 3 * C, device="cuda", dtype=torch.bfloat16)
+    raw[:, 0, :C] = 1.0
+    raw[..., 2 * C:] = (3 + torch.arange(B, device="cuda") / 64)[:, None, None]  # open gates, one per row of the batch
+    one, zero = torch.ones(C, device="cuda"), torch.zeros(C, device="cuda")
+
+    def call(steps):
+        read = torch.empty(B, steps, 4 * C, device="cuda", dtype=torch.bfloat16)
+        state, sums = torch.empty(B, 2 * C, device="cuda"), torch.empty(B, steps, 1, device="cuda")
+        n, x = lib.fields_read_workspace_bytes(B, steps, C, 0), raw[:, :steps].contiguous()
+        ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+        assert lib.fields_read_forward_bf16_stats(*[t.data_ptr() for t in (x, one, zero, one)], None, read.data_ptr(), sums.data_ptr(),
+                                                  state.data_ptr(), ws.data_ptr(), n, B, steps, C,
+                                                  torch.cuda.current_stream().cuda_stream) == 0
+        return state[:, 0].double(), sums[..., 0].double()
+
+    (first, _), (last, sums) = call(1), call(L)
+    keep = (last / first) ** (1 / (L - 1))
+    k = torch.arange(L - 1, device="cuda")
+    off = (sums[:, 1:] / (sums[:, 1:2] * keep[:, None] ** (2 * k)) - 1).abs()
+    # squared twice the relative error: of the product of each step in the recurrence and in the map behind `keep`, three in the
+    # squares and their sum
+    assert bool((off <= 2.0 ** -24 * (4 * k + 6)).all()), off.amax(0)
+
+
 @pytest.mark.parametrize("wanted", [("x",), ("x", "write_proj.bias"), ("gate_proj.weight",), ("write_proj.weight",),
                                     ("out_proj.weight", "gate_proj.bias"), ("read_norm.weight",), ("radius_logit",),
                                     ("theta", "out_proj.bias"), ("write_proj.weight", "gate_proj.weight")])
