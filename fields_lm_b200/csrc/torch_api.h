@@ -83,6 +83,8 @@ inline Tensor f32(const Tensor& t) {
     return t.contiguous().to(at::kFloat);
 }
 inline Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+// ... on the 16 bytes that row kernels and TMA need (a dense view may begin anywhere in its storage)
+inline Tensor aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 ? t.clone() : t; }
 inline float* fp(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 inline void* vp(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline void* stream_of(const Tensor& t) {

@@ -14,7 +14,8 @@ namespace fields_torch {
 
 enum { kX, kWriteW, kWriteB, kRadius, kTheta, kNormW, kOutW, kOutB, kGateW, kGateB, kMixerInputs };
 
-// Whether every input is what the node works on: dense, aligned fp32 on one GPU, sizes that fit.
+// Whether every input is what the node works on: fp32 on one GPU, sizes that fit, parameters dense and aligned (x and the incoming
+// gradient, which may be any views, are copied where they are not).
 static bool mixer_applies(const std::vector<Tensor>& in) {
     const Tensor& x = in[kX];
     if (x.dim() != 3 || x.numel() == 0 || !x.is_cuda()) return false;
@@ -38,7 +39,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
                                  const Tensor& radius, const Tensor& theta, const Tensor& norm_w, const Tensor& out_w,
                                  const Tensor& out_b, const Tensor& gate_w, const Tensor& gate_b, double eps) {
         const Api& f = api();
-        const Tensor x = dense(x_);
+        const Tensor x = aligned(dense(x_));
         const int64_t B = x.size(0), L = x.size(1), D = x.size(2), N = B * L, C = D / 2, W = 3 * C + D, G = (C + 127) / 128;
         const c10::Device dev = x.device();
         const c10::cuda::CUDAGuard guard(dev);
@@ -100,7 +101,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         const Tensor &xb = s[0], &u = s[1], &read = s[2], &groups = s[3], &acc = s[4], &in_w = s[5], &out16 = s[6],
                      &par = s[7], &radius = s[8], &theta = s[9], &norm_w = s[10], &out_w = s[11], &out_b = s[12],
                      &gate_b = s[13];
-        const Tensor gy = f32(grads[0]);
+        const Tensor gy = aligned(f32(grads[0]));
         const int64_t N = xb.size(0), D = xb.size(1), C = D / 2, W = 3 * C + D, G = groups.size(1);
         const int64_t L = ctx->saved_data["length"].toInt(), B = N / L;
         const float eps = (float)ctx->saved_data["eps"].toDouble();
@@ -151,7 +152,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         Tensor grad_x;
         if (need(kX)) {
             grad_x = f32s({B, L, D});
-            if (fused && reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 == 0) {
+            if (fused) {
                 fields_product_args q{};
                 q.a = vp(grad_u); q.b = vp(in_w); q.rows = N; q.cols = (int)D; q.depth = (int)W;
                 q.x = fp(gy); q.y = fp(grad_x);

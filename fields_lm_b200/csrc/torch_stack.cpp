@@ -370,8 +370,7 @@ class FieldStack {
         const c10::Device dev = blocks_[0].src[0].t.device();
         TORCH_CHECK(x.dim() == dims && x.size(dims - 1) == D_ && x.scalar_type() == at::kFloat && x.device() == dev,
                     "activations of shape ", shape(x), " on ", x.device(), " do not fit blocks of width ", D_, " on ", dev);
-        const Tensor d = dense(x);
-        return reinterpret_cast<uintptr_t>(d.data_ptr()) % 16 ? d.clone() : d;
+        return aligned(dense(x));
     }
 
     template <class F>

@@ -48,6 +48,25 @@ def test_native_mixer_matches_the_composed_one(dim, B, L):
         assert rel_err(got[name].float().cpu().numpy(), want[name].float().cpu().numpy()) < BF16_TOL, name
 
 
+@pytest.mark.parametrize("dim", [200, 256])  # library products, fused ones
+@pytest.mark.parametrize("which", ["x", "gradient", "both"])
+def test_views_that_begin_anywhere(dim, which):
+    """x and the incoming gradient as dense views one float into their storage: the results of aligned ones."""
+    torch.manual_seed(dim)
+    m = mirror.IndependentVacancyField(dim).cuda()
+
+    def shifted(t):
+        return torch.zeros(t.numel() + 1, device="cuda")[1:].view_as(t).copy_(t)
+
+    x, gy = torch.randn(3, 37, dim, device="cuda"), torch.randn(3, 37, dim, device="cuda")
+    want = _grads(m, x.clone().requires_grad_(), gy, True)
+    x, gy = x if which == "gradient" else shifted(x), gy if which == "x" else shifted(gy)
+    assert x.is_contiguous() and gy.is_contiguous() and bool(x.data_ptr() % 16 or gy.data_ptr() % 16)
+    got = _grads(m, x.requires_grad_(), gy, True)
+    for name in want:  # (the recurrence is reproducible to rounding)
+        assert rel_err(got[name].float().cpu().numpy(), want[name].float().cpu().numpy()) < 2 ** -8, name
+
+
 # rows from which the products of a wide mixer have fused epilogues, at the edge of a tile and a ragged number; the last
 # width for which they have
 # where fused and library products take turns
