@@ -40,9 +40,12 @@ struct OpenGradParams {
 };
 
 // OWN groups of four columns per thread; R rows are loaded together, under the rows before them (without that, four rows at a time and
-// three blocks per SM: 46.4 us at 16,384 rows of 1,024, 37.9 now).
+// three blocks per SM: 48.5 us at 16,384 rows of 1,024, 38.8 now; one row at a time, four groups and three blocks per SM: 87.3 us
+// of 2,048 columns and 128 of 3,072). Up to 2,048 columns two groups and three blocks per SM, 69.4 us: with four groups, whose
+// registers hold two rows for two blocks, 95.5 (4,096 rows 20.4 and 30.0; two groups, two rows and two blocks 88.3). Above that four and two
+// blocks, 121 us of 3,072 and 147 of 4,096 (168 before).
 template <int OWN, int R>
-__global__ void __launch_bounds__(kRowThreads, OWN > 1 ? 2 : 3) open_grad(const OpenGradParams p) {
+__global__ void __launch_bounds__(kRowThreads, OWN > 2 ? 2 : 3) open_grad(const OpenGradParams p) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float dots[kGradRowsMax][kRowThreads / 32];
     __shared__ float rstds[kGradRowsMax];

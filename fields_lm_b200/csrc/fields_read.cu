@@ -2115,6 +2115,7 @@ int fields_mixer_open_grad(const float* grad_y, const void* acc, const void* gat
         if (threads < kGradRowsMax) threads = kGradRowsMax;  // one thread per row at the end
         return launch_on<OpenGradParams>(open_grad<1, 2>, (unsigned)blocks, (unsigned)threads, 0, st, p);
     }
+    if (D <= 8 * kRowThreads) return launch_on<OpenGradParams>(open_grad<2, 1>, (unsigned)blocks, kRowThreads, 0, st, p);
     return launch_on<OpenGradParams>(open_grad<4, 1>, (unsigned)blocks, kRowThreads, 0, st, p);
 }
 
