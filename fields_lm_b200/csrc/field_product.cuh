@@ -57,9 +57,9 @@ struct ProductParams {
     float inv_features, eps;
     const float* row;        // [M] factor of a row
     float* sums_out;         // [M, ceil(N / 32)]: a warp's columns in the first of their entries, zero in the other
-    // The bfloat16 tensors beside the matrix, for rows that TMA does not address (`direct`), and h and acc where both
-    // are wanted: in16 is gate or read, h the output.
-    int direct;
+    // The bfloat16 tensors beside the matrix, for rows that TMA does not address (`direct_in`, `direct_out`), and h and acc where
+    // both are wanted: in16 is gate or read, h the output.
+    int direct_in, direct_out;
     const uint16_t* in16;
     long long in_pitch;
     uint16_t* h;
@@ -88,12 +88,15 @@ __device__ __forceinline__ uint4 lds16(unsigned addr) {
 __device__ __forceinline__ void sts16(unsigned addr, const uint4& v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// Eight bfloat16 values of a row in global memory that may lie on 8 bytes only, the second four where they exist.
-__device__ __forceinline__ uint4 load_halves(const uint16_t* p, bool second) {
-    const uint2 a = *reinterpret_cast<const uint2*>(p);
-    const uint2 b = second ? *reinterpret_cast<const uint2*>(p + 4) : make_uint2(0u, 0u);
-    return make_uint4(a.x, a.y, b.x, b.y);
+__device__ __forceinline__ uint2 lds8(unsigned addr) {
+    uint2 r;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr) : "memory");
+    return r;
 }
+__device__ __forceinline__ void sts8(unsigned addr, const uint2& v) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+}
+// Eight bfloat16 values of a row in global memory that may lie on 8 bytes only, the second four where they exist.
 __device__ __forceinline__ void store_halves(uint16_t* p, const uint4& v, bool second) {
     *reinterpret_cast<uint2*>(p) = make_uint2(v.x, v.y);
     if (second) *reinterpret_cast<uint2*>(p + 4) = make_uint2(v.z, v.w);
@@ -326,7 +329,7 @@ struct ProductWarp {
     // Inputs of the 32 rows from row0 on and the chunk's columns from col on.
     __device__ void load(unsigned buf, unsigned bar, long long row0, int col) const {
         if (!leader || dead) return;
-        const bool in = Epi::kIn && !p.direct;
+        const bool in = Epi::kIn && !p.direct_in;
         const int bytes = T::kF32Bytes + (in ? 32 * T::kHalfRow : 0);
         if (bytes == 0) return;
         mbar_expect(bar, (unsigned)bytes);
@@ -336,6 +339,36 @@ struct ProductWarp {
     __device__ void buffer_read() const {  // what was sent from the buffer has left it
         if (leader) bulk_wait_read();
         __syncwarp();
+    }
+    // Bfloat16 rows that lie on 8 bytes only, from row0 and hcol on: lanes along the rows, between global memory and where TMA would
+    // have them. (With a lane per row, which touches 32 rows at once, the bias product of 16,384 rows of 1,300 columns and depth 520
+    // took 64.6 us, of 8,192 32.2, the gate of 520 columns 53.3 and 36.0; now 37.8, 21.6, 41.1 and 27.4.)
+    static constexpr int kAcross = T::kHalfRow / 8;  // lanes of a row, and accesses of a lane
+    struct Halves {
+        uint2 w[kAcross];
+    };
+    template <class F>
+    __device__ void along_rows(unsigned buf, int left, int hcol, int cols, F f) const {
+        const int q = lane % kAcross;
+#pragma unroll
+        for (int i = 0; i < kAcross; ++i) {
+            const int r = (i * 32 + lane) / kAcross;
+            f(i, r, hcol + 4 * q, buf + T::kF32Bytes + product_unit<T::kHalfRow>(r, q / 2) + (unsigned)(q & 1) * 8,
+              r < left && hcol + 4 * q < cols);
+        }
+    }
+    __device__ void fetch_halves(Halves& to, long long row0, int left, int hcol) const {
+        along_rows(0, left, hcol, p.N, [&](int i, int r, int c, unsigned, bool in) {
+            to.w[i] = in ? *reinterpret_cast<const uint2*>(p.in16 + (row0 + r) * p.in_pitch + c) : make_uint2(0u, 0u);
+        });
+    }
+    __device__ void put_halves(const Halves& from, unsigned buf) const {
+        along_rows(buf, 0, 0, 0, [&](int i, int, int, unsigned at, bool) { sts8(at, from.w[i]); });
+    }
+    __device__ void send_halves(unsigned buf, uint16_t* to, long long pitch, long long row0, int left, int hcol, int cols) const {
+        along_rows(buf, left, hcol, cols, [&](int, int r, int c, unsigned at, bool in) {
+            if (in) *reinterpret_cast<uint2*>(to + (row0 + r) * pitch + c) = lds8(at);
+        });
     }
     // 32 columns of the row, `k` of the chunk on, which begins at the warp's column `c0` and the matrix's column `col0`. (Loads,
     // arithmetic and stores one after the other: in turns for eight columns the loads' latency was waited for four times,
@@ -355,11 +388,7 @@ struct ProductWarp {
         }
         if constexpr (Epi::kIn) {
 #pragma unroll
-            for (int j = 0; j < kUnits; ++j) {
-                in[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (!p.direct) in[j] = lds16(half_at(j));
-                else if (inside(j)) in[j] = load_halves(p.in16 + (long long)row * p.in_pitch + hcol + 8 * j, second(j));
-            }
+            for (int j = 0; j < kUnits; ++j) in[j] = lds16(half_at(j));
         }
 #pragma unroll
         for (int j = 0; j < kUnits; ++j) {
@@ -381,18 +410,14 @@ struct ProductWarp {
             if (p.has_acc) {
 #pragma unroll
                 for (int j = 0; j < kUnits; ++j) {
-                    if (!p.direct && !p.has_h) sts16(half_at(j), acc[j]);
+                    if (!p.has_h) sts16(half_at(j), acc[j]);
                     else if (inside(j)) store_halves(p.acc + (long long)row * p.N + hcol + 8 * j, acc[j], second(j));
                 }
             }
         }
         if (p.has_h) {
 #pragma unroll
-            for (int j = 0; j < kUnits; ++j) {
-                const uint4 t = pack8(v + j * kWide);
-                if (!p.direct) sts16(half_at(j), t);
-                else if (inside(j)) store_halves(p.h + (long long)row * p.h_pitch + hcol + 8 * j, t, second(j));
-            }
+            for (int j = 0; j < kUnits; ++j) sts16(half_at(j), pack8(v + j * kWide));
         }
     }
     // A tile: tmem is the warp's lanes and first column, acc_full is done where the product is, released where to say that
@@ -404,6 +429,9 @@ struct ProductWarp {
             buffer_read();
             if (any) load(own, bars, row0, col0);
         }
+        Halves in16;
+        constexpr bool kAhead = Epi::kIn && kAcross == 8;  // (sixteen accesses ahead do not fit the registers)
+        if (kAhead && p.direct_in && any) fetch_halves(in16, row0, left, col0);
         const float factor = in_rows ? Epi::factor(p, row) : 1.0f;
         const typename Epi::Kept kept =
             Epi::keep(p, col0 + lane * 4, lane * 4 < T::kColumns && col0 + lane * 4 < p.N, constants + lane * 4);
@@ -428,7 +456,12 @@ struct ProductWarp {
                 buffer_read();
                 load(own, bars, row0, col);
             }
-            if (here && kLoads && (Epi::kF32 || !p.direct)) {
+            if (Epi::kIn && p.direct_in && here) {
+                if (!kAhead) fetch_halves(in16, row0, left, col);
+                put_halves(in16, buf);
+                if (kAhead && c + 1 < kChunks) fetch_halves(in16, row0, left, col + T::kChunk);
+            }
+            if (here && kLoads && (Epi::kF32 || !p.direct_in)) {
                 if (last && c > 0) {
                     mbar_wait_local(bars + c * 8, 0, dead);
                 } else {
@@ -460,10 +493,13 @@ struct ProductWarp {
                 __syncwarp();
                 if (leader) {
                     if constexpr (Epi::kF32) tma_store2(&maps.y, buf, col, (int)row0);
-                    if (!p.direct && (p.has_h || p.has_acc))
+                    if (!p.direct_out && (p.has_h || p.has_acc))
                         tma_store2(&maps.out16, buf + T::kF32Bytes, Epi::kSwiglu ? col / 2 : col, (int)row0);
                     bulk_commit();
                 }
+                const int hcol = Epi::kSwiglu ? col / 2 : col, cols = Epi::kSwiglu ? p.N / 2 : p.N;
+                if (p.direct_out && p.has_h) send_halves(buf, p.h, p.h_pitch, row0, left, hcol, cols);
+                else if (p.direct_out && p.has_acc) send_halves(buf, p.acc, p.N, row0, left, hcol, cols);
             }
         }
         if constexpr (Epi::kSums) {

@@ -2243,8 +2243,8 @@ static int launch_product(const struct fields_product_args& g, ProductParams p, 
     bool ok = operand_map(&maps.a, g.a, p.M, g.depth, kProductRows) &&
               (BY_DEPTH ? operand_map(&maps.b, g.b, g.depth, p.N, T::kBox) : operand_map(&maps.b, g.b, p.N, g.depth, NT / 2));
     if (Epi::kF32) ok = ok && box_map(&maps.x, g.x, p.M, p.N, p.N, T::kChunk, true) && box_map(&maps.y, g.y, p.M, p.N, p.N, T::kChunk, true);
-    if (!p.direct) {
-        if (Epi::kIn) ok = ok && box_map(&maps.in16, p.in16, p.M, p.N, p.in_pitch, T::kHalfColumns, false);
+    if (Epi::kIn && !p.direct_in) ok = ok && box_map(&maps.in16, p.in16, p.M, p.N, p.in_pitch, T::kHalfColumns, false);
+    if (!p.direct_out) {
         if (p.has_h) ok = ok && box_map(&maps.out16, p.h, p.M, Epi::kSwiglu ? p.N / 2 : p.N, p.h_pitch, T::kHalfColumns, false);
         else if (p.has_acc) ok = ok && box_map(&maps.out16, p.acc, p.M, p.N, p.N, T::kHalfColumns, false);
     }
@@ -2550,8 +2550,8 @@ int fields_product(const struct fields_product_args* g, int kind, void* stream) 
     p.in16 = h(gated ? g->gate : g->read); p.in_pitch = gated ? gate_pitch : p.N;
     p.h = static_cast<uint16_t*>(g->h); p.h_pitch = h_pitch; p.acc = static_cast<uint16_t*>(g->acc);
     p.has_h = p.h != nullptr; p.has_acc = gated && p.acc;
-    p.direct = !aligned16(p.in16) || p.in_pitch % 8 || (p.has_h && (!aligned16(p.h) || h_pitch % 8)) ||
-               (p.has_acc && !p.has_h && (!aligned16(p.acc) || p.N % 8));
+    p.direct_in = !aligned16(p.in16) || p.in_pitch % 8;
+    p.direct_out = p.has_h ? !aligned16(p.h) || h_pitch % 8 : p.has_acc && (!aligned16(p.acc) || p.N % 8);
     Stream st = reinterpret_cast<Stream>(stream);
     switch (kind) {
         case FIELDS_PRODUCT_BIAS:

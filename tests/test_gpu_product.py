@@ -170,6 +170,41 @@ def test_rows_that_tma_does_not_address(kind, M, N, K):
         assert all(torch.equal(got[k], want[k]) for k in got)
 
 
+# the same sizes; the input alone or the output alone lies on 8 bytes
+@pytest.mark.parametrize("kind", [BIAS, GATE, NORM_GRAD])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (33, 80, 72), (97, 272, 200), (12000, 1040, 72)])
+def test_one_of_the_tensors_that_tma_does_not_address(kind, M, N, K):
+    """... gives the same bits as both aligned, and what lies between the rows stays as it was."""
+    torch.manual_seed(M + kind)
+    lib = _lib.load()
+
+    def rand(*shape):
+        return torch.randn(*shape, device="cuda")
+
+    t = dict(a=rand(M, K).bfloat16(), b=rand(N, K).bfloat16(), bias16=rand(N).bfloat16(), x=rand(M, N), bias=rand(N),
+             gate_bias=rand(N), sums=rand(M, 3).square(), row=rand(M))
+    values = rand(M, N).bfloat16()
+
+    def off(pitch, shift):
+        return torch.full((M * pitch + 8,), float("nan"), device="cuda", dtype=torch.bfloat16)[shift:shift + M * pitch].view(M, pitch)
+
+    def call(in_shift, out_shift):
+        gate, read, h, y = off(N + 8 + in_shift, in_shift), off(N, in_shift), off(N + 8 + out_shift, out_shift), rand(M, N)
+        gate[:, :N].copy_(values)
+        read.copy_(values)
+        args = Args(rows=M, cols=N, depth=K, entries=3, features=10, eps=1e-3, gate_pitch=gate.stride(0), h_pitch=h.stride(0),
+                    y=y.data_ptr(), h=h.data_ptr(), gate=gate.data_ptr(), read=read.data_ptr(), **{k: v.data_ptr() for k, v in t.items()})
+        assert lib.fields_product(ctypes.byref(args), kind, _stream()) == 0
+        torch.cuda.synchronize()
+        assert bool(h[:, N:].isnan().all())
+        return [h[:, :N], y] if kind == GATE else [h[:, :N]]
+
+    want = call(0, 0)
+    assert not any(bool(v.isnan().any()) for v in want)
+    for shifts in [(4, 0), (0, 4)]:
+        assert all(torch.equal(a, b) for a, b in zip(call(*shifts), want)), shifts
+
+
 # columns and depth around the edges of 64 (a box of the weights), of both tile widths; several tiles of a pair
 @pytest.mark.parametrize("kind", [RESIDUAL, NORM_GRAD])
 @pytest.mark.parametrize("M,N,K", [(1, 16, 16), (130, 72, 64), (257, 200, 136), (300, 1024, 2528), (16000, 272, 72), (9000, 1024, 200)])
