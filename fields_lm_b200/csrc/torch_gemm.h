@@ -11,25 +11,33 @@
 namespace fields_torch {
 
 // Whether products with fused epilogues (field_product.cuh) take the place of the library's with row kernels between
-// them: up to `narrow` always, where the host's launches bound the library's; up to `widest` from `least` rows on, as their
+// them: in narrow models, where the host's launches bound the library's, and in wider ones where there are rows enough, as their
 // tiles of 256 rows leave much of the GPU idle when there are few.
 struct ProductRule {
-    int64_t narrow, least, widest;
+    int64_t narrow;            // up to this width always
+    int64_t less_narrow, few;  // up to this one for so few rows
+    int64_t widest, least;     // up to this one from so many rows on
 };
-// Prefill, us against the library's. Eight blocks: d_model 256 438 to 355 against 524 and 512 374 to 461 against 527 (128 to
-// 2,048 rows); 640 424 at 256 rows, 453 at 1,024 and 506 at 2,048 against 506, 510 and 545; 768 469, 497 and 561 against 512, 514
-// and 607 (544 and 531 at 1,536); 1,024 562, 585 and 648 at 256, 512 and 1,024 rows against 514, 520 and 601, but 673 against 703 at
-// 1,536 and 752 against 792 at 2,048. Two blocks: 1,536 304 against 318 at 1,536 rows, 2,048 511 and 1,512 against 534 and 1,646 at 2,048
-// and 8,192. Wider: all column tiles follow one another for each 256 rows, and the weights of a product no
-// longer stay in L2 meanwhile: 2,560 854 and 1,354 against 741 and 1,343 at 2,048 and 4,096 rows, 3,072 3,697 against 3,474 at 8,192,
-// 4,096 6,460 against 6,003.
-constexpr ProductRule kPrefillProducts{768, 1536, 2048};
-// Mixer, forward and backward: 640 to 2,048 wide 202 to 297 against 244 to 337 from 512 to 2,048 rows, 2,048 869 against 936 at 8,192; 2,560
-// 495 against 479 at 2,048 rows, but 726 against 753 at 4,096, 3,072 968 and 1,931 against 1,048 and 2,018 at 4,096 and 8,192, 4,096 1,750 and
-// 3,378 against 1,813 and 3,398.
-constexpr ProductRule kMixerProducts{2048, 4096, 4096};
+// Prefill, us against the library's. Eight blocks: d_model 256 432, 335 and 357 against 543, 560 and 549 at 128, 512 and 2,048 rows; 576
+// 401, 435 and 486 against 487, 498 and 507 at 256, 1,024 and 2,048; 640 428, 455 and 508 against 486, 499 and 543, 704 453, 480 and 544 against
+// 492, 504 and 585 (at 1,408 rows, the least gain, 493 and 496, 523 and 525); 768 452, 472 and 494 against 531, 501 and 502 at 64, 512 and 768
+// rows, but 496 against 495 at 896 and 534 against 512 at 1,028 (75 tiles where 74 pairs run), 553 against 545 at 1,536 and 577 against
+// 635 at 2,048; 896 596 against 560 at 1,280, 612 against 633 at 1,536; 1,024 662 against 641 at 1,280, 679 against 704 at 1,536, 754
+// against 797 at 2,044. Two blocks: 1,536 305 against 320 and 359 against 374 at 1,536 and 2,044 rows (340 and 338 at 1,792), 2,048 435
+// against 418 at 1,280, 468 and 465 at 1,536, 486 and 507 at 1,792, 1,583 and 1,741 at 8,192. Wider: all column tiles follow one another for
+// each 256 rows, and the weights of a product no longer stay in L2 meanwhile: 2,560 850 against 785 at 2,048 rows, 1,426 and 1,428
+// at 4,096, 2,611 and 2,616 at 8,192 (2,473 and 2,555 in another run), 3,072 3,673 and 3,546.
+constexpr ProductRule kPrefillProducts{704, 768, 768, 2048, 1536};
+// Mixer, forward and backward. As calls 200 to 290 us against 240 to 380 for 256 to 2,048 wide ones of 64 to 1,024 rows (1,024 wide: 213 and
+// 261, 215 and 302, 207 and 341 at 64, 128 and 256 rows; 2,048: 246 and 347, 242 and 344, 234 and 349). Where the host's launches
+// do not count, in a captured graph, the library's are faster by 2 to 7 % below 1,024 rows: 1,024 wide 90 and 86, 93 and 88, 98 and
+// 92, 103 and 100, 118 and 117 us at 64, 128, 256, 512 and 1,024 rows; 2,048 160 and 155, 165 and 158, 171 and 168, 186 and 180, 220 and
+// 228. Wider ones: 2,560 496 and 492 at 2,048 rows, 759 and 807 at 4,096, 1,480 and 1,522 at 8,192; 3,072 632 and 629, 1,084 and 1,120,
+// 2,080 and 2,108; 3,584 1,517 and 1,541 at 4,096, 5,456 and 5,464 at 16,384; 3,840 1,738 and 1,723, 6,230 and 6,045; 4,096 1,938 and 1,911, 3,668
+// and 3,501 at 8,192, 7,186 and 6,796.
+constexpr ProductRule kMixerProducts{2048, 0, 0, 3072, 4096};
 inline bool fused_products(int64_t rows, int64_t dim, ProductRule rule) {
-    return dim <= rule.narrow || (rows >= rule.least && dim <= rule.widest);
+    return dim <= rule.narrow || (dim <= rule.less_narrow && rows <= rule.few) || (dim <= rule.widest && rows >= rule.least);
 }
 
 // A bfloat16 matrix as a product takes it: `rows x cols` after the transposition, if any; rows as stored are

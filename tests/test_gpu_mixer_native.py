@@ -70,7 +70,8 @@ def test_views_that_begin_anywhere(dim, which):
 # rows from which the products of a wide mixer have fused epilogues, at the edge of a tile and a ragged number; the last
 # width for which they have
 # where fused and library products take turns
-@pytest.mark.parametrize("dim,B,L", [(2048, 1, 3), (2056, 1, 40), (2064, 1, 4095), (2064, 1, 4096), (1024, 1, 129), (1032, 2, 301)])
+@pytest.mark.parametrize("dim,B,L", [(2048, 1, 3), (2056, 1, 40), (2064, 1, 4095), (2064, 1, 4096), (1024, 1, 129), (1032, 2, 301), (3072, 1, 4096),
+                                     (3088, 1, 4096)])
 def test_edges_of_the_rule(dim, B, L):
     test_native_mixer_matches_the_composed_one(dim, B, L)
 

@@ -65,7 +65,8 @@ def test_native_stack_matches_the_modules(dim, hidden, B, L):
 # where one launch and four, fused and library products take turns: rows and tiles of steps, rows of prefills
 @pytest.mark.parametrize("dim,hidden,B,L", [(64, 40, 65, 2), (64, 40, 257, 2), (80, 24, 128, 2), (1024, 704, 512, 2), (1280, 64, 384, 4),
                                             (1280, 64, 385, 4), (2048, 96, 256, 2), (2560, 64, 64, 3), (2560, 64, 65, 3),
-                                            (768, 352, 3, 5), (1024, 704, 4, 384)])
+                                            (768, 352, 3, 5), (1024, 704, 4, 384), (768, 352, 3, 256), (768, 352, 1, 769), (768, 352, 3, 512),
+                                            (704, 352, 4, 193), (712, 360, 4, 192), (712, 360, 1, 769)])
 def test_edges_of_the_rules(dim, hidden, B, L):
     test_native_stack_matches_the_modules(dim, hidden, B, L)
 
