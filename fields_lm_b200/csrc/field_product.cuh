@@ -128,7 +128,7 @@ __device__ __forceinline__ void bits_float(const uint4& w, float* v) {
 struct ProductBias {
     static constexpr bool kDependents = false;
     static constexpr int kChunk = 64;
-    static constexpr bool kF32 = false, kIn = false, kScaled = false, kSums = false, kSwiglu = false, kAcc = false;
+    static constexpr bool kF32 = false, kIn = false, kSums = false, kSwiglu = false, kAcc = false;
     __device__ static float factor(const ProductParams&, long long) { return 1.0f; }
     // A lane keeps four columns' biases, and all take them from there: a load of the same address by all lanes is as slow as
     // any (5,000 cycles of a tile's epilogue against 3,300).
