@@ -67,19 +67,19 @@ def test_views_that_begin_anywhere(dim, which):
         assert rel_err(got[name].float().cpu().numpy(), want[name].float().cpu().numpy()) < 2 ** -8, name
 
 
-# rows from which the products of a wide mixer have fused epilogues, at the edge of a tile and a ragged number; the last
-# width for which they have
-# where fused and library products take turns
+# widths and rows where fused and library products take turns, and where the columns of a thread of open_grad change
 @pytest.mark.parametrize("dim,B,L", [(2048, 1, 3), (2056, 1, 40), (2064, 1, 4095), (2064, 1, 4096), (1024, 1, 129), (1032, 2, 301), (3072, 1, 4096),
                                      (3088, 1, 4096)])
 def test_edges_of_the_rule(dim, B, L):
     test_native_mixer_matches_the_composed_one(dim, B, L)
 
 
-@pytest.mark.parametrize("dim,B,L", [(1024, 7, 1003), (1040, 1, 6145), (3072, 3, 2048)])
+# products with fused epilogues: several tiles of a pair, ragged rows, the widest; library products: a width that TMA does not
+# address throughout, one beyond the rule
+@pytest.mark.parametrize("dim,B,L", [(1024, 7, 1003), (1040, 1, 6145), (3072, 3, 2048), (1032, 3, 411), (2064, 1, 300)])
 @pytest.mark.parametrize("x_grad", [True, False])
 def test_mixer_with_fused_products(dim, B, L, x_grad):
-    """... where x needs a gradient, and where it does not, which leaves one weight to transpose."""
+    """... where x needs a gradient, and where it does not, which leaves the product of its gradient out."""
     torch.manual_seed(dim)
     m = mirror.IndependentVacancyField(dim).cuda()
     with torch.no_grad():
@@ -218,11 +218,12 @@ def test_open_gates_of_the_bf16_forward():
 @pytest.mark.parametrize("wanted", [("x",), ("x", "write_proj.bias"), ("gate_proj.weight",), ("write_proj.weight",),
                                     ("out_proj.weight", "gate_proj.bias"), ("read_norm.weight",), ("radius_logit",),
                                     ("theta", "out_proj.bias"), ("write_proj.weight", "gate_proj.weight")])
-def test_frozen_parameters_cost_nothing(wanted):
+@pytest.mark.parametrize("D", [1024, 1032])  # products with fused epilogues, the library's
+def test_frozen_parameters_cost_nothing(wanted, D):
     """Gradients of some inputs alone are those of the full pass, and what only the others need is not computed: a
     third of the weights' gradients is more than the difference that the allocator sees."""
     torch.manual_seed(6)
-    D, B, L = 1024, 1, 40
+    B, L = 1, 40
     m = mirror.IndependentVacancyField(D).cuda()
     x = torch.randn(B, L, D, device="cuda", requires_grad=True)
     gy = torch.randn(B, L, D, device="cuda")
