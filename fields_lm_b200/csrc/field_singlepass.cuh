@@ -10,7 +10,7 @@
 // block with a smaller index, which the hardware has already started.
 //
 // Forward, per block:
-//   1. load the warp's TS steps into registers, turn them into (b_r, b_i, vacancy) in
+//   1. load the warp's TS steps into registers, turn them into (b_r, b_i, sigmoid(z_v)) in
 //      place and compose the warp's affine map (gates: reference :493-501);
 //   2. 128 threads (one per channel) compose the tile's map from the warp maps and
 //      publish it, then walk back over earlier tiles of the chain, composing published

@@ -8,13 +8,12 @@
 //   EpiFf   f = act @ w3^T                  -> x' = y + f, bf16 copy
 //
 // A step of a few hundred rows is bound by latency: the 25 MB of weights of a block of d_model 1,024 take
-// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 4.3 to 6.5 us, in its first form 6 to 8 (256 rows: 2,400 to 3,000
-// cycles from the last tile of one phase to the first load of the next, 1,700 until its operands are there, 3,100 to 4,100
-// until the product is done, 5,900 in the 160-column product, 1,600 to 2,700 for the exchange of partial sums, 1,000 to
-// 4,100 for the epilogue, 1,300 to 1,800 until it is published). As four launches per block (field_step_phase.cuh, where that is still the faster way) a phase took 8 to 9.4:
-// 18 blocks of d_model 1,024 took 429 us at 1 row (589 before), 471 at 16 (626), 502 at 128 (590), 602 at
-// 256 (682); of d_model 512 376 (456) at 1 row and 450 (453) at 256; with what follows a tile spread over warps and the
-// partial sums loaded together 312 at 1 row and 471 at 256. What is done about it:
+// 3.9 us at the copy bandwidth, its products 4 us. A phase takes 7,100 to 7,800 cycles at 1 row and 9,900 to 14,300 at 256: there
+// 1,200 from a block's publication to the count that lets the next phase's loads go (800 for the last block to publish, and the
+// others wait for it), 1,400 until its operands are there, 3,200 to 3,900 until the product is done, 5,700 in the 160-column product,
+// 1,400 to 2,600 for the exchange of partial sums, 700 to 2,600 for the epilogue, 1,100 until it is published. 18 blocks of d_model
+// 1,024 take 312 us at 1 row and 471 at 256; the first form of this launch 429 and 602, four launches per block
+// (field_step_phase.cuh, where that is still the faster way) 589 and 682. What is done about it:
 //   - all blocks of the stack in one cooperative launch. A row tile (128 rows) is a chain of its own: its
 //     thread blocks count the finished tiles of a phase in global memory, and the loads of the next phase's
 //     activations wait for that count;
