@@ -34,9 +34,9 @@ constexpr ProductRule kPrefillProducts{704, 768, 768, 2048, 1536};
 // Mixer, forward and backward. As calls 200 to 290 us against 240 to 380 for 256 to 2,048 wide ones of 64 to 1,024 rows (1,024 wide: 213 and
 // 261, 215 and 302, 207 and 341 at 64, 128 and 256 rows; 2,048: 246 and 347, 242 and 344, 234 and 349). In a graph
 // 1,024 wide 90 and 86, 93 and 88, 98 and 92, 103 and 100, 118 and 117 us at 64, 128, 256, 512 and 1,024 rows, 133 and 137 at 1,536; 2,048
-// 160 and 155, 165 and 158, 171 and 168, 186 and 180, 220 and 228. Wider ones: 2,560 496 and 492 at 2,048 rows, 759 and 807 at 4,096, 1,480 and 1,522 at 8,192; 3,072 632 and 629, 1,084 and 1,120,
-// 2,080 and 2,108; 3,584 1,517 and 1,541 at 4,096, 5,456 and 5,464 at 16,384; 3,840 1,738 and 1,723, 6,230 and 6,045; 4,096 1,938 and 1,911, 3,668
-// and 3,501 at 8,192, 7,186 and 6,796.
+// 160 and 155, 165 and 158, 171 and 168, 186 and 180, 220 and 228. Wider ones, calls: 2,560 496 and 492 at 2,048 rows, 759 and 807 at
+// 4,096, 1,480 and 1,522 at 8,192; 3,072 632 and 629, 1,084 and 1,120, 2,080 and 2,108; 3,584 1,517 and 1,541 at 4,096, 5,456 and 5,464 at
+// 16,384; 3,840 1,738 and 1,723, 6,230 and 6,045; 4,096 1,938 and 1,911, 3,668 and 3,501 at 8,192, 7,186 and 6,796.
 constexpr ProductRule kMixerProducts{2048, 0, 0, 3072, 4096};
 inline bool fused_products(int64_t rows, int64_t dim, ProductRule rule) {
     return dim <= rule.narrow || (dim <= rule.less_narrow && rows <= rule.few) || (dim <= rule.widest && rows >= rule.least);

@@ -4,8 +4,8 @@
 // by the host (1.2 - 1.3 ms at 8 x 2,048 x 1,024 against 0.9 ms of kernels). Here it is two matrix
 // products forward and four backward (the two projections of x are one product over
 // [write_w | gate_w], and so are their two gradients) and the kernels of field_rows.cuh and
-// field_mixer_grad.cuh between them. With rows enough the products of the forward pass and the gradients of read and x have
-// fused epilogues (field_product.cuh); the others are library calls. Weight gradients come out of the products in fp32.
+// field_mixer_grad.cuh between them. Where kMixerProducts (torch_gemm.h) says so the products of the forward pass and the gradients
+// of read and x have fused epilogues (field_product.cuh); the others are library calls. Weight gradients come out of the products in fp32.
 #include "torch_gemm.h"
 
 #include <ATen/ops/addmm_cuda_dispatch.h>
@@ -124,7 +124,7 @@ struct FusedMixer : torch::autograd::Function<FusedMixer> {
         auto need = [&](int i) { return ctx->needs_input_grad(i); };
         const bool recurrence = need(kX) || need(kWriteW) || need(kWriteB) || need(kRadius) || need(kTheta);
         float* p = fp(par);
-        // The products of the gradients of read and x have epilogues where there are rows enough.
+        // The products of the gradients of read and x have epilogues where those of the forward pass have.
         const bool fused = fused_products(N, D);
         if (recurrence) {
             const Tensor grad_read = empty({N, 4 * C}, at::kBFloat16, dev);
